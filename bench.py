@@ -51,8 +51,8 @@ REFIT_DRAM_BYTES_PER_TRIANGLE = (372.71e6 + 452.25e6) / 15520000
 # DRAM bytes per vertex of one k_transform_multi launch (ncu, 64 batched pairs:
 # 124.3 MB read, 74.0 MB written for 7,760,256 vertices)
 TRANSFORM_DRAM_BYTES_PER_VERTEX = (124.32e6 + 73.98e6) / 7760256
-# DRAM bytes (read + written) of the traversal kernels (k_init_front, k_top and
-# the k_walk rounds) of one frame per BVTT node pair tested, measured with ncu
+# DRAM bytes (read + written) of the traversal kernels (k_begin and the
+# k_walk launches) of one frame per BVTT node pair tested, measured with ncu
 # on 64 batched pairs (206.9 MB per frame, 15,594,052 pairs tested)
 TRAVERSAL_DRAM_BYTES_PER_TESTED = (204.71e6 + 1.54e6 + 0.30e6 + 0.30e6) / 15594052
 
@@ -838,7 +838,7 @@ def frame_rooflines(w, prof, cands, hits, tested, peaks, refit_alone_ms, refit_b
                   REFIT_DRAM_BYTES_PER_TRIANGLE * tri_total,
                   "12 B per vertex + 12 B per face read, 24 B per tree node written (the reference layout; this "
                   "layout stores internal nodes only, 32 B each, and reads 16 B per face and per vertex)"),
-        "traversal": ("k_init_front + k_top + k_walk rounds (broad phase, fused 17-axis narrow phase)",
+        "traversal": ("k_begin + k_walk (broad phase, fused 17-axis narrow phase)",
                       broad + 112 * cands + 8 * hits, prof["start_ms"] + prof["walk_ms"],
                       TRAVERSAL_DRAM_BYTES_PER_TESTED * tested if TRAVERSAL_DRAM_BYTES_PER_TESTED else None,
                       "24 B per node of both trees of every pair + 112 B per candidate + 8 B per hit"),

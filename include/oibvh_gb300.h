@@ -231,7 +231,7 @@ int oibvh_scene_transform(oibvh_scene_t s, const float* d_rest_xyzw, const float
 /* Traversal tuning (also chosen by oibvh_scene_autotune). */
 typedef struct oibvh_tuning {
     uint32_t start_pairs_log2;    /* start cross product ~ 2^this node pairs per pass (8..24, default 16) */
-    uint32_t handoff;             /* front width at which one CTA hands the walk to all warps (32..8192, 2048) */
+    uint32_t handoff;             /* 32..8192 (2048); no effect: the traversal has no separate top walk */
     uint32_t walk_blocks_per_sm;  /* walker CTAs per SM, 0 = as many as fit */
     uint32_t front_capacity;      /* starting work-list capacity (entries), 0 = keep */
     uint32_t hit_capacity;        /* starting hit-queue capacity (records), 0 = keep */
@@ -241,14 +241,14 @@ typedef struct oibvh_tuning {
                                      diagonals are within this factor, else only the larger (1..2^30, 16;
                                      2^30: always together; 0 = keep) */
     uint32_t claim_min;           /* walkers claim work-list items dynamically (up to 32 at a time) when a
-                                     list holds at least this many items per warp, else each takes a
-                                     static interleaved share (1..2^20, 1; 0 = keep) */
+                                     list holds at least this many items per warp (and at least 16), else
+                                     each takes a static interleaved share (1..2^20, 1; 0 = keep) */
 } oibvh_tuning;
 int oibvh_scene_set_tuning(oibvh_scene_t s, const oibvh_tuning* t);
 int oibvh_scene_get_tuning(oibvh_scene_t s, oibvh_tuning* t);
 /* Project-written autotuner: times `reps` scene refits per refit level-group
  * depth, then `reps` detects of the scene's current state per setting, by
- * coordinate descent (start size x handoff, then the walkers' per-warp queue
+ * coordinate descent (start size, then the walkers' per-warp queue
  * capacity, then the descend ratio, then the claim threshold, then walker
  * CTAs per SM), keeps the fastest, and sizes the queues
  * from the observed peaks with 2x headroom. Blocking; *chosen may be NULL. */
@@ -256,7 +256,7 @@ int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t reps, o
 
 /* A whole frame as one CUDA graph: [oibvh_scene_transform(d_rest, d_mats)]
  * + [oibvh_scene_refit] (when refit != 0) + the detect of every pair (at most
- * 16384 pairs, fixed number of traversal rounds, results to pinned memory).
+ * 16384 pairs, results to pinned memory).
  * capture_frame runs one ordinary frame first (it sizes the queues with 2x
  * headroom and uploads the tables), then captures. launch_frame replays the
  * graph (re-capturing first if the scene or tuning changed); finish_frame
@@ -275,10 +275,10 @@ int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream);
 typedef struct oibvh_frame_profile {
     float transform_ms;    /* rigid transforms of every tree (0 without) */
     float refit_ms;        /* the one refit launch (0 without) */
-    float start_ms;        /* start front + top walk */
-    float walk_ms;         /* every captured walk round */
+    float start_ms;        /* counters cleared */
+    float walk_ms;         /* the traversal: every walk launch */
     float narrow_ms;       /* precision mode's narrow phase (0 in float mode) */
-    uint32_t walk_rounds;  /* walk rounds launched */
+    uint32_t walk_rounds;  /* walk launches (the last one walks every round that is left) */
     uint32_t kernels;      /* kernels launched */
 } oibvh_frame_profile;
 /* One frame of the captured work (oibvh_scene_capture_frame) enqueued stage
@@ -309,13 +309,13 @@ int oibvh_scene_get_precision(oibvh_scene_t s);
 /* Per-detect diagnostics: passes, BVTT steps, queue regrowths, nodes tested. */
 typedef struct oibvh_detect_stats {
     uint32_t passes;         /* pair batches */
-    uint32_t steps;          /* BVTT steps of the last pass */
+    uint32_t steps;          /* walk rounds of the last pass */
     uint32_t retries;        /* queue regrowths */
     uint32_t frame_redos;    /* captured frames redone synchronously, since the scene was created */
     uint64_t nodes_tested;   /* BVTT nodes tested, all passes */
     uint64_t candidates;
     uint64_t hits;
-    uint64_t front_peak;     /* largest front */
+    uint64_t front_peak;     /* largest list between two walk rounds */
     uint64_t fp64_axes;      /* precision mode: axis tests evaluated again in FP64 */
     uint64_t fp64_candidates;     /* precision mode: candidates with at least one such axis */
     uint64_t fp32_disagreements;  /* precision mode: candidates where float and FP64 answers differ */

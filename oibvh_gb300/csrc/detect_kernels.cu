@@ -6,15 +6,14 @@
 // triangle_intersect_kernel (src/cuda/collide.cu:248-299) with
 // triangleIntersection2 (third/gProximity/cuda_intersect_tritri.h:350-434).
 //
-// The broad phase is three kernels: k_init_front tests the cross product of
-// the node pairs at a start level and lists the overlapping ones; k_top (one
-// CTA) walks the narrow top levels until the front is wide; in k_walk every
-// warp claims 32 items of that front at a time and walks them to the leaves
-// through a private FIFO ring in shared memory (its capacity a tuning
-// parameter); what outgrows it spills to the next round's list, so no grid-wide
-// synchronisation is needed. The host enqueues the rounds and reads the
-// counters back once. Appends (next front, spills, hits) are warp-aggregated:
-// one atomic per warp, positions from ballot/shuffle prefix sums.
+// The broad phase is one kernel, k_walk, after k_begin has set its counters:
+// warps claim start-level node pairs 32 at a time, test them, and walk the
+// overlapping ones down through a private ring in shared memory. It goes in
+// rounds with a grid-wide barrier between them (a cooperative launch): a warp
+// that has nothing more to claim goes on for a few levels only and leaves the
+// rest to the next round's list, which all warps share out anew. Appends
+// (next list, hits, candidates) are warp-aggregated: one atomic per warp,
+// positions from ballot/shuffle prefix sums.
 //
 // Narrow phase: overlapping leaf pairs are buffered per warp in shared memory
 // and, 32 at a time, tested inside the traversal (the kernels' <true>
@@ -29,6 +28,8 @@
 // contracted to FMA), so the GPU pair set is the CPU pair set bit for bit.
 #include "oibvh_common.cuh"
 #include "oibvh_launch.h"
+
+#include <algorithm>
 
 namespace oibvh {
 
@@ -295,6 +296,21 @@ __device__ __forceinline__ V3 load_vertex(const float4* __restrict__ pos, uint32
     return V3{p.x, p.y, p.z};
 }
 
+// The record of mesh pair `p`. kOne: the pass holds one pair, which comes with
+// the kernel's arguments (constant cache) instead of the pair table: one
+// dependent load less per step, and no table to upload.
+template <bool kOne>
+__device__ __forceinline__ void pair_refs(const DetectArgs& a, uint32_t p, TreeRef& TA, TreeRef& TB)
+{
+    if constexpr (kOne) {
+        TA = tree_ref(a.one.ta);
+        TB = tree_ref(a.one.tb);
+    } else {
+        TA = load_tree_ref(a.pairs[p].ta);
+        TB = load_tree_ref(a.pairs[p].tb);
+    }
+}
+
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool pred, uint32_t lane)
 {
     const uint32_t mask = __ballot_sync(0xffffffffu, pred);
@@ -324,36 +340,44 @@ __device__ __forceinline__ void expand_side(const TreeShape& S, uint32_t ia, uin
     count = min(1u << d, right_valid - first + 1u);
 }
 
+// Child x (0, 1) of implicit node i (level l) when `down`, else the node itself
+// (for x = 0); false: there is none (only a level's last node lacks its second
+// child).
+__device__ __forceinline__ bool child_of(const TreeRef& T, uint32_t i, uint32_t l, bool down, uint32_t x, uint32_t& c,
+                                         uint32_t& lc)
+{
+    lc = down ? l + 1u : l;
+    c = down ? 2u * i + 1u + x : i;
+    // implicit nodes of level lc: [2^lc - 1, 2^(lc+1) - 2 - virtual ones]
+    return down ? c <= (2u << lc) - 2u - (T.vl >> (T.L - lc)) : x == 0;
+}
+
 // ---------------------------------------------------------------------------
 // Per-warp candidate buffer: leaf pairs whose boxes overlap are queued in
 // shared memory and tested 32 at a time, one per lane, so the 17-axis test
 // runs at full SIMT width however sparse the candidates are.
 // ---------------------------------------------------------------------------
 constexpr int kCandBuf = 160;  // <= 31 left over + up to 4 per lane added by one expansion step
-constexpr uint32_t kTopThreads = 1024;  // the single CTA of the top levels
-constexpr uint32_t kTopCap = 8192;      // its front capacity (two buffers: 128 KB)
-constexpr uint32_t kHandoff = 2048;     // front width at which the walkers take over
-constexpr uint32_t kWalkCap = 128;      // default per-warp ring capacity of the walkers (node pairs)
+constexpr uint32_t kWalkCap = 128;      // default per-warp capacity of the walkers (node pairs)
 constexpr uint32_t kWalkCapMax = 512;
-// Ring entries per warp for a requested capacity (0: the default): at least
-// 64, so that a top-up of 32 list items always fits beside up to 31 queued.
+constexpr uint32_t kWarps = kDetectThreads / 32;
+// Ring entries per warp for a requested capacity (0: the default): a power of
+// two (slots by masking), twice the capacity: a step's children are appended
+// beside up to 32 pairs that are still queued. 256 entries against 128 take
+// the walk of 512 mesh pairs from 1.75 to 1.63 ms (less goes to the lists).
 __host__ __device__ __forceinline__ uint32_t walk_ring(uint32_t cap)
 {
     cap = cap ? cap : kWalkCap;
-    return cap < 64u ? 64u : cap;
+    return cap <= 64u ? 128u : cap <= 128u ? 256u : 512u;
 }
 
 struct WarpCands {
     uint64_t* buf;       // kCandBuf entries
     uint32_t n;          // warp-uniform
-    uint32_t found = 0;  // candidates found by this warp (added to the counter once, at the end)
+    uint32_t found = 0;  // candidates found by this warp (added to the counter once a round)
 };
 
-__device__ __forceinline__ void flush_found(const DetectArgs& a, const WarpCands& wc, uint32_t lane)
-{
-    if (lane == 0 && wc.found) atomicAdd(a.counts + kCountCands, wc.found);
-}
-
+template <bool kOne>
 __device__ __forceinline__ void test_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count,
                                                 uint32_t lane)
 {
@@ -361,9 +385,9 @@ __device__ __forceinline__ void test_candidates(const DetectArgs& a, const uint6
     uint4 rec = make_uint4(0, 0, 0, 0);
     if (lane < count) {
         const uint64_t c = buf[lane];
-        const PairView& pv = a.pairs[bvtt_pair(c)];
-        const TreeRef TA = load_tree_ref(pv.ta);
-        const TreeRef TB = load_tree_ref(pv.tb);
+        const PairView& pv = kOne ? a.one : a.pairs[bvtt_pair(c)];
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, bvtt_pair(c), TA, TB);
         const uint4 fa = __ldg(TA.face + bvtt_a(c));
         const uint4 fb = __ldg(TB.face + bvtt_b(c));
         hit = tri_intersect_exact(load_vertex(TA.pos, fa.x), load_vertex(TA.pos, fa.y), load_vertex(TA.pos, fa.z),
@@ -396,18 +420,17 @@ __device__ __forceinline__ void store_candidates(const DetectArgs& a, const uint
 // kFused: the narrow phase is compiled into the traversal kernel (tested
 // here); otherwise the candidates are stored, and the kernel carries no
 // triangle-test code (fewer registers, more warps per SM).
-template <bool kFused>
+template <bool kFused, bool kOne>
 __device__ __forceinline__ void flush_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count,
                                                  uint32_t lane)
 {
-    if constexpr (kFused) test_candidates(a, buf, count, lane);
+    if constexpr (kFused) test_candidates<kOne>(a, buf, count, lane);
     else store_candidates(a, buf, count, lane);
 }
 
 // Queue one candidate per lane where `pred` in the warp's buffer (at most 4
 // per lane between two drains).
-template <bool kFused>
-__device__ __forceinline__ void push_candidate(const DetectArgs& a, WarpCands& wc, bool pred, uint64_t cval,
+__device__ __forceinline__ void push_candidate(WarpCands& wc, bool pred, uint64_t cval,
                                                uint32_t lane)
 {
     const uint32_t mask = __ballot_sync(0xffffffffu, pred);
@@ -420,11 +443,11 @@ __device__ __forceinline__ void push_candidate(const DetectArgs& a, WarpCands& w
 
 // Every 32 queued candidates are tested (fused narrow phase) or stored (broad
 // phase only) at once; called once per step, where little else is live.
-template <bool kFused>
+template <bool kFused, bool kOne>
 __device__ __forceinline__ void drain_candidates(const DetectArgs& a, WarpCands& wc, uint32_t lane)
 {
     while (wc.n >= 32) {
-        flush_candidates<kFused>(a, wc.buf + wc.n - 32, 32, lane);
+        flush_candidates<kFused, kOne>(a, wc.buf + wc.n - 32, 32, lane);
         wc.n -= 32;
         __syncwarp();
     }
@@ -440,7 +463,7 @@ __device__ __forceinline__ void drain_candidates(const DetectArgs& a, WarpCands&
 struct Expansion {
     uint32_t pair, fa, fb, m, dm;
 };
-template <bool kFused>
+template <bool kOne>
 __device__ __forceinline__ Expansion expand_test(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node,
                                                  uint32_t lane, uint32_t& tested)
 {
@@ -450,9 +473,8 @@ __device__ __forceinline__ Expansion expand_test(const DetectArgs& a, WarpCands&
     if (valid) {
         pair = bvtt_pair(node);
         const uint32_t ia = bvtt_a(node), ib = bvtt_b(node);
-        const PairView& pv = a.pairs[pair];
-        const TreeRef TA = load_tree_ref(pv.ta);
-        const TreeRef TB = load_tree_ref(pv.tb);
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, pair, TA, TB);
         const uint32_t la = ilog2(ia + 1u), lb = ilog2(ib + 1u);
         // the sides to descend: the key's, never a leaf (a leaf side stays and
         // the other one descends), so every expansion goes one level down
@@ -499,9 +521,52 @@ __device__ __forceinline__ Expansion expand_test(const DetectArgs& a, WarpCands&
             cm &= cm - 1;
             c = bvtt_pack(pair, leaf_a + (k >> 1), leaf_b + (k & 1));
         }
-        push_candidate<kFused>(a, wc, pred, c, lane);
+        push_candidate(wc, pred, c, lane);
     }
     return Expansion{pair, fa, fb, leaves ? 0u : m, dm};
+}
+
+// The same for up to 8 pairs, four lanes each: lane 2x + y of an item tests its
+// child pair (first child of A + x, of B + y), so a lane has one overlap test,
+// one descent rule and one ballot where a lane with all four child pairs has
+// them four times over, a scan and loops: 2.2x fewer cycles from a step's start
+// to its end. Warps of small traversals mostly hold fewer than 8 pairs.
+// Returns whether `child` is an overlapping pair to expand next.
+constexpr uint32_t kFewPairs = 8;
+template <bool kOne>
+__device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node,
+                                           uint32_t lane, uint64_t& child, uint32_t& tested)
+{
+    const uint32_t x = (lane >> 1) & 1u, y = lane & 1u;
+    bool ov = false, leaves = false, active = false;
+    uint64_t cval = 0;
+    child = 0;
+    if (valid) {
+        const uint32_t pair = bvtt_pair(node), ia = bvtt_a(node), ib = bvtt_b(node);
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, pair, TA, TB);
+        const uint32_t la = ilog2(ia + 1u), lb = ilog2(ib + 1u);
+        const uint32_t d = bvtt_desc(node);
+        const bool down_a = la != TA.L && (d != kDescendB || lb == TB.L);
+        const bool down_b = lb != TB.L && (d != kDescendA || la == TA.L);
+        uint32_t ca, lca, cb, lcb;
+        const bool va = child_of(TA, ia, la, down_a, x, ca, lca);
+        const bool vb = child_of(TB, ib, lb, down_b, y, cb, lcb);
+        active = va && vb;
+        if (active) {
+            const Box A = node_box(TA, ca, lca), B = node_box(TB, cb, lcb);
+            ov = overlap(A, B);
+            const bool a_leaf = lca == TA.L, b_leaf = lcb == TB.L;
+            leaves = a_leaf && b_leaf;
+            // leaf indices in Morton order, or the pair to expand next
+            cval = bvtt_pack(pair, ca - ((1u << lca) - 1u), cb - ((1u << lcb) - 1u));
+            child = bvtt_pack(pair, ca, cb, descend_side(A, a_leaf, B, b_leaf, a.descend_ratio));
+        }
+    }
+    const uint32_t t = __popc(__ballot_sync(0xffffffffu, active));
+    tested = lane == 0 ? t : 0u;
+    push_candidate(wc, ov && leaves, cval, lane);
+    return ov && !leaves;
 }
 
 // The key of child pair k (bit 2x + y) of an expansion.
@@ -547,247 +612,276 @@ __device__ __forceinline__ void write_children(const DetectArgs& a, const Expans
     if (overflow) atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
 }
 
-// expand_test, then the overlapping internal pairs go to the CTA's next
-// front in shared memory (one shared atomic per warp); what does not fit
-// goes to the spill list of the next round. Returns the number of child
-// pairs tested (lane 0 only, else 0).
-template <bool kFused>
-__device__ __forceinline__ uint32_t expand_pair(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node,
-                                                uint64_t* next, uint32_t* next_cnt, uint32_t next_cap,
-                                                uint64_t* __restrict__ spill, uint32_t* spill_cnt, uint32_t lane)
+// ---------------------------------------------------------------------------
+// The traversal's rounds. Round 0 takes the start tests, round r >= 1 the list
+// that round r - 1 appended (two arrays in turn). A round's words (list size
+// and, in the upper half of the same 64 bits, the CTAs that have finished
+// appending to it; items claimed) are one of four slots in turn: round r
+// appends to slot r + 1 and clears slot r + 2, which nobody looks at then.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t ld_acquire(const uint64_t* p)
 {
-    uint32_t tested;
-    const Expansion e = expand_test<kFused>(a, wc, valid, node, lane, tested);
-    uint32_t total;
-    const uint32_t ex = child_prefix((uint32_t)__popc(e.m), lane, total);
-    if (total == 0) return tested;
-    uint32_t wbase = 0, sbase = 0;
-    if (lane == 31) {
-        wbase = atomicAdd(next_cnt, total);
-        const uint32_t fit = wbase >= next_cap ? 0u : min(total, next_cap - wbase);
-        if (total > fit) sbase = atomicAdd(spill_cnt, total - fit);
-    }
-    wbase = __shfl_sync(0xffffffffu, wbase, 31);
-    sbase = __shfl_sync(0xffffffffu, sbase, 31);
-    // warp-relative positions: [0, fit) in the front from wbase, the rest spill
-    const uint32_t fit = wbase >= next_cap ? 0u : min(total, next_cap - wbase);
-    write_children(a, e, ex, fit, spill, sbase, [&](uint32_t p) { return next + wbase + p; });
-    return tested;
+    uint64_t v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(uint64_t* p, uint64_t v)
+{
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t* round_slot(uint32_t* counts, uint32_t r)
+{
+    return counts + kCtlRound + (r & 3u) * kCtlRoundWords;
 }
 
-// Initial work list: every start-level node pair of every mesh pair (the
-// reference's Scene::expandBvttNodes cross product, src/cuda/scene.cu:192-223)
-// is tested here; overlapping internal pairs go to work list 0, overlapping
-// leaf pairs straight to the candidates.
-template <bool kFused>
-__global__ void __launch_bounds__(kDetectThreads) k_init_front(DetectArgs a, uint32_t total0)
+// Counters before a traversal.
+__global__ void __launch_bounds__(256) k_begin(DetectArgs a, uint32_t hits_before)
 {
-    __shared__ uint64_t s_cand[kDetectThreads / 32][kCandBuf];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    WarpCands wc{s_cand[wib], 0};
-    for (uint32_t base = warp * 32; base < total0; base += n_warps * 32) {
-        const uint32_t i = base + lane;
-        bool ov = false, leafpair = false;
-        uint64_t node = 0, cval = 0;
-        if (i < total0) {
-            uint32_t lo = 0, hi = a.n_pairs - 1;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1) >> 1;
-                if (a.pairs[mid].front_off <= i) lo = mid;
-                else hi = mid - 1;
-            }
-            const PairView& pv = a.pairs[lo];
-            const uint32_t k = i - pv.front_off;
-            const uint32_t x = k / pv.front_cnt_b, y = k - x * pv.front_cnt_b;
-            const uint32_t ia = (1u << pv.entry_a) - 1u + x, ib = (1u << pv.entry_b) - 1u + y;
-            const TreeRef TA = load_tree_ref(pv.ta);
-            const TreeRef TB = load_tree_ref(pv.tb);
-            const Box ba = node_box(TA, ia, pv.entry_a), bb = node_box(TB, ib, pv.entry_b);
-            ov = overlap(ba, bb);
-            leafpair = ov && pv.entry_a == TA.L && pv.entry_b == TB.L;
-            node = bvtt_pack(lo, ia, ib, descend_side(ba, pv.entry_a == TA.L, bb, pv.entry_b == TB.L, a.descend_ratio));
-            cval = bvtt_pack(lo, x, y);
-        }
-        push_candidate<kFused>(a, wc, leafpair, cval, lane);
-        drain_candidates<kFused>(a, wc, lane);
-        const bool push = ov && !leafpair;
-        const uint32_t pos = warp_append(a.counts + kCountWork0, push, lane);
-        if (push) {
-            if (pos < a.work_cap) a.work[0][pos] = node;
-            else atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.counts + kCountTested, total0);
-    flush_found(a, wc, lane);
-    if (wc.n > 0) flush_candidates<kFused>(a, wc.buf, wc.n, lane);
+    for (uint32_t i = threadIdx.x; i < kCountTotal; i += blockDim.x) a.counts[i] = i == kCountHits ? hits_before : 0u;
 }
 
-// The narrow top of the traversal: ONE CTA of kTopThreads walks the start
-// list level by level with its front in shared memory (__syncthreads between
-// levels) until the front holds more than kHandoff pairs; that front becomes
-// the next work list. The first levels hold a few hundred pairs at most, so
-// one CTA covers them with one round of loads per level and no grid-wide
-// synchronisation.
-template <bool kFused>
-__global__ void __launch_bounds__(kTopThreads) k_top(DetectArgs a)
+// Counters to pinned host memory, at the end of a frame.
+__global__ void k_publish(const uint32_t* __restrict__ counts, uint32_t* __restrict__ host)
 {
-    extern __shared__ uint64_t s_dyn[];  // two front buffers of kTopCap
-    __shared__ uint64_t s_cand[kTopThreads / 32][kCandBuf];
-    __shared__ uint32_t s_cnt[2];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    constexpr uint32_t kWarps = kTopThreads / 32;
-    WarpCands wc{s_cand[wib], 0};
-    uint64_t* out = a.work[1];
-    uint32_t* out_cnt = a.counts + kCountWork0 + 1;
-    const uint32_t n0 = min(a.counts[kCountWork0], a.work_cap);
-    uint32_t tested = 0;
-    // the start list fits the front buffer, or goes straight to the walkers
-    const uint32_t handoff = a.handoff ? min(a.handoff, kTopCap) : kHandoff;
-    if (n0 > handoff) {
-        for (uint32_t i = threadIdx.x; i < n0; i += kTopThreads) out[i] = __ldcg(a.work[0] + i);
-        if (threadIdx.x == 0) *out_cnt = n0;
-        return;
-    }
-    for (uint32_t i = threadIdx.x; i < n0; i += kTopThreads) s_dyn[i] = __ldcg(a.work[0] + i);
-    uint32_t cur = 0, c = n0;
+    if (threadIdx.x < kCountHost) host[threadIdx.x] = counts[threadIdx.x];
+}
+
+// The grid's barrier after round r (every CTA is resident: a cooperative
+// launch). The CTA that arrives last has the list's final size from the word
+// it arrives at, and releases the others with it: one atomic and one poll
+// between a CTA's last append and the next round's first load. Returns the
+// next round's items, 0 to stop (also when the list has overflowed). A CTA
+// that has polled for several seconds raises kFlagTimeout and stops.
+constexpr uint32_t kBarrierPolls = 1u << 24;
+__device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t r, uint32_t* s_next)
+{
     __syncthreads();
-    while (c > 0) {
-        uint64_t* fc = cur ? s_dyn + kTopCap : s_dyn;
-        uint64_t* fn = cur ? s_dyn : s_dyn + kTopCap;
-        if (c > handoff) {
-            // wide enough: hand the front to the walkers, after the children the
-            // last level spilled to the list (a handoff above kTopCap / 4 lets a
-            // level outgrow the buffer); the count is stable: every spill
-            // happened before the last __syncthreads
-            const uint32_t base = *(volatile uint32_t*)out_cnt;
-            const uint32_t room = base < a.work_cap ? min(c, a.work_cap - base) : 0u;
-            for (uint32_t i = threadIdx.x; i < room; i += kTopThreads) out[base + i] = fc[i];
-            __syncthreads();  // every thread has read the count before it moves
-            if (threadIdx.x == 0) {
-                *out_cnt = base + c;
-                if (room < c) atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
+    if (threadIdx.x == 0) {
+        uint32_t* ctl = a.counts;
+        uint64_t* release = (uint64_t*)(ctl + kCtlRelease);  // (rounds finished, items of the next)
+        __threadfence();
+        const uint64_t w = atomicAdd((unsigned long long*)round_slot(ctl, r + 1), 1ull << 32);
+        uint32_t next = (uint32_t)w;
+        if ((uint32_t)(w >> 32) == gridDim.x - 1u) {
+            if (next > a.work_cap) next = 0;
+            st_release(release, (uint64_t)(r + 1u) << 32 | next);
+            ctl[kCountPeak] = max(ctl[kCountPeak], (uint32_t)w);
+            ctl[kCountRounds] = r + 1u;
+        } else {
+            uint64_t v = 0;
+            uint32_t polls = 0;
+            while ((uint32_t)((v = ld_acquire(release)) >> 32) <= r && ++polls < kBarrierPolls) __nanosleep(20);
+            next = (uint32_t)v;
+            if ((uint32_t)(v >> 32) <= r) {
+                atomicOr(ctl + kCountFlags, (uint32_t)kFlagTimeout);
+                next = 0;
             }
-            break;
         }
-        if (threadIdx.x == 0) s_cnt[cur ^ 1] = 0;
-        __syncthreads();
-        for (uint32_t base = wib * 32; base < c; base += kWarps * 32) {
-            const uint32_t i = base + lane;
-            const bool valid = i < c;
-            const uint64_t node = valid ? fc[i] : 0ull;
-            // what outgrows the buffer goes to the walkers' list directly
-            tested += expand_pair<kFused>(a, wc, valid, node, fn, &s_cnt[cur ^ 1], kTopCap, out, out_cnt, lane);
-            drain_candidates<kFused>(a, wc, lane);
-        }
-        __syncthreads();
-        c = min(s_cnt[cur ^ 1], kTopCap);
-        cur ^= 1;
+        *s_next = next;
     }
-    if (lane == 0 && tested) atomicAdd(a.counts + kCountTested, tested);
-    flush_found(a, wc, lane);
-    if (wc.n > 0) flush_candidates<kFused>(a, wc.buf, wc.n, lane);
+    __syncthreads();
+    return *s_next;
 }
 
-// The wide bottom of the traversal, round `round` (>= 1): every warp claims
-// up to 32 consecutive work-list items at a time (one atomic on the round's
-// claim counter; a list with fewer than claim_min items per warp, a tuning
-// parameter, is dealt out statically instead, one interleaved share per
-// warp) and walks them to the leaves through a private FIFO ring of node
-// pairs in shared memory: each step pops up to 32 pairs (one per lane),
-// expands them and appends the overlapping children at the tail, with no
-// barrier between tree levels, so lanes stay busy as long as a warp's worth
-// of pairs is queued (a level-by-level front leaves the last chunk of every
-// level part empty). The ring is topped up with the next claim whenever it
-// holds fewer than 32 pairs, so warps whose items expand less take more of
-// the list. Warps never wait for each other; children that do not fit in the
-// ring spill to the next round's list (consecutively per warp, so a claim of
-// consecutive items keeps one subtree's spill together).
-// kDense: compiled for 4 CTAs per SM (64 registers; the fused form spills a
-// few bytes), used when the grid asks for 4; otherwise the register budget of
-// 3 CTAs per SM (no spills).
-template <bool kFused, bool kDense>
-__global__ void __launch_bounds__(kDetectThreads, kDense ? 4 : 3) k_walk(DetectArgs a, uint32_t round)
+// One start pair per lane (test i of the start-level cross products, the
+// reference's Scene::expandBvttNodes, src/cuda/scene.cu:192-223): overlapping
+// internal pairs are appended to the ring, overlapping leaf pairs are
+// candidates. Returns the number appended.
+template <bool kOne>
+__device__ __forceinline__ uint32_t start_pairs(const DetectArgs& a, WarpCands& wc, uint32_t i, bool valid,
+                                                uint64_t* ring, uint32_t mask, uint32_t at, uint32_t lane)
 {
-    extern __shared__ uint64_t s_front[];  // [warp][walk_ring(cap)]: one ring per warp
-    __shared__ uint64_t s_cand[kDetectThreads / 32][kCandBuf];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    WarpCands wc{s_cand[wib], 0};
-    const uint64_t* __restrict__ src = (round & 1) ? a.work[1] : a.work[0];
-    uint64_t* __restrict__ spill = (round & 1) ? a.work[0] : a.work[1];
-    uint32_t* spill_cnt = a.counts + kCountWork0 + round + 1;
-    const uint32_t n_src = min(*(volatile uint32_t*)(a.counts + kCountWork0 + round), a.work_cap);
-    uint32_t* claim = a.counts + kCountClaim0 + round;
-    const uint32_t R = walk_ring(a.walk_cap);  // ring entries (>= 64)
-    uint64_t* ring = s_front + (size_t)wib * R;
-    // A list of at least claim_min items per warp is claimed `chunk`
-    // consecutive items at a time (its items per warp, 1..32); a shorter one
-    // is dealt out statically, items w, w + W, w + 2W, ... to warp w (W warps),
-    // so that every warp gets work.
-    const uint32_t W = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const bool claiming = n_src >= max(1u, a.claim_min) * W;
-    const uint32_t chunk = min(32u, max(1u, n_src / W));
-    const uint32_t n_mine = claiming ? 0u : (n_src > w ? (n_src - w + W - 1) / W : 0u);
-    uint32_t next_item = 0;
-    bool drained = !claiming;     // warp-uniform: no unclaimed item left (claiming lists)
-    uint32_t head = 0, live = 0;  // warp-uniform: ring[head .. head + live) mod R is queued
-    uint32_t tested = 0;
-    auto slot = [&](uint32_t off) {  // ring index of the entry `off` after head (off < R)
-        const uint32_t i = head + off;
-        return i >= R ? i - R : i;
-    };
-    for (;;) {
-        if (live < 32 && !drained) {
-            // the next `chunk` items of the list, claimed with one atomic per
-            // warp: warps whose items expand less come back sooner and take
-            // more, and neighbouring items (often one subtree's spill) stay together
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(claim, chunk);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            const uint32_t take = base < n_src ? min(chunk, n_src - base) : 0u;  // live + take <= 63 < R
-            drained = base + chunk >= n_src;
-            if (lane < take) ring[slot(live + lane)] = __ldcg(src + base + lane);
-            live += take;
-            __syncwarp();
-        } else if (live < 32 && next_item < n_mine) {
-            const uint32_t take = min(32u, n_mine - next_item);  // live + take <= 63 < R
-            if (lane < take) ring[slot(live + lane)] = __ldcg(src + w + (size_t)(next_item + lane) * W);
-            next_item += take;
-            live += take;
-            __syncwarp();
+    bool ov = false, leafpair = false;
+    uint64_t node = 0, cval = 0;
+    if (valid) {
+        uint32_t lo = 0, hi = kOne ? 0u : a.n_pairs - 1;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1) >> 1;
+            if (a.pairs[mid].front_off <= i) lo = mid;
+            else hi = mid - 1;
         }
-        if (live == 0) break;
-        const uint32_t n = min(32u, live);
-        const bool valid = lane < n;
-        const uint64_t node = valid ? ring[slot(lane)] : 0ull;
-        __syncwarp();  // every lane has read its entry before the slots are reused
-        head = slot(n);
-        live -= n;
-        uint32_t t;
-        const Expansion e = expand_test<kFused>(a, wc, valid, node, lane, t);
-        tested += t;
-        uint32_t total;
-        const uint32_t ex = child_prefix((uint32_t)__popc(e.m), lane, total);
-        if (total > 0) {
-            const uint32_t fit = min(total, R - live);
-            uint32_t sbase = 0;
-            if (total > fit) {
-                if (lane == 31) sbase = atomicAdd(spill_cnt, total - fit);
-                sbase = __shfl_sync(0xffffffffu, sbase, 31);
-            }
-            write_children(a, e, ex, fit, spill, sbase, [&](uint32_t p) { return ring + slot(live + p); });
-            live += fit;
-            __syncwarp();  // appended entries are visible to the lanes that pop them
-        }
-        // the step's candidates are tested (or stored) after its children are
-        // queued, where little else is live
-        drain_candidates<kFused>(a, wc, lane);
+        const PairView& pv = kOne ? a.one : a.pairs[lo];
+        const uint32_t k = i - pv.front_off;
+        const uint32_t x = k / pv.front_cnt_b, y = k - x * pv.front_cnt_b;
+        const uint32_t ia = (1u << pv.entry_a) - 1u + x, ib = (1u << pv.entry_b) - 1u + y;
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, lo, TA, TB);
+        const Box ba = node_box(TA, ia, pv.entry_a), bb = node_box(TB, ib, pv.entry_b);
+        ov = overlap(ba, bb);
+        leafpair = ov && pv.entry_a == TA.L && pv.entry_b == TB.L;
+        node = bvtt_pack(lo, ia, ib, descend_side(ba, pv.entry_a == TA.L, bb, pv.entry_b == TB.L, a.descend_ratio));
+        cval = bvtt_pack(lo, x, y);
     }
-    if (lane == 0 && tested) atomicAdd(a.counts + kCountTested, tested);
-    flush_found(a, wc, lane);
-    if (wc.n > 0) flush_candidates<kFused>(a, wc.buf, wc.n, lane);
+    push_candidate(wc, leafpair, cval, lane);
+    const uint32_t m = __ballot_sync(0xffffffffu, ov && !leafpair);
+    if (ov && !leafpair) ring[(at + __popc(m & ((1u << lane) - 1u))) & mask] = node;
+    __syncwarp();
+    return __popc(m);
+}
+
+// Pairs per warp from which a round's list is claimed: below it, a warp's few
+// pairs are better spread out than walked together (16 against 1: two pairs of
+// meshes 94 to 81 us a detect, 24 bodies 92 to 80, 64 pairs 306 to 297).
+constexpr uint32_t kClaimMin = 16;
+
+// Rounds first .. last of the traversal (fewer when a round leaves nothing);
+// more than one round needs a cooperative launch. Each step pops up to 32 pairs
+// of the warp's ring (one per lane), expands them and appends the overlapping
+// children at the tail, with no barrier between tree levels.
+//
+// What bounds it: the latency of a step's chain (ring entry, boxes, at the
+// leaves faces and then vertices; 1.5 us with few warps busy) times the steps
+// in a row of the busiest warp; DRAM stays below 10 %. So a warp cuts its walk
+// six steps after it has last claimed something and the rest is shared out
+// anew: a barrier costs about 3 us, a warp left alone with a deep subtree tens
+// (2, 4, 6, 8, 12 steps: two meshes of 1.31 M triangles 141, 104, 96, 103, 119 us
+// a detect). Measured, whole detects, against one kernel for the start tests,
+// one CTA for the top levels and several launches that each walk to the leaves:
+// two meshes of 20 k triangles 91 to 44 us, of 1.31 M 158 to 79, 24 bodies
+// 115 to 78, a frame of 64 pairs 360 to 270 us for the traversal, of 512
+// pairs 1.52 to 1.50 ms. A queue that idle warps wait on, instead of rounds,
+// was slower (20 k: 112 us): a hand-over costs its giver about 3 us.
+template <bool kFused, bool kOne>
+__global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32_t total0, uint32_t first, uint32_t last)
+{
+    extern __shared__ uint64_t s_ring[];  // [warp][walk_ring(cap)]
+    __shared__ uint64_t s_cand[kWarps][kCandBuf];
+    __shared__ uint32_t s_next, s_found, s_tested;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_found = s_tested = 0;
+    __syncthreads();
+    WarpCands wc{s_cand[wib], 0};
+    const uint32_t R = walk_ring(a.walk_cap), mask = R - 1u;
+    uint64_t* ring = s_ring + (size_t)wib * R;
+    const uint32_t W = gridDim.x * kWarps;
+    const uint32_t w = wib * gridDim.x + blockIdx.x;  // neighbouring items go to different SMs
+    uint32_t n_src = first == 0 ? total0 : min(*(volatile uint32_t*)round_slot(a.counts, first), a.work_cap);
+    for (uint32_t r = first;; ++r) {
+        uint32_t* claim = round_slot(a.counts, r) + kCtlRoundClaim;
+        uint32_t* spill_cnt = round_slot(a.counts, r + 1);
+        const uint64_t* src = r & 1u ? a.work[1] : a.work[0];
+        uint64_t* spill = r & 1u ? a.work[0] : a.work[1];
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *(uint64_t*)round_slot(a.counts, r + 2) = 0;
+            round_slot(a.counts, r + 2)[kCtlRoundClaim] = 0;
+        }
+        // A long list is claimed `chunk` consecutive items at a time; a short one (start tests:
+        // at most a warp's worth per warp; pairs: fewer than kClaimMin per warp) is dealt out
+        // statically, items w, w + W, .., so that it spreads over all warps.
+        const uint32_t per_warp = n_src / W;
+        const bool claiming = r == 0 ? per_warp >= 32u : per_warp >= max(kClaimMin, a.claim_min);
+        const uint32_t chunk = claiming ? min(32u, max(1u, per_warp)) : 0u;
+        uint32_t next = w;  // static share: the next item
+        bool more = claiming ? n_src > 0 : w < n_src;
+        // pairs a warp may queue (the rest goes to the next round): few items, few pairs each
+        const uint32_t cap = claiming ? R - 32u : 32u;
+        uint32_t head = 0, live = 0, steps = 0, tested = 0;
+        for (;;) {
+            while (live < 32u && more) {
+                uint32_t i, n_take;  // this lane's item; items taken
+                steps = 0;
+                if (claiming) {
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(claim, chunk);
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    n_take = base < n_src ? min(chunk, n_src - base) : 0u;
+                    i = base + lane;
+                    more = base + chunk < n_src;
+                } else {
+                    const uint32_t left = (n_src - next + W - 1u) / W;
+                    n_take = min(32u, left);
+                    i = next + lane * W;
+                    next += n_take * W;
+                    more = left > 32u;
+                }
+                if (r == 0) {
+                    live += start_pairs<kOne>(a, wc, i, lane < n_take, ring, mask, head + live, lane);
+                    drain_candidates<kFused, kOne>(a, wc, lane);
+                } else {
+                    if (lane < n_take) ring[(head + live + lane) & mask] = __ldcg(src + i);
+                    live += n_take;
+                    __syncwarp();
+                }
+            }
+            if (live == 0) break;
+            bool cut = false;
+            // some steps since the last claim (two more with few pairs, which may be about to end):
+            // is anything left to claim?
+            if (steps >= a.walk_steps && (live > kFewPairs || steps >= a.walk_steps + 2u)) {
+                if (more && claiming) {
+                    uint32_t c = 0;
+                    if (lane == 0) c = *(volatile uint32_t*)claim;
+                    more = __shfl_sync(0xffffffffu, c, 0) < n_src;
+                }
+                cut = !more;
+                steps = 0;
+            }
+            ++steps;
+            if (cut) {
+                // no: other warps may be idle, and what this one holds is shared out anew
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(spill_cnt, live);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                for (uint32_t k = lane; k < live; k += 32)
+                    if (base + k < a.work_cap) spill[base + k] = ring[(head + k) & mask];
+                if (lane == 0 && base + live > a.work_cap) atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
+                break;
+            }
+            uint32_t t;
+            if (live <= kFewPairs) {
+                const uint64_t node = ring[(head + (lane >> 2)) & mask];
+                const uint32_t n = live;
+                __syncwarp();  // every lane has read its entry before the slots are reused
+                head += n;
+                uint64_t child;
+                const bool keep = expand_few<kOne>(a, wc, (lane >> 2) < n, node, lane, child, t);
+                const uint32_t km = __ballot_sync(0xffffffffu, keep);
+                live = __popc(km);  // at most 32: fits any ring
+                if (keep) ring[(head + __popc(km & ((1u << lane) - 1u))) & mask] = child;
+            } else {
+                const uint32_t n = min(32u, live);
+                const bool valid = lane < n;
+                const uint64_t node = valid ? ring[(head + lane) & mask] : 0ull;
+                __syncwarp();
+                head += n;
+                live -= n;
+                const Expansion e = expand_test<kOne>(a, wc, valid, node, lane, t);
+                uint32_t total;
+                const uint32_t ex = child_prefix((uint32_t)__popc(e.m), lane, total);
+                const uint32_t fit = live < cap ? min(total, cap - live) : 0u;
+                uint32_t sbase = 0;
+                if (total > fit) {
+                    if (lane == 31) sbase = atomicAdd(spill_cnt, total - fit);
+                    sbase = __shfl_sync(0xffffffffu, sbase, 31);
+                }
+                write_children(a, e, ex, fit, spill, sbase, [&](uint32_t p) { return ring + ((head + live + p) & mask); });
+                live += fit;
+            }
+            tested += t;
+            __syncwarp();  // appended entries are visible to the lanes that pop them
+            // the step's candidates are tested (or stored) after its children are
+            // queued, where little else is live
+            drain_candidates<kFused, kOne>(a, wc, lane);
+        }
+        // the warp's last candidates and the CTA's totals, before the wait for the slowest warp
+        if (wc.n > 0) flush_candidates<kFused, kOne>(a, wc.buf, wc.n, lane);
+        wc.n = 0;
+        if (lane == 0 && (tested | wc.found)) {
+            atomicAdd(&s_tested, tested);
+            atomicAdd(&s_found, wc.found);
+        }
+        wc.found = 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (r == 0 && blockIdx.x == 0) s_tested += total0;
+            if (s_tested) atomicAdd(a.counts + kCountTested, s_tested);
+            if (s_found) atomicAdd(a.counts + kCountCands, s_found);
+            s_tested = s_found = 0;
+        }
+        if (r == last) break;
+        n_src = round_barrier(a, r, &s_next);
+        if (n_src == 0) break;
+    }
 }
 
 // Narrow phase over stored candidates (the split broad/narrow API):
@@ -800,7 +894,7 @@ __global__ void __launch_bounds__(kDetectThreads) k_narrow(DetectArgs a)
     const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t base = warp * 32; base < n; base += n_warps * 32) {
         const uint32_t cnt = min(32u, n - base);
-        test_candidates(a, a.cand + base, cnt, lane);
+        test_candidates<false>(a, a.cand + base, cnt, lane);
     }
 }
 
@@ -1509,47 +1603,27 @@ __global__ void __launch_bounds__(kDetectThreads) k_prec_fp64(DetectArgs a)
 // mode runs the broad phase alone and then its narrow-phase passes.
 static inline bool fused_precision(const DetectArgs& a) { return a.precision && a.fuse_narrow; }
 
-cudaError_t launch_init_front(const DetectArgs& a, uint32_t total0, cudaStream_t s)
+cudaError_t launch_begin(const DetectArgs& a, uint32_t hits_before, cudaStream_t s)
 {
     if (fused_precision(a)) return cudaErrorInvalidValue;
-    uint32_t blocks = (total0 + kDetectThreads - 1) / kDetectThreads;
-    if (blocks > (uint32_t)a.grid) blocks = (uint32_t)a.grid;
-    if (blocks == 0) blocks = 1;
     note_launches(1);
-    if (a.fuse_narrow) k_init_front<true><<<blocks, kDetectThreads, 0, s>>>(a, total0);
-    else k_init_front<false><<<blocks, kDetectThreads, 0, s>>>(a, total0);
+    k_begin<<<1, 256, 0, s>>>(a, hits_before);
     return cudaGetLastError();
 }
 
-cudaError_t launch_top(const DetectArgs& a, cudaStream_t s)
+cudaError_t launch_publish(const DetectArgs& a, uint32_t* host, cudaStream_t s)
 {
-    if (fused_precision(a)) return cudaErrorInvalidValue;
-    const int smem = (int)(2 * kTopCap * sizeof(uint64_t));
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_top<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_top<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
     note_launches(1);
-    if (a.fuse_narrow) k_top<true><<<1, kTopThreads, smem, s>>>(a);
-    else k_top<false><<<1, kTopThreads, smem, s>>>(a);
+    k_publish<<<1, 32, 0, s>>>(a.counts, host);
     return cudaGetLastError();
 }
 
-static size_t walk_smem(uint32_t cap) { return (size_t)(kDetectThreads / 32) * walk_ring(cap) * 8; }  // one ring per warp
+static size_t walk_smem(uint32_t cap) { return (size_t)kWarps * walk_ring(cap) * 8; }  // one ring per warp
 
-static int walk_sm_count()
+typedef void (*WalkKernel)(DetectArgs, uint32_t, uint32_t, uint32_t);
+static WalkKernel walk_kernel(bool fused, bool one)
 {
-    static int sms[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return 1;
-    if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    return sms[dev] > 0 ? sms[dev] : 1;
+    return fused ? (one ? k_walk<true, true> : k_walk<true, false>) : (one ? k_walk<false, true> : k_walk<false, false>);
 }
 
 static cudaError_t walk_configure()
@@ -1559,40 +1633,42 @@ static cudaError_t walk_configure()
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
     const int smem = (int)walk_smem(kWalkCapMax);
-    cudaError_t e = cudaFuncSetAttribute(k_walk<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_walk<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_walk<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_walk<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = true;
-    return e;
+    for (int k = 0; k < 4; ++k) {
+        const cudaError_t e = cudaFuncSetAttribute(walk_kernel(k & 1, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+    return cudaSuccess;
 }
 
-cudaError_t launch_walk(const DetectArgs& a, uint32_t round, cudaStream_t s)
+cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, uint32_t last, cudaStream_t s)
 {
     if (fused_precision(a)) return cudaErrorInvalidValue;
     if (a.walk_cap > kWalkCapMax || (a.walk_cap % 32) != 0) return cudaErrorInvalidValue;
     cudaError_t e = walk_configure();
     if (e != cudaSuccess) return e;
     note_launches(1);
-    const size_t smem = walk_smem(a.walk_cap);
-    const bool dense = a.grid > 3u * (uint32_t)walk_sm_count();  // 4 walker CTAs per SM asked for
-    if (a.fuse_narrow) {
-        if (dense) k_walk<true, true><<<a.grid, kDetectThreads, smem, s>>>(a, round);
-        else k_walk<true, false><<<a.grid, kDetectThreads, smem, s>>>(a, round);
-    } else {
-        if (dense) k_walk<false, true><<<a.grid, kDetectThreads, smem, s>>>(a, round);
-        else k_walk<false, false><<<a.grid, kDetectThreads, smem, s>>>(a, round);
-    }
-    return cudaGetLastError();
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)a.grid);
+    cfg.blockDim = dim3(kDetectThreads);
+    cfg.dynamicSmemBytes = walk_smem(a.walk_cap);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = first != last ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, walk_kernel(a.fuse_narrow, a.n_pairs == 1), a, total0, first, last);
 }
 
 int walk_blocks_per_sm(uint32_t walk_cap, bool fused)
 {
     if (walk_configure() != cudaSuccess) return 1;
-    int n = 0;
-    const cudaError_t e =
-        fused ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_walk<true, true>, kDetectThreads, walk_smem(walk_cap))
-              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_walk<false, true>, kDetectThreads, walk_smem(walk_cap));
+    int n = 0, m = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_kernel(fused, false), kDetectThreads, walk_smem(walk_cap));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, walk_kernel(fused, true), kDetectThreads, walk_smem(walk_cap));
+    n = std::min(n, m);
     if (e != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }

@@ -5,9 +5,9 @@
 // (include/cuda/scene.cuh:44-61, src/cuda/scene.cu). Differences by design:
 //   * the tree stays resident in device memory; nothing is copied back to
 //     the host after build or refit unless asked (oibvh_tree_get_aabbs);
-//   * the BVTT loop is enqueued whole: each level reads its front size on
-//     the device, so detect reads counters back once per pass, not once per
-//     level (the reference reads after every level, src/cuda/scene.cu:302);
+//   * the BVTT loop is one launch, so detect reads counters back once per
+//     pass, not once per level (the reference reads after every level,
+//     src/cuda/scene.cu:302);
 //   * queues are sized by demand: an overflow is detected, the queue grows,
 //     and the pass reruns (the reference writes past fixed 10M-entry buffers
 //     unchecked, src/cuda/scene.cu:15-21, src/cuda/collide.cu:160-161);
@@ -166,15 +166,13 @@ struct oibvh_scene_s {
     bool all_pairs = true;
     std::vector<uint32_t> pairs;  // flattened (a, b)
 
-    DevBuf<TreeView> views;
     DevBuf<PairView> pairv;
-    DevBuf<uint64_t> front0, front1, cand;
+    DevBuf<uint64_t> work0, work1, cand;
     DevBuf<uint4> hits;
     DevBuf<uint32_t> counts;
     DevBuf<uint32_t> prec_lists;  // precision narrow phase: float-hit, recheck and FP64 lists (4 x cand_cap)
     DevBuf<double> fp64_tri;      // precision narrow phase: FP64 setups (kFp64TriRows x fp64_tri_cap)
     uint32_t fp64_tri_cap = 0;
-    PinnedBuf<TreeView> h_views;
     PinnedBuf<PairView> h_pairs;
     PinnedBuf<uint32_t> h_counts;
 
@@ -199,7 +197,7 @@ struct oibvh_scene_s {
 
     // tuning (oibvh_scene_set_tuning / oibvh_scene_autotune)
     uint32_t tune_start_log2 = 16;  // start cross product ~ 2^this node pairs per pass
-    uint32_t tune_handoff = 2048;   // front width at which k_top hands over to the walkers
+    uint32_t tune_handoff = 2048;   // kept for callers: the traversal has no separate top walk
     uint32_t precision = 0;         // OIBVH_PRECISION_*
     uint32_t tune_walk_per_sm = 0;  // walker CTAs per SM, 0 = as many as fit
     uint32_t tune_walk_cap = 128;   // per-warp front entries of the walkers
@@ -314,26 +312,6 @@ uint32_t grow_cap(uint64_t need, uint32_t cur)
     return (uint32_t)c;
 }
 
-int upload_views(oibvh_scene_s* s, cudaStream_t st)
-{
-    const size_t n = s->trees.size();
-    OK_TRY(s->h_views.ensure(n, "cudaMallocHost(views)"));
-    OK_TRY(s->views.ensure(n, "cudaMalloc(views)"));
-    CUDA_TRY(cudaStreamSynchronize(st));  // the pinned staging buffer may still feed an earlier copy
-    for (size_t i = 0; i < n; ++i) {
-        const oibvh_tree_t t = s->trees[i];
-        TreeView v{};
-        v.box = t->box.p;
-        v.face = t->face.p;
-        v.pos = t->cur_pos;
-        v.shape = t->shape;
-        v.nV = t->nV;
-        s->h_views.p[i] = v;
-    }
-    CUDA_TRY(cudaMemcpyAsync(s->views.p, s->h_views.p, n * sizeof(TreeView), cudaMemcpyHostToDevice, st));
-    return OIBVH_OK;
-}
-
 int walk_grid(const oibvh_scene_s* s, bool fused = true)
 {
     const int fit = walk_blocks_per_sm(s->tune_walk_cap, fused);
@@ -350,6 +328,15 @@ int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_
 enum DetectMode { kDetectFused = 0, kDetectBroad = 1, kDetectSplit = 2 };
 inline int full_detect_mode(const oibvh_scene_s* s) { return s->precision ? kDetectSplit : kDetectFused; }
 
+// Work lists for the scene's capacity, and the counters.
+int ensure_lists(oibvh_scene_s* s)
+{
+    OK_TRY(s->work0.ensure(s->front_cap, "cudaMalloc(work list)"));
+    OK_TRY(s->work1.ensure(s->front_cap, "cudaMalloc(work list)"));
+    OK_TRY(s->counts.ensure(kCountTotal, "cudaMalloc(counts)"));
+    return OIBVH_OK;
+}
+
 // Broad phase (+ narrow phase unless kDetectBroad) over every pair, pass by pass.
 int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expand, int mode, cudaStream_t st)
 {
@@ -364,15 +351,15 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
     DeviceGuard g(s->device);
     struct StaleIfMoved {
         oibvh_scene_s* s;
-        const void* p[6];
+        const void* p[5];
         explicit StaleIfMoved(oibvh_scene_s* sc)
-            : s(sc), p{sc->front0.p, sc->front1.p, sc->hits.p, sc->counts.p, sc->pairv.p, sc->views.p}
+            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->pairv.p}
         {
         }
         ~StaleIfMoved()
         {
-            const void* q[6] = {s->front0.p, s->front1.p, s->hits.p, s->counts.p, s->pairv.p, s->views.p};
-            for (int i = 0; i < 6; ++i)
+            const void* q[5] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->pairv.p};
+            for (int i = 0; i < 5; ++i)
                 if (p[i] != q[i]) s->frame_stale = true;
         }
     } stale_guard(s);
@@ -387,7 +374,6 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         if (pr[2 * i] >= s->trees.size() || pr[2 * i + 1] >= s->trees.size() || pr[2 * i] == pr[2 * i + 1])
             return fail(OIBVH_ERR_ARG, "pair list refers to a missing tree or pairs a tree with itself");
     if (n_pairs == 0) return OIBVH_OK;
-    OK_TRY(upload_views(s, st));
     OK_TRY(s->hits.ensure(s->hit_cap, "cudaMalloc(hits)"));
 
     const int grid = walk_grid(s, narrow);
@@ -395,31 +381,25 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         const uint32_t np = std::min(kMaxPairsPerPass, n_pairs - p0);
         PassPlan plan;
         OK_TRY(plan_pass(s, pr.data() + 2 * (size_t)p0, np, entry, plan));
-        OK_TRY(s->counts.ensure(kCountTotal, "cudaMalloc(counts)"));
-        OK_TRY(s->h_counts.ensure(kCountTotal, "cudaMallocHost(counts)"));
+        OK_TRY(s->h_counts.ensure(kCountHost, "cudaMallocHost(counts)"));
         OK_TRY(s->h_pairs.ensure(np, "cudaMallocHost(pairs)"));
         OK_TRY(s->pairv.ensure(np, "cudaMalloc(pairs)"));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        std::memcpy(s->h_pairs.p, plan.pv.data(), np * sizeof(PairView));
-        CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
+        if (np > 1 || !narrow) {  // one pair goes with the walk's arguments; the narrow-phase kernels read the table
+            CUDA_TRY(cudaStreamSynchronize(st));  // the staging buffer may feed an earlier copy
+            std::memcpy(s->h_pairs.p, plan.pv.data(), np * sizeof(PairView));
+            CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
+        }
         const uint64_t hits_before = s->hit_count;
         for (int attempt = 0;; ++attempt) {
             if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "BVTT queues kept overflowing after regrowing");
-            OK_TRY(s->front0.ensure(s->front_cap, "cudaMalloc(work list)"));
-            OK_TRY(s->front1.ensure(s->front_cap, "cudaMalloc(work list)"));
+            OK_TRY(ensure_lists(s));
             if (!narrow) OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
-            CUDA_TRY(cudaMemsetAsync(s->counts.p, 0, kCountTotal * sizeof(uint32_t), st));
-            if (hits_before) {
-                s->h_counts.p[0] = (uint32_t)hits_before;
-                CUDA_TRY(cudaMemcpyAsync(s->counts.p, s->h_counts.p, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            }
             DetectArgs a{};
-            a.trees = s->views.p;
             a.pairs = s->pairv.p;
             a.n_pairs = np;
-            a.expand_levels = 1;
-            a.work[0] = s->front0.p;
-            a.work[1] = s->front1.p;
+            a.one = plan.pv[0];
+            a.work[0] = s->work0.p;
+            a.work[1] = s->work1.p;
             a.work_cap = s->front_cap;
             a.cand = narrow ? nullptr : s->cand.p;
             a.cand_cap = narrow ? 0 : s->cand_cap;
@@ -428,29 +408,20 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.counts = s->counts.p;
             a.fuse_narrow = narrow ? 1u : 0u;
             a.grid = grid;
-            a.handoff = s->tune_handoff;
             a.walk_cap = s->tune_walk_cap;
             a.precision = s->precision;
-            a.descend_ratio = (float)s->tune_descend;
             a.claim_min = s->tune_claim;
-            CUDA_TRY(launch_init_front(a, (uint32_t)plan.front0, st));
-            CUDA_TRY(launch_top(a, st));
-            uint32_t rounds = 1;  // list 1 is the first walk round's input
-            for (;;) {
-                // two walk rounds go out with the first read-back; later ones one by one
-                const uint32_t upto = std::min(kMaxRounds, rounds == 1 ? 3u : rounds + 1);
-                for (; rounds < upto; ++rounds) CUDA_TRY(launch_walk(a, rounds, st));
-                CUDA_TRY(cudaMemcpyAsync(s->h_counts.p, s->counts.p, kCountTotal * sizeof(uint32_t),
-                                         cudaMemcpyDeviceToHost, st));
-                CUDA_TRY(cudaStreamSynchronize(st));
-                const uint32_t* c = s->h_counts.p;
-                if (c[kCountFlags] || c[kCountWork0 + rounds] == 0) break;
-                if (rounds >= kMaxRounds) return fail(OIBVH_ERR_OVERFLOW, "BVTT traversal needed too many rounds");
-            }
+            a.descend_ratio = (float)s->tune_descend;
+            const uint32_t front0 = (uint32_t)plan.front0;
+            CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
+            CUDA_TRY(launch_walk(a, front0, 0, kAllRounds, st));
+            CUDA_TRY(cudaMemcpyAsync(s->h_counts.p, s->counts.p, kCountHost * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                     st));
+            CUDA_TRY(cudaStreamSynchronize(st));
             const uint32_t* c = s->h_counts.p;
-            const uint32_t flags = c[kCountFlags];
-            uint64_t peak = 0;
-            for (uint32_t k = 0; k <= rounds; ++k) peak = std::max<uint64_t>(peak, c[kCountWork0 + k]);
+            const uint32_t flags = c[kCountFlags], rounds = c[kCountRounds];
+            const uint64_t peak = c[kCountPeak];
+            if (flags & kFlagTimeout) return fail(OIBVH_ERR_TIMEOUT, "the BVTT traversal's barrier timed out");
             if (flags) {
                 s->stats.retries++;
                 if (flags & kFlagFrontOverflow) s->front_cap = grow_cap(peak, s->front_cap);
@@ -510,18 +481,17 @@ int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_
         if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "hit queue kept overflowing");
         // counts[kCountCandSlots] still holds the candidate count of the broad phase;
         // hits (from hits_before), flags and the precision-mode counters are reset
-        std::memset(s->h_counts.p, 0, kCountWork0 * sizeof(uint32_t));
+        std::memset(s->h_counts.p, 0, kCountNarrowEnd * sizeof(uint32_t));
         s->h_counts.p[kCountHits] = (uint32_t)hits_before;
         CUDA_TRY(cudaMemcpyAsync(s->counts.p, s->h_counts.p, 2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(s->counts.p + kCountFp64Axes, s->h_counts.p + kCountFp64Axes,
-                                 (kCountWork0 - kCountFp64Axes) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+                                 (kCountNarrowEnd - kCountFp64Axes) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         const void* lists_before = s->prec_lists.p;
         if (s->precision) OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
         if (s->prec_lists.p != lists_before) s->frame_stale = true;  // a captured frame used the old lists
         DetectArgs a{};
         a.precision = s->precision;
         a.prec_lists = s->precision ? s->prec_lists.p : nullptr;
-        a.trees = s->views.p;
         a.pairs = s->pairv.p;
         a.n_pairs = np;
         a.cand = s->cand.p;
@@ -536,8 +506,7 @@ int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_
             a.fp64_tri_cap = s->fp64_tri_cap;
         }
         CUDA_TRY(launch_narrow(a, st));
-        CUDA_TRY(cudaMemcpyAsync(s->h_counts.p, s->counts.p, kCountTotal * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                 st));
+        CUDA_TRY(cudaMemcpyAsync(s->h_counts.p, s->counts.p, kCountHost * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
         const uint32_t* c = s->h_counts.p;
         if (c[kCountFlags] & kFlagHitOverflow) {
@@ -1010,8 +979,8 @@ API int oibvh_scene_set_queue_capacity(oibvh_scene_t s, uint32_t front, uint32_t
     // shrinking the hit queue would drop hits of the last detect
     if (front) {
         s->front_cap = front;
-        s->front0.release();
-        s->front1.release();
+        s->work0.release();
+        s->work1.release();
     }
     if (candidates) {
         s->cand_cap = candidates;
@@ -1242,9 +1211,10 @@ API int oibvh_scene_get_tuning(oibvh_scene_t s, oibvh_tuning* t)
 }
 
 // Times `reps` detects per candidate setting with CUDA events and keeps the
-// fastest. Coordinate descent: the start size x handoff grid first, then the
-// walkers' front capacity, then walker CTAs per SM, each with the others at
-// their best so far.
+// fastest. Coordinate descent: the start size first, then the walkers' ring
+// capacity, the descent ratio, the claim threshold and the walker CTAs per SM,
+// each with the others at their best so far. The handoff width has no effect
+// on this traversal and keeps its default.
 API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t reps, oibvh_tuning* chosen)
 {
     GUARD_BEGIN
@@ -1295,22 +1265,21 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
         if (st == OIBVH_OK) st = oibvh_scene_refit(s, 0);
     }
     float best = 1e30f;
-    uint32_t b_start = s->tune_start_log2, b_handoff = s->tune_handoff, b_cap = 128, b_per = 0;
+    uint32_t b_start = s->tune_start_log2, b_cap = 128, b_per = 0;
+    const uint32_t b_handoff = 2048;
     uint32_t b_desc = 16, b_claim = 1;
     s->tune_walk_cap = 128;
     s->tune_walk_per_sm = 0;
     s->tune_descend = 16;
     s->tune_claim = 1;
-    for (uint32_t sl : {12u, 14u, 16u, 18u, 20u})
-        for (uint32_t h : {512u, 2048u, 8192u}) {
-            s->tune_start_log2 = sl;
-            s->tune_handoff = h;
-            float ms;
-            if (!time_setting(ms)) break;
-            if (ms < best) best = ms, b_start = sl, b_handoff = h;
-        }
-    s->tune_start_log2 = b_start;
     s->tune_handoff = b_handoff;
+    for (uint32_t sl : {12u, 14u, 16u, 18u, 20u}) {
+        s->tune_start_log2 = sl;
+        float ms;
+        if (!time_setting(ms)) break;
+        if (ms < best) best = ms, b_start = sl;
+    }
+    s->tune_start_log2 = b_start;
     for (uint32_t cap : {64u, 256u, 512u}) {
         if (st != OIBVH_OK) break;
         s->tune_walk_cap = cap;
@@ -1327,7 +1296,7 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
         if (ms < best) best = ms, b_desc = r;
     }
     s->tune_descend = b_desc;
-    for (uint32_t c : {4u, 32u}) {
+    for (uint32_t c : {32u, 64u}) {  // (below 16 items per warp lists are never claimed)
         if (st != OIBVH_OK) break;
         s->tune_claim = c;
         float ms;
@@ -1358,7 +1327,7 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
             s->tune_descend = 16;
             s->tune_claim = 1;
             if (time_setting(ms_default) && ms_default < ms_chosen) {
-                b_start = 16, b_handoff = 2048, b_cap = 128, b_per = 0, b_desc = 16, b_claim = 1;
+                b_start = 16, b_cap = 128, b_per = 0, b_desc = 16, b_claim = 1;
             }
         }
         reps = reps0;
@@ -1400,10 +1369,9 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
 namespace {
 
 // The frame's work on `st`, as captured: [transform of every tree], [refit
-// of every tree], the detect of every pair (start front, top walk, the
-// captured walk rounds), [the precision narrow phase], the counters to the
-// host. `ev` (optional, 6 events) brackets the stages for per-stage times:
-// ev[0] | transform | ev[1] | refit | ev[2] | start + top | ev[3] | walk
+// of every tree], the detect of every pair (counters cleared, the walk),
+// [the precision narrow phase], the counters to the host. `ev` (optional, 6 events) brackets the stages for per-stage times:
+// ev[0] | transform | ev[1] | refit | ev[2] | start | ev[3] | walk
 // rounds | ev[4] | narrow | ev[5].
 cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, uint32_t* kernels)
 {
@@ -1426,13 +1394,11 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
         ++k;
     }
     mark(2);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->counts.p, 0, kCountTotal * sizeof(uint32_t), st);
-    if (e == cudaSuccess) e = launch_init_front(a, s->frame_front0, st);
-    if (e == cudaSuccess) e = launch_top(a, st);
-    k += 2;
+    if (e == cudaSuccess) e = launch_begin(a, 0, st);
+    ++k;
     mark(3);
-    for (uint32_t r = 1; r <= s->frame_rounds && e == cudaSuccess; ++r) {
-        e = launch_walk(a, r, st);
+    for (uint32_t r = 0; r < s->frame_rounds && e == cudaSuccess; ++r) {  // the last launch walks all rounds left
+        e = launch_walk(a, s->frame_front0, r, r + 1 < s->frame_rounds ? r : kAllRounds, st);
         ++k;
     }
     mark(4);
@@ -1444,9 +1410,8 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
         k += narrow_kernels(n);
     }
     mark(5);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(s->h_frame_counts.p, s->counts.p, kCountTotal * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                            st);
+    if (e == cudaSuccess) e = launch_publish(a, s->h_frame_counts.p, st);
+    ++k;
     if (kernels) *kernels = k;
     return e;
 }
@@ -1467,13 +1432,9 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     if (s->frame_rest) OK_TRY(oibvh_scene_transform(s, (const float*)s->frame_rest, s->frame_mats, st));
     if (s->frame_refit) OK_TRY(oibvh_scene_refit(s, st));
     OK_TRY(detect_impl(s, s->device, s->frame_entry, s->frame_expand, full_detect_mode(s), st));
-    // walk rounds: the warm-up frame used steps - 1 of them; two more for headroom
-    // (a round with an empty input list returns at once)
-    s->frame_rounds = std::min(kMaxRounds - 1, std::max(3u, s->stats.steps + 1));
     // headroom, then the exact tables the graph will read
     s->front_cap = std::max(s->front_cap, grow_cap(2 * s->stats.front_peak, s->front_cap));
-    OK_TRY(s->front0.ensure(s->front_cap, "cudaMalloc(work list)"));
-    OK_TRY(s->front1.ensure(s->front_cap, "cudaMalloc(work list)"));
+    OK_TRY(ensure_lists(s));
     if (s->hit_count * 2 > s->hit_cap) {
         const uint32_t want = grow_cap(2 * s->hit_count, s->hit_cap);
         OK_TRY(s->hits.ensure(want, "cudaMalloc(hits)"));
@@ -1485,13 +1446,12 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
         OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
         OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
     }
-    OK_TRY(s->h_frame_counts.ensure(kCountTotal, "cudaMallocHost(frame counts)"));
+    OK_TRY(s->h_frame_counts.ensure(kCountHost, "cudaMallocHost(frame counts)"));
     PassPlan plan;
     OK_TRY(plan_pass(s, pr.data(), np, s->frame_entry, plan));
     CUDA_TRY(cudaStreamSynchronize(st));
     std::memcpy(s->h_pairs.p, plan.pv.data(), np * sizeof(PairView));
     CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
-    OK_TRY(upload_views(s, st));
     if (s->frame_rest) {
         OK_TRY(ensure_build_jobs(s, st));
         // the graph reads the rest positions in each tree's vertex order: one
@@ -1504,12 +1464,11 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     CUDA_TRY(cudaStreamSynchronize(st));
 
     DetectArgs a{};
-    a.trees = s->views.p;
     a.pairs = s->pairv.p;
     a.n_pairs = np;
-    a.expand_levels = 1;
-    a.work[0] = s->front0.p;
-    a.work[1] = s->front1.p;
+    a.one = plan.pv[0];
+    a.work[0] = s->work0.p;
+    a.work[1] = s->work1.p;
     a.work_cap = s->front_cap;
     a.hits = s->hits.p;
     a.hit_cap = s->hit_cap;
@@ -1521,11 +1480,10 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     a.fp64_tri = s->precision ? s->fp64_tri.p : nullptr;
     a.fp64_tri_cap = s->precision ? s->fp64_tri_cap : 0u;
     a.grid = walk_grid(s, !s->precision);
-    a.handoff = s->tune_handoff;
     a.walk_cap = s->tune_walk_cap;
     a.precision = s->precision;
-    a.descend_ratio = (float)s->tune_descend;
     a.claim_min = s->tune_claim;
+    a.descend_ratio = (float)s->tune_descend;
 
     s->frame_args = a;
     s->frame_front0 = (uint32_t)plan.front0;
@@ -1598,7 +1556,7 @@ API int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream)
     CUDA_TRY(cudaStreamSynchronize(st));
     const uint32_t* c = s->h_frame_counts.p;
     if (!c) return fail(OIBVH_ERR_STATE, "no frame was launched");
-    if (c[kCountFlags] || c[kCountWork0 + s->frame_rounds + 1] != 0) {
+    if (c[kCountFlags]) {
         // the captured queues were too small for this frame: redo the detect the
         // synchronous way (the refit already ran) and capture again next frame
         s->frame_stale = true;
@@ -1609,15 +1567,13 @@ API int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream)
     }
     s->stats = oibvh_detect_stats{};
     s->stats.passes = 1;
-    s->stats.steps = s->frame_rounds;
+    s->stats.steps = c[kCountRounds];
     s->stats.nodes_tested = c[kCountTested];
     s->stats.fp64_axes = c[kCountFp64Axes];
     s->stats.fp64_candidates = c[kCountFp64Cands];
     s->stats.fp32_disagreements = c[kCountDisagree];
     s->stats.bounded_candidates = (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck];
-    uint64_t peak = 0;
-    for (uint32_t k = 0; k <= s->frame_rounds + 1; ++k) peak = std::max<uint64_t>(peak, c[kCountWork0 + k]);
-    s->stats.front_peak = peak;
+    s->stats.front_peak = c[kCountPeak];
     s->hit_count = c[kCountHits];
     s->cand_count = c[kCountCands];
     s->stats.candidates = s->cand_count;

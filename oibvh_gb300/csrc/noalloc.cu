@@ -32,16 +32,11 @@ namespace oibvh {
 
 // Fixed capacity of each of the two traversal work lists (BVTT node pairs).
 constexpr uint32_t kNoAllocItems = 1u << 18;
-// Header: the two tree views, the pair view and the counters, rounded up.
+// Header: the counters, rounded up (the pair's record goes with the kernels' arguments).
 constexpr size_t kNoAllocHeader = 4096;
 constexpr size_t kNoAllocBytes = kNoAllocHeader + 2 * (size_t)kNoAllocItems * sizeof(uint64_t);
 
-struct NoAllocHeader {
-    TreeView trees[2];
-    PairView pair;
-    uint32_t counts[kCountTotal];
-};
-static_assert(sizeof(NoAllocHeader) <= kNoAllocHeader, "header fits");
+static_assert(kCountTotal * sizeof(uint32_t) <= kNoAllocHeader, "header fits");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -115,12 +110,12 @@ extern "C" __attribute__((visibility("default"))) int oibvh_pair_detect_noalloc(
         if (((uintptr_t)d_out4) % 16)
             return noalloc_fail(OIBVH_ERR_ARG, "d_out4 must be 16-byte aligned (the kernels store 16-byte records)");
         *n_hits = 0;
-        NoAllocHeader h;
-        std::memset(&h, 0, sizeof(h));
+        TreeView trees[2] = {};
+        PairView pair{};
         int dev_a = -1, dev_b = -1;
         bool built_a = false, built_b = false;
-        int st = tree_device_view(a, &h.trees[0], &dev_a, &built_a);
-        if (st == OIBVH_OK) st = tree_device_view(b, &h.trees[1], &dev_b, &built_b);
+        int st = tree_device_view(a, &trees[0], &dev_a, &built_a);
+        if (st == OIBVH_OK) st = tree_device_view(b, &trees[1], &dev_b, &built_b);
         if (st != OIBVH_OK) return st;
         if (!built_a || !built_b) return noalloc_fail(OIBVH_ERR_STATE, "both trees must be built");
         if (dev_a != dev_b) return noalloc_fail(OIBVH_ERR_ARG, "the trees live on different devices");
@@ -140,57 +135,46 @@ extern "C" __attribute__((visibility("default"))) int oibvh_pair_detect_noalloc(
         if (st != OIBVH_OK) return st;
 
         // start level: the entry level, deepened to a ~2^16-pair cross product (as oibvh_scene_detect)
-        const TreeShape& A = h.trees[0].shape;
-        const TreeShape& B = h.trees[1].shape;
+        const TreeShape& A = trees[0].shape;
+        const TreeShape& B = trees[1].shape;
         const uint32_t start = entry_level > 8u ? entry_level : 8u;
-        h.pair.a = 0;
-        h.pair.b = 1;
-        h.pair.ta = h.trees[0];
-        h.pair.tb = h.trees[1];
-        h.pair.front_off = 0;
-        h.pair.entry_a = start < A.L ? start : A.L;
-        h.pair.entry_b = start < B.L ? start : B.L;
-        h.pair.front_cnt_a = A.level_count(h.pair.entry_a);
-        h.pair.front_cnt_b = B.level_count(h.pair.entry_b);
-        const uint64_t total0 = (uint64_t)h.pair.front_cnt_a * h.pair.front_cnt_b;
+        pair.a = 0;
+        pair.b = 1;
+        pair.ta = trees[0];
+        pair.tb = trees[1];
+        pair.front_off = 0;
+        pair.entry_a = start < A.L ? start : A.L;
+        pair.entry_b = start < B.L ? start : B.L;
+        pair.front_cnt_a = A.level_count(pair.entry_a);
+        pair.front_cnt_b = B.level_count(pair.entry_b);
+        const uint64_t total0 = (uint64_t)pair.front_cnt_a * pair.front_cnt_b;
         if (total0 > (uint64_t)64 * kNoAllocItems)
             return noalloc_fail(OIBVH_ERR_ARG, "entry level " + std::to_string(entry_level) + " starts from " +
                                                    std::to_string(total0) + " node pairs; the fixed scratch allows " +
                                                    std::to_string((uint64_t)64 * kNoAllocItems));
 
         cudaStream_t s = (cudaStream_t)stream;
-        NoAllocHeader* dh = (NoAllocHeader*)base;
-        // header (views, pair, zeroed counters): the previous call's contents are overwritten
-        NA_CUDA(cudaMemcpyAsync(dh, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-
+        uint32_t* d_counts = (uint32_t*)base;
         DetectArgs args{};
-        args.trees = dh->trees;
-        args.pairs = &dh->pair;
         args.n_pairs = 1;
-        args.expand_levels = 1;
+        args.one = pair;
         args.work[0] = (uint64_t*)(base + kNoAllocHeader);
         args.work[1] = args.work[0] + kNoAllocItems;
         args.work_cap = kNoAllocItems;
         args.hits = (uint4*)d_out4;
         args.hit_cap = out_cap;
-        args.counts = dh->counts;
+        args.counts = d_counts;
         args.fuse_narrow = 1;
         int sms = 1, per_sm = walk_blocks_per_sm();
         NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_a));
         args.grid = sms * per_sm;
 
-        NA_CUDA(launch_init_front(args, (uint32_t)total0, s));
-        NA_CUDA(launch_top(args, s));
-        uint32_t counts[kCountTotal];
-        uint32_t rounds = 1;
-        for (;;) {
-            const uint32_t upto = rounds == 1 ? 3u : rounds + 1;
-            for (; rounds < upto && rounds < kMaxRounds; ++rounds) NA_CUDA(launch_walk(args, rounds, s));
-            NA_CUDA(cudaMemcpyAsync(counts, dh->counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
-            NA_CUDA(cudaStreamSynchronize(s));
-            if (counts[kCountFlags] || counts[kCountWork0 + rounds] == 0) break;
-            if (rounds >= kMaxRounds) return noalloc_fail(OIBVH_ERR_OVERFLOW, "traversal needed too many rounds");
-        }
+        NA_CUDA(launch_begin(args, 0, s));
+        NA_CUDA(launch_walk(args, (uint32_t)total0, 0, kAllRounds, s));
+        uint32_t counts[kCountHost];
+        NA_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
+        NA_CUDA(cudaStreamSynchronize(s));
+        if (counts[kCountFlags] & kFlagTimeout) return noalloc_fail(OIBVH_ERR_TIMEOUT, "the traversal's barrier timed out");
         *n_hits = counts[kCountHits];
         if (counts[kCountFlags] & kFlagFrontOverflow)
             return noalloc_fail(OIBVH_ERR_OVERFLOW, "the pair needs more than " + std::to_string(kNoAllocItems) +

@@ -286,6 +286,18 @@ __device__ __forceinline__ TreeRef load_tree_ref(const TreeView& T)
     return t;
 }
 
+// The same of a view among a kernel's arguments.
+__device__ __forceinline__ TreeRef tree_ref(const TreeView& T)
+{
+    TreeRef t;
+    t.box = T.box;
+    t.face = T.face;
+    t.pos = T.pos;
+    t.L = T.shape.L;
+    t.vl = T.shape.vl;
+    return t;
+}
+
 // How to expand an overlapping node pair next: both sides while their boxes
 // are of similar size (squared diagonals within `ratio`), else only the
 // larger box's side; a leaf never descends. The pair set does not depend on

@@ -98,10 +98,9 @@ cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total
 
 // detect_kernels.cu
 struct DetectArgs {
-    const TreeView* trees;
-    const PairView* pairs;
+    const PairView* pairs;  // n_pairs records (the walk of one pair reads `one` instead)
     uint32_t n_pairs;
-    uint32_t expand_levels;
+    PairView one;           // the record of the only pair when n_pairs == 1
     uint64_t* work[2];     // traversal work lists (ping-pong between rounds)
     uint32_t work_cap;
     uint64_t* cand;        // broad-only mode: candidate leaf pairs
@@ -116,16 +115,21 @@ struct DetectArgs {
     uint32_t fp64_tri_cap;
     uint32_t fuse_narrow;  // 1: test candidates in the traversal; 0: store them
     int grid;              // CTAs of the grid-stride / persistent kernels
-    uint32_t handoff;      // front width at which k_top hands over to the walkers (<= 8192)
     uint32_t precision;    // 0: float triangle test (reference arithmetic); 1: FP64-filtered
-    uint32_t walk_cap;     // per-warp front entries of the walkers (multiple of 32, <= 512; 0: 128)
+    uint32_t walk_cap;     // per-warp ring entries of the walkers (multiple of 32, <= 512; 0: the default)
+    uint32_t walk_steps = 6;  // steps a warp goes on for when its round has nothing more to claim
+    uint32_t claim_min = 1;   // a round's pairs are claimed dynamically from this many per warp
     float descend_ratio = kDescendRatio;  // both sides descend while the boxes' squared diagonals are within it
-    uint32_t claim_min = 1;  // walkers claim list items dynamically from this many items per warp
 };
-cudaError_t launch_init_front(const DetectArgs& a, uint32_t total0, cudaStream_t s);
-cudaError_t launch_top(const DetectArgs& a, cudaStream_t s);
-cudaError_t launch_walk(const DetectArgs& a, uint32_t round, cudaStream_t s);
-// walker CTAs that fit on one SM with fronts of `walk_cap` entries (0:
+// A traversal of `total0` start pairs: launch_begin (counters set, hits from
+// hits_before), then launch_walk of round 0 .. kAllRounds, or of rounds 0, 1,
+// .. one at a time and then r .. kAllRounds.
+cudaError_t launch_begin(const DetectArgs& a, uint32_t hits_before, cudaStream_t s);
+constexpr uint32_t kAllRounds = 0xffffffffu;  // until a round leaves nothing (a cooperative launch)
+cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, uint32_t last, cudaStream_t s);
+// the first kCountHost counters to pinned host memory
+cudaError_t launch_publish(const DetectArgs& a, uint32_t* host, cudaStream_t s);
+// walker CTAs that fit on one SM with rings of `walk_cap` entries (0:
 // default), for the fused (narrow phase inside) or the broad-only walker
 int walk_blocks_per_sm(uint32_t walk_cap = 0, bool fused = true);
 cudaError_t launch_narrow(const DetectArgs& a, cudaStream_t s);
@@ -138,16 +142,15 @@ constexpr uint32_t kFp64TriRows = 23;
 // BVTT pairs tested, (precision mode) axes evaluated in FP64, candidates with
 // at least one such axis, candidates whose float and FP64 answers differ,
 // the sizes of the float-hit, recheck and FP64 lists of the precision narrow phase
-// and of the list its double-float pass leaves to FP64,
-// then the work-list size of each traversal round (list
-// 0: the overlapping start pairs; list 1: the front k_top hands over; list
-// r+1: what walk round r spilled), then how many items of each list the
-// walkers have claimed.
-constexpr uint32_t kMaxRounds = 16;
+// and of the list its double-float pass leaves to FP64; then the largest list
+// of a walk round and the rounds walked. Past the words that the host reads:
+// the walk's control words, each on a cache line of its own.
 constexpr uint32_t kCountHits = 0, kCountFlags = 1, kCountCands = 2, kCountCandSlots = 3, kCountTested = 4,
                    kCountFp64Axes = 5, kCountFp64Cands = 6, kCountDisagree = 7, kCountPrecHits = 8,
-                   kCountPrecRecheck = 9, kCountPrecFp64 = 10, kCountPrecLeft = 11, kCountWork0 = 12,
-                   kCountClaim0 = kCountWork0 + kMaxRounds + 1,  // items of list r claimed so far
-                   kCountTotal = kCountClaim0 + kMaxRounds + 1;
+                   kCountPrecRecheck = 9, kCountPrecFp64 = 10, kCountPrecLeft = 11, kCountNarrowEnd = 12,
+                   kCountPeak = 12, kCountRounds = 13, kCountHost = 16,
+                   kCtlRelease = 32,
+                   kCtlRound = 64, kCtlRoundWords = 64, kCtlRoundClaim = 32,  // four slots
+                   kCountTotal = kCtlRound + 4 * kCtlRoundWords;
 
 } // namespace oibvh

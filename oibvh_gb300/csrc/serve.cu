@@ -13,7 +13,7 @@
 //     lists) is idle and queries are waiting, all waiting queries whose slots
 //     fit in the arena (up to max_batch) form a batch and are launched at
 //     once: one transform launch for all slots, one refit launch for all
-//     slots, one detect (start front, top walk, walk rounds) for all pairs,
+//     slots, one detect for all pairs,
 //     and the counters copied back; so queries that arrive while earlier
 //     batches are on the GPU are admitted as lanes and memory free up, and
 //     batches on different lanes overlap on the device;
@@ -22,9 +22,8 @@
 //     the grouped pairs, 8 B each) tracked by events, each query's pairs then
 //     one block copy on the host; the loop never waits on the device while
 //     other work can be launched;
-//   * a batch whose queues were too small (flags, or spill beyond the
-//     launched walk rounds) is redone on its lane with larger queues, so
-//     results are never truncated.
+//   * a batch whose queues were too small is redone on its lane with larger
+//     queues, so results are never truncated.
 //
 // A query's pair set does not depend on what it was batched with: the
 // traversal and the triangle test of a pair read only that pair's trees.
@@ -47,7 +46,6 @@ using Clock = std::chrono::steady_clock;
 
 constexpr size_t kArenaAlign = 256;
 static_assert(kArenaAlign % 32 == 0, "node arrays in the arena must be 32-byte aligned (256-bit node loads)");
-constexpr uint32_t kServeWalkRoundsInit = 8;
 
 size_t align_up(size_t x) { return (x + kArenaAlign - 1) / kArenaAlign * kArenaAlign; }
 
@@ -116,8 +114,6 @@ struct Lane {
     cudaEvent_t ev = nullptr;
     int phase = 0;  // 0 idle, 1 detect in flight, 2 hit copy in flight
     std::vector<Query*> batch;
-    PinnedBuf<TreeView> h_views;
-    DevBuf<TreeView> views;
     PinnedBuf<PairView> h_pairs;
     DevBuf<PairView> pairv;
     PinnedBuf<BuildJob> h_jobs;
@@ -127,7 +123,7 @@ struct Lane {
     PinnedBuf<float> h_mats;
     DevBuf<float> mats;
     DevBuf<uint32_t> rcount;
-    DevBuf<uint64_t> front0, front1;
+    DevBuf<uint64_t> work0, work1;
     DevBuf<uint4> hits;
     DevBuf<uint32_t> counts;
     PinnedBuf<uint32_t> h_counts;
@@ -137,11 +133,16 @@ struct Lane {
     PinnedBuf<uint2> h_out;
     uint32_t front_cap = 0, hit_cap = 0;  // set from the server's capacities at the first batch
     uint32_t cap_gen = ~0u;  // queue capacities follow the server's settings of this generation
-    uint32_t rounds = kServeWalkRoundsInit;
     uint64_t front0_count = 0;
     uint32_t n_pairs = 0;
     uint64_t n_hits = 0;
 
+    int ensure_lists()
+    {
+        OK_TRY(work0.ensure(front_cap, "cudaMalloc(work list)"));
+        OK_TRY(work1.ensure(front_cap, "cudaMalloc(work list)"));
+        return counts.ensure(kCountTotal, "cudaMalloc(counts)");
+    }
     ~Lane()
     {
         if (ev) cudaEventDestroy(ev);
@@ -302,8 +303,6 @@ int oibvh_server_s::reserve_lanes()
     const size_t n = max_batch;
     for (auto& Lp : lanes) {
         Lane& L = *Lp;
-        OK_TRY(ensure_pow2(L.h_views, 2 * n, "cudaMallocHost(views)"));
-        OK_TRY(ensure_pow2(L.views, 2 * n, "cudaMalloc(views)"));
         OK_TRY(ensure_pow2(L.h_pairs, n, "cudaMallocHost(pairs)"));
         OK_TRY(ensure_pow2(L.pairv, n, "cudaMalloc(pairs)"));
         OK_TRY(ensure_pow2(L.h_jobs, n, "cudaMallocHost(jobs)"));
@@ -313,13 +312,11 @@ int oibvh_server_s::reserve_lanes()
         OK_TRY(ensure_pow2(L.h_mats, 12 * n, "cudaMallocHost(matrices)"));
         OK_TRY(ensure_pow2(L.mats, 12 * n, "cudaMalloc(matrices)"));
         OK_TRY(ensure_pow2(L.rcount, (size_t)per * n, "cudaMalloc(refit counters)"));
-        OK_TRY(L.counts.ensure(kCountTotal, "cudaMalloc(counts)"));
-        OK_TRY(L.h_counts.ensure(kCountTotal, "cudaMallocHost(counts)"));
+        OK_TRY(L.h_counts.ensure(kCountHost, "cudaMallocHost(counts)"));
         L.front_cap = init_front_cap;
         L.hit_cap = init_hit_cap;
         L.cap_gen = cap_gen;
-        OK_TRY(L.front0.ensure(L.front_cap, "cudaMalloc(work list)"));
-        OK_TRY(L.front1.ensure(L.front_cap, "cudaMalloc(work list)"));
+        OK_TRY(L.ensure_lists());
         OK_TRY(L.hits.ensure(L.hit_cap, "cudaMalloc(hits)"));
         OK_TRY(L.qcount.ensure(n + 1, "cudaMalloc(query counts)"));
         OK_TRY(L.qcursor.ensure(n + 1, "cudaMalloc(query cursors)"));
@@ -336,8 +333,6 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
 {
     const uint32_t n = (uint32_t)batch.size();
     const uint32_t per = refit_counters_per_tree();
-    OK_TRY(ensure_pow2(L.h_views, 2 * n, "cudaMallocHost(views)"));
-    OK_TRY(ensure_pow2(L.views, 2 * n, "cudaMalloc(views)"));
     OK_TRY(ensure_pow2(L.h_pairs, n, "cudaMallocHost(pairs)"));
     OK_TRY(ensure_pow2(L.pairv, n, "cudaMalloc(pairs)"));
     OK_TRY(ensure_pow2(L.h_jobs, n, "cudaMallocHost(jobs)"));
@@ -347,8 +342,7 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
     OK_TRY(ensure_pow2(L.h_mats, 12 * (size_t)n, "cudaMallocHost(matrices)"));
     OK_TRY(ensure_pow2(L.mats, 12 * (size_t)n, "cudaMalloc(matrices)"));
     OK_TRY(ensure_pow2(L.rcount, (size_t)per * n, "cudaMalloc(refit counters)"));
-    OK_TRY(L.counts.ensure(kCountTotal, "cudaMalloc(counts)"));
-    OK_TRY(L.h_counts.ensure(kCountTotal, "cudaMallocHost(counts)"));
+    OK_TRY(L.h_counts.ensure(kCountHost, "cudaMallocHost(counts)"));
     OK_TRY(L.qcount.ensure((size_t)n + 1, "cudaMalloc(query counts)"));
     OK_TRY(L.qcursor.ensure((size_t)n + 1, "cudaMalloc(query cursors)"));
     OK_TRY(L.qoff.ensure((size_t)n + 1, "cudaMalloc(query offsets)"));
@@ -376,8 +370,6 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
         vb.pos = q->pos;
         vb.shape = B->shape;
         vb.nV = B->nV;
-        L.h_views.p[2 * i] = va;
-        L.h_views.p[2 * i + 1] = vb;
         PairView pv{};
         pv.a = 2 * i;
         pv.b = 2 * i + 1;
@@ -419,8 +411,8 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
         if (L.cap_gen != cap_gen) {
             // adopt the server's capacities (set by the caller, or raised by a lane that grew)
             if (L.front_cap != init_front_cap) {
-                L.front0.release();
-                L.front1.release();
+                L.work0.release();
+                L.work1.release();
             }
             if (L.hit_cap != init_hit_cap) L.hits.release();
             L.front_cap = init_front_cap;
@@ -429,7 +421,6 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
         }
     }
     cudaStream_t st = L.st;
-    CUDA_TRY(cudaMemcpyAsync(L.views.p, L.h_views.p, 2 * n * sizeof(TreeView), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(L.pairv.p, L.h_pairs.p, n * sizeof(PairView), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(L.jobs.p, L.h_jobs.p, n * sizeof(BuildJob), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(L.rjobs.p, L.h_rjobs.p, n * sizeof(RefitJob), cudaMemcpyHostToDevice, st));
@@ -451,29 +442,24 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
 int oibvh_server_s::enqueue_detect(Lane& L)
 {
     cudaStream_t st = L.st;
-    OK_TRY(L.front0.ensure(L.front_cap, "cudaMalloc(work list)"));
-    OK_TRY(L.front1.ensure(L.front_cap, "cudaMalloc(work list)"));
+    OK_TRY(L.ensure_lists());
     OK_TRY(L.hits.ensure(L.hit_cap, "cudaMalloc(hits)"));
     OK_TRY(L.out.ensure(L.hit_cap, "cudaMalloc(grouped pairs)"));
-    CUDA_TRY(cudaMemsetAsync(L.counts.p, 0, kCountTotal * sizeof(uint32_t), st));
     CUDA_TRY(cudaMemsetAsync(L.qcount.p, 0, L.n_pairs * sizeof(uint32_t), st));
     DetectArgs a{};
-    a.trees = L.views.p;
     a.pairs = L.pairv.p;
     a.n_pairs = L.n_pairs;
-    a.expand_levels = 1;
-    a.work[0] = L.front0.p;
-    a.work[1] = L.front1.p;
+    a.one = L.h_pairs.p[0];
+    a.work[0] = L.work0.p;
+    a.work[1] = L.work1.p;
     a.work_cap = L.front_cap;
     a.hits = L.hits.p;
     a.hit_cap = L.hit_cap;
     a.counts = L.counts.p;
     a.fuse_narrow = 1;
     a.grid = sm_count(device) * walk_blocks_per_sm();
-    a.handoff = 0;
-    CUDA_TRY(launch_init_front(a, (uint32_t)L.front0_count, st));
-    CUDA_TRY(launch_top(a, st));
-    for (uint32_t r = 1; r <= L.rounds; ++r) CUDA_TRY(launch_walk(a, r, st));
+    CUDA_TRY(launch_begin(a, 0, st));
+    CUDA_TRY(launch_walk(a, (uint32_t)L.front0_count, 0, kAllRounds, st));
     // the hits grouped by query (discarded if the batch is redone)
     const uint32_t bgrid = (uint32_t)sm_count(device) * 2;
     k_bucket_count<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, L.counts.p, L.hit_cap, L.qcount.p);
@@ -481,7 +467,7 @@ int oibvh_server_s::enqueue_detect(Lane& L)
     k_bucket_scatter<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, L.counts.p, L.hit_cap, L.qcursor.p, L.out.p);
     CUDA_TRY(cudaGetLastError());
     note_launches(3);
-    CUDA_TRY(cudaMemcpyAsync(L.h_counts.p, L.counts.p, kCountTotal * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(L.h_counts.p, L.counts.p, kCountHost * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaMemcpyAsync(L.h_qoff.p, L.qoff.p, ((size_t)L.n_pairs + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaEventRecord(L.ev, st));
     L.phase = 1;
@@ -513,14 +499,11 @@ int oibvh_server_s::advance(Lane& L)
 {
     if (L.phase == 1) {
         const uint32_t* c = L.h_counts.p;
-        const bool spill = c[kCountWork0 + L.rounds + 1] != 0;
-        if (c[kCountFlags] || spill) {
-            // queues too small or more walk rounds needed: grow and redo the detect
-            uint64_t peak = 0;
-            for (uint32_t k = 0; k <= L.rounds + 1; ++k) peak = std::max<uint64_t>(peak, c[kCountWork0 + k]);
+        if (c[kCountFlags]) {
+            // queues too small: grow and redo the detect
+            const uint64_t peak = c[kCountPeak];
             if (c[kCountFlags] & kFlagFrontOverflow) L.front_cap = grow(peak, L.front_cap);
             if (c[kCountFlags] & kFlagHitOverflow) L.hit_cap = grow(c[kCountHits], L.hit_cap);
-            if (spill) L.rounds = std::min(kMaxRounds - 1, L.rounds + 4);
             if (c[kCountFlags] & ~(uint32_t)(kFlagFrontOverflow | kFlagHitOverflow))
                 return fail(OIBVH_ERR_CUDA, "unexpected traversal flags");
             if (L.front_cap == 0x7fffffffu && (c[kCountFlags] & kFlagFrontOverflow))
