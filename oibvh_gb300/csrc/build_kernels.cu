@@ -1,7 +1,7 @@
-// Build-time kernels: mesh bounds, leaf boxes + Morton codes, the stable
-// LSD radix sort of the codes, and the gather of Morton-ordered faces; the
-// same stages for any number of trees in one launch each (scene builds);
-// and the rigid transform of every tree's vertices in one launch.
+// Build-time kernels: mesh bounds, Morton codes, their stable LSD radix sort,
+// the sorted face records and the vertex renumbering, for any number of trees
+// in one launch a stage; and the rigid transform of every tree's vertices in
+// one launch.
 //
 // Reference: src/cuda/oibvh.cu:6-70 (strech_by_3, morton3D,
 // calculate_aabb_and_morton_kernel) and src/cuda/oibvhTree.cu:253-299
@@ -15,10 +15,7 @@
 
 namespace oibvh {
 
-// ---------------------------------------------------------------------------
-// Mesh bounds (src/utils/mesh.cpp:91-98): exact min/max over every vertex,
-// accumulated as order-preserving unsigned keys with atomicMin/atomicMax.
-// ---------------------------------------------------------------------------
+// Floats as unsigned keys of the same order.
 __device__ __forceinline__ uint32_t float_to_ordered(float f)
 {
     const uint32_t b = __float_as_uint(f);
@@ -28,14 +25,6 @@ __device__ __forceinline__ float ordered_to_float(uint32_t k)
 {
     const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
     return __uint_as_float(b);
-}
-
-__global__ void k_bounds_init(uint32_t* keys)
-{
-    if (threadIdx.x < 3) {
-        keys[threadIdx.x] = 0xffffffffu;  // min accumulators
-        keys[3 + threadIdx.x] = 0u;       // max accumulators
-    }
 }
 
 // Positions as given (x, y, z) to the device layout (x, y, z, 0): one
@@ -58,109 +47,7 @@ __global__ void __launch_bounds__(256) k_gather_pos4(const float4* __restrict__ 
     pos[v] = __ldg(src + (vperm ? __ldg(vperm + v) : v));
 }
 
-// ---------------------------------------------------------------------------
-// Vertex order: after the faces are sorted, a tree renumbers its vertices in
-// the order the sorted faces first use them, so that the refit's and the
-// traversal's vertex gathers for consecutive leaves fall on nearby positions
-// (the caller's order is arbitrary). Unreferenced vertices go last, in their
-// previous order. Results do not depend on it: faces keep their order and
-// original indices, and a face's three corners keep theirs.
-// ---------------------------------------------------------------------------
-constexpr uint32_t kUnused = (1u << 25) - 1u;  // above every 3 f + slot (f < 2^23): 25-bit sort keys
-
-__global__ void __launch_bounds__(256) k_first_use_init(uint32_t* __restrict__ first, uint32_t* __restrict__ idx,
-                                                        uint32_t nV)
-{
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nV) return;
-    first[v] = kUnused;
-    idx[v] = v;
-}
-__global__ void __launch_bounds__(256) k_first_use(const uint4* __restrict__ face, uint32_t nT,
-                                                   uint32_t* __restrict__ first)
-{
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nT) return;
-    const uint4 r = __ldg(face + f);
-    atomicMin(first + r.x, 3u * f);
-    atomicMin(first + r.y, 3u * f + 1u);
-    atomicMin(first + r.z, 3u * f + 2u);
-}
-// order[j] = the current index of new vertex j: inv[order[j]] = j, the new
-// positions and the new caller-order map.
-__global__ void __launch_bounds__(256) k_apply_order(const uint32_t* __restrict__ order, uint32_t nV,
-                                                     uint32_t* __restrict__ inv, const float4* __restrict__ pos,
-                                                     float4* __restrict__ pos_new, const uint32_t* __restrict__ vperm,
-                                                     uint32_t* __restrict__ vperm_new)
-{
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nV) return;
-    const uint32_t o = __ldg(order + j);
-    inv[o] = j;
-    pos_new[j] = __ldg(pos + o);
-    vperm_new[j] = vperm ? __ldg(vperm + o) : o;
-}
-__global__ void __launch_bounds__(256) k_renumber_faces(uint4* __restrict__ face, uint32_t* __restrict__ tri,
-                                                        uint32_t nT, const uint32_t* __restrict__ inv)
-{
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nT) return;
-    uint4 r = face[f];
-    r.x = __ldg(inv + r.x);
-    r.y = __ldg(inv + r.y);
-    r.z = __ldg(inv + r.z);
-    face[f] = r;
-    tri[3 * (size_t)f] = __ldg(inv + tri[3 * (size_t)f]);
-    tri[3 * (size_t)f + 1] = __ldg(inv + tri[3 * (size_t)f + 1]);
-    tri[3 * (size_t)f + 2] = __ldg(inv + tri[3 * (size_t)f + 2]);
-}
-
-__global__ void __launch_bounds__(256) k_mesh_bounds(const float4* __restrict__ pos, uint32_t nV, uint32_t* keys)
-{
-    uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    uint32_t mx[3] = {0u, 0u, 0u};
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nV; v += gridDim.x * blockDim.x) {
-        const float4 p = __ldg(pos + v);
-        const float c[3] = {p.x, p.y, p.z};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const uint32_t o = float_to_ordered(c[k]);
-            mn[k] = min(mn[k], o);
-            mx[k] = max(mx[k], o);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        for (int s = 16; s > 0; s >>= 1) {
-            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], s));
-            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], s));
-        }
-    }
-    __shared__ uint32_t smn[3][8], smx[3][8];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0)
-        for (int k = 0; k < 3; ++k) {
-            smn[k][w] = mn[k];
-            smx[k][w] = mx[k];
-        }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        const int k = threadIdx.x;
-        uint32_t a = 0xffffffffu, b = 0u;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
-            a = min(a, smn[k][i]);
-            b = max(b, smx[k][i]);
-        }
-        atomicMin(keys + k, a);
-        atomicMax(keys + 3 + k, b);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Leaf boxes + Morton codes (src/cuda/oibvh.cu:6-22,42-70). The float ops are
-// the reference's, each rounded on its own (the *0.5f and *1024.0f scalings
-// are exact, the one division is IEEE round-to-nearest).
-// ---------------------------------------------------------------------------
+// Morton codes (src/cuda/oibvh.cu:6-22).
 __device__ __forceinline__ uint32_t stretch3(uint32_t x)
 {
     x &= 0x3ffu;
@@ -218,188 +105,575 @@ __device__ __forceinline__ void morton_key(const float u[3], bool wide, uint32_t
     hi = (uint32_t)(k >> 32);
 }
 
-__global__ void __launch_bounds__(256) k_leaf_morton(const uint32_t* __restrict__ tri, const float4* __restrict__ pos,
-                                                     uint32_t nT, const uint32_t* __restrict__ bound_keys,
-                                                     uint32_t* __restrict__ codes, uint32_t* __restrict__ idx,
-                                                     uint32_t* __restrict__ codes_hi)
+// ---------------------------------------------------------------------------
+// The build of any number of trees: every stage is one launch for all of them
+// (a scene build) or for one (a tree build). Faces and vertices are cut into
+// tiles of 4096 that never straddle trees; a host-built map names a tile's
+// tree.
+//
+//   k_build_vertices  mesh bounds; first-use slots cleared
+//   k_build_codes     Morton codes, and the digit histograms of every pass
+//   k_build_sort x 4  one stable radix pass over 8 bits each (x 8 for 63-bit
+//                     keys); the last one writes the sorted face records and
+//                     each vertex's first use instead of keys
+//   k_build_mark, k_build_count, k_build_place
+//                     new vertex numbers in order of first use
+//   k_build_apply     faces and positions in the new numbering
+//
+// A tile's share of a running count (digits of a pass, first uses) is its
+// tree's sum over the tiles before it, taken by decoupled look-back (Merrill
+// and Garland, "Single-pass parallel prefix scan with decoupled look-back",
+// 2016; for radix passes Adinets and Merrill, "Onesweep", 2022): a tile
+// publishes its own count, then adds up its predecessors' from the nearest on
+// until one has published its whole sum. CTAs take their tiles from a counter,
+// so the tiles waited for are running or done; a wait has a limit, after which
+// the build is given up (BuildScratch::fail).
+// ---------------------------------------------------------------------------
+constexpr uint32_t kNoUse = 0xffffffffu;
+constexpr uint32_t kTileWords = 3 * kBuildTile / 32;  // a bit per face corner of a tile
+constexpr uint32_t kStateSum = 1u << 30, kStateTotal = 2u << 30, kStateValue = kStateSum - 1u;
+constexpr uint32_t kLookbackPolls = 1u << 20;
+
+__device__ __forceinline__ const BuildJob& job_of(const BuildArgs& a, const uint32_t* map, uint32_t tile, uint32_t& j)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nT) return;
-    float bmin[3], bmax[3];
+    j = a.jobs ? __ldg(map + tile) : 0u;
+    return a.jobs ? a.jobs[j] : a.one;
+}
+__device__ __forceinline__ uint32_t ld_state(const uint32_t* p) { return *(const volatile uint32_t*)p; }
+__device__ __forceinline__ void st_state(uint32_t* p, uint32_t v) { *(volatile uint32_t*)p = v; }
+__device__ __forceinline__ void give_up(const BuildArgs& a)
+{
+    st_state(a.sc.fail, 1u);
+    *(volatile uint32_t*)a.host_error = 1u;  // pinned host memory
+    __threadfence_system();
+}
+
+// Bounds of each mesh (src/utils/mesh.cpp:91-98) as order-preserving keys:
+// maxima of the coordinates and of their complements (so 0 is neutral for
+// both). One atomic per CTA and bound: with one per warp the 14 M vertices of
+// 128 meshes took 573 us, queueing at six words a mesh.
+__global__ void __launch_bounds__(256) k_build_vertices(const __grid_constant__ BuildArgs a)
+{
+    __shared__ uint32_t s_red[6][8];
+    uint32_t j;
+    const BuildJob& job = job_of(a, a.vtile_job, blockIdx.x >> 2, j);
+    const uint32_t base = ((blockIdx.x >> 2) - job.vtile_begin) * kBuildTile + (blockIdx.x & 3u) * 1024u;
+    if (base >= job.nV) return;
+    uint32_t red[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        bmin[k] = ordered_to_float(bound_keys[k]);
-        bmax[k] = ordered_to_float(bound_keys[3 + k]);
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t v = base + k * 256u + threadIdx.x;
+        if (v >= job.nV) continue;
+        const float4 p = __ldg(job.pos + v);
+        const float c[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t o = float_to_ordered(c[i]);
+            red[i] = max(red[i], ~o);
+            red[3 + i] = max(red[3 + i], o);
+        }
+        a.sc.first[job.vert_off + v] = kNoUse;
     }
-    const uint32_t f0 = __ldg(tri + 3 * (size_t)i), f1 = __ldg(tri + 3 * (size_t)i + 1),
-                   f2 = __ldg(tri + 3 * (size_t)i + 2);
-    const float4 p0 = __ldg(pos + f0), p1 = __ldg(pos + f1), p2 = __ldg(pos + f2);
-    const float va[3] = {p0.x, p0.y, p0.z}, vb[3] = {p1.x, p1.y, p1.z}, vc[3] = {p2.x, p2.y, p2.z};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        red[i] = __reduce_max_sync(0xffffffffu, red[i]);
+        if ((threadIdx.x & 31) == 0) s_red[i][threadIdx.x >> 5] = red[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        uint32_t m = 0;
+        for (int w = 0; w < 8; ++w) m = max(m, s_red[threadIdx.x][w]);
+        atomicMax(a.sc.bounds + 6 * j + threadIdx.x, m);
+    }
+}
+
+// The leaf's Morton code (src/cuda/oibvh.cu:6-22,42-70): the float operations
+// are the reference's, each rounded on its own (the *0.5f and the quantiser's
+// scaling are exact, the one division is IEEE round-to-nearest).
+__device__ __forceinline__ void leaf_code(const float va[3], const float vb[3], const float vc[3], const float bmin[3],
+                                          const float bmax[3], bool wide, uint32_t& lo, uint32_t& hi)
+{
     float u[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const float a = va[k], b = vb[k], c = vc[k];
-        const float mn = gmin(gmin(a, b), c), mx = gmax(gmax(a, b), c);
+        const float mn = gmin(gmin(va[k], vb[k]), vc[k]), mx = gmax(gmax(va[k], vb[k]), vc[k]);
         const float centroid = __fmul_rn(__fadd_rn(mn, mx), 0.5f);
-        const float off = __fsub_rn(centroid, bmin[k]);
-        const float len = __fsub_rn(bmax[k], bmin[k]);
-        u[k] = __fdiv_rn(off, len);
+        u[k] = __fdiv_rn(__fsub_rn(centroid, bmin[k]), __fsub_rn(bmax[k], bmin[k]));
     }
-    uint32_t lo, hi;
-    morton_key(u, codes_hi != nullptr, lo, hi);
-    codes[i] = lo;
-    if (codes_hi) codes_hi[i] = hi;
-    idx[i] = i;
+    morton_key(u, wide, lo, hi);
 }
 
-// ---------------------------------------------------------------------------
-// Stable LSD radix sort, 8-bit digits. A tile is 2048 consecutive items
-// (8 warps x 8 rounds x 32 lanes); ranks inside a tile come from
-// __match_any_sync peer groups in item order, so equal digits keep their
-// input order and the sort is stable, as thrust::stable_sort_by_key is.
-// ---------------------------------------------------------------------------
-constexpr int kRsThreads = 256;
-constexpr int kRsRounds = 8;
-constexpr int kRsTile = kRsThreads * kRsRounds;
-
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
-                                                        uint32_t* __restrict__ hist, uint32_t n_tiles)
+template <bool kWide>
+__global__ void __launch_bounds__(256) k_build_codes(const __grid_constant__ BuildArgs a)
 {
-    __shared__ uint32_t cnt[256];
-    cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t base = blockIdx.x * kRsTile;
+    constexpr uint32_t P = kWide ? 8 : 4;
+    __shared__ uint32_t s_hist[P * 256];
+    uint32_t j;
+    const BuildJob& job = job_of(a, a.ftile_job, blockIdx.x >> 2, j);
+    const uint32_t base = ((blockIdx.x >> 2) - job.ftile_begin) * kBuildTile + (blockIdx.x & 3u) * 1024u;
+    if (base >= job.nT) return;
+    for (uint32_t i = threadIdx.x; i < P * 256; i += 256) s_hist[i] = 0;
+    float bmin[3], bmax[3];
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
-        const uint32_t i = base + r * kRsThreads + threadIdx.x;
-        if (i < n) atomicAdd(&cnt[(__ldg(keys + i) >> shift) & 255u], 1u);
+    for (int k = 0; k < 3; ++k) {
+        bmin[k] = ordered_to_float(~a.sc.bounds[6 * j + k]);
+        bmax[k] = ordered_to_float(a.sc.bounds[6 * j + 3 + k]);
+    }
+    uint32_t f[4][3];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t i = base + k * 256u + threadIdx.x;
+        const uint32_t* t = job.tri + 3 * (size_t)(i < job.nT ? i : 0u);
+        f[k][0] = __ldg(t);
+        f[k][1] = __ldg(t + 1);
+        f[k][2] = __ldg(t + 2);
     }
     __syncthreads();
-    hist[(size_t)threadIdx.x * n_tiles + blockIdx.x] = cnt[threadIdx.x];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t i = base + k * 256u + threadIdx.x;
+        if (i >= job.nT) continue;
+        const float4 p0 = __ldg(job.pos + f[k][0]), p1 = __ldg(job.pos + f[k][1]), p2 = __ldg(job.pos + f[k][2]);
+        const float va[3] = {p0.x, p0.y, p0.z}, vb[3] = {p1.x, p1.y, p1.z}, vc[3] = {p2.x, p2.y, p2.z};
+        uint32_t lo, hi;
+        leaf_code(va, vb, vc, bmin, bmax, kWide, lo, hi);
+        a.sc.keys[0][job.face_off + i] = lo;
+        if (kWide) a.sc.hi[job.face_off + i] = hi;
+#pragma unroll
+        for (uint32_t p = 0; p < P; ++p) atomicAdd(&s_hist[p * 256 + (((p < 4 ? lo : hi) >> (8 * (p & 3))) & 255u)], 1u);
+    }
+    __syncthreads();
+    uint32_t* hist = a.sc.hist + (size_t)j * P * 256;
+    for (uint32_t i = threadIdx.x; i < P * 256; i += 256)
+        if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
 }
 
-// Block-wide exclusive scan of one value per thread (256 threads).
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total, uint32_t* sh /*[8]*/)
+// Exclusive scan of one value per thread over threads 0..255 of the CTA (every
+// thread calls; the others pass anything and get garbage).
+__device__ __forceinline__ uint32_t scan_256(uint32_t v, uint32_t* sh /*[8]*/)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint32_t x = v;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, s);
-        if (lane >= s) x += y;
+        if ((int)lane >= s) x += y;
     }
-    if (lane == 31) sh[w] = x;
+    if (lane == 31 && w < 8) sh[w] = x;
     __syncthreads();
-    uint32_t wpre = 0, tot = 0;
+    uint32_t pre = 0;
 #pragma unroll
-    for (int i = 0; i < kRsThreads / 32; ++i) {
-        const uint32_t t = sh[i];
-        if (i < w) wpre += t;
-        tot += t;
-    }
+    for (uint32_t i = 0; i < 8; ++i) pre += i < w ? sh[i] : 0u;
     __syncthreads();
-    *total = tot;
-    return wpre + x - v;
+    return pre + x - v;
 }
 
-// One CTA per digit: exclusive scan of hist[d][0..n_tiles) in place, digit total out.
-__global__ void __launch_bounds__(kRsThreads) k_rs_scan_digit(uint32_t* __restrict__ hist, uint32_t n_tiles,
-                                                              uint32_t* __restrict__ totals)
-{
-    __shared__ uint32_t sh[8];
-    uint32_t* row = hist + (size_t)blockIdx.x * n_tiles;
-    uint32_t carry = 0;
-    for (uint32_t s = 0; s < n_tiles; s += kRsThreads) {
-        const uint32_t i = s + threadIdx.x;
-        const uint32_t v = (i < n_tiles) ? row[i] : 0u;
-        uint32_t tot;
-        const uint32_t ex = block_exclusive_scan(v, &tot, sh);
-        if (i < n_tiles) row[i] = carry + ex;
-        carry += tot;
-    }
-    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
-}
+// One pass of the stable LSD radix sort: a CTA ranks a tile of 4096 items
+// (groups of equal digits in item order), reorders them in shared memory
+// so that each digit's items leave as one run, and writes them behind those of
+// the tree's earlier tiles. kFirst: the values are the item numbers (not read);
+// kLast: the sorted faces are gathered and written with each vertex's first
+// use, instead of keys and values. `swap_hi`: the key written is the item's
+// high word (the pass between the two halves of a 63-bit key).
+constexpr uint32_t kSortThreads = 512, kSortWarps = kSortThreads / 32, kSortItems = kBuildTile / kSortThreads;
 
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                           uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                           uint32_t n, int shift, const uint32_t* __restrict__ hist,
-                                                           uint32_t n_tiles, const uint32_t* __restrict__ totals)
+template <bool kFirst, bool kLast>
+__global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_constant__ BuildArgs a, uint32_t pass, bool swap_hi)
 {
-    __shared__ uint32_t warp_cnt[kRsThreads / 32][256];
-    __shared__ uint32_t base[256];
-    __shared__ uint32_t sh[8];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < (kRsThreads / 32) * 256; i += kRsThreads) (&warp_cnt[0][0])[i] = 0;
-    {
-        uint32_t tot;
-        const uint32_t ex = block_exclusive_scan(totals[threadIdx.x], &tot, sh);
-        base[threadIdx.x] = ex + hist[(size_t)threadIdx.x * n_tiles + blockIdx.x];
+    __shared__ uint16_t s_cnt[kSortWarps][256];
+    __shared__ uint32_t s_key[kBuildTile], s_val[kBuildTile];
+    __shared__ uint32_t s_base[256], s_start[256], s_sh[8], s_tile, s_bad;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t shift = 8 * (pass & 3u);
+    if (tid == 0) {
+        s_tile = atomicAdd(a.sc.tickets + pass, 1u);
+        s_bad = ld_state(a.sc.fail);
     }
+    for (uint32_t i = tid; i < kSortWarps * 128; i += kSortThreads) ((uint32_t*)s_cnt)[i] = 0;
     __syncthreads();
+    if (s_bad) return;
+    const uint32_t tile = s_tile;
+    uint32_t j;
+    const BuildJob& job = job_of(a, a.ftile_job, tile, j);
+    const uint32_t t0 = tile - job.ftile_begin, n = min(kBuildTile, job.nT - t0 * kBuildTile);
+    const uint32_t* kin = a.sc.keys[pass & 1] + job.face_off + t0 * kBuildTile;
+    const uint32_t* vin = a.sc.vals[pass & 1] + job.face_off + t0 * kBuildTile;
+    uint32_t* state = a.sc.sort_state[pass & 1];
+    uint32_t key[kSortItems], val[kSortItems];
+    uint16_t rank[kSortItems];
+    const uint32_t i0 = w * (32 * kSortItems) + lane;
+#pragma unroll
+    for (uint32_t r = 0; r < kSortItems; ++r) {
+        const uint32_t i = i0 + 32 * r;
+        key[r] = i < n ? kin[i] : 0u;
+        val[r] = kFirst ? t0 * kBuildTile + i : i < n ? vin[i] : 0u;
+    }
     const uint32_t lt = (1u << lane) - 1u;
-    uint32_t key[kRsRounds], val[kRsRounds], rank[kRsRounds];
-    const uint32_t tile0 = blockIdx.x * kRsTile + w * (kRsRounds * 32);
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
-        const uint32_t i = tile0 + r * 32 + lane;
-        const bool valid = i < n;
-        key[r] = valid ? kin[i] : 0u;
-        val[r] = valid ? vin[i] : 0u;
-        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-        rank[r] = 0;
-        if (valid) {
-            const uint32_t d = (key[r] >> shift) & 255u;
-            const uint32_t peers = __match_any_sync(vmask, d);
-            const uint32_t b = warp_cnt[w][d];
-            rank[r] = b + __popc(peers & lt);
-            __syncwarp(vmask);
-            if (lane == __ffs(peers) - 1) warp_cnt[w][d] = b + __popc(peers);
+    for (uint32_t r = 0; r < kSortItems; ++r) {
+        const bool valid = i0 + 32 * r < n;
+        const uint32_t d = (key[r] >> shift) & 255u;
+        // the valid lanes of the same digit (eight ballots; __match_any_sync was twice as slow a pass)
+        uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (uint32_t b = 0; b < 8; ++b) {
+            const uint32_t set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+            peers &= (d >> b) & 1u ? set : ~set;
         }
+        uint32_t b = 0;
+        if (valid) b = s_cnt[w][d];
+        rank[r] = (uint16_t)(b + __popc(peers & lt));
+        __syncwarp();
+        if (valid && (peers & lt) == 0) s_cnt[w][d] = (uint16_t)(b + __popc(peers));
         __syncwarp();
     }
     __syncthreads();
-    {
-        const int d = threadIdx.x;
-        uint32_t s = 0;
+    uint32_t cnt = 0, digits = 0;
+    if (tid < 256) {
 #pragma unroll
-        for (int i = 0; i < kRsThreads / 32; ++i) {
-            const uint32_t t = warp_cnt[i][d];
-            warp_cnt[i][d] = s;
-            s += t;
+        for (uint32_t i = 0; i < kSortWarps; ++i) {
+            const uint32_t c = s_cnt[i][tid];
+            s_cnt[i][tid] = (uint16_t)cnt;
+            cnt += c;
         }
+        st_state(state + (size_t)tile * 256 + tid, (t0 == 0 ? kStateTotal : kStateSum) | cnt);
+        a.sc.sort_state[(pass + 1) & 1][(size_t)tile * 256 + tid] = 0;  // for the next pass
+        digits = a.sc.hist[((size_t)j * a.passes + pass) * 256 + tid];
     }
+    const uint32_t start = scan_256(cnt, s_sh);
+    const uint32_t first = scan_256(digits, s_sh);
+    if (tid < 256) s_start[tid] = start;
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
-        const uint32_t i = tile0 + r * 32 + lane;
-        if (i < n) {
+    for (uint32_t r = 0; r < kSortItems; ++r) {
+        if (i0 + 32 * r < n) {
             const uint32_t d = (key[r] >> shift) & 255u;
-            const uint32_t dst = base[d] + warp_cnt[w][d] + rank[r];
-            kout[dst] = key[r];
-            vout[dst] = val[r];
+            const uint32_t q = s_start[d] + s_cnt[w][d] + rank[r];
+            s_key[q] = key[r];
+            s_val[q] = val[r];
+        }
+    }
+    if (tid < 256) {
+        // this digit's items in the tree's earlier tiles: eight predecessors per round of loads
+        uint32_t before = 0, polls = 0;
+        bool done = t0 == 0;
+        for (uint32_t k = tile; !done;) {
+            uint32_t v[8];
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q)
+                v[q] = q < k - job.ftile_begin ? ld_state(state + (size_t)(k - q - 1) * 256 + tid) : 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q) {
+                if (done || v[q] == 0) break;
+                before += v[q] & kStateValue;
+                done = (v[q] & kStateTotal) != 0;
+                --k;
+            }
+            if (!done && ++polls > kLookbackPolls) {
+                s_bad = 1;
+                break;
+            }
+        }
+        if (t0 != 0 && done) st_state(state + (size_t)tile * 256 + tid, kStateTotal | (before + cnt));
+        s_base[tid] = first + before - start;
+    }
+    __syncthreads();
+    if (s_bad) {
+        if (tid == 0) give_up(a);
+        return;
+    }
+    uint32_t* kout = a.sc.keys[(pass + 1) & 1] + job.face_off;
+    uint32_t* vout = a.sc.vals[(pass + 1) & 1] + job.face_off;
+    const uint32_t* hi = a.sc.hi + job.face_off;
+#pragma unroll
+    for (uint32_t r = 0; r < kSortItems; ++r) {
+        const uint32_t q = r * kSortThreads + tid;
+        if (q >= n) break;
+        const uint32_t k = s_key[q], o = s_val[q], dst = s_base[(k >> shift) & 255u] + q;
+        if (kLast) {
+            const uint32_t* t = job.tri + 3 * (size_t)o;
+            const uint32_t x = __ldg(t), y = __ldg(t + 1), z = __ldg(t + 2);
+            job.face_out[dst] = make_uint4(x, y, z, o);
+            uint32_t* use = a.sc.first + job.vert_off;
+            atomicMin(use + x, 3u * dst);
+            atomicMin(use + y, 3u * dst + 1u);
+            atomicMin(use + z, 3u * dst + 2u);
+        } else {
+            kout[dst] = swap_hi ? __ldg(hi + o) : k;
+            vout[dst] = o;
         }
     }
 }
 
-// Morton-ordered face records: (v0, v1, v2, original face index).
-__global__ void __launch_bounds__(256) k_gather_faces(const uint32_t* __restrict__ tri, const uint32_t* __restrict__ perm,
-                                                      uint32_t nT, uint4* __restrict__ out)
+// This block's running count: `mine` (of the whole CTA) published, and the sum
+// over the chain's earlier blocks [chain, block). Called by warp 0; false: gave up.
+__device__ __forceinline__ bool lookback(const BuildArgs& a, uint32_t* state, uint32_t chain, uint32_t block, uint32_t mine,
+                                         uint32_t& before)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nT) return;
-    const uint32_t o = perm[i];
-    out[i] = make_uint4(__ldg(tri + 3 * (size_t)o), __ldg(tri + 3 * (size_t)o + 1), __ldg(tri + 3 * (size_t)o + 2), o);
+    const uint32_t lane = threadIdx.x & 31;
+    before = 0;
+    if (block == chain) {
+        if (lane == 0) st_state(state + block, kStateTotal | mine);
+        return true;
+    }
+    if (lane == 0) st_state(state + block, kStateSum | mine);
+    uint32_t polls = 0;
+    for (uint32_t b = block;;) {  // lane l looks at block b - 1 - l
+        const bool in = b > chain + lane;
+        const uint32_t v = in ? ld_state(state + b - 1 - lane) : kStateTotal;
+        const uint32_t empty = __ballot_sync(0xffffffffu, v == 0), total = __ballot_sync(0xffffffffu, (v & kStateTotal) != 0);
+        const uint32_t upto = total ? (uint32_t)__ffs(total) - 1u : 31u;  // lanes 0 .. upto count
+        if (empty & (0xffffffffu >> (31u - upto))) {
+            if (++polls > kLookbackPolls) return false;
+            continue;
+        }
+        before += __reduce_add_sync(0xffffffffu, lane <= upto ? v & kStateValue : 0u);
+        if (total) break;
+        b -= 32;
+    }
+    if (lane == 0) st_state(state + block, kStateTotal | (before + mine));
+    return true;
+}
+
+// New vertex numbers, in the order in which the sorted faces first use them (so
+// that the refit's and the traversal's vertex gathers for neighbouring leaves
+// fall on nearby positions; the caller's order is arbitrary), unused vertices
+// last in their previous order. A vertex's number is the count of first uses
+// (of unused vertices) before its own: a bit per face corner marks the first
+// uses, running counts are kept per 32 corners, and everything that follows
+// works vertex by vertex. (Going through the faces instead, each corner looking
+// up whether it is its vertex's first use, took 361 us for 14 M faces against
+// 64 us for these three kernels.)
+__global__ void __launch_bounds__(256) k_build_mark(const __grid_constant__ BuildArgs a)
+{
+    if (ld_state(a.sc.fail)) return;
+    uint32_t j;
+    const BuildJob& job = job_of(a, a.vtile_job, blockIdx.x >> 2, j);
+    const uint32_t base = ((blockIdx.x >> 2) - job.vtile_begin) * kBuildTile + (blockIdx.x & 3u) * 1024u + threadIdx.x;
+    uint32_t* marks = a.sc.marks + (size_t)job.ftile_begin * kTileWords;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t v = base + 256u * k;
+        const uint32_t s = v < job.nV ? __ldg(a.sc.first + job.vert_off + v) : kNoUse;
+        if (s != kNoUse) atomicOr(marks + (s >> 5), 1u << (s & 31));
+    }
+}
+
+// Running counts: CTAs [0, f_tiles) of the marks (per word), the rest of the
+// unused vertices (per 1024), in ticket order.
+__global__ void __launch_bounds__(128) k_build_count(const __grid_constant__ BuildArgs a)
+{
+    __shared__ uint32_t s_w[4], s_tile, s_before, s_bad;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (tid == 0) {
+        s_tile = atomicAdd(a.sc.tickets + 8, 1u);
+        s_bad = ld_state(a.sc.fail);
+    }
+    __syncthreads();
+    if (s_bad) return;
+    const bool faces = s_tile < a.f_tiles;
+    const uint32_t tile = faces ? s_tile : s_tile - a.f_tiles;
+    uint32_t j;
+    const BuildJob& job = faces ? job_of(a, a.ftile_job, tile, j) : job_of(a, a.vtile_job, tile, j);
+    const uint32_t chain = faces ? job.ftile_begin : job.vtile_begin;
+    constexpr uint32_t kPer = kTileWords / 128;  // words of a thread
+    uint32_t c[kPer] = {}, cnt = 0;
+    if (faces) {
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            c[k] = __popc(a.sc.marks[(size_t)tile * kTileWords + kPer * tid + k]);
+            cnt += c[k];
+        }
+    } else {
+        // thread t: 32 vertices; a warp's 1024 are one block of k_build_place
+        const uint32_t v0 = (tile - chain) * kBuildTile + 32u * tid;
+        const uint32_t* first = a.sc.first + job.vert_off;
+        for (uint32_t k = 0; k < 32 && v0 + k < job.nV; ++k) cnt += __ldg(first + v0 + k) == kNoUse ? 1u : 0u;
+    }
+    uint32_t x = cnt;  // inclusive scan over the CTA
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, s);
+        if ((int)lane >= s) x += y;
+    }
+    if (lane == 31) s_w[w] = x;
+    __syncthreads();
+    uint32_t pre = 0, sum = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        pre += i < w ? s_w[i] : 0u;
+        sum += s_w[i];
+    }
+    if (w == 0) {
+        uint32_t before;
+        const bool ok = lookback(a, a.sc.order_state + (faces ? 0u : a.f_tiles), chain, tile, sum, before);
+        if (lane == 0) {
+            s_before = before;
+            s_bad = ok ? 0u : 1u;
+        }
+    }
+    __syncthreads();
+    if (s_bad) {
+        if (tid == 0) give_up(a);
+        return;
+    }
+    uint32_t run = s_before + pre + x - cnt;
+    if (faces) {
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            a.sc.counts[(size_t)tile * kTileWords + kPer * tid + k] = run;
+            run += c[k];
+        }
+    } else if (lane == 0) {
+        a.sc.unused[4 * tile + w] = run;
+    }
+}
+
+// Every vertex to its number: the map from old to new, positions and the
+// caller-order map in the new order (to the scratch).
+__global__ void __launch_bounds__(256) k_build_place(const __grid_constant__ BuildArgs a)
+{
+    __shared__ uint32_t s_w[8];
+    if (ld_state(a.sc.fail)) return;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    uint32_t j;
+    const BuildJob& job = job_of(a, a.vtile_job, blockIdx.x >> 2, j);
+    const uint32_t base = ((blockIdx.x >> 2) - job.vtile_begin) * kBuildTile + (blockIdx.x & 3u) * 1024u;
+    const uint32_t* marks = a.sc.marks + (size_t)job.ftile_begin * kTileWords;
+    const uint32_t* counts = a.sc.counts + (size_t)job.ftile_begin * kTileWords;
+    uint32_t s[4], v[4], unused = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        v[k] = base + 256u * k + tid;
+        s[k] = v[k] < job.nV ? __ldg(a.sc.first + job.vert_off + v[k]) : 0u;
+        unused |= v[k] < job.nV && s[k] == kNoUse ? 1u << k : 0u;
+    }
+    if (__syncthreads_or(unused)) {
+        // number the unused ones after the used ones: in vertex order, 256 at a time
+        const uint32_t last = job.ftile_begin + (job.nT + kBuildTile - 1) / kBuildTile;
+        uint32_t run = (ld_state(a.sc.order_state + last - 1) & kStateValue) + a.sc.unused[blockIdx.x];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t m = __ballot_sync(0xffffffffu, (unused >> k) & 1u);
+            if (lane == 0) s_w[w] = __popc(m);
+            __syncthreads();
+            uint32_t pre = 0, sum = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                pre += i < w ? s_w[i] : 0u;
+                sum += s_w[i];
+            }
+            __syncthreads();
+            if ((unused >> k) & 1u) s[k] = run + pre + __popc(m & ((1u << lane) - 1u));
+            run += sum;
+        }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        if (v[k] >= job.nV) continue;
+        const uint32_t nv = (unused >> k) & 1u ? s[k]
+                                               : __ldg(counts + (s[k] >> 5)) + __popc(__ldg(marks + (s[k] >> 5)) & ((1u << (s[k] & 31)) - 1u));
+        a.sc.inv[job.vert_off + v[k]] = nv;
+        a.sc.pos_new[job.vert_off + nv] = __ldg(job.pos_out + v[k]);
+        a.sc.vperm_new[job.vert_off + nv] = job.vperm ? __ldg(job.vperm + v[k]) : v[k];
+    }
+}
+
+// Face records and the caller-order faces to the new numbering, positions and
+// the map back into each tree's own buffers.
+__global__ void __launch_bounds__(256) k_build_apply(const __grid_constant__ BuildArgs a)
+{
+    if (ld_state(a.sc.fail)) return;
+    const bool faces = blockIdx.x < 4 * a.f_tiles;
+    const uint32_t block = faces ? blockIdx.x : blockIdx.x - 4 * a.f_tiles;
+    uint32_t j;
+    const BuildJob& job = faces ? job_of(a, a.ftile_job, block >> 2, j) : job_of(a, a.vtile_job, block >> 2, j);
+    const uint32_t base = (block - 4 * (faces ? job.ftile_begin : job.vtile_begin)) * 1024u + threadIdx.x;
+    if (faces) {
+        const uint32_t* inv = a.sc.inv + job.vert_off;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t f = base + 256u * k;
+            if (f >= job.nT) break;
+            uint4 r = job.face_out[f];
+            r.x = __ldg(inv + r.x);
+            r.y = __ldg(inv + r.y);
+            r.z = __ldg(inv + r.z);
+            job.face_out[f] = r;
+            uint32_t* t = job.tri_rw + 3 * (size_t)r.w;
+            t[0] = r.x;
+            t[1] = r.y;
+            t[2] = r.z;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t v = base + 256u * k;
+            if (v >= job.nV) break;
+            job.pos_out[v] = a.sc.pos_new[job.vert_off + v];
+            job.vperm_out[v] = a.sc.vperm_new[job.vert_off + v];
+        }
+    }
+}
+
+// The scratch of a build: `p` (256-byte aligned) laid out; returns the bytes,
+// of which the first `zero_bytes` have to be zero when the build starts.
+size_t build_scratch(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t n_verts, void* p)
+{
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        void* q = (uint8_t*)p + off;
+        off += (bytes + 255) / 256 * 256;
+        return q;
+    };
+    BuildScratch& s = a.sc;
+    s.fail = (uint32_t*)take(256);
+    s.tickets = s.fail + 16;  // one per sort pass (8), one of k_build_count
+    s.bounds = (uint32_t*)take(6 * (size_t)n_jobs * 4);
+    s.hist = (uint32_t*)take((size_t)n_jobs * a.passes * 256 * 4);
+    s.order_state = (uint32_t*)take(((size_t)a.f_tiles + a.v_tiles) * 4);
+    s.marks = (uint32_t*)take((size_t)a.f_tiles * kTileWords * 4);
+    s.sort_state[0] = (uint32_t*)take((size_t)a.f_tiles * 256 * 4);
+    s.zero_bytes = off;
+    s.sort_state[1] = (uint32_t*)take((size_t)a.f_tiles * 256 * 4);
+    for (int i = 0; i < 2; ++i) {
+        s.keys[i] = (uint32_t*)take((size_t)n_faces * 4);
+        s.vals[i] = (uint32_t*)take((size_t)n_faces * 4);
+    }
+    s.hi = a.passes == 8 ? (uint32_t*)take((size_t)n_faces * 4) : s.keys[0];
+    s.counts = (uint32_t*)take((size_t)a.f_tiles * kTileWords * 4);
+    s.unused = (uint32_t*)take(4 * (size_t)a.v_tiles * 4);
+    s.first = (uint32_t*)take((size_t)n_verts * 4);
+    s.inv = (uint32_t*)take((size_t)n_verts * 4);
+    s.vperm_new = (uint32_t*)take((size_t)n_verts * 4);
+    s.pos_new = (float4*)take((size_t)n_verts * 16);
+    return off;
+}
+
+cudaError_t launch_build(const BuildArgs& a, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(a.sc.fail, 0, a.sc.zero_bytes, s);
+    if (e != cudaSuccess) return e;
+    const bool wide = a.passes == 8;
+    note_launches(6 + a.passes);
+    k_build_vertices<<<4 * a.v_tiles, 256, 0, s>>>(a);
+    if (wide) k_build_codes<true><<<4 * a.f_tiles, 256, 0, s>>>(a);
+    else k_build_codes<false><<<4 * a.f_tiles, 256, 0, s>>>(a);
+    for (uint32_t p = 0; p < a.passes; ++p) {
+        if (p == 0) k_build_sort<true, false><<<a.f_tiles, kSortThreads, 0, s>>>(a, p, false);
+        else if (p + 1 < a.passes) k_build_sort<false, false><<<a.f_tiles, kSortThreads, 0, s>>>(a, p, p == 3);
+        else k_build_sort<false, true><<<a.f_tiles, kSortThreads, 0, s>>>(a, p, false);
+    }
+    k_build_mark<<<4 * a.v_tiles, 256, 0, s>>>(a);
+    k_build_count<<<a.f_tiles + a.v_tiles, 128, 0, s>>>(a);
+    k_build_place<<<4 * a.v_tiles, 256, 0, s>>>(a);
+    k_build_apply<<<4 * (a.f_tiles + a.v_tiles), 256, 0, s>>>(a);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
-size_t radix_sort_scratch_bytes(uint32_t n)
-{
-    const uint32_t n_tiles = (n + kRsTile - 1) / kRsTile;
-    return (size_t)256 * n_tiles * sizeof(uint32_t) + 256 * sizeof(uint32_t) + 2 * (size_t)n * sizeof(uint32_t);
-}
-
 cudaError_t launch_xyz_to_pos4(const float* xyz, const uint32_t* vperm, uint32_t nV, float4* pos, cudaStream_t s)
 {
     note_launches(1);
@@ -414,433 +688,17 @@ cudaError_t launch_gather_pos4(const float4* src, const uint32_t* vperm, uint32_
     return cudaGetLastError();
 }
 
-size_t reorder_scratch_bytes(uint32_t nV)
-{
-    const size_t arr = ((size_t)nV * 4 + 255) / 256 * 256;
-    return 4 * arr + ((size_t)nV * 16 + 255) / 256 * 256 + radix_sort_scratch_bytes(nV);
-}
-
-cudaError_t launch_reorder_vertices(uint4* face, uint32_t* tri, uint32_t nT, uint32_t nV, float4* pos,
-                                    uint32_t* vperm, bool has_vperm, void* scratch, cudaStream_t s)
-{
-    const size_t arr = ((size_t)nV * 4 + 255) / 256 * 256;
-    uint8_t* base = (uint8_t*)scratch;
-    uint32_t* first = (uint32_t*)base;
-    uint32_t* order = (uint32_t*)(base + arr);
-    uint32_t* inv = (uint32_t*)(base + 2 * arr);
-    uint32_t* vperm_new = (uint32_t*)(base + 3 * arr);
-    float4* pos_new = (float4*)(base + 4 * arr);
-    void* sort_scratch = base + 4 * arr + ((size_t)nV * 16 + 255) / 256 * 256;
-    const uint32_t vb = (nV + 255) / 256, fb = (nT + 255) / 256;
-    note_launches(3);
-    k_first_use_init<<<vb, 256, 0, s>>>(first, order, nV);
-    k_first_use<<<fb, 256, 0, s>>>(face, nT, first);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    e = launch_radix_sort(first, order, nV, 25, sort_scratch, s);  // stable: unused vertices keep their order
-    if (e != cudaSuccess) return e;
-    k_apply_order<<<vb, 256, 0, s>>>(order, nV, inv, pos, pos_new, has_vperm ? vperm : nullptr, vperm_new);
-    k_renumber_faces<<<fb, 256, 0, s>>>(face, tri, nT, inv);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    e = cudaMemcpyAsync(pos, pos_new, (size_t)nV * sizeof(float4), cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(vperm, vperm_new, (size_t)nV * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
-}
-
-cudaError_t launch_mesh_bounds(const float4* xyz, uint32_t nV, uint32_t* bound_keys, int num_sms, cudaStream_t s)
-{
-    note_launches(1);
-    k_bounds_init<<<1, 32, 0, s>>>(bound_keys);
-    uint32_t blocks = (nV + 255) / 256;
-    const uint32_t cap = (uint32_t)num_sms * 8u;
-    if (blocks > cap) blocks = cap;
-    if (blocks == 0) blocks = 1;
-    note_launches(1);
-    k_mesh_bounds<<<blocks, 256, 0, s>>>(xyz, nV, bound_keys);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_leaf_morton(const uint32_t* tri, const float4* xyz, uint32_t nT, const uint32_t* bound_keys,
-                               uint32_t* codes, uint32_t* idx, uint32_t* codes_hi, cudaStream_t s)
-{
-    note_launches(1);
-    k_leaf_morton<<<(nT + 255) / 256, 256, 0, s>>>(tri, xyz, nT, bound_keys, codes, idx, codes_hi);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_radix_sort(uint32_t* keys, uint32_t* vals, uint32_t n, int key_bits, void* scratch,
-                              cudaStream_t s)
-{
-    if (n <= 1) return cudaSuccess;
-    const uint32_t n_tiles = (n + kRsTile - 1) / kRsTile;
-    uint32_t* hist = (uint32_t*)scratch;
-    uint32_t* totals = hist + (size_t)256 * n_tiles;
-    uint32_t* k2 = totals + 256;
-    uint32_t* v2 = k2 + n;
-    uint32_t *ki = keys, *vi = vals, *ko = k2, *vo = v2;
-    int passes = 0;
-    for (int shift = 0; shift < key_bits; shift += 8) {
-        note_launches(1);
-        k_rs_hist<<<n_tiles, kRsThreads, 0, s>>>(ki, n, shift, hist, n_tiles);
-        note_launches(1);
-        k_rs_scan_digit<<<256, kRsThreads, 0, s>>>(hist, n_tiles, totals);
-        note_launches(1);
-        k_rs_scatter<<<n_tiles, kRsThreads, 0, s>>>(ki, vi, ko, vo, n, shift, hist, n_tiles, totals);
-        uint32_t* t = ki; ki = ko; ko = t;
-        t = vi; vi = vo; vo = t;
-        ++passes;
-    }
-    if (passes & 1) {
-        cudaMemcpyAsync(keys, ki, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(vals, vi, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gather_faces(const uint32_t* tri, const uint32_t* perm, uint32_t nT, uint4* out, cudaStream_t s)
-{
-    note_launches(1);
-    k_gather_faces<<<(nT + 255) / 256, 256, 0, s>>>(tri, perm, nT, out);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Multi-tree build: every stage is one launch for all trees of a scene. A CTA
-// finds its tree with a binary search over the jobs' first-CTA numbers.
-// Faces of all trees are numbered globally (tree t owns [face_off, +nT)); one
-// stable sort by Morton code followed by one stable sort by tree id gives,
-// per tree, the order of the single-tree build: (code, original index).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t find_job(const BuildJob* jobs, uint32_t n, uint32_t block, bool faces,
+__device__ __forceinline__ uint32_t find_job(const BuildJob* jobs, uint32_t n, uint32_t block,
                                              const uint32_t* __restrict__ table)
 {
     if (table) return __ldg(table + block);  // host-built block -> job map: one load
     uint32_t lo = 0, hi = n - 1;
     while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
-        const uint32_t b = faces ? jobs[mid].fblock_begin : jobs[mid].vblock_begin;
-        if (b <= block) lo = mid;
+        if (jobs[mid].vblock_begin <= block) lo = mid;
         else hi = mid - 1;
     }
     return lo;
-}
-
-__global__ void k_bounds_init_multi(const BuildJob* __restrict__ jobs, uint32_t n_jobs)
-{
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_jobs) return;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        jobs[j].bound_keys[k] = 0xffffffffu;
-        jobs[j].bound_keys[3 + k] = 0u;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_mesh_bounds_multi(const BuildJob* __restrict__ jobs, uint32_t n_jobs,
-                                                           const uint32_t* __restrict__ vjob)
-{
-    const uint32_t j = find_job(jobs, n_jobs, blockIdx.x, false, vjob);
-    const BuildJob job = jobs[j];
-    const uint32_t v = (blockIdx.x - job.vblock_begin) * blockDim.x + threadIdx.x;
-    uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    uint32_t mx[3] = {0u, 0u, 0u};
-    if (v < job.nV) {
-        const float4 p = __ldg(job.pos + v);
-        const float c[3] = {p.x, p.y, p.z};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) mn[k] = mx[k] = float_to_ordered(c[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        for (int s = 16; s > 0; s >>= 1) {
-            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], s));
-            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], s));
-        }
-    }
-    if ((threadIdx.x & 31) == 0 && (v - (threadIdx.x & 31)) < job.nV) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            atomicMin(job.bound_keys + k, mn[k]);
-            atomicMax(job.bound_keys + 3 + k, mx[k]);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) k_leaf_morton_multi(const BuildJob* __restrict__ jobs, uint32_t n_jobs,
-                                                           const uint32_t* __restrict__ fjob,
-                                                           uint32_t* __restrict__ codes, uint32_t* __restrict__ idx,
-                                                           uint32_t* __restrict__ tree_of, uint32_t* __restrict__ codes_hi)
-{
-    const uint32_t j = find_job(jobs, n_jobs, blockIdx.x, true, fjob);
-    const BuildJob job = jobs[j];
-    const uint32_t i = (blockIdx.x - job.fblock_begin) * blockDim.x + threadIdx.x;
-    if (i >= job.nT) return;
-    float bmin[3], bmax[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        bmin[k] = ordered_to_float(job.bound_keys[k]);
-        bmax[k] = ordered_to_float(job.bound_keys[3 + k]);
-    }
-    const uint32_t f0 = __ldg(job.tri + 3 * (size_t)i), f1 = __ldg(job.tri + 3 * (size_t)i + 1),
-                   f2 = __ldg(job.tri + 3 * (size_t)i + 2);
-    const float4 p0 = __ldg(job.pos + f0), p1 = __ldg(job.pos + f1), p2 = __ldg(job.pos + f2);
-    const float va[3] = {p0.x, p0.y, p0.z}, vb[3] = {p1.x, p1.y, p1.z}, vc[3] = {p2.x, p2.y, p2.z};
-    float u[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float mn = gmin(gmin(va[k], vb[k]), vc[k]), mx = gmax(gmax(va[k], vb[k]), vc[k]);
-        const float centroid = __fmul_rn(__fadd_rn(mn, mx), 0.5f);
-        u[k] = __fdiv_rn(__fsub_rn(centroid, bmin[k]), __fsub_rn(bmax[k], bmin[k]));
-    }
-    const uint32_t g = job.face_off + i;
-    uint32_t lo, hi;
-    morton_key(u, codes_hi != nullptr, lo, hi);
-    codes[g] = lo;
-    if (codes_hi) codes_hi[g] = hi;
-    idx[g] = g;
-    tree_of[g] = j;
-}
-
-__global__ void __launch_bounds__(256) k_gather_u32(const uint32_t* __restrict__ src, const uint32_t* __restrict__ idx,
-                                                    uint32_t n, uint32_t* __restrict__ dst)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = __ldg(src + __ldg(idx + i));
-}
-
-// Sorted position i (grouped by tree, trees in job order) -> that tree's face records.
-__global__ void __launch_bounds__(256) k_gather_faces_multi(const BuildJob* __restrict__ jobs, uint32_t n_jobs,
-                                                            const uint32_t* __restrict__ idx,
-                                                            const uint32_t* __restrict__ tree_of, uint32_t n)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t g = __ldg(idx + i);
-    const BuildJob& job = jobs[__ldg(tree_of + g)];
-    const uint32_t o = g - job.face_off;
-    job.face_out[i - job.face_off] =
-        make_uint4(__ldg(job.tri + 3 * (size_t)o), __ldg(job.tri + 3 * (size_t)o + 1), __ldg(job.tri + 3 * (size_t)o + 2), o);
-}
-
-// ---------------------------------------------------------------------------
-// Multi-tree vertex renumbering: the order of launch_reorder_vertices (used
-// vertices in the order of their first use by the sorted faces, then unused
-// ones in their previous order) for every tree at once, without a sort. A
-// vertex's new index is the number of first uses before its own: each
-// 256-face block counts the corners that are a first use, one scan over the
-// block counts gives every block its offset, and the tree's own offset is
-// that of its first block (blocks never straddle trees). Unused vertices are
-// ranked the same way over 256-vertex blocks, after the tree's used ones.
-// Global vertex index g = vert_off + v; six launches for any number of trees.
-// ---------------------------------------------------------------------------
-constexpr uint32_t kNoUse = 0xffffffffu;
-
-struct RenumberScratch {
-    uint32_t* first;     // n_verts: first-use slot (3 f + corner) of each vertex
-    uint32_t* inv;       // n_verts: new index of each vertex
-    float4* pos_new;     // n_verts
-    uint32_t* vperm_new; // n_verts
-    uint32_t* fscan;     // f_blocks + 1: first uses per face block, then their exclusive scan
-    uint32_t* vscan;     // v_blocks + 1: unused vertices per vertex block, then the scan
-};
-
-__host__ __device__ inline size_t rn_align(size_t b) { return (b + 255) / 256 * 256; }
-
-__host__ __device__ inline RenumberScratch rn_scratch(void* base, uint32_t n_verts, uint32_t v_blocks,
-                                                      uint32_t f_blocks)
-{
-    uint8_t* p = (uint8_t*)base;
-    RenumberScratch r;
-    const size_t a4 = rn_align((size_t)n_verts * 4);
-    r.first = (uint32_t*)p;
-    r.inv = (uint32_t*)(p + a4);
-    r.vperm_new = (uint32_t*)(p + 2 * a4);
-    r.pos_new = (float4*)(p + 3 * a4);
-    r.fscan = (uint32_t*)(p + 3 * a4 + rn_align((size_t)n_verts * 16));
-    r.vscan = r.fscan + rn_align((size_t)(f_blocks + 1) * 4) / 4;
-    return r;
-}
-
-__global__ void __launch_bounds__(256) k_rn_init(const BuildJob* __restrict__ jobs, const uint32_t* __restrict__ vjob,
-                                                 uint32_t* __restrict__ first)
-{
-    const BuildJob& job = jobs[__ldg(vjob + blockIdx.x)];
-    const uint32_t v = (blockIdx.x - job.vblock_begin) * 256u + threadIdx.x;
-    if (v < job.nV) first[job.vert_off + v] = kNoUse;
-}
-
-__global__ void __launch_bounds__(256) k_rn_first_use(const BuildJob* __restrict__ jobs,
-                                                      const uint32_t* __restrict__ fjob, uint32_t* __restrict__ first)
-{
-    const BuildJob& job = jobs[__ldg(fjob + blockIdx.x)];
-    const uint32_t f = (blockIdx.x - job.fblock_begin) * 256u + threadIdx.x;
-    if (f >= job.nT) return;
-    const uint4 r = job.face_out[f];
-    uint32_t* fj = first + job.vert_off;
-    atomicMin(fj + r.x, 3u * f);
-    atomicMin(fj + r.y, 3u * f + 1u);
-    atomicMin(fj + r.z, 3u * f + 2u);
-}
-
-// This thread's count (first-use corners of its face, or 1 for an unused
-// vertex) for the block kinds below: CTAs [0, f_blocks) are face blocks,
-// the rest vertex blocks.
-struct RnItem {
-    const BuildJob* job;
-    bool face_block;
-    uint32_t i;      // face or vertex of the job
-    uint32_t cnt;
-    uint32_t mask;   // face blocks: which corners are first uses
-    uint4 r;         // face blocks: the face record
-};
-__device__ __forceinline__ RnItem rn_item(const BuildJob* jobs, const uint32_t* vjob, const uint32_t* fjob,
-                                          uint32_t f_blocks, const uint32_t* first)
-{
-    RnItem it{};
-    it.face_block = blockIdx.x < f_blocks;
-    if (it.face_block) {
-        it.job = jobs + __ldg(fjob + blockIdx.x);
-        it.i = (blockIdx.x - it.job->fblock_begin) * 256u + threadIdx.x;
-        if (it.i < it.job->nT) {
-            it.r = it.job->face_out[it.i];
-            const uint32_t* fj = first + it.job->vert_off;
-            it.mask = (__ldg(fj + it.r.x) == 3u * it.i ? 1u : 0u) | (__ldg(fj + it.r.y) == 3u * it.i + 1u ? 2u : 0u) |
-                      (__ldg(fj + it.r.z) == 3u * it.i + 2u ? 4u : 0u);
-            it.cnt = __popc(it.mask);
-        }
-    } else {
-        const uint32_t b = blockIdx.x - f_blocks;
-        it.job = jobs + __ldg(vjob + b);
-        it.i = (b - it.job->vblock_begin) * 256u + threadIdx.x;
-        if (it.i < it.job->nV) it.cnt = __ldg(first + it.job->vert_off + it.i) == kNoUse ? 1u : 0u;
-    }
-    return it;
-}
-
-__global__ void __launch_bounds__(256) k_rn_count(const BuildJob* __restrict__ jobs, const uint32_t* __restrict__ vjob,
-                                                  const uint32_t* __restrict__ fjob, uint32_t f_blocks,
-                                                  RenumberScratch sc)
-{
-    __shared__ uint32_t sh[8];
-    const RnItem it = rn_item(jobs, vjob, fjob, f_blocks, sc.first);
-    uint32_t tot;
-    block_exclusive_scan(it.cnt, &tot, sh);
-    if (threadIdx.x == 0) {
-        if (it.face_block) sc.fscan[blockIdx.x] = tot;
-        else sc.vscan[blockIdx.x - f_blocks] = tot;
-    }
-}
-
-// CTA 0 scans fscan[0..f_blocks), CTA 1 vscan[0..v_blocks), in place
-// (exclusive; the total goes to entry n), 4 entries per thread per step.
-__global__ void __launch_bounds__(256) k_rn_scan(RenumberScratch sc, uint32_t f_blocks, uint32_t v_blocks)
-{
-    __shared__ uint32_t sh[8];
-    uint32_t* a = blockIdx.x == 0 ? sc.fscan : sc.vscan;
-    const uint32_t n = blockIdx.x == 0 ? f_blocks : v_blocks;
-    uint32_t carry = 0;
-    for (uint32_t s = 0; s < n; s += 4 * 256) {
-        const uint32_t i0 = s + 4 * threadIdx.x;
-        uint32_t v[4], sum = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            v[k] = i0 + k < n ? a[i0 + k] : 0u;
-            sum += v[k];
-        }
-        uint32_t tot;
-        uint32_t ex = carry + block_exclusive_scan(sum, &tot, sh);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (i0 + k < n) a[i0 + k] = ex;
-            ex += v[k];
-        }
-        carry += tot;
-    }
-    if (threadIdx.x == 0) a[n] = carry;
-}
-
-// New index of every vertex; positions and the caller-order map in the new
-// order into the scratch.
-__global__ void __launch_bounds__(256) k_rn_assign(const BuildJob* __restrict__ jobs, const uint32_t* __restrict__ vjob,
-                                                   const uint32_t* __restrict__ fjob, uint32_t f_blocks,
-                                                   RenumberScratch sc)
-{
-    __shared__ uint32_t sh[8];
-    const RnItem it = rn_item(jobs, vjob, fjob, f_blocks, sc.first);
-    uint32_t tot;
-    const uint32_t ex = block_exclusive_scan(it.cnt, &tot, sh);
-    if (it.cnt == 0) return;
-    const BuildJob& job = *it.job;
-    const uint32_t vo = job.vert_off;
-    const uint32_t f_first = job.fblock_begin, f_end = job.fblock_begin + (job.nT + 255u) / 256u;
-    auto place = [&](uint32_t v, uint32_t nv) {
-        sc.inv[vo + v] = nv;
-        sc.pos_new[vo + nv] = __ldg(job.pos_out + v);
-        sc.vperm_new[vo + nv] = job.vperm ? __ldg(job.vperm + v) : v;
-    };
-    if (it.face_block) {
-        uint32_t rank = sc.fscan[blockIdx.x] - sc.fscan[f_first] + ex;
-        if (it.mask & 1u) place(it.r.x, rank++);
-        if (it.mask & 2u) place(it.r.y, rank++);
-        if (it.mask & 4u) place(it.r.z, rank);
-    } else {
-        const uint32_t used = sc.fscan[f_end] - sc.fscan[f_first];
-        const uint32_t b = blockIdx.x - f_blocks;
-        place(it.i, used + sc.vscan[b] - sc.vscan[job.vblock_begin] + ex);
-    }
-}
-
-// Faces and `tri` to the new numbering; positions and the map copied back
-// into each tree's own buffers.
-__global__ void __launch_bounds__(256) k_rn_apply(const BuildJob* __restrict__ jobs, const uint32_t* __restrict__ vjob,
-                                                  const uint32_t* __restrict__ fjob, uint32_t f_blocks,
-                                                  RenumberScratch sc)
-{
-    if (blockIdx.x < f_blocks) {
-        const BuildJob& job = jobs[__ldg(fjob + blockIdx.x)];
-        const uint32_t f = (blockIdx.x - job.fblock_begin) * 256u + threadIdx.x;
-        if (f >= job.nT) return;
-        const uint32_t* inv = sc.inv + job.vert_off;
-        uint4 r = job.face_out[f];
-        r.x = __ldg(inv + r.x);
-        r.y = __ldg(inv + r.y);
-        r.z = __ldg(inv + r.z);
-        job.face_out[f] = r;
-        uint32_t* t = job.tri_rw + 3 * (size_t)f;
-        t[0] = __ldg(inv + t[0]);
-        t[1] = __ldg(inv + t[1]);
-        t[2] = __ldg(inv + t[2]);
-    } else {
-        const uint32_t b = blockIdx.x - f_blocks;
-        const BuildJob& job = jobs[__ldg(vjob + b)];
-        const uint32_t v = (b - job.vblock_begin) * 256u + threadIdx.x;
-        if (v >= job.nV) return;
-        job.pos_out[v] = sc.pos_new[job.vert_off + v];
-        job.vperm_out[v] = sc.vperm_new[job.vert_off + v];
-    }
-}
-
-size_t reorder_multi_scratch_bytes(uint32_t n_verts, uint32_t v_blocks, uint32_t f_blocks)
-{
-    return 3 * rn_align((size_t)n_verts * 4) + rn_align((size_t)n_verts * 16) + rn_align((size_t)(f_blocks + 1) * 4) +
-           rn_align((size_t)(v_blocks + 1) * 4);
-}
-
-cudaError_t launch_reorder_vertices_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks,
-                                          uint32_t f_blocks, const uint32_t* vjob, const uint32_t* fjob,
-                                          uint32_t n_verts, void* scratch, cudaStream_t s)
-{
-    if (n_jobs == 0 || v_blocks == 0 || f_blocks == 0) return cudaSuccess;
-    const RenumberScratch sc = rn_scratch(scratch, n_verts, v_blocks, f_blocks);
-    note_launches(6);
-    k_rn_init<<<v_blocks, 256, 0, s>>>(d_jobs, vjob, sc.first);
-    k_rn_first_use<<<f_blocks, 256, 0, s>>>(d_jobs, fjob, sc.first);
-    k_rn_count<<<f_blocks + v_blocks, 256, 0, s>>>(d_jobs, vjob, fjob, f_blocks, sc);
-    k_rn_scan<<<2, 256, 0, s>>>(sc, f_blocks, v_blocks);
-    k_rn_assign<<<f_blocks + v_blocks, 256, 0, s>>>(d_jobs, vjob, fjob, f_blocks, sc);
-    k_rn_apply<<<f_blocks + v_blocks, 256, 0, s>>>(d_jobs, vjob, fjob, f_blocks, sc);
-    return cudaGetLastError();
 }
 
 // Rigid transforms of every tree: pos = M * rest, M a row-major 3x4 matrix per
@@ -862,7 +720,7 @@ __global__ void __launch_bounds__(256, 8) k_transform_multi(const BuildJob* __re
         const uint32_t vb = blockIdx.x * kTransformUnroll + k;
         jj[k] = 0xffffffffu;
         if (vb >= v_blocks) continue;
-        const uint32_t j = find_job(jobs, n_jobs, vb, false, vjob);
+        const uint32_t j = find_job(jobs, n_jobs, vb, vjob);
         const uint32_t v = (vb - jobs[j].vblock_begin) * 256u + threadIdx.x;
         if (v >= jobs[j].nV) continue;
         jj[k] = j;
@@ -886,45 +744,6 @@ __global__ void __launch_bounds__(256, 8) k_transform_multi(const BuildJob* __re
     }
 }
 
-cudaError_t launch_build_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, uint32_t f_blocks,
-                               const uint32_t* vjob, const uint32_t* fjob, uint32_t n_faces, uint32_t tree_bits,
-                               bool wide, void* scratch, cudaStream_t s)
-{
-    // scratch: codes, idx, tree_of, keys2, codes_hi (5 x n_faces u32), then the sort scratch
-    uint32_t* codes = (uint32_t*)scratch;
-    uint32_t* idx = codes + n_faces;
-    uint32_t* tree_of = idx + n_faces;
-    uint32_t* keys2 = tree_of + n_faces;
-    uint32_t* codes_hi = keys2 + n_faces;
-    void* sort_scratch = codes_hi + n_faces;
-    note_launches(4);
-    k_bounds_init_multi<<<(n_jobs + 255) / 256, 256, 0, s>>>(d_jobs, n_jobs);
-    k_mesh_bounds_multi<<<v_blocks, 256, 0, s>>>(d_jobs, n_jobs, vjob);
-    k_leaf_morton_multi<<<f_blocks, 256, 0, s>>>(d_jobs, n_jobs, fjob, codes, idx, tree_of, wide ? codes_hi : nullptr);
-    // stable LSD order: low key bits, [high key bits,] then the tree id
-    cudaError_t e = launch_radix_sort(codes, idx, n_faces, wide ? 32 : 30, sort_scratch, s);
-    if (e != cudaSuccess) return e;
-    if (wide) {
-        note_launches(1);
-        k_gather_u32<<<(n_faces + 255) / 256, 256, 0, s>>>(codes_hi, idx, n_faces, keys2);
-        e = launch_radix_sort(keys2, idx, n_faces, 31, sort_scratch, s);
-        if (e != cudaSuccess) return e;
-    }
-    k_gather_u32<<<(n_faces + 255) / 256, 256, 0, s>>>(tree_of, idx, n_faces, keys2);
-    if (tree_bits > 0) {
-        e = launch_radix_sort(keys2, idx, n_faces, (int)tree_bits, sort_scratch, s);
-        if (e != cudaSuccess) return e;
-    }
-    note_launches(1);
-    k_gather_faces_multi<<<(n_faces + 255) / 256, 256, 0, s>>>(d_jobs, n_jobs, idx, tree_of, n_faces);
-    return cudaGetLastError();
-}
-
-size_t build_multi_scratch_bytes(uint32_t n_faces)
-{
-    return 5 * (size_t)n_faces * sizeof(uint32_t) + radix_sort_scratch_bytes(n_faces);
-}
-
 cudaError_t launch_transform_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, const uint32_t* vjob,
                                    const float4* rest, const float* mats, bool rest_tree_order, cudaStream_t s)
 {
@@ -941,7 +760,7 @@ __global__ void __launch_bounds__(256) k_gather_rest_multi(const BuildJob* __res
                                                            const uint32_t* __restrict__ vjob,
                                                            const float4* __restrict__ rest, float4* __restrict__ out)
 {
-    const uint32_t j = find_job(jobs, n_jobs, blockIdx.x, false, vjob);
+    const uint32_t j = find_job(jobs, n_jobs, blockIdx.x, vjob);
     const uint32_t v = (blockIdx.x - jobs[j].vblock_begin) * 256u + threadIdx.x;
     if (v >= jobs[j].nV) return;
     const uint32_t* vp = jobs[j].vperm;
@@ -957,13 +776,5 @@ cudaError_t launch_gather_rest_multi(const BuildJob* d_jobs, uint32_t n_jobs, ui
     return cudaGetLastError();
 }
 
-
-cudaError_t launch_gather_u32(const uint32_t* src, const uint32_t* idx, uint32_t n, uint32_t* out, cudaStream_t s)
-{
-    if (n == 0) return cudaSuccess;
-    note_launches(1);
-    k_gather_u32<<<(n + 255) / 256, 256, 0, s>>>(src, idx, n, out);
-    return cudaGetLastError();
-}
 
 } // namespace oibvh

@@ -103,22 +103,36 @@ static int sync_positions(oibvh_tree_t t, cudaStream_t s)
     return OIBVH_OK;
 }
 
-// After the faces are sorted: vertices renumbered in the order the sorted
-// faces first use them (faces, `tri`, positions and the caller-order map).
-// `scratch` (reorder_scratch_bytes(nV) or more) may be shared by trees
-// renumbered one after another on the same stream; nullptr: a private one.
-static int reorder_vertices(oibvh_tree_t t, cudaStream_t s, void* scratch = nullptr)
+// A pinned word per build that a build kernel sets when it gives up (a wait
+// that ran out). The words outlive the builds: one page, taken in turn.
+static uint32_t* build_error_word()
 {
-    DevBuf<uint8_t> own;
-    if (!scratch) {
-        OK_TRY(own.ensure(reorder_scratch_bytes(t->nV), "cudaMalloc(reorder scratch)"));
-        scratch = own.p;
-    }
-    OK_TRY(t->vperm.ensure(t->nV, "cudaMalloc(vertex order)"));
-    CUDA_TRY(launch_reorder_vertices(t->face.p, t->tri.p, t->nT, t->nV, t->pos4.p, t->vperm.p, t->reordered,
-                                     scratch, s));
-    if (own.p) CUDA_TRY(cudaStreamSynchronize(s));  // the private scratch is freed on return
-    t->reordered = true;
+    static uint32_t* page = [] {
+        void* p = nullptr;
+        return cudaHostAlloc(&p, 4096, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess ? (uint32_t*)p : nullptr;
+    }();
+    static std::atomic<uint32_t> next{0};
+    if (!page) return nullptr;
+    uint32_t* w = page + next.fetch_add(1, std::memory_order_relaxed) % 1024u;
+    *(volatile uint32_t*)w = 0;
+    return w;
+}
+
+// The faces sorted and the vertices renumbered, for the jobs of `a` (which
+// holds everything but the scratch and the error word). Blocking.
+static int build_impl(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t n_verts, int device, cudaStream_t s)
+{
+    a.host_error = build_error_word();
+    if (!a.host_error) return fail(OIBVH_ERR_OOM, "cudaHostAlloc(build error words)");
+    PoolBuf scratch(device, s);
+    OK_TRY(scratch.ensure(build_scratch(a, n_jobs, n_faces, n_verts, nullptr), "build scratch"));
+    build_scratch(a, n_jobs, n_faces, n_verts, scratch.p);
+    CUDA_TRY(launch_build(a, s));
+    return OIBVH_OK;
+}
+static int build_check(const BuildArgs& a)
+{
+    if (*(volatile uint32_t*)a.host_error) return fail(OIBVH_ERR_TIMEOUT, "a wait between the build's tiles ran out");
     return OIBVH_OK;
 }
 
@@ -126,33 +140,18 @@ static int tree_build_impl(oibvh_tree_t t, cudaStream_t s)
 {
     if (!t) return fail(OIBVH_ERR_ARG, "tree is NULL");
     DeviceGuard g(t->device);
-    const uint32_t nT = t->nT;
-    // scratch: bounds keys, codes, indices, sort buffers
-    DevBuf<uint8_t> scratch;
-    const bool wide = t->morton_bits == 63;
-    const size_t sort_bytes = radix_sort_scratch_bytes(nT);
-    const size_t arr = ((size_t)nT * 4 + 255) / 256 * 256;
-    const size_t codes_off = 256, idx_off = codes_off + arr, hi_off = idx_off + arr, gath_off = hi_off + arr;
-    const size_t sort_off = gath_off + arr;
-    OK_TRY(scratch.ensure(sort_off + sort_bytes, "cudaMalloc(build scratch)"));
-    uint32_t* keys6 = (uint32_t*)scratch.p;
-    uint32_t* codes = (uint32_t*)(scratch.p + codes_off);
-    uint32_t* idx = (uint32_t*)(scratch.p + idx_off);
-    uint32_t* hi = (uint32_t*)(scratch.p + hi_off);
-    uint32_t* hi_sorted = (uint32_t*)(scratch.p + gath_off);
+    OK_TRY(t->vperm.ensure(t->nV, "cudaMalloc(vertex order)"));
     OK_TRY(sync_positions(t, s));
-    CUDA_TRY(launch_mesh_bounds(t->cur_pos, t->nV, keys6, sm_count(t->device), s));
-    CUDA_TRY(launch_leaf_morton(t->tri.p, t->cur_pos, nT, keys6, codes, idx, wide ? hi : nullptr, s));
-    // stable LSD order by (key, original index): low key bits first, then the high ones
-    CUDA_TRY(launch_radix_sort(codes, idx, nT, wide ? 32 : 30, scratch.p + sort_off, s));
-    if (wide) {
-        CUDA_TRY(launch_gather_u32(hi, idx, nT, hi_sorted, s));
-        CUDA_TRY(launch_radix_sort(hi_sorted, idx, nT, 31, scratch.p + sort_off, s));
-    }
-    CUDA_TRY(launch_gather_faces(t->tri.p, idx, nT, t->face.p, s));
-    OK_TRY(reorder_vertices(t, s));
+    BuildArgs a{};
+    a.one = t->build_job();
+    a.f_tiles = (t->nT + kBuildTile - 1) / kBuildTile;
+    a.v_tiles = (t->nV + kBuildTile - 1) / kBuildTile;
+    a.passes = t->morton_bits == 63 ? 8 : 4;
+    OK_TRY(build_impl(a, 1, t->nT, t->nV, t->device, s));
     CUDA_TRY(launch_refit_one(t->job(), s));
     CUDA_TRY(cudaStreamSynchronize(s));
+    OK_TRY(build_check(a));
+    t->reordered = true;
     t->built = true;
     return OIBVH_OK;
 }
@@ -190,10 +189,10 @@ struct oibvh_scene_s {
 
     // multi-tree build / transform: job table for the current tree list
     DevBuf<BuildJob> build_jobs;
-    DevBuf<uint32_t> vblock_job, fblock_job;  // 256-vertex / 256-face block -> job
-    DevBuf<uint32_t> bound_keys;
+    DevBuf<uint32_t> vblock_job;            // 256-vertex block -> job
+    DevBuf<uint32_t> ftile_job, vtile_job;  // kBuildTile-face / -vertex tile -> job
     std::vector<BuildJob> build_cache;
-    uint32_t v_blocks = 0, f_blocks = 0, n_faces = 0, n_verts = 0;
+    uint32_t v_blocks = 0, f_tiles = 0, v_tiles = 0, n_faces = 0, n_verts = 0;
 
     // tuning (oibvh_scene_set_tuning / oibvh_scene_autotune)
     uint32_t tune_start_log2 = 16;  // start cross product ~ 2^this node pairs per pass
@@ -1059,27 +1058,18 @@ int ensure_build_jobs(oibvh_scene_s* s, cudaStream_t st)
 {
     const size_t n = s->trees.size();
     std::vector<BuildJob> jobs(n);
-    uint32_t vb = 0, fb = 0, fo = 0, vo = 0;
-    OK_TRY(s->bound_keys.ensure(6 * std::max<size_t>(n, 1), "cudaMalloc(bounds)"));
+    uint32_t vb = 0, ft = 0, vt = 0, fo = 0, vo = 0;
     for (size_t i = 0; i < n; ++i) {
         const oibvh_tree_t t = s->trees[i];
-        BuildJob j{};
-        j.pos = t->cur_pos;
-        j.tri = t->tri.p;
-        j.face_out = t->face.p;
-        j.bound_keys = s->bound_keys.p + 6 * i;
-        j.pos_out = t->pos4.p;
-        j.nV = t->nV;
-        j.nT = t->nT;
+        BuildJob j = t->build_job();
         j.vblock_begin = vb;
-        j.fblock_begin = fb;
+        j.ftile_begin = ft;
+        j.vtile_begin = vt;
         j.face_off = fo;
         j.vert_off = vo;
-        j.vperm = t->vmap();
-        j.vperm_out = t->vperm.p;
-        j.tri_rw = t->tri.p;
         vb += (t->nV + 255) / 256;
-        fb += (t->nT + 255) / 256;
+        ft += (t->nT + kBuildTile - 1) / kBuildTile;
+        vt += (t->nV + kBuildTile - 1) / kBuildTile;
         if ((uint64_t)fo + t->nT > 0xffffffffull || (uint64_t)vo + t->nV > 0xffffffffull)
             return fail(OIBVH_ERR_ARG, "the scene holds more than 2^32 faces or vertices");
         fo += t->nT;
@@ -1087,7 +1077,8 @@ int ensure_build_jobs(oibvh_scene_s* s, cudaStream_t st)
         jobs[i] = j;
     }
     s->v_blocks = vb;
-    s->f_blocks = fb;
+    s->f_tiles = ft;
+    s->v_tiles = vt;
     s->n_faces = fo;
     s->n_verts = vo;
     bool same = s->build_cache.size() == n && s->build_jobs.p;
@@ -1095,18 +1086,19 @@ int ensure_build_jobs(oibvh_scene_s* s, cudaStream_t st)
     if (!same) {
         OK_TRY(s->build_jobs.ensure(std::max<size_t>(n, 1), "cudaMalloc(build jobs)"));
         OK_TRY(s->vblock_job.ensure(std::max(1u, vb), "cudaMalloc(vertex block map)"));
-        OK_TRY(s->fblock_job.ensure(std::max(1u, fb), "cudaMalloc(face block map)"));
-        std::vector<uint32_t> vmap(vb), fmap(fb);
+        OK_TRY(s->ftile_job.ensure(std::max(1u, ft), "cudaMalloc(face tile map)"));
+        OK_TRY(s->vtile_job.ensure(std::max(1u, vt), "cudaMalloc(vertex tile map)"));
+        std::vector<uint32_t> vmap(vb), fmap(ft), wmap(vt);
         for (size_t i = 0; i < n; ++i) {
-            const oibvh_tree_t t = s->trees[i];
-            std::fill(vmap.begin() + jobs[i].vblock_begin, vmap.begin() + jobs[i].vblock_begin + (t->nV + 255) / 256,
-                      (uint32_t)i);
-            std::fill(fmap.begin() + jobs[i].fblock_begin, fmap.begin() + jobs[i].fblock_begin + (t->nT + 255) / 256,
-                      (uint32_t)i);
+            const bool end = i + 1 == n;
+            std::fill(vmap.begin() + jobs[i].vblock_begin, end ? vmap.end() : vmap.begin() + jobs[i + 1].vblock_begin, (uint32_t)i);
+            std::fill(fmap.begin() + jobs[i].ftile_begin, end ? fmap.end() : fmap.begin() + jobs[i + 1].ftile_begin, (uint32_t)i);
+            std::fill(wmap.begin() + jobs[i].vtile_begin, end ? wmap.end() : wmap.begin() + jobs[i + 1].vtile_begin, (uint32_t)i);
         }
         CUDA_TRY(cudaMemcpyAsync(s->build_jobs.p, jobs.data(), n * sizeof(BuildJob), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(s->vblock_job.p, vmap.data(), vb * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(s->fblock_job.p, fmap.data(), fb * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(s->ftile_job.p, fmap.data(), ft * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(s->vtile_job.p, wmap.data(), vt * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaStreamSynchronize(st));  // jobs and the maps are pageable host vectors
         s->build_cache = jobs;
     }
@@ -1124,31 +1116,31 @@ API int oibvh_scene_build(oibvh_scene_t s, void* stream)
     cudaStream_t st = (cudaStream_t)stream;
     for (auto t : s->trees) OK_TRY(sync_positions(t, st));
     OK_TRY(ensure_build_jobs(s, st));
-    DevBuf<uint8_t> scratch;  // the build stages, then (in stream order) the renumbering
-    OK_TRY(scratch.ensure(std::max(build_multi_scratch_bytes(s->n_faces),
-                                   reorder_multi_scratch_bytes(s->n_verts, s->v_blocks, s->f_blocks)),
-                          "cudaMalloc(build scratch)"));
     const uint32_t n = (uint32_t)s->trees.size();
-    const uint32_t tree_bits = n <= 1 ? 0u : ilog2(next_pow2(n));
     const bool wide = s->trees[0]->morton_bits == 63;
     for (auto t : s->trees)
         if ((t->morton_bits == 63) != wide)
             return fail(OIBVH_ERR_UNSUPPORTED, "a scene build needs the same Morton key width for every tree");
-    CUDA_TRY(launch_build_multi(s->build_jobs.p, n, s->v_blocks, s->f_blocks, s->vblock_job.p, s->fblock_job.p,
-                                s->n_faces, tree_bits, wide, scratch.p, st));
-    // every tree's vertices renumbered in the order its sorted faces first use
-    // them: six launches for all trees
-    CUDA_TRY(launch_reorder_vertices_multi(s->build_jobs.p, n, s->v_blocks, s->f_blocks, s->vblock_job.p,
-                                           s->fblock_job.p, s->n_verts, scratch.p, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    BuildArgs a{};
+    a.jobs = s->build_jobs.p;
+    a.ftile_job = s->ftile_job.p;
+    a.vtile_job = s->vtile_job.p;
+    a.f_tiles = s->f_tiles;
+    a.v_tiles = s->v_tiles;
+    a.passes = wide ? 8 : 4;
+    OK_TRY(build_impl(a, n, s->n_faces, s->n_verts, s->device, st));
     for (auto t : s->trees) {
         t->reordered = true;
         t->built = true;
     }
-    const int r = oibvh_scene_refit(s, stream);
-    if (r != OIBVH_OK) return r;
-    CUDA_TRY(cudaStreamSynchronize(st));
-    return OIBVH_OK;
+    int r = oibvh_scene_refit(s, stream);
+    if (r == OIBVH_OK) {
+        CUDA_TRY(cudaStreamSynchronize(st));
+        r = build_check(a);
+    }
+    if (r != OIBVH_OK)
+        for (auto t : s->trees) t->built = false;
+    return r;
     GUARD_END
 }
 

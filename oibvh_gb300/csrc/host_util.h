@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include <cuda_runtime.h>
@@ -140,6 +141,58 @@ struct DevBuf {
     }
 };
 
+// Scratch memory for one call, stream-ordered, from a pool of its own per
+// device that keeps up to 512 MB between calls (cudaMalloc and cudaFree of a
+// call's scratch cost more than a small build, and synchronise the device).
+inline cudaMemPool_t scratch_pool(int dev)
+{
+    struct Pools {
+        cudaMemPool_t p[64] = {};
+        std::once_flag once[64];
+    };
+    static Pools pools;
+    if (dev < 0 || dev >= 64) return nullptr;
+    std::call_once(pools.once[dev], [dev] {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        uint64_t keep = 512ull << 20;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools.p[dev] = pool;
+    });
+    return pools.p[dev];
+}
+struct PoolBuf {
+    uint8_t* p = nullptr;
+    int dev;
+    cudaStream_t s;
+    PoolBuf(int device, cudaStream_t stream) : dev(device), s(stream) {}
+    PoolBuf(const PoolBuf&) = delete;
+    PoolBuf& operator=(const PoolBuf&) = delete;
+    ~PoolBuf()
+    {
+        if (p) cudaFreeAsync(p, s);
+    }
+    int ensure(size_t bytes, const char* what)
+    {
+        cudaMemPool_t pool = scratch_pool(dev);
+        cudaError_t e = injected_alloc_failure() || !pool ? cudaErrorMemoryAllocation
+                                                         : cudaMallocFromPoolAsync((void**)&p, bytes, pool, s);
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();
+            return cuda_fail(e, what);
+        }
+        return OIBVH_OK;
+    }
+};
+
 template <class T>
 struct PinnedBuf {
     T* p = nullptr;
@@ -195,6 +248,22 @@ struct oibvh_tree_s {
     uint32_t morton_bits = 30;  // 30 (the reference's key) or 63 (21 bits per axis)
 
     const uint32_t* vmap() const { return reordered ? vperm.p : nullptr; }
+
+    // this tree alone (a scene sets the first tiles and offsets)
+    BuildJob build_job() const
+    {
+        BuildJob j{};
+        j.pos = cur_pos;
+        j.tri = tri.p;
+        j.face_out = face.p;
+        j.pos_out = pos4.p;
+        j.nV = nV;
+        j.nT = nT;
+        j.vperm = vmap();
+        j.vperm_out = vperm.p;
+        j.tri_rw = tri.p;
+        return j;
+    }
 
     RefitJob job() const
     {

@@ -29,27 +29,51 @@ struct BuildJob {
     const float4* pos;      // positions to build from (transform source when no packed rest array is given)
     const uint32_t* tri;    // faces as given (3 * nT)
     uint4* face_out;        // Morton-ordered face records
-    uint32_t* bound_keys;   // 6 words of scratch (mesh bounds)
     float4* pos_out;        // transform target (the tree's own positions)
     uint32_t nV, nT;
     uint32_t vblock_begin;  // first CTA of this tree in vertex-chunk launches (256 vertices per CTA)
-    uint32_t fblock_begin;  // first CTA of this tree in face-chunk launches (256 faces per CTA)
-    uint32_t face_off;      // first face of this tree in the global face numbering
+    uint32_t ftile_begin;   // first tile of this tree in the build's face tiles (kBuildTile faces each)
+    uint32_t vtile_begin;   // the same for its vertex tiles
+    uint32_t face_off;      // first face of this tree in the build's keys
     uint32_t vert_off;      // first vertex of this tree in packed rest positions
+    uint32_t pad0;
     const uint32_t* vperm;  // tree vertex v is the caller's vertex vperm[v] (nullptr: the same order)
     uint32_t* vperm_out;    // the tree's map buffer (nV entries), rewritten by the renumbering
     uint32_t* tri_rw;       // the tree's faces (3 * nT), rewritten by the renumbering (tri, writable)
 };
 
 // build_kernels.cu
-size_t radix_sort_scratch_bytes(uint32_t n);
-size_t build_multi_scratch_bytes(uint32_t n_faces);
-// vjob / fjob: optional host-built maps from a 256-vertex / 256-face block
-// to its job (nullptr: each CTA binary-searches the job table).
-// wide: 63-bit Morton keys (21 bits per axis) instead of the reference's 30.
-cudaError_t launch_build_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, uint32_t f_blocks,
-                               const uint32_t* vjob, const uint32_t* fjob, uint32_t n_faces, uint32_t tree_bits,
-                               bool wide, void* scratch, cudaStream_t s);
+constexpr uint32_t kBuildTile = 4096;  // faces (vertices) of a tile
+struct BuildScratch {
+    uint32_t* fail;           // a wait ran out: the build's later kernels return at once
+    uint32_t* tickets;        // next tile of each sort pass, next block of the renumbering
+    uint32_t* bounds;         // 6 words per job
+    uint32_t* hist;           // per job and pass: 256 digit counts
+    uint32_t* order_state;    // per face tile, then per vertex tile: look-back states
+    uint32_t* marks;          // a bit per face corner (sorted faces): a vertex's first use
+    uint32_t* counts;         // per word of marks: the tree's marks before it
+    uint32_t* unused;         // per 1024 vertices: the tree's unused vertices before them
+    uint32_t* sort_state[2];  // per face tile: 256 look-back states, in turn between passes
+    size_t zero_bytes;
+    uint32_t *keys[2], *vals[2], *hi;  // n_faces each (hi: 63-bit keys only)
+    uint32_t *first, *inv, *vperm_new; // n_verts: first-use slot, new number, caller-order map in the new order
+    float4* pos_new;                   // n_verts
+};
+struct BuildArgs {
+    const BuildJob* jobs;   // one job: nullptr, and the job in `one`
+    BuildJob one;
+    const uint32_t *ftile_job, *vtile_job;  // tile -> job
+    uint32_t f_tiles, v_tiles;
+    uint32_t passes;        // 4: the reference's 30-bit keys; 8: 63 bits (21 per axis)
+    uint32_t* host_error;   // pinned word, set when the build gave up
+    BuildScratch sc;
+};
+// Bytes of the build's scratch, and its parts set from `p`.
+size_t build_scratch(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t n_verts, void* p);
+// Bounds, codes, sort, sorted faces and vertex renumbering of every job: face
+// records, `tri` and positions get the new vertex numbers, vperm_out the new
+// caller-order map.
+cudaError_t launch_build(const BuildArgs& a, cudaStream_t s);
 // rest: packed positions of all jobs in each caller's vertex order (read
 // through the jobs' vperm), or in each tree's order (rest_tree_order), or
 // nullptr (each job's own pos). Writes each job's pos_out.
@@ -61,29 +85,6 @@ cudaError_t launch_gather_rest_multi(const BuildJob* d_jobs, uint32_t n_jobs, ui
 cudaError_t launch_xyz_to_pos4(const float* xyz, const uint32_t* vperm, uint32_t nV, float4* pos, cudaStream_t s);
 // pos[v] = src[vperm[v]] (vperm == nullptr: a copy)
 cudaError_t launch_gather_pos4(const float4* src, const uint32_t* vperm, uint32_t nV, float4* pos, cudaStream_t s);
-// Renumber a built tree's vertices in the order its sorted faces first use
-// them: face records and `tri` get the new indices, `pos` the new order and
-// vperm (nV entries; read first when has_vperm) the new caller-order map.
-size_t reorder_scratch_bytes(uint32_t nV);
-cudaError_t launch_reorder_vertices(uint4* face, uint32_t* tri, uint32_t nT, uint32_t nV, float4* pos,
-                                    uint32_t* vperm, bool has_vperm, void* scratch, cudaStream_t s);
-// The same renumbering for every tree of a multi-tree build, in a fixed
-// number of launches: each job's face_out, tri_rw, pos_out (the positions,
-// read and rewritten) and vperm_out (from vperm, or the identity when nullptr).
-size_t reorder_multi_scratch_bytes(uint32_t n_verts, uint32_t v_blocks, uint32_t f_blocks);
-cudaError_t launch_reorder_vertices_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks,
-                                          uint32_t f_blocks, const uint32_t* vjob, const uint32_t* fjob,
-                                          uint32_t n_verts, void* scratch, cudaStream_t s);
-cudaError_t launch_mesh_bounds(const float4* pos, uint32_t nV, uint32_t* bound_keys, int num_sms, cudaStream_t s);
-// codes_hi != nullptr: 63-bit keys, low 32 bits in codes and high 31 in codes_hi
-cudaError_t launch_leaf_morton(const uint32_t* tri, const float4* pos, uint32_t nT, const uint32_t* bound_keys,
-                               uint32_t* codes, uint32_t* idx, uint32_t* codes_hi, cudaStream_t s);
-cudaError_t launch_radix_sort(uint32_t* keys, uint32_t* vals, uint32_t n, int key_bits, void* scratch,
-                              cudaStream_t s);
-// out[i] = src[idx[i]]
-cudaError_t launch_gather_u32(const uint32_t* src, const uint32_t* idx, uint32_t n, uint32_t* out, cudaStream_t s);
-cudaError_t launch_gather_faces(const uint32_t* tri, const uint32_t* perm, uint32_t nT, uint4* out, cudaStream_t s);
-
 // refit_kernels.cu
 // refit CTAs of a tree of nT leaves with level groups of group_log2 levels
 // (9, 10 or 11; 0 = 10, the single-tree refit's)
