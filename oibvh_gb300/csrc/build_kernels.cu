@@ -12,6 +12,9 @@
 // 63 bits (21 per axis) as an option, sorted as two stable 32-bit passes.
 #include "oibvh_common.cuh"
 #include "oibvh_launch.h"
+#include "refit_device.cuh"
+
+#include <atomic>
 
 namespace oibvh {
 
@@ -668,6 +671,237 @@ cudaError_t launch_build(const BuildArgs& a, cudaStream_t s)
     k_build_count<<<a.f_tiles + a.v_tiles, 128, 0, s>>>(a);
     k_build_place<<<4 * a.v_tiles, 256, 0, s>>>(a);
     k_build_apply<<<4 * (a.f_tiles + a.v_tiles), 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// The whole build of one small tree in one CTA: positions, keys, sort and
+// renumbering in shared memory, then every node of the tree. A build of a few
+// thousand faces is a chain of a dozen launches otherwise, each a few
+// microseconds of latency for less work than one SM has threads for (1,280
+// faces: 83 us, against 32 here; up to 4,096 faces and vertices, what the
+// shared memory holds).
+// ---------------------------------------------------------------------------
+constexpr uint32_t kSmallMax = 4096, kSmallThreads = 1024;
+struct SmallShared {
+    float4 pos[kSmallMax];
+    uint32_t first[kSmallMax], lo[kSmallMax], hi[kSmallMax];
+    uint16_t idx[2][kSmallMax], inv[kSmallMax];
+    uint16_t cnt[kSmallThreads / 32][256];
+    uint32_t base[256], w[32], red[6][32];
+    Box boxes[32];
+};
+
+// Exclusive scan of one value per thread over the CTA of 1024; `sum` = the total.
+__device__ __forceinline__ uint32_t scan_1024(uint32_t v, uint32_t* sh /*[32]*/, uint32_t& sum)
+{
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, s);
+        if ((int)lane >= s) x += y;
+    }
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    const uint32_t t = sh[lane];
+    const uint32_t pre = __reduce_add_sync(0xffffffffu, lane < w ? t : 0u);
+    sum = __reduce_add_sync(0xffffffffu, t);
+    __syncthreads();
+    return pre + x - v;
+}
+
+template <bool kWide>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_build_small(const BuildJob job, const TreeShape S, float4* box)
+{
+    extern __shared__ uint4 s_mem[];
+    SmallShared& sh = *(SmallShared*)s_mem;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t nT = job.nT, nV = job.nV;
+    // positions and bounds
+    uint32_t red[6] = {0, 0, 0, 0, 0, 0}, from[kSmallMax / kSmallThreads];
+#pragma unroll
+    for (uint32_t k = 0; k < kSmallMax / kSmallThreads; ++k) {
+        const uint32_t v = k * kSmallThreads + tid;
+        if (v >= nV) break;
+        const float4 p = job.pos[v];
+        from[k] = job.vperm ? job.vperm[v] : v;
+        sh.pos[v] = p;
+        sh.first[v] = kNoUse;
+        const float c[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t o = float_to_ordered(c[i]);
+            red[i] = max(red[i], ~o);
+            red[3 + i] = max(red[3 + i], o);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        red[i] = __reduce_max_sync(0xffffffffu, red[i]);
+        if (lane == 0) sh.red[i][w] = red[i];
+    }
+    __syncthreads();
+    float bmin[3], bmax[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        bmin[k] = ordered_to_float(~__reduce_max_sync(0xffffffffu, sh.red[k][lane]));
+        bmax[k] = ordered_to_float(__reduce_max_sync(0xffffffffu, sh.red[3 + k][lane]));
+    }
+    // keys
+    for (uint32_t i = tid; i < nT; i += kSmallThreads) {
+        const uint32_t* t = job.tri + 3 * (size_t)i;
+        const float4 p0 = sh.pos[t[0]], p1 = sh.pos[t[1]], p2 = sh.pos[t[2]];
+        const float va[3] = {p0.x, p0.y, p0.z}, vb[3] = {p1.x, p1.y, p1.z}, vc[3] = {p2.x, p2.y, p2.z};
+        uint32_t lo, hi;
+        leaf_code(va, vb, vc, bmin, bmax, kWide, lo, hi);
+        sh.lo[i] = lo;
+        if (kWide) sh.hi[i] = hi;
+        sh.idx[0][i] = (uint16_t)i;
+    }
+    // stable LSD radix sort of the item numbers, 8 bits a pass; warp w ranks the items from w * 32 * rounds on
+    const uint32_t rounds = (nT + kSmallThreads - 1) / kSmallThreads, lt = (1u << lane) - 1u;
+    for (uint32_t p = 0; p < (kWide ? 8u : 4u); ++p) {
+        const uint32_t* key = p < 4 ? sh.lo : sh.hi;
+        const uint32_t shift = 8 * (p & 3u);
+        for (uint32_t i = tid; i < 32 * 128; i += kSmallThreads) ((uint32_t*)sh.cnt)[i] = 0;
+        __syncthreads();
+        uint32_t item[4], rank[4], dig[4];
+#pragma unroll
+        for (uint32_t r = 0; r < 4; ++r) {
+            if (r >= rounds) break;
+            const uint32_t i = (w * rounds + r) * 32 + lane;
+            const bool valid = i < nT;
+            item[r] = valid ? sh.idx[p & 1][i] : 0u;
+            const uint32_t d = valid ? (key[item[r]] >> shift) & 255u : 0u;
+            uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+            for (uint32_t b = 0; b < 8; ++b) {
+                const uint32_t set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+                peers &= (d >> b) & 1u ? set : ~set;
+            }
+            const uint32_t before = valid ? sh.cnt[w][d] : 0u;
+            rank[r] = before + __popc(peers & lt);
+            dig[r] = valid ? d : 256u;
+            __syncwarp();
+            if (valid && (peers & lt) == 0) sh.cnt[w][d] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        // four threads a digit, eight warps each: counts to exclusive sums over the warps, then over the digits
+        const uint32_t d = tid >> 2, w0 = 8 * (tid & 3u);
+        uint32_t c[8], sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            c[k] = sh.cnt[w0 + k][d];
+            sum += c[k];
+        }
+        uint32_t x = sum;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, s);
+            if ((int)lane >= s) x += y;
+        }
+        if (lane == 31) sh.w[w] = x;
+        const uint32_t group = __shfl_sync(0xffffffffu, x - sum, lane & ~3u);  // the digit's start within the warp
+        uint32_t run = x - sum - group;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            sh.cnt[w0 + k][d] = (uint16_t)run;
+            run += c[k];
+        }
+        __syncthreads();
+        const uint32_t pre = __reduce_add_sync(0xffffffffu, lane < w ? sh.w[lane] : 0u);
+        if ((tid & 3u) == 0) sh.base[d] = pre + group;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t r = 0; r < 4; ++r)
+            if (r < rounds && dig[r] < 256u)
+                sh.idx[(p + 1) & 1][sh.base[dig[r]] + sh.cnt[w][dig[r]] + rank[r]] = (uint16_t)item[r];
+        __syncthreads();
+    }
+    // first uses; four consecutive sorted faces a thread
+    uint32_t f[4][4], m[4], cnt = 0, used, unused;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t i = 4 * tid + k;
+        if (i >= nT) continue;
+        f[k][3] = sh.idx[0][i];  // an even number of passes
+#pragma unroll
+        for (uint32_t c = 0; c < 3; ++c) {
+            f[k][c] = job.tri[3 * (size_t)f[k][3] + c];
+            atomicMin(&sh.first[f[k][c]], 3 * i + c);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t i = 4 * tid + k;
+        m[k] = 0;
+        if (i < nT)
+#pragma unroll
+            for (uint32_t c = 0; c < 3; ++c) m[k] |= sh.first[f[k][c]] == 3 * i + c ? 1u << c : 0u;
+        cnt += __popc(m[k]);
+    }
+    uint32_t nv = scan_1024(cnt, sh.w, used);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+#pragma unroll
+        for (uint32_t c = 0; c < 3; ++c)
+            if ((m[k] >> c) & 1u) sh.inv[f[k][c]] = (uint16_t)nv++;
+    cnt = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) cnt += 4 * tid + k < nV && sh.first[4 * tid + k] == kNoUse ? 1u : 0u;
+    nv = scan_1024(cnt, sh.w, unused) + used;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+        if (4 * tid + k < nV && sh.first[4 * tid + k] == kNoUse) sh.inv[4 * tid + k] = (uint16_t)nv++;
+    __syncthreads();  // (also: every thread has read its part of the map before it is rewritten)
+#pragma unroll
+    for (uint32_t k = 0; k < kSmallMax / kSmallThreads; ++k) {
+        const uint32_t v = k * kSmallThreads + tid;
+        if (v >= nV) break;
+        job.pos_out[sh.inv[v]] = sh.pos[v];
+        job.vperm_out[sh.inv[v]] = from[k];
+    }
+    // faces, and the leaves' boxes
+    Box b[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        b[k] = Box{0, 0, 0, 0, 0, 0};
+        const uint32_t i = 4 * tid + k;
+        if (i >= nT) continue;
+        const uint4 r = make_uint4(sh.inv[f[k][0]], sh.inv[f[k][1]], sh.inv[f[k][2]], f[k][3]);
+        job.face_out[i] = r;
+        uint32_t* t = job.tri_rw + 3 * (size_t)r.w;
+        t[0] = r.x;
+        t[1] = r.y;
+        t[2] = r.z;
+        const float4 p0 = sh.pos[f[k][0]], p1 = sh.pos[f[k][1]], p2 = sh.pos[f[k][2]];
+        b[k] = Box{gmin(gmin(p0.x, p1.x), p2.x), gmin(gmin(p0.y, p1.y), p2.y), gmin(gmin(p0.z, p1.z), p2.z),
+                   gmax(gmax(p0.x, p1.x), p2.x), gmax(gmax(p0.y, p1.y), p2.y), gmax(gmax(p0.z, p1.z), p2.z)};
+    }
+    if (S.L > 0) reduce_block<12>(b, S, box, S.L, 0, S.L, sh.boxes);
+}
+
+bool build_is_small(uint32_t nT, uint32_t nV) { return nT <= kSmallMax && nV <= kSmallMax; }
+
+cudaError_t launch_build_small(const BuildJob& job, const TreeShape& shape, float4* box, bool wide, cudaStream_t s)
+{
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+        e = cudaFuncSetAttribute(k_build_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_build_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared));
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+    }
+    note_launches(1);
+    if (wide) k_build_small<true><<<1, kSmallThreads, sizeof(SmallShared), s>>>(job, shape, box);
+    else k_build_small<false><<<1, kSmallThreads, sizeof(SmallShared), s>>>(job, shape, box);
     return cudaGetLastError();
 }
 

@@ -142,6 +142,13 @@ static int tree_build_impl(oibvh_tree_t t, cudaStream_t s)
     DeviceGuard g(t->device);
     OK_TRY(t->vperm.ensure(t->nV, "cudaMalloc(vertex order)"));
     OK_TRY(sync_positions(t, s));
+    if (build_is_small(t->nT, t->nV)) {
+        CUDA_TRY(launch_build_small(t->build_job(), t->shape, t->box.p, t->morton_bits == 63, s));
+        CUDA_TRY(cudaStreamSynchronize(s));
+        t->reordered = true;
+        t->built = true;
+        return OIBVH_OK;
+    }
     BuildArgs a{};
     a.one = t->build_job();
     a.f_tiles = (t->nT + kBuildTile - 1) / kBuildTile;

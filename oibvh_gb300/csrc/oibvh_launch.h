@@ -74,6 +74,10 @@ size_t build_scratch(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t n
 // records, `tri` and positions get the new vertex numbers, vperm_out the new
 // caller-order map.
 cudaError_t launch_build(const BuildArgs& a, cudaStream_t s);
+// The whole build of one tree, boxes included, in one launch, for trees that
+// build_is_small() (up to 4,096 faces and vertices).
+bool build_is_small(uint32_t nT, uint32_t nV);
+cudaError_t launch_build_small(const BuildJob& job, const TreeShape& shape, float4* box, bool wide, cudaStream_t s);
 // rest: packed positions of all jobs in each caller's vertex order (read
 // through the jobs' vperm), or in each tree's order (rest_tree_order), or
 // nullptr (each job's own pos). Writes each job's pos_out.
