@@ -30,6 +30,7 @@
 #include "oibvh_launch.h"
 
 #include <algorithm>
+#include <atomic>
 
 namespace oibvh {
 
@@ -640,11 +641,17 @@ __global__ void __launch_bounds__(256) k_begin(DetectArgs a, uint32_t hits_befor
     for (uint32_t i = threadIdx.x; i < kCountTotal; i += blockDim.x) a.counts[i] = i == kCountHits ? hits_before : 0u;
 }
 
-// Counters to pinned host memory, at the end of a frame.
-__global__ void k_publish(const uint32_t* __restrict__ counts, uint32_t* __restrict__ host)
+// The counters and, when there are at most host_hit_cap, the hits to pinned
+// host memory (one CTA): a result that a program reads at once is then there
+// without a copy of its own (about 18 us a call, for a few hundred records).
+__device__ __forceinline__ void publish(const DetectArgs& a)
 {
-    if (threadIdx.x < kCountHost) host[threadIdx.x] = counts[threadIdx.x];
+    for (uint32_t i = threadIdx.x; i < kCountHost; i += blockDim.x) a.host[i] = __ldcg(a.counts + i);
+    const uint32_t n = __ldcg(a.counts + kCountHits);
+    if (n > a.host_hit_cap || n > a.hit_cap) return;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) a.host_hits[i] = __ldcg(a.hits + i);
 }
+__global__ void __launch_bounds__(256) k_publish(DetectArgs a) { publish(a); }
 
 // The grid's barrier after round r (every CTA is resident: a cooperative
 // launch). The CTA that arrives last has the list's final size from the word
@@ -653,16 +660,18 @@ __global__ void k_publish(const uint32_t* __restrict__ counts, uint32_t* __restr
 // next round's items, 0 to stop (also when the list has overflowed). A CTA
 // that has polled for several seconds raises kFlagTimeout and stops.
 constexpr uint32_t kBarrierPolls = 1u << 24;
-__device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t r, uint32_t* s_next)
+__device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t r, uint32_t* s_next, uint32_t* s_last)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
+        *s_last = 0;
         uint32_t* ctl = a.counts;
         uint64_t* release = (uint64_t*)(ctl + kCtlRelease);  // (rounds finished, items of the next)
         __threadfence();
         const uint64_t w = atomicAdd((unsigned long long*)round_slot(ctl, r + 1), 1ull << 32);
         uint32_t next = (uint32_t)w;
         if ((uint32_t)(w >> 32) == gridDim.x - 1u) {
+            *s_last = 1;
             if (next > a.work_cap) next = 0;
             st_release(release, (uint64_t)(r + 1u) << 32 | next);
             ctl[kCountPeak] = max(ctl[kCountPeak], (uint32_t)w);
@@ -746,7 +755,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
 {
     extern __shared__ uint64_t s_ring[];  // [warp][walk_ring(cap)]
     __shared__ uint64_t s_cand[kWarps][kCandBuf];
-    __shared__ uint32_t s_next, s_found, s_tested;
+    __shared__ uint32_t s_next, s_last, s_found, s_tested;
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_found = s_tested = 0;
     __syncthreads();
@@ -879,8 +888,14 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             s_tested = s_found = 0;
         }
         if (r == last) break;
-        n_src = round_barrier(a, r, &s_next);
+        n_src = round_barrier(a, r, &s_next, &s_last);
         if (n_src == 0) break;
+    }
+    // the CTA that was last to finish hands over the results, and clears the
+    // other counter block for the next traversal (nobody uses it now)
+    if (a.host && s_last) {
+        publish(a);
+        for (uint32_t i = threadIdx.x; i < kCountTotal; i += blockDim.x) a.counts_next[i] = 0;
     }
 }
 
@@ -1611,10 +1626,10 @@ cudaError_t launch_begin(const DetectArgs& a, uint32_t hits_before, cudaStream_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_publish(const DetectArgs& a, uint32_t* host, cudaStream_t s)
+cudaError_t launch_publish(const DetectArgs& a, cudaStream_t s)
 {
     note_launches(1);
-    k_publish<<<1, 32, 0, s>>>(a.counts, host);
+    k_publish<<<1, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -1663,14 +1678,19 @@ cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, ui
 
 int walk_blocks_per_sm(uint32_t walk_cap, bool fused)
 {
-    if (walk_configure() != cudaSuccess) return 1;
+    static std::atomic<int> known[64][2][kWalkCapMax / 32 + 1];
+    int dev = 0;
+    if (walk_cap > kWalkCapMax || cudaGetDevice(&dev) != cudaSuccess || walk_configure() != cudaSuccess) return 1;
+    std::atomic<int>* cached = dev >= 0 && dev < 64 ? &known[dev][fused][walk_cap / 32] : nullptr;
+    if (cached && cached->load(std::memory_order_relaxed)) return cached->load(std::memory_order_relaxed);
     int n = 0, m = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_kernel(fused, false), kDetectThreads, walk_smem(walk_cap));
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, walk_kernel(fused, true), kDetectThreads, walk_smem(walk_cap));
     n = std::min(n, m);
-    if (e != cudaSuccess) return 1;
-    return n > 0 ? n : 1;
+    if (e != cudaSuccess || n < 1) return 1;
+    if (cached) cached->store(n, std::memory_order_relaxed);
+    return n;
 }
 
 uint32_t narrow_kernels(const DetectArgs& a) { return a.precision ? (a.fp64_tri_cap ? 5u : 4u) : 1u; }

@@ -179,8 +179,13 @@ struct oibvh_scene_s {
     DevBuf<uint32_t> prec_lists;  // precision narrow phase: float-hit, recheck and FP64 lists (4 x cand_cap)
     DevBuf<double> fp64_tri;      // precision narrow phase: FP64 setups (kFp64TriRows x fp64_tri_cap)
     uint32_t fp64_tri_cap = 0;
+    DevBuf<uint32_t> walk_counts;  // two counter blocks, in turn between direct detects: each clears the other one
+    uint32_t walk_turn = 0;
+    bool walk_clean = false;       // the block of this turn is zero
     PinnedBuf<PairView> h_pairs;
     PinnedBuf<uint32_t> h_counts;
+    PinnedBuf<uint4> h_hits;       // the last detect's hits, when there are at most kHostHits
+    bool h_hits_valid = false;
 
     uint32_t front_cap = 1u << 20;
     uint32_t cand_cap = 1u << 20;
@@ -238,6 +243,9 @@ struct oibvh_scene_s {
 };
 
 namespace {
+
+// Hits that come to the host with the counters (64 KB).
+constexpr uint32_t kHostHits = 4096;
 
 struct PassPlan {
     std::vector<PairView> pv;
@@ -339,7 +347,7 @@ int ensure_lists(oibvh_scene_s* s)
 {
     OK_TRY(s->work0.ensure(s->front_cap, "cudaMalloc(work list)"));
     OK_TRY(s->work1.ensure(s->front_cap, "cudaMalloc(work list)"));
-    OK_TRY(s->counts.ensure(kCountTotal, "cudaMalloc(counts)"));
+    OK_TRY(s->counts.ensure(2 * kCountTotal, "cudaMalloc(counts)"));
     return OIBVH_OK;
 }
 
@@ -373,6 +381,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
     s->hit_count = 0;
     s->cand_count = 0;
     s->cands_valid = false;
+    s->h_hits_valid = false;
     std::vector<uint32_t> pr;
     list_pairs(s, pr);
     const uint32_t n_pairs = (uint32_t)(pr.size() / 2);
@@ -388,6 +397,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         PassPlan plan;
         OK_TRY(plan_pass(s, pr.data() + 2 * (size_t)p0, np, entry, plan));
         OK_TRY(s->h_counts.ensure(kCountHost, "cudaMallocHost(counts)"));
+        OK_TRY(s->h_hits.ensure(kHostHits, "cudaMallocHost(hits)"));
         OK_TRY(s->h_pairs.ensure(np, "cudaMallocHost(pairs)"));
         OK_TRY(s->pairv.ensure(np, "cudaMalloc(pairs)"));
         if (np > 1 || !narrow) {  // one pair goes with the walk's arguments; the narrow-phase kernels read the table
@@ -419,11 +429,30 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.claim_min = s->tune_claim;
             a.descend_ratio = (float)s->tune_descend;
             const uint32_t front0 = (uint32_t)plan.front0;
-            CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
-            CUDA_TRY(launch_walk(a, front0, 0, kAllRounds, st));
-            CUDA_TRY(cudaMemcpyAsync(s->h_counts.p, s->counts.p, kCountHost * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                     st));
-            CUDA_TRY(cudaStreamSynchronize(st));
+            s->h_counts.p[kCountFlags] = kFlagTimeout;  // overwritten when the walk hands over its counters
+            a.host = s->h_counts.p;
+            a.host_hits = s->h_hits.p;
+            a.host_hit_cap = narrow ? kHostHits : 0u;
+            if (narrow && hits_before == 0) {
+                // one launch: the counter block was cleared by the detect before
+                if (!s->walk_counts.p) {
+                    OK_TRY(s->walk_counts.ensure(2 * kCountTotal, "cudaMalloc(counts)"));
+                    s->walk_clean = false;
+                }
+                a.counts = s->walk_counts.p + s->walk_turn * kCountTotal;
+                a.counts_next = s->walk_counts.p + (s->walk_turn ^ 1u) * kCountTotal;
+                if (!s->walk_clean) CUDA_TRY(launch_begin(a, 0, st));
+                s->walk_clean = false;
+                CUDA_TRY(launch_walk(a, front0, 0, kAllRounds, st));
+                CUDA_TRY(cudaStreamSynchronize(st));
+                s->walk_clean = !(s->h_counts.p[kCountFlags] & kFlagTimeout);
+                if (s->walk_clean) s->walk_turn ^= 1u;
+            } else {
+                a.counts_next = a.counts + kCountTotal;  // (cleared to no purpose)
+                CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
+                CUDA_TRY(launch_walk(a, front0, 0, kAllRounds, st));
+                CUDA_TRY(cudaStreamSynchronize(st));
+            }
             const uint32_t* c = s->h_counts.p;
             const uint32_t flags = c[kCountFlags], rounds = c[kCountRounds];
             const uint64_t peak = c[kCountPeak];
@@ -446,7 +475,10 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             s->stats.front_peak = std::max(s->stats.front_peak, peak);
             s->stats.steps = rounds;
             s->cand_count += c[kCountCands];
-            if (narrow) s->hit_count = c[kCountHits];
+            if (narrow) {
+                s->hit_count = c[kCountHits];
+                s->h_hits_valid = s->hit_count <= kHostHits && hits_before == 0;
+            }
             break;
         }
         s->stats.passes++;
@@ -522,6 +554,7 @@ int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_
             continue;
         }
         s->hit_count = c[kCountHits];
+        s->h_hits_valid = false;
         s->stats.hits = s->hit_count;
         s->stats.fp64_axes += c[kCountFp64Axes];
         s->stats.fp64_candidates += c[kCountFp64Cands];
@@ -948,6 +981,10 @@ API int oibvh_scene_get_int_tri_pairs(oibvh_scene_t s, uint32_t* out4, uint64_t 
     const uint64_t k = std::min(cap, s->hit_count);
     if (k == 0) return OIBVH_OK;
     if (!out4) return fail(OIBVH_ERR_ARG, "out4 is NULL");
+    if (s->h_hits_valid) {  // they came with the counters
+        std::memcpy(out4, s->h_hits.p, k * sizeof(uint4));
+        return OIBVH_OK;
+    }
     DeviceGuard g(s->device);
     CUDA_TRY(cudaMemcpy(out4, s->hits.p, k * sizeof(uint4), cudaMemcpyDeviceToHost));
     return OIBVH_OK;
@@ -997,6 +1034,7 @@ API int oibvh_scene_set_queue_capacity(oibvh_scene_t s, uint32_t front, uint32_t
         s->hit_cap = hits;
         s->hits.release();
         s->hit_count = 0;
+        s->h_hits_valid = false;
     }
     s->frame_stale = true;  // a captured frame points at the released buffers
     return OIBVH_OK;
@@ -1409,7 +1447,13 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
         k += narrow_kernels(n);
     }
     mark(5);
-    if (e == cudaSuccess) e = launch_publish(a, s->h_frame_counts.p, st);
+    if (e == cudaSuccess) {
+        DetectArgs p = a;
+        p.host = s->h_frame_counts.p;
+        p.host_hits = s->h_hits.p;
+        p.host_hit_cap = kHostHits;
+        e = launch_publish(p, st);
+    }
     ++k;
     if (kernels) *kernels = k;
     return e;
@@ -1574,6 +1618,7 @@ API int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream)
     s->stats.bounded_candidates = (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck];
     s->stats.front_peak = c[kCountPeak];
     s->hit_count = c[kCountHits];
+    s->h_hits_valid = s->hit_count <= kHostHits;
     s->cand_count = c[kCountCands];
     s->stats.candidates = s->cand_count;
     s->stats.hits = s->hit_count;

@@ -113,6 +113,10 @@ struct DetectArgs {
     uint4* hits;
     uint32_t hit_cap;
     uint32_t* counts;      // see kCount* below
+    uint32_t* host;        // pinned: where the walk of all rounds (or launch_publish) puts the counters; nullptr: nowhere
+    uint4* host_hits;      // pinned: and the hits, when there are at most host_hit_cap
+    uint32_t host_hit_cap;
+    uint32_t* counts_next; // with host: the counter block that the walk clears for the next traversal
     uint32_t* prec_lists;  // precision mode, 4 x cand_cap words: float-hit list, recheck list (candidate
                            // indices), then the FP64 list ((candidate index, axis mask) pairs)
     double* fp64_tri;      // precision mode: the FP64 list's setups, kFp64TriRows rows of fp64_tri_cap
@@ -126,14 +130,14 @@ struct DetectArgs {
     uint32_t claim_min = 1;   // a round's pairs are claimed dynamically from this many per warp
     float descend_ratio = kDescendRatio;  // both sides descend while the boxes' squared diagonals are within it
 };
-// A traversal of `total0` start pairs: launch_begin (counters set, hits from
-// hits_before), then launch_walk of round 0 .. kAllRounds, or of rounds 0, 1,
+// A traversal of `total0` start pairs: counters cleared (launch_begin, which
+// sets the hits to hits_before, or the traversal before), then launch_walk of round 0 .. kAllRounds, or of rounds 0, 1,
 // .. one at a time and then r .. kAllRounds.
 cudaError_t launch_begin(const DetectArgs& a, uint32_t hits_before, cudaStream_t s);
 constexpr uint32_t kAllRounds = 0xffffffffu;  // until a round leaves nothing (a cooperative launch)
 cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, uint32_t last, cudaStream_t s);
-// the first kCountHost counters to pinned host memory
-cudaError_t launch_publish(const DetectArgs& a, uint32_t* host, cudaStream_t s);
+// the counters (and few hits) to the pinned host memory
+cudaError_t launch_publish(const DetectArgs& a, cudaStream_t s);
 // walker CTAs that fit on one SM with rings of `walk_cap` entries (0:
 // default), for the fused (narrow phase inside) or the broad-only walker
 int walk_blocks_per_sm(uint32_t walk_cap = 0, bool fused = true);
