@@ -838,8 +838,8 @@ def frame_rooflines(w, prof, cands, hits, tested, peaks, refit_alone_ms, refit_b
                   REFIT_DRAM_BYTES_PER_TRIANGLE * tri_total,
                   "12 B per vertex + 12 B per face read, 24 B per tree node written (the reference layout; this "
                   "layout stores internal nodes only, 32 B each, and reads 16 B per face and per vertex)"),
-        "traversal": ("k_begin + k_walk (broad phase, fused 17-axis narrow phase)",
-                      broad + 112 * cands + 8 * hits, prof["start_ms"] + prof["walk_ms"],
+        "traversal": ("k_begin + k_walk + k_narrow (broad phase, 17-axis narrow phase)",
+                      broad + 112 * cands + 8 * hits, prof["start_ms"] + prof["walk_ms"] + prof["narrow_ms"],
                       TRAVERSAL_DRAM_BYTES_PER_TESTED * tested if TRAVERSAL_DRAM_BYTES_PER_TESTED else None,
                       "24 B per node of both trees of every pair + 112 B per candidate + 8 B per hit"),
     }
@@ -858,7 +858,7 @@ def frame_rooflines(w, prof, cands, hits, tested, peaks, refit_alone_ms, refit_b
     dominant = max(("transform", "refit", "traversal"), key=lambda k: out[k]["launch_ms"])
     top = dict(out[dominant])
     top.update({"stage": dominant, "peak_source": src, "stages": out,
-                "stages_ms_sum": round(sum(prof[k] for k in ("transform_ms", "refit_ms", "start_ms", "walk_ms")), 4),
+                "stages_ms_sum": round(sum(prof[k] for k in ("transform_ms", "refit_ms", "start_ms", "walk_ms", "narrow_ms")), 4),
                 "stages_cover_of_step": round(sum(out[k]["launch_ms"] for k in out) / ms_step, 4),
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per stage on 64 batched pairs "
                                   "(profiles/), scaled by the units the stage processes",

@@ -277,7 +277,7 @@ typedef struct oibvh_frame_profile {
     float refit_ms;        /* the one refit launch (0 without) */
     float start_ms;        /* counters cleared */
     float walk_ms;         /* the traversal: every walk launch */
-    float narrow_ms;       /* precision mode's narrow phase (0 in float mode) */
+    float narrow_ms;       /* the narrow phase where it is a launch of its own (precision mode, large frames; else 0) */
     uint32_t walk_rounds;  /* walk launches (the last one walks every round that is left) */
     uint32_t kernels;      /* kernels launched */
 } oibvh_frame_profile;

@@ -70,7 +70,10 @@ __device__ __forceinline__ bool project6(const V3& ax, const V3& p1, const V3& p
     return true;
 }
 // triangleIntersect (src/utils/utils.cpp:97-169); the 17 tests are a
-// conjunction, so evaluating the axes lazily does not change the result.
+// conjunction, so evaluating the axes lazily, or in two goes, does not change
+// the result. kPart: all axes, the two face normals, or the 15 others.
+enum SatPart { kSatAll = 0, kSatNormals = 1, kSatEdges = 2 };
+template <int kPart = kSatAll>
 __device__ __forceinline__ bool tri_intersect_exact(const V3& P1, const V3& P2, const V3& P3, const V3& Q1,
                                                     const V3& Q2, const V3& Q3)
 {
@@ -80,9 +83,10 @@ __device__ __forceinline__ bool tri_intersect_exact(const V3& P1, const V3& P2, 
     const V3 e1 = vsub(p2, p1), e2 = vsub(p3, p2), e3 = vsub(p1, p3);
     const V3 f1 = vsub(q2, q1), f2 = vsub(q3, q2), f3 = vsub(q1, q3);
     const V3 n1 = vcross(e1, e2);
-    if (!project6(n1, p1, p2, p3, q1, q2, q3)) return false;
+    if (kPart != kSatEdges && !project6(n1, p1, p2, p3, q1, q2, q3)) return false;
     const V3 m1 = vcross(f1, f2);
-    if (!project6(m1, p1, p2, p3, q1, q2, q3)) return false;
+    if (kPart != kSatEdges && !project6(m1, p1, p2, p3, q1, q2, q3)) return false;
+    if (kPart == kSatNormals) return true;
     if (!project6(vcross(e1, f1), p1, p2, p3, q1, q2, q3)) return false;
     if (!project6(vcross(e1, f2), p1, p2, p3, q1, q2, q3)) return false;
     if (!project6(vcross(e1, f3), p1, p2, p3, q1, q2, q3)) return false;
@@ -372,15 +376,24 @@ __host__ __device__ __forceinline__ uint32_t walk_ring(uint32_t cap)
     return cap <= 64u ? 128u : cap <= 128u ? 256u : 512u;
 }
 
+// Candidates are tested in two goes: the face normals first, which separate four
+// of five (batched meshes: 78 %), and what is left, 32 at a time again, against
+// the other 15 axes. In one go a warp ran all 17 axes nearly always, for the
+// one lane in nine that needs them: 900 instructions for 32 candidates, against
+// about 360 so.
+constexpr int kLateBuf = 64;  // <= 31 left over + up to 32 that pass the normals
 struct WarpCands {
     uint64_t* buf;       // kCandBuf entries
+    uint64_t* late;      // kLateBuf entries: past the normals
     uint32_t n;          // warp-uniform
+    uint32_t n_late = 0;
     uint32_t found = 0;  // candidates found by this warp (added to the counter once a round)
 };
 
-template <bool kOne>
-__device__ __forceinline__ void test_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count,
-                                                uint32_t lane)
+// `count` buffered candidates, one per lane: against kPart's axes. Hits go to
+// the hit list (not with kSatNormals alone); returns whether this lane's passed.
+template <bool kOne, int kPart>
+__device__ __forceinline__ bool test_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count, uint32_t lane)
 {
     bool hit = false;
     uint4 rec = make_uint4(0, 0, 0, 0);
@@ -391,18 +404,20 @@ __device__ __forceinline__ void test_candidates(const DetectArgs& a, const uint6
         pair_refs<kOne>(a, bvtt_pair(c), TA, TB);
         const uint4 fa = __ldg(TA.face + bvtt_a(c));
         const uint4 fb = __ldg(TB.face + bvtt_b(c));
-        hit = tri_intersect_exact(load_vertex(TA.pos, fa.x), load_vertex(TA.pos, fa.y), load_vertex(TA.pos, fa.z),
-                                  load_vertex(TB.pos, fb.x), load_vertex(TB.pos, fb.y), load_vertex(TB.pos, fb.z));
-        rec = make_uint4(pv.a, pv.b, fa.w, fb.w);
+        hit = tri_intersect_exact<kPart>(load_vertex(TA.pos, fa.x), load_vertex(TA.pos, fa.y), load_vertex(TA.pos, fa.z),
+                                         load_vertex(TB.pos, fb.x), load_vertex(TB.pos, fb.y), load_vertex(TB.pos, fb.z));
+        if (kPart != kSatNormals) rec = make_uint4(pv.a, pv.b, fa.w, fb.w);
     }
-    const uint32_t pos = warp_append(a.counts + kCountHits, hit, lane);
-    if (hit) {
-        if (pos < a.hit_cap) a.hits[pos] = rec;
-        else atomicOr(a.counts + kCountFlags, (uint32_t)kFlagHitOverflow);
+    if (kPart != kSatNormals) {
+        const uint32_t pos = warp_append(a.counts + kCountHits, hit, lane);
+        if (hit) {
+            if (pos < a.hit_cap) a.hits[pos] = rec;
+            else atomicOr(a.counts + kCountFlags, (uint32_t)kFlagHitOverflow);
+        }
     }
+    return hit;
 }
 
-// Queue (or, in broad-only mode, store) one candidate per lane where `pred`.
 // Broad phase only: `count` buffered candidates (one per lane) to the global
 // candidate queue with one atomic for the warp.
 __device__ __forceinline__ void store_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count,
@@ -417,16 +432,39 @@ __device__ __forceinline__ void store_candidates(const DetectArgs& a, const uint
     }
 }
 
-// The warp's buffered candidates: tested (fused narrow phase) or stored.
-// kFused: the narrow phase is compiled into the traversal kernel (tested
-// here); otherwise the candidates are stored, and the kernel carries no
-// triangle-test code (fewer registers, more warps per SM).
+// 32 buffered candidates: tested (kFused: the narrow phase is compiled into the
+// traversal) or stored (the kernel carries no triangle-test code).
 template <bool kFused, bool kOne>
-__device__ __forceinline__ void flush_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count,
-                                                 uint32_t lane)
+__device__ __forceinline__ void take_candidates(const DetectArgs& a, WarpCands& wc, const uint64_t* buf, uint32_t lane)
 {
-    if constexpr (kFused) test_candidates<kOne>(a, buf, count, lane);
-    else store_candidates(a, buf, count, lane);
+    if constexpr (kFused) {
+        const bool pass = test_candidates<kOne, kSatNormals>(a, buf, 32, lane);
+        const uint32_t m = __ballot_sync(0xffffffffu, pass);
+        if (pass) wc.late[wc.n_late + __popc(m & ((1u << lane) - 1u))] = buf[lane];
+        wc.n_late += __popc(m);
+        __syncwarp();
+        if (wc.n_late >= 32) {
+            test_candidates<kOne, kSatEdges>(a, wc.late + wc.n_late - 32, 32, lane);
+            wc.n_late -= 32;
+            __syncwarp();
+        }
+    } else {
+        store_candidates(a, buf, 32, lane);
+    }
+}
+
+// What is left in the buffers (fewer than 32 each).
+template <bool kFused, bool kOne>
+__device__ __forceinline__ void flush_candidates(const DetectArgs& a, WarpCands& wc, uint32_t lane)
+{
+    if (wc.n > 0) {
+        if constexpr (kFused) test_candidates<kOne, kSatAll>(a, wc.buf, wc.n, lane);
+        else store_candidates(a, wc.buf, wc.n, lane);
+    }
+    if constexpr (kFused)
+        if (wc.n_late > 0) test_candidates<kOne, kSatEdges>(a, wc.late, wc.n_late, lane);
+    wc.n = wc.n_late = 0;
+    __syncwarp();
 }
 
 // Queue one candidate per lane where `pred` in the warp's buffer (at most 4
@@ -448,7 +486,7 @@ template <bool kFused, bool kOne>
 __device__ __forceinline__ void drain_candidates(const DetectArgs& a, WarpCands& wc, uint32_t lane)
 {
     while (wc.n >= 32) {
-        flush_candidates<kFused, kOne>(a, wc.buf + wc.n - 32, 32, lane);
+        take_candidates<kFused, kOne>(a, wc, wc.buf + wc.n - 32, lane);
         wc.n -= 32;
         __syncwarp();
     }
@@ -657,10 +695,13 @@ __global__ void __launch_bounds__(256) k_publish(DetectArgs a) { publish(a); }
 // launch). The CTA that arrives last has the list's final size from the word
 // it arrives at, and releases the others with it: one atomic and one poll
 // between a CTA's last append and the next round's first load. Returns the
-// next round's items, 0 to stop (also when the list has overflowed). A CTA
+// next round's items, kStop to stop: after a round that may be the last and
+// left nothing, or when the list has overflowed. A CTA
 // that has polled for several seconds raises kFlagTimeout and stops.
 constexpr uint32_t kBarrierPolls = 1u << 24;
-__device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t r, uint32_t* s_next, uint32_t* s_last)
+constexpr uint32_t kStop = 0xffffffffu;
+__device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t r, bool may_stop, uint32_t* s_next,
+                                                  uint32_t* s_last)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -671,8 +712,10 @@ __device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t 
         const uint64_t w = atomicAdd((unsigned long long*)round_slot(ctl, r + 1), 1ull << 32);
         uint32_t next = (uint32_t)w;
         if ((uint32_t)(w >> 32) == gridDim.x - 1u) {
-            *s_last = 1;
-            if (next > a.work_cap) next = 0;
+            if (next > a.work_cap || (next == 0 && may_stop)) {
+                next = kStop;
+                *s_last = 1;
+            }
             st_release(release, (uint64_t)(r + 1u) << 32 | next);
             ctl[kCountPeak] = max(ctl[kCountPeak], (uint32_t)w);
             ctl[kCountRounds] = r + 1u;
@@ -683,7 +726,7 @@ __device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t 
             next = (uint32_t)v;
             if ((uint32_t)(v >> 32) <= r) {
                 atomicOr(ctl + kCountFlags, (uint32_t)kFlagTimeout);
-                next = 0;
+                next = kStop;
             }
         }
         *s_next = next;
@@ -754,12 +797,12 @@ template <bool kFused, bool kOne>
 __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32_t total0, uint32_t first, uint32_t last)
 {
     extern __shared__ uint64_t s_ring[];  // [warp][walk_ring(cap)]
-    __shared__ uint64_t s_cand[kWarps][kCandBuf];
+    __shared__ uint64_t s_cand[kWarps][kCandBuf], s_late[kFused ? kWarps : 1][kLateBuf];
     __shared__ uint32_t s_next, s_last, s_found, s_tested;
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_found = s_tested = 0;
     __syncthreads();
-    WarpCands wc{s_cand[wib], 0};
+    WarpCands wc{s_cand[wib], s_late[kFused ? wib : 0], 0};
     const uint32_t R = walk_ring(a.walk_cap), mask = R - 1u;
     uint64_t* ring = s_ring + (size_t)wib * R;
     const uint32_t W = gridDim.x * kWarps;
@@ -872,9 +915,10 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             // queued, where little else is live
             drain_candidates<kFused, kOne>(a, wc, lane);
         }
-        // the warp's last candidates and the CTA's totals, before the wait for the slowest warp
-        if (wc.n > 0) flush_candidates<kFused, kOne>(a, wc.buf, wc.n, lane);
-        wc.n = 0;
+        // before the wait for the slowest warp: the warp's last candidates (but for rounds that
+        // claim: a partial buffer costs as much as a full one, so those keep theirs, and
+        // another round follows even if nothing is left), and the CTA's totals
+        if (!claiming || r == last) flush_candidates<kFused, kOne>(a, wc, lane);
         if (lane == 0 && (tested | wc.found)) {
             atomicAdd(&s_tested, tested);
             atomicAdd(&s_found, wc.found);
@@ -888,8 +932,8 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             s_tested = s_found = 0;
         }
         if (r == last) break;
-        n_src = round_barrier(a, r, &s_next, &s_last);
-        if (n_src == 0) break;
+        n_src = round_barrier(a, r, !claiming, &s_next, &s_last);
+        if (n_src == kStop) break;
     }
     // the CTA that was last to finish hands over the results, and clears the
     // other counter block for the next traversal (nobody uses it now)
@@ -903,14 +947,17 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
 // triangle_intersect_kernel (src/cuda/collide.cu:248-299).
 __global__ void __launch_bounds__(kDetectThreads) k_narrow(DetectArgs a)
 {
+    __shared__ uint64_t s_late[kWarps][kLateBuf];
     const uint32_t n = min(a.counts[kCountCandSlots], a.cand_cap);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+    WarpCands wc{nullptr, s_late[threadIdx.x >> 5], 0};
     for (uint32_t base = warp * 32; base < n; base += n_warps * 32) {
-        const uint32_t cnt = min(32u, n - base);
-        test_candidates<false>(a, a.cand + base, cnt, lane);
+        if (n - base >= 32) take_candidates<true, false>(a, wc, a.cand + base, lane);
+        else test_candidates<false, kSatAll>(a, a.cand + base, n - base, lane);
     }
+    flush_candidates<true, false>(a, wc, lane);
 }
 
 // Precision mode's narrow phase over stored candidates: one candidate's

@@ -244,6 +244,7 @@ struct oibvh_scene_s {
 
 namespace {
 
+constexpr uint64_t kSplitTriangles = 1ull << 20;  // split_narrow
 // Hits that come to the host with the counters (64 KB).
 constexpr uint32_t kHostHits = 4096;
 
@@ -335,6 +336,26 @@ int walk_grid(const oibvh_scene_s* s, bool fused = true)
 
 int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_t st);
 
+// Whether a pass's float narrow phase runs as a kernel of its own after the
+// walk instead of inside it: for several pairs of a million triangles in all.
+// The walk then carries no triangle test, and the tests run with every lane
+// busy: a frame of 512 pairs 3.13 to 3.06 ms, of 64 pairs 461 to 446 us, of 4
+// pairs 101 to 96 us. Below that, and for one pair, the launch costs what it
+// gives. Without room for the candidates the walk tests them itself.
+bool split_narrow(const oibvh_scene_s* s, const PassPlan& plan)
+{
+    if (plan.pv.size() == 1) return false;
+    std::vector<bool> seen(s->trees.size(), false);
+    uint64_t triangles = 0;
+    for (const PairView& v : plan.pv)
+        for (uint32_t t : {v.a, v.b})
+            if (!seen[t]) {
+                seen[t] = true;
+                triangles += s->trees[t]->nT;
+            }
+    return triangles >= kSplitTriangles;
+}
+
 // How detect_impl runs the narrow phase: fused into the traversal (float
 // test), not at all (broad phase only, candidates kept), or as a separate
 // kernel over each pass's candidates (precision mode: the filtered test
@@ -365,15 +386,15 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
     DeviceGuard g(s->device);
     struct StaleIfMoved {
         oibvh_scene_s* s;
-        const void* p[5];
+        const void* p[6];
         explicit StaleIfMoved(oibvh_scene_s* sc)
-            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->pairv.p}
+            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->pairv.p, sc->cand.p}
         {
         }
         ~StaleIfMoved()
         {
-            const void* q[5] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->pairv.p};
-            for (int i = 0; i < 5; ++i)
+            const void* q[6] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->pairv.p, s->cand.p};
+            for (int i = 0; i < 6; ++i)
                 if (p[i] != q[i]) s->frame_stale = true;
         }
     } stale_guard(s);
@@ -391,7 +412,6 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
     if (n_pairs == 0) return OIBVH_OK;
     OK_TRY(s->hits.ensure(s->hit_cap, "cudaMalloc(hits)"));
 
-    const int grid = walk_grid(s, narrow);
     for (uint32_t p0 = 0; p0 < n_pairs; p0 += kMaxPairsPerPass) {
         const uint32_t np = std::min(kMaxPairsPerPass, n_pairs - p0);
         PassPlan plan;
@@ -406,10 +426,13 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
         }
         const uint64_t hits_before = s->hit_count;
+        bool split = narrow && split_narrow(s, plan);
         for (int attempt = 0;; ++attempt) {
             if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "BVTT queues kept overflowing after regrowing");
             OK_TRY(ensure_lists(s));
+            if (split && s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)") != OIBVH_OK) split = false;
             if (!narrow) OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
+            const bool fused = narrow && !split;
             DetectArgs a{};
             a.pairs = s->pairv.p;
             a.n_pairs = np;
@@ -417,13 +440,13 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.work[0] = s->work0.p;
             a.work[1] = s->work1.p;
             a.work_cap = s->front_cap;
-            a.cand = narrow ? nullptr : s->cand.p;
-            a.cand_cap = narrow ? 0 : s->cand_cap;
+            a.cand = fused ? nullptr : s->cand.p;
+            a.cand_cap = fused ? 0 : s->cand_cap;
             a.hits = s->hits.p;
             a.hit_cap = s->hit_cap;
             a.counts = s->counts.p;
-            a.fuse_narrow = narrow ? 1u : 0u;
-            a.grid = grid;
+            a.fuse_narrow = fused ? 1u : 0u;
+            a.grid = walk_grid(s, fused);
             a.walk_cap = s->tune_walk_cap;
             a.precision = s->precision;
             a.claim_min = s->tune_claim;
@@ -433,7 +456,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.host = s->h_counts.p;
             a.host_hits = s->h_hits.p;
             a.host_hit_cap = narrow ? kHostHits : 0u;
-            if (narrow && hits_before == 0) {
+            if (fused && hits_before == 0) {
                 // one launch: the counter block was cleared by the detect before
                 if (!s->walk_counts.p) {
                     OK_TRY(s->walk_counts.ensure(2 * kCountTotal, "cudaMalloc(counts)"));
@@ -447,6 +470,15 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
                 CUDA_TRY(cudaStreamSynchronize(st));
                 s->walk_clean = !(s->h_counts.p[kCountFlags] & kFlagTimeout);
                 if (s->walk_clean) s->walk_turn ^= 1u;
+            } else if (split) {
+                DetectArgs w = a, n = a;
+                w.host = nullptr;
+                n.grid = sm_count(s->device) * 8;
+                CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
+                CUDA_TRY(launch_walk(w, front0, 0, kAllRounds, st));
+                CUDA_TRY(launch_narrow(n, st));
+                CUDA_TRY(launch_publish(a, st));
+                CUDA_TRY(cudaStreamSynchronize(st));
             } else {
                 a.counts_next = a.counts + kCountTotal;  // (cleared to no purpose)
                 CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
@@ -1439,7 +1471,7 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
         ++k;
     }
     mark(4);
-    if (s->precision && e == cudaSuccess) {
+    if (!a.fuse_narrow && e == cudaSuccess) {
         DetectArgs n = a;
         n.fuse_narrow = 1;
         n.grid = sm_count(s->device) * 8;
@@ -1483,15 +1515,22 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
         OK_TRY(s->hits.ensure(want, "cudaMalloc(hits)"));
         s->hit_cap = want;
     }
-    if (s->precision) {
-        // split narrow phase: the candidates of the whole frame are stored
-        s->cand_cap = std::max(s->cand_cap, grow_cap(2 * s->cand_count, s->cand_cap));
-        OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
-        OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
-    }
-    OK_TRY(s->h_frame_counts.ensure(kCountHost, "cudaMallocHost(frame counts)"));
     PassPlan plan;
     OK_TRY(plan_pass(s, pr.data(), np, s->frame_entry, plan));
+    bool split = s->precision || split_narrow(s, plan);
+    if (split) {
+        // a narrow phase of its own: the candidates of the whole frame are stored
+        const uint32_t cap = s->cand_cap;
+        s->cand_cap = std::max(s->cand_cap, grow_cap(2 * s->cand_count, s->cand_cap));
+        const int r = s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)");
+        if (r != OIBVH_OK && s->precision) return r;
+        if (r != OIBVH_OK) {
+            split = false;
+            s->cand_cap = cap;
+        }
+    }
+    if (s->precision) OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
+    OK_TRY(s->h_frame_counts.ensure(kCountHost, "cudaMallocHost(frame counts)"));
     CUDA_TRY(cudaStreamSynchronize(st));
     std::memcpy(s->h_pairs.p, plan.pv.data(), np * sizeof(PairView));
     CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
@@ -1516,13 +1555,13 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     a.hits = s->hits.p;
     a.hit_cap = s->hit_cap;
     a.counts = s->counts.p;
-    a.fuse_narrow = s->precision ? 0u : 1u;
-    a.cand = s->precision ? s->cand.p : nullptr;
-    a.cand_cap = s->precision ? s->cand_cap : 0u;
+    a.fuse_narrow = split ? 0u : 1u;
+    a.cand = split ? s->cand.p : nullptr;
+    a.cand_cap = split ? s->cand_cap : 0u;
     a.prec_lists = s->precision ? s->prec_lists.p : nullptr;
     a.fp64_tri = s->precision ? s->fp64_tri.p : nullptr;
     a.fp64_tri_cap = s->precision ? s->fp64_tri_cap : 0u;
-    a.grid = walk_grid(s, !s->precision);
+    a.grid = walk_grid(s, !split);
     a.walk_cap = s->tune_walk_cap;
     a.precision = s->precision;
     a.claim_min = s->tune_claim;
