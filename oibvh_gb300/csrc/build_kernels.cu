@@ -877,9 +877,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_build_small(const BuildJob
         t[0] = r.x;
         t[1] = r.y;
         t[2] = r.z;
-        const float4 p0 = sh.pos[f[k][0]], p1 = sh.pos[f[k][1]], p2 = sh.pos[f[k][2]];
-        b[k] = Box{gmin(gmin(p0.x, p1.x), p2.x), gmin(gmin(p0.y, p1.y), p2.y), gmin(gmin(p0.z, p1.z), p2.z),
-                   gmax(gmax(p0.x, p1.x), p2.x), gmax(gmax(p0.y, p1.y), p2.y), gmax(gmax(p0.z, p1.z), p2.z)};
+        b[k] = box_of(sh.pos[f[k][0]], sh.pos[f[k][1]], sh.pos[f[k][2]]);
     }
     if (S.L > 0) reduce_block<12>(b, S, box, S.L, 0, S.L, sh.boxes);
 }

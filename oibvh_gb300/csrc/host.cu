@@ -51,6 +51,7 @@ static int tree_alloc(oibvh_tree_t t)
     OK_TRY(t->vperm.ensure(t->nV, "cudaMalloc(vertex order)"));
     OK_TRY(t->box.ensure(2 * (size_t)std::max(1u, t->shape.size - t->nT), "cudaMalloc(tree)"));
     OK_TRY(t->counters.ensure(refit_counters_per_tree(), "cudaMalloc(counters)"));
+    CUDA_TRY(cudaMemset(t->counters.p, 0, refit_counters_per_tree() * sizeof(uint32_t)));
     return OIBVH_OK;
 }
 
@@ -155,7 +156,7 @@ static int tree_build_impl(oibvh_tree_t t, cudaStream_t s)
     a.v_tiles = (t->nV + kBuildTile - 1) / kBuildTile;
     a.passes = t->morton_bits == 63 ? 8 : 4;
     OK_TRY(build_impl(a, 1, t->nT, t->nV, t->device, s));
-    CUDA_TRY(launch_refit_one(t->job(), s));
+    CUDA_TRY(launch_refit_one(t->job(), RefitSource{}, s));
     CUDA_TRY(cudaStreamSynchronize(s));
     OK_TRY(build_check(a));
     t->reordered = true;
@@ -714,17 +715,20 @@ API int oibvh_tree_build(oibvh_tree_t t, void* stream)
     GUARD_END
 }
 
-// Positions as given (xyz, host or device) into the tree's own device layout.
-static int stage_xyz(oibvh_tree_t t, const float* xyz, bool on_device, cudaStream_t s)
+// Positions as given (xyz, host or device) into the tree's own device layout;
+// with `refit`, and then the boxes (a small tree in one launch).
+static int stage_xyz(oibvh_tree_t t, const float* xyz, bool on_device, bool refit, cudaStream_t s)
 {
     const float* src = xyz;
     if (!on_device) {
         CUDA_TRY(cudaMemcpyAsync(t->xyz.p, xyz, 3 * (size_t)t->nV * sizeof(float), cudaMemcpyHostToDevice, s));
         src = t->xyz.p;
     }
-    CUDA_TRY(launch_xyz_to_pos4(src, t->vmap(), t->nV, t->pos4.p, s));
+    const bool direct = refit && refit_takes_xyz(t->nT);
+    if (!direct) CUDA_TRY(launch_xyz_to_pos4(src, t->vmap(), t->nV, t->pos4.p, s));
     t->cur_pos = t->pos4.p;
     t->borrowed = nullptr;
+    if (refit) CUDA_TRY(launch_refit_one(t->job(), direct ? RefitSource{src, t->vmap(), t->nV} : RefitSource{}, s));
     return OIBVH_OK;
 }
 
@@ -745,9 +749,9 @@ API int oibvh_tree_refit(oibvh_tree_t t, const float* xyz, void* stream)
     if (!t->built) return fail(OIBVH_ERR_STATE, "refit before build");
     DeviceGuard g(t->device);
     cudaStream_t s = (cudaStream_t)stream;
-    if (xyz) OK_TRY(stage_xyz(t, xyz, false, s));
-    else OK_TRY(sync_positions(t, s));
-    CUDA_TRY(launch_refit_one(t->job(), s));
+    if (xyz) return stage_xyz(t, xyz, false, true, s);
+    OK_TRY(sync_positions(t, s));
+    CUDA_TRY(launch_refit_one(t->job(), RefitSource{}, s));
     return OIBVH_OK;
     GUARD_END
 }
@@ -759,9 +763,7 @@ API int oibvh_tree_refit_device(oibvh_tree_t t, const float* d_xyz, void* stream
     if (!t->built) return fail(OIBVH_ERR_STATE, "refit before build");
     DeviceGuard g(t->device);
     OK_TRY(check_device_ptr(d_xyz, 4));
-    OK_TRY(stage_xyz(t, d_xyz, true, (cudaStream_t)stream));
-    CUDA_TRY(launch_refit_one(t->job(), (cudaStream_t)stream));
-    return OIBVH_OK;
+    return stage_xyz(t, d_xyz, true, true, (cudaStream_t)stream);
     GUARD_END
 }
 
@@ -770,7 +772,7 @@ API int oibvh_tree_set_positions(oibvh_tree_t t, const float* xyz, void* stream)
     GUARD_BEGIN
     if (!t || !xyz) return fail(OIBVH_ERR_ARG, "tree or xyz is NULL");
     DeviceGuard g(t->device);
-    return stage_xyz(t, xyz, false, (cudaStream_t)stream);
+    return stage_xyz(t, xyz, false, false, (cudaStream_t)stream);
     GUARD_END
 }
 
@@ -780,7 +782,7 @@ API int oibvh_tree_set_positions_device(oibvh_tree_t t, const float* d_xyz, void
     if (!t || !d_xyz) return fail(OIBVH_ERR_ARG, "tree or d_xyz is NULL");
     DeviceGuard g(t->device);
     OK_TRY(check_device_ptr(d_xyz, 4));
-    return stage_xyz(t, d_xyz, true, (cudaStream_t)stream);
+    return stage_xyz(t, d_xyz, true, false, (cudaStream_t)stream);
     GUARD_END
 }
 
@@ -975,7 +977,10 @@ API int oibvh_scene_refit(oibvh_scene_t s, void* stream)
         jobs[i] = j;
     }
     const size_t per = refit_counters_per_tree();
-    OK_TRY(s->refit_counters.ensure(per * n, "cudaMalloc(refit counters)"));
+    if (!s->refit_counters.p || s->refit_counters.n < per * n) {
+        OK_TRY(s->refit_counters.ensure(per * n, "cudaMalloc(refit counters)"));
+        CUDA_TRY(cudaMemsetAsync(s->refit_counters.p, 0, s->refit_counters.n * sizeof(uint32_t), st));
+    }
     for (size_t i = 0; i < n; ++i) jobs[i].counters = s->refit_counters.p + per * i;
     bool same = s->refit_cache.size() == n && s->refit_jobs.p;
     for (size_t i = 0; same && i < n; ++i) same = std::memcmp(&jobs[i], &s->refit_cache[i], sizeof(RefitJob)) == 0;
@@ -996,8 +1001,7 @@ API int oibvh_scene_refit(oibvh_scene_t s, void* stream)
         s->refit_cache = jobs;
     }
     s->refit_blocks = blocks;
-    CUDA_TRY(launch_refit(s->refit_jobs.p, (uint32_t)n, blocks, s->refit_block_job.p, s->refit_counters.p, per * n,
-                          s->tune_refit_log, st));
+    CUDA_TRY(launch_refit(s->refit_jobs.p, (uint32_t)n, blocks, s->refit_block_job.p, s->tune_refit_log, st));
     return OIBVH_OK;
     GUARD_END
 }
@@ -1459,7 +1463,7 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
     mark(1);
     if (s->frame_refit && e == cudaSuccess) {
         e = launch_refit(s->refit_jobs.p, (uint32_t)s->trees.size(), s->refit_blocks, s->refit_block_job.p,
-                         s->refit_counters.p, refit_counters_per_tree() * s->trees.size(), s->tune_refit_log, st);
+                         s->tune_refit_log, st);
         ++k;
     }
     mark(2);

@@ -178,14 +178,17 @@ __device__ __forceinline__ Box merge(const Box& l, const Box& r)
                gmax(l.xx, r.xx), gmax(l.xy, r.xy), gmax(l.xz, r.xz)};
 }
 
-// Box of one face (v0, v1, v2, .): glm::min(glm::min(v0, v1), v2) and the
-// max likewise, as calculate_aabb_kernel (src/cuda/oibvh.cu:24-40); one
-// 16-byte load per vertex.
-__device__ __forceinline__ Box leaf_box(const float4* __restrict__ pos, uint4 f)
+// Box of a triangle: glm::min(glm::min(v0, v1), v2) and the max likewise, as
+// calculate_aabb_kernel (src/cuda/oibvh.cu:24-40).
+__device__ __forceinline__ Box box_of(const float4& a, const float4& b, const float4& c)
 {
-    const float4 a = __ldg(pos + f.x), b = __ldg(pos + f.y), c = __ldg(pos + f.z);
     return Box{gmin(gmin(a.x, b.x), c.x), gmin(gmin(a.y, b.y), c.y), gmin(gmin(a.z, b.z), c.z),
                gmax(gmax(a.x, b.x), c.x), gmax(gmax(a.y, b.y), c.y), gmax(gmax(a.z, b.z), c.z)};
+}
+// Box of one face (v0, v1, v2, .); one 16-byte load per vertex.
+__device__ __forceinline__ Box leaf_box(const float4* __restrict__ pos, uint4 f)
+{
+    return box_of(__ldg(pos + f.x), __ldg(pos + f.y), __ldg(pos + f.z));
 }
 
 // Internal nodes are 32 bytes, (min.xyz, 0, max.xyz, 0), and 32-byte

@@ -20,8 +20,16 @@ struct RefitJob {
     TreeShape shape;
     uint32_t block_begin;  // first CTA of this tree in the launch
     uint32_t n_blocks;
-    uint32_t* counters;    // refit_counters_per_tree() zeroed words
+    uint32_t* counters;    // refit_counters_per_tree() words, zero before the first refit (each leaves them zero)
     uint32_t pad0;
+};
+
+// A refit's positions as the caller gave them (xyz; tree vertex v is the
+// caller's vperm[v]); xyz == nullptr: the tree's own positions.
+struct RefitSource {
+    const float* xyz;
+    const uint32_t* vperm;
+    uint32_t nV;
 };
 
 // One tree of a multi-tree build / transform launch.
@@ -94,12 +102,13 @@ cudaError_t launch_gather_pos4(const float4* src, const uint32_t* vperm, uint32_
 // (9, 10 or 11; 0 = 10, the single-tree refit's)
 uint32_t refit_blocks_for(uint32_t nT, uint32_t group_log2 = 0);
 uint32_t refit_counters_per_tree();
-cudaError_t launch_refit_one(const RefitJob& job, cudaStream_t s);
+bool refit_takes_xyz(uint32_t nT);  // whether launch_refit_one should be given `src` rather than converted positions
+cudaError_t launch_refit_one(const RefitJob& job, const RefitSource& src, cudaStream_t s);
 cudaError_t launch_leaf_boxes(const uint4* face, const float4* pos, uint32_t nT, float4* out, cudaStream_t s);
 // block_job: optional host-built map from a refit CTA to its job (nullptr:
 // each CTA binary-searches the job table).
 cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks, const uint32_t* block_job,
-                         uint32_t* d_counters, size_t n_counters, uint32_t group_log2, cudaStream_t s);
+                         uint32_t group_log2, cudaStream_t s);
 
 // detect_kernels.cu
 struct DetectArgs {

@@ -31,11 +31,15 @@ namespace oibvh {
 constexpr uint32_t kRefitLogDefault = 10;
 constexpr int kStageCounters = 64;  // counters per climbing stage and tree (groups of the widest stage, kLog 9)
 
-// `jobs` == nullptr: a single tree passed by value in `one`.
-template <int kLog>
+// `jobs` == nullptr: a single tree passed by value in `one`. kXyz: its positions
+// are still the caller's, in `src`: the CTAs convert them (a slice of the
+// vertices each) and take the leaves' corners from the source, so a small
+// tree's refit is one launch (320 triangles: a refit and detect pass 62 to
+// 55 us). Corners cost four loads so instead of one, which larger trees feel.
+template <int kLog, bool kXyz>
 __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
     k_refit(const RefitJob* __restrict__ jobs, uint32_t n_jobs, const uint32_t* __restrict__ block_job,
-            const RefitJob one)
+            const RefitJob one, const RefitSource src)
 {
     constexpr uint32_t kRefitLog = kLog, kRefitChunk = 1u << kLog;
     __shared__ Box sm8[(1 << kLog) / 128];
@@ -54,8 +58,15 @@ __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
         job = jobs[lo];
     }
     const TreeShape S = job.shape;
-    if (S.L == 0) return;  // a single leaf: no internal node
     const uint32_t chunk = blockIdx.x - job.block_begin;
+    if constexpr (kXyz) {
+        float4* pos = const_cast<float4*>(job.pos);
+        for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < src.nV; v += gridDim.x * blockDim.x) {
+            const float* p = src.xyz + 3 * (size_t)(src.vperm ? __ldg(src.vperm + v) : v);
+            pos[v] = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), 0.0f);
+        }
+    }
+    if (S.L == 0) return;  // a single leaf: no internal node
 
     // ---- leaves: calculate_aabb_kernel (src/cuda/oibvh.cu:24-40), in registers ----
     const uint32_t leaf0 = (chunk << kRefitLog) + 4 * threadIdx.x;
@@ -69,7 +80,17 @@ __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
     }
     Box v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = leaf_box(job.pos, f[k]);
+    for (int k = 0; k < 4; ++k) {
+        if constexpr (kXyz) {
+            auto corner = [&](uint32_t i) {
+                const float* p = src.xyz + 3 * (size_t)(src.vperm ? __ldg(src.vperm + i) : i);
+                return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), 0.0f);
+            };
+            v[k] = box_of(corner(f[k].x), corner(f[k].y), corner(f[k].z));
+        } else {
+            v[k] = leaf_box(job.pos, f[k]);
+        }
+    }
 
     uint32_t levels = min((uint32_t)kRefitLog, S.L);
     reduce_block<kLog>(v, S, job.box, S.L, chunk << kRefitLog, levels, sm8);
@@ -83,7 +104,8 @@ __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
         const uint32_t gcnt = min(kRefitChunk, S.level_count(lvl) - (g << kRefitLog));
         if (threadIdx.x == 0) {
             __threadfence();
-            const uint32_t old = atomicAdd(job.counters + stage * kStageCounters + g, 1u);
+            // (wraps to 0 with the last arrival: nobody has to clear it for the next refit)
+            const uint32_t old = atomicInc(job.counters + stage * kStageCounters + g, gcnt - 1);
             s_last = (old == gcnt - 1) ? 1u : 0u;
         }
         __syncthreads();
@@ -124,42 +146,33 @@ uint32_t refit_blocks_for(uint32_t nT, uint32_t group_log2)
 }
 uint32_t refit_counters_per_tree() { return 4 * kStageCounters; }
 
-template <int kLog>
-static void refit_launch(uint32_t blocks, const RefitJob* jobs, uint32_t n_jobs, const uint32_t* block_job,
-                         const RefitJob& one, cudaStream_t s)
-{
-    k_refit<kLog><<<blocks, (1 << kLog) / 4, 0, s>>>(jobs, n_jobs, block_job, one);
-}
+// A tree of up to this many faces is refitted from the caller's positions in one launch.
+constexpr uint32_t kRefitXyzMax = 32768;
+bool refit_takes_xyz(uint32_t nT) { return nT <= kRefitXyzMax; }
 
-static cudaError_t refit_dispatch(uint32_t group_log2, uint32_t blocks, const RefitJob* jobs, uint32_t n_jobs,
-                                  const uint32_t* block_job, const RefitJob& one, cudaStream_t s)
+cudaError_t launch_refit_one(const RefitJob& job, const RefitSource& src, cudaStream_t s)
 {
-    switch (group_log2 ? group_log2 : kRefitLogDefault) {
-    case 9: refit_launch<9>(blocks, jobs, n_jobs, block_job, one, s); break;
-    case 10: refit_launch<10>(blocks, jobs, n_jobs, block_job, one, s); break;
-    case 11: refit_launch<11>(blocks, jobs, n_jobs, block_job, one, s); break;
-    default: return cudaErrorInvalidValue;
-    }
+    note_launches(1);
+    constexpr uint32_t kThreads = (1u << kRefitLogDefault) / 4;
+    if (src.xyz) k_refit<kRefitLogDefault, true><<<job.n_blocks, kThreads, 0, s>>>(nullptr, 1, nullptr, job, src);
+    else k_refit<kRefitLogDefault, false><<<job.n_blocks, kThreads, 0, s>>>(nullptr, 1, nullptr, job, src);
     return cudaGetLastError();
 }
 
-cudaError_t launch_refit_one(const RefitJob& job, cudaStream_t s)
-{
-    cudaError_t e = cudaMemsetAsync(job.counters, 0, refit_counters_per_tree() * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    note_launches(1);
-    return refit_dispatch(kRefitLogDefault, job.n_blocks, nullptr, 1, nullptr, job, s);
-}
-
 cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks, const uint32_t* block_job,
-                         uint32_t* d_counters, size_t n_counters, uint32_t group_log2, cudaStream_t s)
+                         uint32_t group_log2, cudaStream_t s)
 {
     if (n_jobs == 0 || total_blocks == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(d_counters, 0, n_counters * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    RefitJob none{};
+    const RefitJob none{};
+    const RefitSource own{};
     note_launches(1);
-    return refit_dispatch(group_log2, total_blocks, d_jobs, n_jobs, block_job, none, s);
+    switch (group_log2 ? group_log2 : kRefitLogDefault) {
+    case 9: k_refit<9, false><<<total_blocks, 128, 0, s>>>(d_jobs, n_jobs, block_job, none, own); break;
+    case 10: k_refit<10, false><<<total_blocks, 256, 0, s>>>(d_jobs, n_jobs, block_job, none, own); break;
+    case 11: k_refit<11, false><<<total_blocks, 512, 0, s>>>(d_jobs, n_jobs, block_job, none, own); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_leaf_boxes(const uint4* face, const float4* xyz, uint32_t nT, float4* out, cudaStream_t s)

@@ -137,6 +137,7 @@ struct Lane {
     uint32_t n_pairs = 0;
     uint64_t n_hits = 0;
 
+    int ensure_refit_counters(size_t words);  // zero when new: refits leave them zero
     int ensure_lists()
     {
         OK_TRY(work0.ensure(front_cap, "cudaMalloc(work list)"));
@@ -158,6 +159,14 @@ int ensure_pow2(Buf& b, size_t want, const char* what)
     size_t n = 64;
     while (n < want) n <<= 1;
     return b.ensure(n, what);
+}
+
+int Lane::ensure_refit_counters(size_t words)
+{
+    if (rcount.p && rcount.n >= words) return OIBVH_OK;
+    OK_TRY(ensure_pow2(rcount, words, "cudaMalloc(refit counters)"));
+    CUDA_TRY(cudaMemsetAsync(rcount.p, 0, rcount.n * sizeof(uint32_t), st));
+    return OIBVH_OK;
 }
 
 uint32_t grow(uint64_t need, uint32_t cur)
@@ -311,7 +320,7 @@ int oibvh_server_s::reserve_lanes()
         OK_TRY(ensure_pow2(L.rjobs, n, "cudaMalloc(refit jobs)"));
         OK_TRY(ensure_pow2(L.h_mats, 12 * n, "cudaMallocHost(matrices)"));
         OK_TRY(ensure_pow2(L.mats, 12 * n, "cudaMalloc(matrices)"));
-        OK_TRY(ensure_pow2(L.rcount, (size_t)per * n, "cudaMalloc(refit counters)"));
+        OK_TRY(L.ensure_refit_counters((size_t)per * n));
         OK_TRY(L.h_counts.ensure(kCountHost, "cudaMallocHost(counts)"));
         L.front_cap = init_front_cap;
         L.hit_cap = init_hit_cap;
@@ -341,7 +350,7 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
     OK_TRY(ensure_pow2(L.rjobs, n, "cudaMalloc(refit jobs)"));
     OK_TRY(ensure_pow2(L.h_mats, 12 * (size_t)n, "cudaMallocHost(matrices)"));
     OK_TRY(ensure_pow2(L.mats, 12 * (size_t)n, "cudaMalloc(matrices)"));
-    OK_TRY(ensure_pow2(L.rcount, (size_t)per * n, "cudaMalloc(refit counters)"));
+    OK_TRY(L.ensure_refit_counters((size_t)per * n));
     OK_TRY(L.h_counts.ensure(kCountHost, "cudaMallocHost(counts)"));
     OK_TRY(L.qcount.ensure((size_t)n + 1, "cudaMalloc(query counts)"));
     OK_TRY(L.qcursor.ensure((size_t)n + 1, "cudaMalloc(query cursors)"));
@@ -427,7 +436,7 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
     CUDA_TRY(cudaMemcpyAsync(L.mats.p, L.h_mats.p, 12 * n * sizeof(float), cudaMemcpyHostToDevice, st));
     // a batch has few jobs: the kernels binary-search them (no block maps)
     CUDA_TRY(launch_transform_multi(L.jobs.p, n, vblocks, nullptr, nullptr, L.mats.p, false, st));
-    CUDA_TRY(launch_refit(L.rjobs.p, n, rblocks, nullptr, L.rcount.p, (size_t)per * n, 0, st));
+    CUDA_TRY(launch_refit(L.rjobs.p, n, rblocks, nullptr, 0, st));
     L.batch = batch;
     const auto now = Clock::now();
     for (uint32_t i = 0; i < n; ++i) {

@@ -86,3 +86,42 @@ def test_scene_build(gpu, sizes, bits):
             _check(t, x, f, bits)
             if bits == 63:
                 assert np.array_equal(t.sorted_faces()[1], _order63(x, f))
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 1023, 1024, 1025, 5000, 32767, 32768, 32769, 60000])
+@pytest.mark.parametrize("where", ["host", "device"])
+def test_refits_in_a_row(gpu, n, where):
+    """Refits from the caller's positions (one launch up to 32,768 faces, two
+    above) follow each other with nothing cleared in between."""
+    import torch
+
+    from oibvh_gb300 import OibvhTree
+
+    xyz, tri = _mesh(n, 900 + n, "unused")
+    t = OibvhTree(xyz=xyz, tri=tri)
+    t.build()
+    f, p = t.sorted_faces()
+    rng = np.random.default_rng(n)
+    for _ in range(4):
+        moved = (xyz + rng.normal(0, 0.1, xyz.shape)).astype(np.float32)
+        if where == "host":
+            t.refit(moved)
+        else:
+            d = torch.from_numpy(moved).cuda()
+            t.refit_device(d.data_ptr())
+        a = moved[f]
+        leaves = np.concatenate([a.min(1), a.max(1)], 1)
+        got = t.aabb_tree()
+        assert np.array_equal(got[-n:], leaves)
+        assert np.array_equal(got[0], np.concatenate([leaves[:, :3].min(0), leaves[:, 3:].max(0)]))
+        level = leaves  # every level: the union of its two children, a lone last one's own box
+        while level.shape[0] > 1:
+            odd = level[-1:] if level.shape[0] % 2 else level[:0]
+            e = level[: level.shape[0] // 2 * 2].reshape(-1, 2, 6)
+            level = np.concatenate([np.concatenate([e[:, :, :3].min(1), e[:, :, 3:].max(1)], 1), odd])
+            at = got.shape[0] - n if level.shape[0] == (n + 1) // 2 else at
+            at -= level.shape[0]
+            assert np.array_equal(got[at : at + level.shape[0]], level)
+    for _ in range(2):  # the positions now held, again
+        t.refit()
+        assert np.array_equal(t.aabb_tree(), got)
