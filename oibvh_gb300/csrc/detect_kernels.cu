@@ -1026,15 +1026,18 @@ __device__ __forceinline__ EV3 axis_of(uint32_t k, const LaneTri& t)
 // ---------------------------------------------------------------------------
 // Precision narrow phase in passes, grouping candidates by how much of the
 // filtered test they need, so that the lanes of a warp run the same code:
-//  1. k_prec_classify, one candidate per thread: the plain float SAT (the
-//     reference's arithmetic), which also names the first separating axis. A
-//     float-separated candidate needs only that axis bounded: a margin above
-//     its error bound separates in every arithmetic (no hit, float and FP64
-//     agree); otherwise it goes to the recheck list. Shared vertices are hits
-//     at once, and so is a float hit whose every axis overlaps beyond a
-//     static bound on the float and FP64 errors; other float hits go to the
-//     float-hit list, whose members need all 17 bounded axes.
-//  2. k_prec_settle over the float-hit list then the recheck list, one per
+//  1. k_prec_classify: the plain float SAT (the reference's arithmetic), which
+//     also names the first separating axis. A float-separated candidate needs
+//     only that axis bounded: a margin above its error bound separates in every
+//     arithmetic (no hit, float and FP64 agree); otherwise it goes to the
+//     recheck list with the axis. Shared vertices are hits at once, and so is a
+//     float hit whose every axis overlaps beyond a static bound on the float
+//     and FP64 errors; other float hits go to the float-hit list, whose members
+//     need all 17 bounded axes.
+//     Then k_prec_recheck: the recheck list's one axis in double-float
+//     arithmetic (3.). Where FP64 separates there too, which is nearly always,
+//     the candidate is done; the others join the float hits.
+//  2. k_prec_settle over the float hits and what the recheck left, one per
 //     lane: pass 1 of the filtered test (all 17 axes bounded, straight-line
 //     for float hits: no lane leaves early); what it leaves undecided goes to
 //     the FP64 list with the mask of its undecided axes.
@@ -1138,57 +1141,108 @@ __device__ __forceinline__ uint32_t bounded_axis_separates(uint32_t k, const V3&
     return project6_bounded(axis_of(k, t), zero, p2, p3, q1, q2, q3, s32) == 0u ? kPass1Separated : kPass1Undecided;
 }
 
+// The lists of the precision passes, in prec_lists (4 x cand_cap words): the
+// float hits (words), what the recheck leaves (words), and the recheck list
+// ((candidate, axis) pairs), whose room the FP64 list takes once it is done.
+struct PrecLists {
+    uint32_t *hits, *left;
+    uint2 *recheck, *fp64;
+    __device__ __forceinline__ explicit PrecLists(const DetectArgs& a)
+        : hits(a.prec_lists), left(a.prec_lists + a.cand_cap), recheck((uint2*)(a.prec_lists + 2 * (size_t)a.cand_cap)),
+          fp64(recheck)
+    {
+    }
+};
+
+// A warp's entries for a global list, gathered in shared memory and appended 32
+// at a time: an atomic for each list and 32 candidates queued up at the counters
+// (3.2 M candidates of 16 pairs of sheets: 140 us so, 127 with this. The test in
+// two goes, the walk's way, took 128, and 18 in place of 15 for 239 k).
+template <typename T>
+struct WarpList {
+    T* buf;          // 64 entries in shared memory
+    uint32_t n = 0;  // warp-uniform
+    template <typename Store>
+    __device__ __forceinline__ void flush(uint32_t count, uint32_t* counter, uint32_t lane, Store store)
+    {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(counter, count);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (lane < count) store(at + lane, buf[n - count + lane]);
+        n -= count;
+        __syncwarp();
+    }
+    template <typename Store>
+    __device__ __forceinline__ void push(bool pred, const T& v, uint32_t* counter, uint32_t lane, Store store)
+    {
+        const uint32_t m = __ballot_sync(0xffffffffu, pred);
+        if (m == 0) return;
+        if (pred) buf[n + __popc(m & ((1u << lane) - 1u))] = v;
+        n += __popc(m);
+        __syncwarp();
+        if (n >= 32) flush(32, counter, lane, store);
+    }
+};
+
 __global__ void __launch_bounds__(kDetectThreads) k_prec_classify(DetectArgs a)
 {
+    __shared__ uint4 s_hit[kWarps][64];
+    __shared__ uint2 s_recheck[kWarps][64];
+    __shared__ uint32_t s_float[kWarps][64];
     const uint32_t n = min(a.counts[kCountCandSlots], a.cand_cap);
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t* hit_list = a.prec_lists;
-    uint32_t* recheck = a.prec_lists + a.cand_cap;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const uint32_t i = base + threadIdx.x;
-        bool hit = false, to_hits = false, to_recheck = false;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const PrecLists lists(a);
+    WarpList<uint4> hits{s_hit[w]};
+    WarpList<uint2> rechecks{s_recheck[w]};
+    WarpList<uint32_t> floats{s_float[w]};
+    auto put_hit = [&](uint32_t at, const uint4& rec) {
+        if (at < a.hit_cap) a.hits[at] = rec;
+        else atomicOr(a.counts + kCountFlags, (uint32_t)kFlagHitOverflow);
+    };
+    auto put_recheck = [&](uint32_t at, const uint2& e) { lists.recheck[at] = e; };
+    auto put_float = [&](uint32_t at, uint32_t i) { lists.hits[at] = i; };
+    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t i = base + lane;
+        bool robust = false, hit = false, to_floats = false, to_recheck = false;
         uint4 rec = make_uint4(0, 0, 0, 0);
+        uint32_t k = 17;
         if (i < n) {
             V3 P1, P2, P3, Q1, Q2, Q3;
             load_tris(a, a.cand[i], P1, P2, P3, Q1, Q2, Q3, rec);
-            if (veq(P1, Q1) || veq(P1, Q2) || veq(P1, Q3) || veq(P2, Q1) || veq(P2, Q2) || veq(P2, Q3) ||
-                veq(P3, Q1) || veq(P3, Q2) || veq(P3, Q3)) {
+            if (veq(P1, Q1) || veq(P1, Q2) || veq(P1, Q3) || veq(P2, Q1) || veq(P2, Q2) || veq(P2, Q3) || veq(P3, Q1) ||
+                veq(P3, Q2) || veq(P3, Q3)) {
                 hit = true;  // a shared vertex: never separated, in any arithmetic
             } else {
-                bool robust;
-                const uint32_t k = tri_first_separating_axis(P1, P2, P3, Q1, Q2, Q3, robust);
-                if (k == 17) {
-                    if (robust) hit = true;  // every axis overlaps beyond the error bounds
-                    else to_hits = true;
-                } else {
-                    to_recheck = bounded_axis_separates(k, P1, P2, P3, Q1, Q2, Q3) != kPass1Separated;
-                }
+                k = tri_first_separating_axis(P1, P2, P3, Q1, Q2, Q3, robust);
+                if (k != 17) to_recheck = bounded_axis_separates(k, P1, P2, P3, Q1, Q2, Q3) != kPass1Separated;
+                else if (robust) hit = true;  // every axis overlaps beyond the error bounds
+                else to_floats = true;
             }
         }
-        append_hit(a, hit, rec, lane);
-        const uint32_t ph = warp_append(a.counts + kCountPrecHits, to_hits, lane);
-        if (to_hits) hit_list[ph] = i;
-        const uint32_t pr = warp_append(a.counts + kCountPrecRecheck, to_recheck, lane);
-        if (to_recheck) recheck[pr] = i;
+        hits.push(hit, rec, a.counts + kCountHits, lane, put_hit);
+        floats.push(to_floats, i, a.counts + kCountPrecHits, lane, put_float);
+        rechecks.push(to_recheck, make_uint2(i, k), a.counts + kCountPrecRecheck, lane, put_recheck);
     }
+    if (hits.n > 0) hits.flush(hits.n, a.counts + kCountHits, lane, put_hit);
+    if (floats.n > 0) floats.flush(floats.n, a.counts + kCountPrecHits, lane, put_float);
+    if (rechecks.n > 0) rechecks.flush(rechecks.n, a.counts + kCountPrecRecheck, lane, put_recheck);
 }
 
 __global__ void __launch_bounds__(kDetectThreads) k_prec_settle(DetectArgs a)
 {
     const uint32_t n_hits = min(a.counts[kCountPrecHits], a.cand_cap);
-    const uint32_t n = n_hits + min(a.counts[kCountPrecRecheck], a.cand_cap);
+    const uint32_t n = n_hits + min(a.counts[kCountPrecAgain], a.cand_cap);
+    const PrecLists lists(a);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    uint2* fp64_list = (uint2*)(a.prec_lists + 2 * (size_t)a.cand_cap);
     for (uint32_t base = warp * 32; base < n; base += n_warps * 32) {
         const uint32_t j = base + lane;
         bool hit = false, queue = false;
         uint4 rec = make_uint4(0, 0, 0, 0);
         uint32_t i = 0, mask = 0;
         if (j < n) {
-            i = j < n_hits ? a.prec_lists[j] : a.prec_lists[a.cand_cap + (j - n_hits)];
+            i = j < n_hits ? lists.hits[j] : lists.left[j - n_hits];
             V3 P1, P2, P3, Q1, Q2, Q3;
             load_tris(a, a.cand[i], P1, P2, P3, Q1, Q2, Q3, rec);
             bool hit32 = false;
@@ -1201,7 +1255,7 @@ __global__ void __launch_bounds__(kDetectThreads) k_prec_settle(DetectArgs a)
         }
         append_hit(a, hit, rec, lane);
         const uint32_t q = warp_append(a.counts + kCountPrecFp64, queue, lane);
-        if (queue) fp64_list[q] = make_uint2(i, mask);
+        if (queue) lists.fp64[q] = make_uint2(i, mask);
     }
 }
 
@@ -1414,10 +1468,10 @@ __device__ __forceinline__ DFB3 dfb_axis(uint32_t k, const DFTri& t, bool edges)
     const DFB3 c = dfb3_cross(dfb3_sel(ef || en, E, F), dfb3_sel(ef, F, dfb3_sel(en, t.n1, t.m1)));
     return dfb3_sel(k == 0, t.n1, dfb3_sel(k == 1, t.m1, c));
 }
-// Axis k of FP64 known from double-floats: 0 = separates, 1 = overlaps, 2 = undecided.
-__device__ __forceinline__ uint32_t dfb_axis_fp64(uint32_t k, const DFTri& t, bool edges)
+// What FP64 finds on the axis, known from double-floats: 0 = separates, 1 =
+// overlaps, 2 = undecided.
+__device__ __forceinline__ uint32_t dfb_decide(const DFB3& ax, const DFTri& t)
 {
-    const DFB3 ax = dfb_axis(k, t, edges);
     const DFB P[3] = {DFB{DF{0.0f, 0.0f}, 0.0f}, dfb3_dot(ax, t.p2), dfb3_dot(ax, t.p3)};
     const DFB Q[3] = {dfb3_dot(ax, t.q1), dfb3_dot(ax, t.q2), dfb3_dot(ax, t.q3)};
     // intervals that hold the FP64 values: value as hi + lo (the sum's rounding
@@ -1437,6 +1491,64 @@ __device__ __forceinline__ uint32_t dfb_axis_fp64(uint32_t k, const DFTri& t, bo
     if (pl > qh || ql > ph) return 0u;             // mn1 > mx2 or mn2 > mx1 for sure
     if (phl < qlh && qhl < plh) return 1u;         // mn1 < mx2 and mn2 < mx1 for sure
     return 2u;
+}
+__device__ __forceinline__ uint32_t dfb_axis_fp64(uint32_t k, const DFTri& t, bool edges)
+{
+    return dfb_decide(dfb_axis(k, t, edges), t);
+}
+__device__ __forceinline__ float max_abs_diff(const V3& a, const V3& b)
+{
+    return fmaxf(fmaxf(fabsf(__fsub_rn(a.x, b.x)), fabsf(__fsub_rn(a.y, b.y))), fabsf(__fsub_rn(a.z, b.z)));
+}
+
+// The recheck list: candidates that an axis separates in float by less than the
+// bound. The same axis with double-floats: where FP64 separates there too the
+// candidate is done, else it needs every axis. (Sending them all through the 17
+// bounded axes and then through the double-float pass took 190 us for the
+// 553 k of 16 pairs of sheets, whose margins of 1e-8 to 1e-7 no float bound
+// decides; with this pass 85 us, 57 of them here.) The normals, nearly every axis here, take one cross product with
+// its factors picked by selects.
+__global__ void __launch_bounds__(kDetectThreads) k_prec_recheck(DetectArgs a)
+{
+    const uint32_t n = min(a.counts[kCountPrecRecheck], a.cand_cap);
+    const uint32_t lane = threadIdx.x & 31;
+    const PrecLists lists(a);
+    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
+        bool again = false;
+        uint2 item = make_uint2(0, 0);
+        if (base + lane < n) {
+            item = lists.recheck[base + lane];
+            V3 P1, P2, P3, Q1, Q2, Q3;
+            uint4 rec;
+            load_tris(a, a.cand[item.x], P1, P2, P3, Q1, Q2, Q3, rec);
+            const float A = fmaxf(fmaxf(max_abs_diff(P2, P1), max_abs_diff(P3, P1)),
+                                  fmaxf(fmaxf(max_abs_diff(Q1, P1), max_abs_diff(Q2, P1)), max_abs_diff(Q3, P1)));
+            // (fmaxf drops a NaN, this sum does not)
+            const float sum = (P2.x + P2.y + P2.z) + (P3.x + P3.y + P3.z) + (Q1.x + Q1.y + Q1.z) + (Q2.x + Q2.y + Q2.z) +
+                              (Q3.x + Q3.y + Q3.z) + (P1.x + P1.y + P1.z);
+            again = true;
+            if (A >= 0x1p-20f && A <= 0x1p20f && fabsf(sum) <= 3e38f) {  // (else the bounds could under- or overflow)
+                DFTri t;
+                t.p2 = dfb3_rel(P2, P1);
+                t.p3 = dfb3_rel(P3, P1);
+                t.q1 = dfb3_rel(Q1, P1);
+                t.q2 = dfb3_rel(Q2, P1);
+                t.q3 = dfb3_rel(Q3, P1);
+                if (item.y < 2) {
+                    const bool nrm = item.y == 0;  // n1 = p2 x (p3 - p2), m1 = (q2 - q1) x (q3 - q2)
+                    const DFB3 c = dfb3_cross(dfb3_sel(nrm, t.p2, dfb3_sub(t.q2, t.q1)),
+                                              dfb3_sub(dfb3_sel(nrm, t.p3, t.q3), dfb3_sel(nrm, t.p2, t.q2)));
+                    again = dfb_decide(c, t) != 0u;
+                } else {
+                    t.n1 = dfb3_cross(t.p2, dfb3_sub(t.p3, t.p2));
+                    t.m1 = dfb3_cross(dfb3_sub(t.q2, t.q1), dfb3_sub(t.q3, t.q2));
+                    again = dfb_axis_fp64(item.y, t, true) != 0u;
+                }
+            }
+        }
+        const uint32_t q = warp_append(a.counts + kCountPrecAgain, again, lane);
+        if (again) lists.left[q] = item.x;
+    }
 }
 
 // Idle lanes that trigger a refill of the double-float pass (a refill forms
@@ -1461,7 +1573,7 @@ __global__ void __launch_bounds__(kDetectThreads) k_prec_df(DetectArgs a)
 {
     const uint32_t n = min(a.counts[kCountPrecFp64], a.cand_cap);
     const uint2* list = (const uint2*)(a.prec_lists + 2 * (size_t)a.cand_cap);
-    uint2* left = (uint2*)a.prec_lists;  // the float-hit and recheck lists' room, free after the bounded pass
+    uint2* left = (uint2*)a.prec_lists;  // the room of the float hits and the recheck's rest, free after the bounded pass
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t W = (gridDim.x * blockDim.x) >> 5;
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1740,7 +1852,7 @@ int walk_blocks_per_sm(uint32_t walk_cap, bool fused)
     return n;
 }
 
-uint32_t narrow_kernels(const DetectArgs& a) { return a.precision ? (a.fp64_tri_cap ? 5u : 4u) : 1u; }
+uint32_t narrow_kernels(const DetectArgs& a) { return a.precision ? (a.fp64_tri_cap ? 6u : 5u) : 1u; }
 
 cudaError_t launch_narrow(const DetectArgs& a, cudaStream_t s)
 {
@@ -1748,6 +1860,7 @@ cudaError_t launch_narrow(const DetectArgs& a, cudaStream_t s)
         if (a.prec_lists == nullptr || (a.fp64_tri_cap && a.fp64_tri == nullptr)) return cudaErrorInvalidValue;
         note_launches(narrow_kernels(a));
         k_prec_classify<<<a.grid, kDetectThreads, 0, s>>>(a);
+        k_prec_recheck<<<a.grid, kDetectThreads, 0, s>>>(a);
         k_prec_settle<<<a.grid, kDetectThreads, 0, s>>>(a);
         k_prec_df<<<a.grid, kDetectThreads, 0, s>>>(a);
         if (a.fp64_tri_cap) k_prec_fp64_setup<<<a.grid, kDetectThreads, 0, s>>>(a);

@@ -126,8 +126,7 @@ struct DetectArgs {
     uint4* host_hits;      // pinned: and the hits, when there are at most host_hit_cap
     uint32_t host_hit_cap;
     uint32_t* counts_next; // with host: the counter block that the walk clears for the next traversal
-    uint32_t* prec_lists;  // precision mode, 4 x cand_cap words: float-hit list, recheck list (candidate
-                           // indices), then the FP64 list ((candidate index, axis mask) pairs)
+    uint32_t* prec_lists;  // precision mode, 4 x cand_cap words: the passes' lists (PrecLists)
     double* fp64_tri;      // precision mode: the FP64 list's setups, kFp64TriRows rows of fp64_tri_cap
                            // (structure of arrays; nullptr: each is formed where it is used)
     uint32_t fp64_tri_cap;
@@ -160,13 +159,14 @@ constexpr uint32_t kFp64TriRows = 23;
 // BVTT pairs tested, (precision mode) axes evaluated in FP64, candidates with
 // at least one such axis, candidates whose float and FP64 answers differ,
 // the sizes of the float-hit, recheck and FP64 lists of the precision narrow phase
-// and of the list its double-float pass leaves to FP64; then the largest list
+// of the list its double-float pass leaves to FP64, and of what its recheck
+// leaves to the bounded pass; then the largest list
 // of a walk round and the rounds walked. Past the words that the host reads:
 // the walk's control words, each on a cache line of its own.
 constexpr uint32_t kCountHits = 0, kCountFlags = 1, kCountCands = 2, kCountCandSlots = 3, kCountTested = 4,
                    kCountFp64Axes = 5, kCountFp64Cands = 6, kCountDisagree = 7, kCountPrecHits = 8,
-                   kCountPrecRecheck = 9, kCountPrecFp64 = 10, kCountPrecLeft = 11, kCountNarrowEnd = 12,
-                   kCountPeak = 12, kCountRounds = 13, kCountHost = 16,
+                   kCountPrecRecheck = 9, kCountPrecFp64 = 10, kCountPrecLeft = 11, kCountPrecAgain = 12,
+                   kCountNarrowEnd = 13, kCountPeak = 13, kCountRounds = 14, kCountHost = 16,
                    kCtlRelease = 32,
                    kCtlRound = 64, kCtlRoundWords = 64, kCtlRoundClaim = 32,  // four slots
                    kCountTotal = kCtlRound + 4 * kCtlRoundWords;

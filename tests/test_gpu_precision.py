@@ -169,6 +169,23 @@ def test_coplanar_soups_take_the_fp64_pass(gpu, seed):
     assert st["fp64_candidates"] > 0 and st["fp64_axes"] > 0  # the FP64 pass ran
 
 
+@pytest.mark.parametrize("scale", [1.0, 1e-8, 1e7])  # relative extents within the bounds' range, below and above
+@pytest.mark.parametrize("n_tri", [1, 7, 8, 9, 33, 300])
+def test_axes_within_the_float_bound(gpu, n_tri, scale):
+    """Lists of a few entries, a warp's and more, on every pass: margins no
+    float bound decides, with extents for which the bounds hold or do not."""
+    from oibvh_gb300 import _native as N
+    from oibvh_gb300.meshes import Mesh
+
+    meshes = [Mesh((m.xyz * np.float32(scale)).astype(np.float32), m.tri) for m in near_degenerate_pair(40 + n_tri, n_tri)]
+    want32, want64, cands = _oracle_sets(meshes, None)
+    sc, _ = _scene(meshes, None)
+    got64, st = _run(sc, N.PRECISION_FP64_FILTERED)
+    assert np.array_equal(got64, want64), f"{_sym(got64, want64)} mismatches against the FP64 oracle"
+    assert st["candidates"] == cands
+    assert st["fp32_disagreements"] == _sym(want32, want64)
+
+
 def test_precision_argument_checks(gpu):
     from oibvh_gb300 import OibvhError, Scene
 
