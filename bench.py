@@ -51,10 +51,13 @@ REFIT_DRAM_BYTES_PER_TRIANGLE = (372.71e6 + 452.25e6) / 15520000
 # DRAM bytes per vertex of one k_transform_multi launch (ncu, 64 batched pairs:
 # 124.3 MB read, 74.0 MB written for 7,760,256 vertices)
 TRANSFORM_DRAM_BYTES_PER_VERTEX = (124.32e6 + 73.98e6) / 7760256
-# DRAM bytes (read + written) of the traversal kernels (k_begin and the
-# k_walk launches) of one frame per BVTT node pair tested, measured with ncu
-# on 64 batched pairs (206.9 MB per frame, 15,594,052 pairs tested)
-TRAVERSAL_DRAM_BYTES_PER_TESTED = (204.71e6 + 1.54e6 + 0.30e6 + 0.30e6) / 15594052
+# The same of a k_refit launch that moves the vertices as well (12,808,960
+# triangles: 307.6 MB read, 500.3 MB written)
+MOVE_REFIT_DRAM_BYTES_PER_TRIANGLE = (307.60e6 + 500.34e6) / 12808960
+# DRAM bytes (read + written) of the traversal kernels (k_begin, the k_walk
+# launches and k_narrow) of one frame per BVTT node pair tested, measured with
+# ncu on 64 batched pairs (146.1 MB per frame, 12,582,398 pairs tested)
+TRAVERSAL_DRAM_BYTES_PER_TESTED = (6.48e6 + 26.00e6 + 85.46e6 + 28.15e6) / 12582398
 
 
 def parse():
@@ -829,20 +832,26 @@ def frame_rooflines(w, prof, cands, hits, tested, peaks, refit_alone_ms, refit_b
     peak, src = peaks
     tri_total = w.info["triangles_total"]
     broad = sum(24 * (_tree_size(w.rest[a].n_triangles) + _tree_size(w.rest[b].n_triangles)) for a, b in w.pairs)
-    stages = {
-        "transform": ("k_transform_multi (one launch: every vertex of every mesh)",
-                      sum(32 * m.n_vertices + 48 for m in w.rest), prof["transform_ms"],
-                      TRANSFORM_DRAM_BYTES_PER_VERTEX * w.info["vertices_total"],
-                      "16 B in + 16 B out per vertex, 48 B of matrix per mesh"),
-        "refit": ("k_refit (one launch: all trees, leaf boxes + every level)", refit_bytes, prof["refit_ms"],
-                  REFIT_DRAM_BYTES_PER_TRIANGLE * tri_total,
-                  "12 B per vertex + 12 B per face read, 24 B per tree node written (the reference layout; this "
-                  "layout stores internal nodes only, 32 B each, and reads 16 B per face and per vertex)"),
+    moved = sum(32 * m.n_vertices + 48 for m in w.rest)
+    refit_rule = ("12 B per vertex + 12 B per face read, 24 B per tree node written (the reference layout; this "
+                  "layout stores internal nodes only, 32 B each, and reads 16 B per face and per vertex)")
+    stages = {}
+    if prof["transform_ms"] > 0.005:
+        stages["transform"] = ("k_transform_multi (one launch: every vertex of every mesh)", moved, prof["transform_ms"],
+                               TRANSFORM_DRAM_BYTES_PER_VERTEX * w.info["vertices_total"],
+                               "16 B in + 16 B out per vertex, 48 B of matrix per mesh")
+        stages["refit"] = ("k_refit (one launch: all trees, leaf boxes + every level)", refit_bytes, prof["refit_ms"],
+                           REFIT_DRAM_BYTES_PER_TRIANGLE * tri_total, refit_rule)
+    else:  # a large frame: the refit moves the vertices it reads
+        stages["refit"] = ("k_refit (one launch: every vertex moved, all trees' leaf boxes + every level)",
+                           refit_bytes + moved, prof["refit_ms"], MOVE_REFIT_DRAM_BYTES_PER_TRIANGLE * tri_total,
+                           "16 B in + 16 B out per vertex, 48 B of matrix per mesh; " + refit_rule)
+    stages.update({
         "traversal": ("k_begin + k_walk + k_narrow (broad phase, 17-axis narrow phase)",
                       broad + 112 * cands + 8 * hits, prof["start_ms"] + prof["walk_ms"] + prof["narrow_ms"],
                       TRAVERSAL_DRAM_BYTES_PER_TESTED * tested if TRAVERSAL_DRAM_BYTES_PER_TESTED else None,
                       "24 B per node of both trees of every pair + 112 B per candidate + 8 B per hit"),
-    }
+    })
     out = {}
     for name, (kern, b, ms, traffic, rule) in stages.items():
         ach = b / (ms / 1e3) / 1e9
@@ -855,7 +864,7 @@ def frame_rooflines(w, prof, cands, hits, tested, peaks, refit_alone_ms, refit_b
         out[name] = e
     out["refit"]["frac_effective"] = out["refit"]["frac"]
     out["refit"]["alone_ms"] = round(refit_alone_ms, 4)
-    dominant = max(("transform", "refit", "traversal"), key=lambda k: out[k]["launch_ms"])
+    dominant = max(out, key=lambda k: out[k]["launch_ms"])
     top = dict(out[dominant])
     top.update({"stage": dominant, "peak_source": src, "stages": out,
                 "stages_ms_sum": round(sum(prof[k] for k in ("transform_ms", "refit_ms", "start_ms", "walk_ms", "narrow_ms")), 4),

@@ -273,8 +273,9 @@ int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream);
 /* Per-stage device times of one frame (milliseconds, CUDA events on the
  * caller's stream between the stages). */
 typedef struct oibvh_frame_profile {
-    float transform_ms;    /* rigid transforms of every tree (0 without) */
-    float refit_ms;        /* the one refit launch (0 without) */
+    float transform_ms;    /* rigid transforms of every tree (about 0 without, and in frames of 2^20 faces or more
+                            * that are refitted too: the refit's launch does them) */
+    float refit_ms;        /* the one refit launch (about 0 without) */
     float start_ms;        /* counters cleared */
     float walk_ms;         /* the traversal: every walk launch */
     float narrow_ms;       /* the narrow phase where it is a launch of its own (precision mode, large frames; else 0) */

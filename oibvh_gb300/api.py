@@ -282,8 +282,9 @@ class Scene:
 
     def profile_frame(self, stream=None) -> dict:
         """One frame stage by stage with CUDA events between the stages:
-        device milliseconds of transform, refit, start (counters cleared),
-        walk (every walk launch) and narrow; the results are the frame's."""
+        device milliseconds of transform (frames of 2^20 faces or more: part
+        of refit), refit, start (counters cleared), walk (every walk launch)
+        and narrow; the results are the frame's."""
         p = N.FrameProfile()
         N.check(N.lib().oibvh_scene_profile_frame(self._h, _stream_handle(stream), ctypes.byref(p)),
                 "oibvh_scene_profile_frame")

@@ -933,8 +933,7 @@ __device__ __forceinline__ uint32_t find_job(const BuildJob* jobs, uint32_t n, u
     return lo;
 }
 
-// Rigid transforms of every tree: pos = M * rest, M a row-major 3x4 matrix per
-// tree, each product and sum rounded on its own: x' = ((m0 x + m1 y) + m2 z) + m3.
+// Rigid transforms of every tree: pos = M * rest, M a row-major 3x4 matrix per tree.
 // Four 256-vertex blocks per CTA (vertex v of block k at thread v): the four
 // loads are issued before any arithmetic, for more bytes in flight.
 constexpr uint32_t kTransformUnroll = 4;
@@ -957,22 +956,15 @@ __global__ void __launch_bounds__(256, 8) k_transform_multi(const BuildJob* __re
         if (v >= jobs[j].nV) continue;
         jj[k] = j;
         vv[k] = v;
-        // packed rest positions of all jobs (the caller's vertex order: through vperm), or
-        // (rest == nullptr) each job's own source (the tree's order)
+        // packed rest positions of all jobs, in the caller's vertex order (through vperm) or the trees'
         const uint32_t* vp = rest_tree_order ? nullptr : jobs[j].vperm;
-        p[k] = rest ? __ldg(rest + jobs[j].vert_off + (vp ? __ldg(vp + v) : v)) : __ldg(jobs[j].pos + v);
+        p[k] = __ldg(rest + jobs[j].vert_off + (vp ? __ldg(vp + v) : v));
     }
 #pragma unroll
     for (uint32_t k = 0; k < kTransformUnroll; ++k) {
         if (jj[k] == 0xffffffffu) continue;
         const float* m = mats + 12 * (size_t)jj[k];
-        float o[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-            o[r] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(__ldg(m + 4 * r), p[k].x), __fmul_rn(__ldg(m + 4 * r + 1), p[k].y)),
-                                       __fmul_rn(__ldg(m + 4 * r + 2), p[k].z)),
-                             __ldg(m + 4 * r + 3));
-        jobs[jj[k]].pos_out[vv[k]] = make_float4(o[0], o[1], o[2], 0.0f);
+        jobs[jj[k]].pos_out[vv[k]] = rigid_move([&](int i) { return __ldg(m + i); }, p[k]);
     }
 }
 

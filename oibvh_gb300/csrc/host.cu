@@ -1442,8 +1442,9 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
 namespace {
 
 // The frame's work on `st`, as captured: [transform of every tree], [refit
-// of every tree], the detect of every pair (counters cleared, the walk),
-// [the precision narrow phase], the counters to the host. `ev` (optional, 6 events) brackets the stages for per-stage times:
+// of every tree] (large frames: both in one), the detect of every pair (counters
+// cleared, the walk), [a narrow phase of its own], the counters to the host. `ev`
+// (optional, 6 events) brackets the stages for per-stage times:
 // ev[0] | transform | ev[1] | refit | ev[2] | start | ev[3] | walk
 // rounds | ev[4] | narrow | ev[5].
 cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, uint32_t* kernels)
@@ -1455,13 +1456,18 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
         if (ev && e == cudaSuccess) e = cudaEventRecord(ev[i], st);
     };
     mark(0);
-    if (s->frame_rest && e == cudaSuccess) {
+    const bool together = s->frame_rest && s->frame_refit && transform_refit_pays(s->n_faces);
+    if (s->frame_rest && !together && e == cudaSuccess) {
         e = launch_transform_multi(s->build_jobs.p, (uint32_t)s->trees.size(), s->v_blocks, s->vblock_job.p,
                                    s->frame_rest_tree.p, s->frame_mats, true, st);
         ++k;
     }
     mark(1);
-    if (s->frame_refit && e == cudaSuccess) {
+    if (together && e == cudaSuccess) {
+        e = launch_transform_refit(s->refit_jobs.p, (uint32_t)s->trees.size(), s->refit_blocks, s->refit_block_job.p,
+                                   s->tune_refit_log, RefitRest{s->build_jobs.p, s->frame_rest_tree.p, s->frame_mats}, st);
+        ++k;
+    } else if (s->frame_refit && e == cudaSuccess) {
         e = launch_refit(s->refit_jobs.p, (uint32_t)s->trees.size(), s->refit_blocks, s->refit_block_job.p,
                          s->tune_refit_log, st);
         ++k;

@@ -185,6 +185,19 @@ __device__ __forceinline__ Box box_of(const float4& a, const float4& b, const fl
     return Box{gmin(gmin(a.x, b.x), c.x), gmin(gmin(a.y, b.y), c.y), gmin(gmin(a.z, b.z), c.z),
                gmax(gmax(a.x, b.x), c.x), gmax(gmax(a.y, b.y), c.y), gmax(gmax(a.z, b.z), c.z)};
 }
+// A position moved by a row-major 3x4 matrix (m(0) .. m(11)), each product and sum
+// rounded on its own: x' = ((m0 x + m1 y) + m2 z) + m3.
+template <typename M>
+__device__ __forceinline__ float4 rigid_move(M m, const float4& p)
+{
+    auto row = [&](int r) {
+        return __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m(4 * r), p.x), __fmul_rn(m(4 * r + 1), p.y)),
+                                   __fmul_rn(m(4 * r + 2), p.z)),
+                         m(4 * r + 3));
+    };
+    return make_float4(row(0), row(1), row(2), 0.0f);
+}
+
 // Box of one face (v0, v1, v2, .); one 16-byte load per vertex.
 __device__ __forceinline__ Box leaf_box(const float4* __restrict__ pos, uint4 f)
 {

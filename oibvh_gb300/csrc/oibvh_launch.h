@@ -32,6 +32,16 @@ struct RefitSource {
     uint32_t nV;
 };
 
+// Rigid transforms done by the refit that follows them (launch_transform_refit):
+// the trees' transform jobs, one for each refit job, the packed rest positions
+// in the trees' vertex order (nullptr: each job's own source) and the matrices.
+struct BuildJob;
+struct RefitRest {
+    const BuildJob* jobs;
+    const float4* rest;
+    const float* mats;
+};
+
 // One tree of a multi-tree build / transform launch.
 struct BuildJob {
     const float4* pos;      // positions to build from (transform source when no packed rest array is given)
@@ -87,8 +97,7 @@ cudaError_t launch_build(const BuildArgs& a, cudaStream_t s);
 bool build_is_small(uint32_t nT, uint32_t nV);
 cudaError_t launch_build_small(const BuildJob& job, const TreeShape& shape, float4* box, bool wide, cudaStream_t s);
 // rest: packed positions of all jobs in each caller's vertex order (read
-// through the jobs' vperm), or in each tree's order (rest_tree_order), or
-// nullptr (each job's own pos). Writes each job's pos_out.
+// through the jobs' vperm), or in each tree's order (rest_tree_order). Writes each job's pos_out.
 cudaError_t launch_transform_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, const uint32_t* vjob,
                                    const float4* rest, const float* mats, bool rest_tree_order, cudaStream_t s);
 cudaError_t launch_gather_rest_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, const uint32_t* vjob,
@@ -109,6 +118,10 @@ cudaError_t launch_leaf_boxes(const uint4* face, const float4* pos, uint32_t nT,
 // each CTA binary-searches the job table).
 cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks, const uint32_t* block_job,
                          uint32_t group_log2, cudaStream_t s);
+// launch_transform_multi and launch_refit in one
+cudaError_t launch_transform_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks,
+                                   const uint32_t* block_job, uint32_t group_log2, const RefitRest& rest, cudaStream_t s);
+bool transform_refit_pays(uint64_t n_faces);  // whether a captured frame should
 
 // detect_kernels.cu
 struct DetectArgs {

@@ -36,18 +36,30 @@ constexpr int kStageCounters = 64;  // counters per climbing stage and tree (gro
 // vertices each) and take the leaves' corners from the source, so a small
 // tree's refit is one launch (320 triangles: a refit and detect pass 62 to
 // 55 us). Corners cost four loads so instead of one, which larger trees feel.
-template <int kLog, bool kXyz>
+// kRest: the trees are moved first, by `mov`: the CTAs write the moved positions
+// (a slice each) and move the leaves' corners themselves, so the positions are
+// not read back and a launch is saved (12.9 M triangles: 38 us of transforms and
+// 155 of refit become 174; 103 M: 314 and 1249 become 1456).
+//
+// What bounds it: the L1 (70 % busy with gathers and the nodes' 32-byte stores)
+// and the chain of a CTA's few steps; DRAM is at 55 %. Measured against four
+// leaves a thread, 12.9 M triangles at 160 us: two leaves a thread 184, eight 179;
+// 32 neighbouring leaves per load 163; corners that siblings share loaded once 240.
+enum RefitFrom { kOwn = 0, kXyz = 1, kRest = 2 };
+template <int kLog, int kFrom>
 __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
     k_refit(const RefitJob* __restrict__ jobs, uint32_t n_jobs, const uint32_t* __restrict__ block_job,
-            const RefitJob one, const RefitSource src)
+            const RefitJob one, const RefitSource src, const RefitRest mov)
 {
     constexpr uint32_t kRefitLog = kLog, kRefitChunk = 1u << kLog;
     __shared__ Box sm8[(1 << kLog) / 128];
     __shared__ uint32_t s_last;
 
     RefitJob job = one;
+    uint32_t ji = 0;
     if (jobs != nullptr && block_job != nullptr) {
-        job = jobs[__ldg(block_job + blockIdx.x)];
+        ji = __ldg(block_job + blockIdx.x);
+        job = jobs[ji];
     } else if (jobs != nullptr) {
         uint32_t lo = 0, hi = n_jobs - 1;
         while (lo < hi) {
@@ -55,16 +67,33 @@ __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
             if (jobs[mid].block_begin <= blockIdx.x) lo = mid;
             else hi = mid - 1;
         }
+        ji = lo;
         job = jobs[lo];
     }
     const TreeShape S = job.shape;
     const uint32_t chunk = blockIdx.x - job.block_begin;
-    if constexpr (kXyz) {
+    if constexpr (kFrom == kXyz) {
         float4* pos = const_cast<float4*>(job.pos);
         for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < src.nV; v += gridDim.x * blockDim.x) {
             const float* p = src.xyz + 3 * (size_t)(src.vperm ? __ldg(src.vperm + v) : v);
             pos[v] = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), 0.0f);
         }
+    }
+    const float4* corners = job.pos;
+    float m[12] = {};
+    bool moved = false;
+    auto move = [&](const float4& p) { return rigid_move([&](int k) { return m[k]; }, p); };
+    if constexpr (kFrom == kRest) {
+        const BuildJob& b = mov.jobs[ji];
+        const float4* rest = mov.rest ? mov.rest + b.vert_off : b.pos;
+        float4* out = b.pos_out;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) m[k] = __ldg(mov.mats + 12 * (size_t)ji + k);
+        moved = job.pos == out;  // (else the tree is refitted from positions of its own)
+        if (moved) corners = rest;
+        const uint32_t per = ((b.nV + job.n_blocks - 1) / job.n_blocks + 7u) & ~7u;
+        const uint32_t end = min(b.nV, (chunk + 1) * per);
+        for (uint32_t v = chunk * per + threadIdx.x; v < end; v += blockDim.x) out[v] = move(__ldg(rest + v));
     }
     if (S.L == 0) return;  // a single leaf: no internal node
 
@@ -81,12 +110,15 @@ __global__ void __launch_bounds__((1 << kLog) / 4, 1536 / ((1 << kLog) / 4))
     Box v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        if constexpr (kXyz) {
+        if constexpr (kFrom == kXyz) {
             auto corner = [&](uint32_t i) {
                 const float* p = src.xyz + 3 * (size_t)(src.vperm ? __ldg(src.vperm + i) : i);
                 return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), 0.0f);
             };
             v[k] = box_of(corner(f[k].x), corner(f[k].y), corner(f[k].z));
+        } else if constexpr (kFrom == kRest) {
+            const float4 a = __ldg(corners + f[k].x), b = __ldg(corners + f[k].y), c = __ldg(corners + f[k].z);
+            v[k] = moved ? box_of(move(a), move(b), move(c)) : box_of(a, b, c);
         } else {
             v[k] = leaf_box(job.pos, f[k]);
         }
@@ -154,25 +186,45 @@ cudaError_t launch_refit_one(const RefitJob& job, const RefitSource& src, cudaSt
 {
     note_launches(1);
     constexpr uint32_t kThreads = (1u << kRefitLogDefault) / 4;
-    if (src.xyz) k_refit<kRefitLogDefault, true><<<job.n_blocks, kThreads, 0, s>>>(nullptr, 1, nullptr, job, src);
-    else k_refit<kRefitLogDefault, false><<<job.n_blocks, kThreads, 0, s>>>(nullptr, 1, nullptr, job, src);
+    if (src.xyz) k_refit<kRefitLogDefault, kXyz><<<job.n_blocks, kThreads, 0, s>>>(nullptr, 1, nullptr, job, src, RefitRest{});
+    else k_refit<kRefitLogDefault, kOwn><<<job.n_blocks, kThreads, 0, s>>>(nullptr, 1, nullptr, job, src, RefitRest{});
     return cudaGetLastError();
 }
 
-cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks, const uint32_t* block_job,
-                         uint32_t group_log2, cudaStream_t s)
+namespace {
+template <int kFrom>
+cudaError_t launch_many(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks, const uint32_t* block_job,
+                        uint32_t group_log2, const RefitRest& rest, cudaStream_t s)
 {
     if (n_jobs == 0 || total_blocks == 0) return cudaSuccess;
     const RefitJob none{};
     const RefitSource own{};
     note_launches(1);
     switch (group_log2 ? group_log2 : kRefitLogDefault) {
-    case 9: k_refit<9, false><<<total_blocks, 128, 0, s>>>(d_jobs, n_jobs, block_job, none, own); break;
-    case 10: k_refit<10, false><<<total_blocks, 256, 0, s>>>(d_jobs, n_jobs, block_job, none, own); break;
-    case 11: k_refit<11, false><<<total_blocks, 512, 0, s>>>(d_jobs, n_jobs, block_job, none, own); break;
+    case 9: k_refit<9, kFrom><<<total_blocks, 128, 0, s>>>(d_jobs, n_jobs, block_job, none, own, rest); break;
+    case 10: k_refit<10, kFrom><<<total_blocks, 256, 0, s>>>(d_jobs, n_jobs, block_job, none, own, rest); break;
+    case 11: k_refit<11, kFrom><<<total_blocks, 512, 0, s>>>(d_jobs, n_jobs, block_job, none, own, rest); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks, const uint32_t* block_job,
+                         uint32_t group_log2, cudaStream_t s)
+{
+    return launch_many<kOwn>(d_jobs, n_jobs, total_blocks, block_job, group_log2, RefitRest{}, s);
+}
+
+// A captured frame of this many faces or more is moved by its refit; in smaller ones
+// the launch saved is about 2 us, and a frame's profile keeps the two stages apart.
+constexpr uint64_t kTransformRefitFaces = 1u << 20;
+bool transform_refit_pays(uint64_t n_faces) { return n_faces >= kTransformRefitFaces; }
+
+cudaError_t launch_transform_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks,
+                                   const uint32_t* block_job, uint32_t group_log2, const RefitRest& rest, cudaStream_t s)
+{
+    return launch_many<kRest>(d_jobs, n_jobs, total_blocks, block_job, group_log2, rest, s);
 }
 
 cudaError_t launch_leaf_boxes(const uint4* face, const float4* xyz, uint32_t nT, float4* out, cudaStream_t s)

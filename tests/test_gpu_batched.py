@@ -360,3 +360,46 @@ def test_scene_build_launches_do_not_grow_with_trees(gpu):
         return N.lib().oibvh_get_launch_count() - before
 
     assert launches(3) == launches(60)
+
+
+@pytest.mark.parametrize("group", [9, 10, 11])
+@pytest.mark.parametrize("faces", [(1 << 20) - 1, 1 << 20, (1 << 20) + 511])
+def test_frames_of_any_size_move_and_refit(gpu, faces, group):
+    """Frames on both sides of the size from which the refit does the
+    transforms: boxes, positions and pairs as with separate calls, for trees of
+    one triangle up; and a tree refitted from positions of its own."""
+    import torch
+
+    from oibvh_gb300 import DeviceType, OibvhTree, Scene
+    from oibvh_gb300.meshes import Mesh
+
+    rng = np.random.default_rng(faces)
+    sizes = [1, 2, 5, 511, 513, 1025, 4097]
+    sizes.append(faces - sum(sizes))
+    rest, scenes = [], []
+    for n in sizes:
+        at = rng.uniform(0, 1, (n + 2, 3)).astype(np.float32) * np.float32(0.3)
+        rest.append(Mesh(at, (np.arange(n, dtype=np.uint32)[:, None] + np.array([0, 1, 2], dtype=np.uint32)) % np.uint32(n + 2)))
+    for _ in range(2):
+        trees = [OibvhTree(m) for m in rest]
+        sc = Scene()
+        for t in trees:
+            sc.addOibvhTree(t)
+        sc.build()
+        sc.set_pairs([(0, 3), (1, 2), (3, 5)])
+        sc.set_tuning(refit_group_log2=group)
+        scenes.append((sc, trees))
+    packed = torch.from_numpy(np.concatenate([np.pad(m.xyz, ((0, 0), (0, 1))) for m in rest], 0)).cuda()
+    mats = torch.zeros((len(sizes), 12), device="cuda")
+    (a, ta), (b, tb) = scenes
+    a.capture_frame(0, 1, True, packed.data_ptr(), mats.data_ptr())
+    for _ in range(3):
+        mats.copy_(torch.from_numpy(rng.normal(0, 1, (len(sizes), 12)).astype(np.float32)))
+        a.launch_frame()
+        a.finish_frame()
+        b.transform(packed.data_ptr(), mats.data_ptr())
+        b.refit()
+        b.detectCollision(DeviceType.GPU0, 0, 1)
+        assert np.array_equal(a.int_tri_pairs(), b.int_tri_pairs()) and a.candidate_count() == b.candidate_count()
+        for x, y in zip(ta, tb):
+            assert np.array_equal(x.aabb_tree().view(np.uint32), y.aabb_tree().view(np.uint32))
