@@ -105,6 +105,30 @@ __device__ __forceinline__ bool tri_intersect_exact(const V3& P1, const V3& P2, 
     return true;
 }
 
+__device__ __forceinline__ V3 vpick(bool p, const V3& a, const V3& b)
+{
+    return V3{p ? a.x : b.x, p ? a.y : b.y, p ? a.z : b.z};
+}
+// Whether axis k (0, 1: the normals, 2 + 3 i + j: E_i x F_j, 11 + i: E_i x n1,
+// 14 + j: F_j x m1) does not separate: the same arithmetic, for a k of the
+// lane's own. Every axis is a cross product (the normals e1 x e2 and f1 x f2).
+__device__ __forceinline__ bool axis_overlaps(uint32_t k, const V3& P1, const V3& P2, const V3& P3, const V3& Q1,
+                                              const V3& Q2, const V3& Q3)
+{
+    const V3 p1{0.0f, 0.0f, 0.0f};
+    const V3 p2 = vsub(P2, P1), p3 = vsub(P3, P1);
+    const V3 q1 = vsub(Q1, P1), q2 = vsub(Q2, P1), q3 = vsub(Q3, P1);
+    const V3 e1 = vsub(p2, p1), e2 = vsub(p3, p2), e3 = vsub(p1, p3);
+    const V3 f1 = vsub(q2, q1), f2 = vsub(q3, q2), f3 = vsub(q1, q3);
+    const bool pairs = k >= 2u && k < 11u;
+    const uint32_t i = pairs ? (k - 2u) / 3u : k >= 11u ? (k - 11u) % 3u : 0u, j = pairs ? (k - 2u) % 3u : i;
+    const V3 E = vpick(i == 0, e1, vpick(i == 1, e2, e3)), F = vpick(j == 0, f1, vpick(j == 1, f2, f3));
+    const bool of_f = k == 1u || k >= 14u;  // F_j x .. (else E_i x ..)
+    const V3 n = vcross(vpick(of_f, f1, e1), vpick(of_f, f2, e2));  // the normal of that side
+    const V3 c = vcross(vpick(of_f, F, E), vpick(pairs, F, n));
+    return project6(vpick(k < 2u, n, c), p1, p2, p3, q1, q2, q3);
+}
+
 // ---------------------------------------------------------------------------
 // Precision mode: the same 17 tests with an FP64 filter.
 //
@@ -345,16 +369,16 @@ __device__ __forceinline__ void expand_side(const TreeShape& S, uint32_t ia, uin
     count = min(1u << d, right_valid - first + 1u);
 }
 
-// Child x (0, 1) of implicit node i (level l) when `down`, else the node itself
-// (for x = 0); false: there is none (only a level's last node lacks its second
-// child).
-__device__ __forceinline__ bool child_of(const TreeRef& T, uint32_t i, uint32_t l, bool down, uint32_t x, uint32_t& c,
+// Descendant x of implicit node i (level l), d levels down (d = 0: the node
+// itself, for x = 0); false: there is none (x past the 2^d, or past the level's
+// last real node).
+__device__ __forceinline__ bool child_of(const TreeRef& T, uint32_t i, uint32_t l, uint32_t d, uint32_t x, uint32_t& c,
                                          uint32_t& lc)
 {
-    lc = down ? l + 1u : l;
-    c = down ? 2u * i + 1u + x : i;
+    lc = l + d;
+    c = ((i + 1u) << d) - 1u + x;
     // implicit nodes of level lc: [2^lc - 1, 2^(lc+1) - 2 - virtual ones]
-    return down ? c <= (2u << lc) - 2u - (T.vl >> (T.L - lc)) : x == 0;
+    return x >> d == 0 && c <= (2u << lc) - 2u - (T.vl >> (T.L - lc));
 }
 
 // ---------------------------------------------------------------------------
@@ -418,6 +442,39 @@ __device__ __forceinline__ bool test_candidates(const DetectArgs& a, const uint6
     return hit;
 }
 
+// Up to 16 candidates, g = 2, 4, .. 32 lanes each: lane q of a candidate's tests the
+// axes q, q + g, ... What is left in the buffers at a round's end is waited for
+// by every warp: one candidate per lane and its 17 axes take 2 us (a few
+// candidates 4, in two lists), so they take about 1.
+template <bool kOne>
+__device__ __forceinline__ void test_few(const DetectArgs& a, const WarpCands& wc, uint32_t lane)
+{
+    const uint32_t count = wc.n + wc.n_late;
+    const uint32_t lg = 5u - (count > 1u ? 32u - __clz(count - 1u) : 0u), g = 1u << lg, item = lane >> lg;
+    bool over = true;
+    uint4 rec = make_uint4(0, 0, 0, 0);
+    if (item < count) {
+        const uint64_t c = item < wc.n ? wc.buf[item] : wc.late[item - wc.n];
+        const PairView& pv = kOne ? a.one : a.pairs[bvtt_pair(c)];
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, bvtt_pair(c), TA, TB);
+        const uint4 fa = __ldg(TA.face + bvtt_a(c));
+        const uint4 fb = __ldg(TB.face + bvtt_b(c));
+        const V3 P1 = load_vertex(TA.pos, fa.x), P2 = load_vertex(TA.pos, fa.y), P3 = load_vertex(TA.pos, fa.z);
+        const V3 Q1 = load_vertex(TB.pos, fb.x), Q2 = load_vertex(TB.pos, fb.y), Q3 = load_vertex(TB.pos, fb.z);
+        rec = make_uint4(pv.a, pv.b, fa.w, fb.w);
+        for (uint32_t k = lane & (g - 1u); over && k < 17u; k += g) over = axis_overlaps(k, P1, P2, P3, Q1, Q2, Q3);
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, over) >> (item << lg);  // this candidate's lanes
+    const uint32_t all = g == 32u ? 0xffffffffu : (1u << g) - 1u;
+    const bool hit = item < count && (lane & (g - 1u)) == 0 && (m & all) == all;
+    const uint32_t pos = warp_append(a.counts + kCountHits, hit, lane);
+    if (hit) {
+        if (pos < a.hit_cap) a.hits[pos] = rec;
+        else atomicOr(a.counts + kCountFlags, (uint32_t)kFlagHitOverflow);
+    }
+}
+
 // Broad phase only: `count` buffered candidates (one per lane) to the global
 // candidate queue with one atomic for the warp.
 __device__ __forceinline__ void store_candidates(const DetectArgs& a, const uint64_t* buf, uint32_t count,
@@ -457,12 +514,17 @@ __device__ __forceinline__ void take_candidates(const DetectArgs& a, WarpCands& 
 template <bool kFused, bool kOne>
 __device__ __forceinline__ void flush_candidates(const DetectArgs& a, WarpCands& wc, uint32_t lane)
 {
-    if (wc.n > 0) {
-        if constexpr (kFused) test_candidates<kOne, kSatAll>(a, wc.buf, wc.n, lane);
-        else store_candidates(a, wc.buf, wc.n, lane);
+    const uint32_t n = wc.n + wc.n_late;
+    if (kFused && n <= 16) {
+        if (n > 0) test_few<kOne>(a, wc, lane);
+    } else {
+        if (wc.n > 0) {
+            if constexpr (kFused) test_candidates<kOne, kSatAll>(a, wc.buf, wc.n, lane);
+            else store_candidates(a, wc.buf, wc.n, lane);
+        }
+        if constexpr (kFused)
+            if (wc.n_late > 0) test_candidates<kOne, kSatEdges>(a, wc.late, wc.n_late, lane);
     }
-    if constexpr (kFused)
-        if (wc.n_late > 0) test_candidates<kOne, kSatEdges>(a, wc.late, wc.n_late, lane);
     wc.n = wc.n_late = 0;
     __syncwarp();
 }
@@ -571,12 +633,16 @@ __device__ __forceinline__ Expansion expand_test(const DetectArgs& a, WarpCands&
 // them four times over, a scan and loops: 2.2x fewer cycles from a step's start
 // to its end. Warps of small traversals mostly hold fewer than 8 pairs.
 // Returns whether `child` is an overlapping pair to expand next.
-constexpr uint32_t kFewPairs = 8;
+//
+// With e = 2: up to 2 pairs, 16 lanes each and two levels at once: the pairs between
+// are not tested (their boxes contain the children's, so nothing is missed), and a
+// warp with a pair or two, as most in small traversals, is down in half the steps.
+constexpr uint32_t kFewPairs = 8, kDeepPairs = 2;
 template <bool kOne>
-__device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node,
+__device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node, uint32_t e,
                                            uint32_t lane, uint64_t& child, uint32_t& tested)
 {
-    const uint32_t x = (lane >> 1) & 1u, y = lane & 1u;
+    const uint32_t x = (lane >> e) & ((1u << e) - 1u), y = lane & ((1u << e) - 1u);
     bool ov = false, leaves = false, active = false;
     uint64_t cval = 0;
     child = 0;
@@ -589,8 +655,8 @@ __device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, b
         const bool down_a = la != TA.L && (d != kDescendB || lb == TB.L);
         const bool down_b = lb != TB.L && (d != kDescendA || la == TA.L);
         uint32_t ca, lca, cb, lcb;
-        const bool va = child_of(TA, ia, la, down_a, x, ca, lca);
-        const bool vb = child_of(TB, ib, lb, down_b, y, cb, lcb);
+        const bool va = child_of(TA, ia, la, down_a ? min(e, TA.L - la) : 0u, x, ca, lca);
+        const bool vb = child_of(TB, ib, lb, down_b ? min(e, TB.L - lb) : 0u, y, cb, lcb);
         active = va && vb;
         if (active) {
             const Box A = node_box(TA, ca, lca), B = node_box(TB, cb, lcb);
@@ -785,9 +851,11 @@ constexpr uint32_t kClaimMin = 16;
 // leaves faces and then vertices; 1.5 us with few warps busy) times the steps
 // in a row of the busiest warp; DRAM stays below 10 %. So a warp cuts its walk
 // six steps after it has last claimed something and the rest is shared out
-// anew: a barrier costs about 3 us, a warp left alone with a deep subtree tens
+// anew: a barrier costs about 2 us, a warp left alone with a deep subtree tens
 // (2, 4, 6, 8, 12 steps: two meshes of 1.31 M triangles 141, 104, 96, 103, 119 us
-// a detect). Measured, whole detects, against one kernel for the start tests,
+// a detect); three steps after start tests that were dealt out, which leave pairs
+// to one warp in ten (six against three: 1.31 M triangles 77 to 71 us, 24 bodies
+// 72 to 66, 20 k triangles 39 to 36, with pairs taken two levels at once). Measured, whole detects, against one kernel for the start tests,
 // one CTA for the top levels and several launches that each walk to the leaves:
 // two meshes of 20 k triangles 91 to 44 us, of 1.31 M 158 to 79, 24 bodies
 // 115 to 78, a frame of 64 pairs 360 to 270 us for the traversal, of 512
@@ -827,6 +895,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
         bool more = claiming ? n_src > 0 : w < n_src;
         // pairs a warp may queue (the rest goes to the next round): few items, few pairs each
         const uint32_t cap = claiming ? R - 32u : 32u;
+        const uint32_t limit = r == 0 && !claiming ? a.start_steps : a.walk_steps;
         uint32_t head = 0, live = 0, steps = 0, tested = 0;
         for (;;) {
             while (live < 32u && more) {
@@ -859,7 +928,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             bool cut = false;
             // some steps since the last claim (two more with few pairs, which may be about to end):
             // is anything left to claim?
-            if (steps >= a.walk_steps && (live > kFewPairs || steps >= a.walk_steps + 2u)) {
+            if (steps >= limit && (live > kFewPairs || steps >= limit + 2u)) {
                 if (more && claiming) {
                     uint32_t c = 0;
                     if (lane == 0) c = *(volatile uint32_t*)claim;
@@ -881,12 +950,13 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             }
             uint32_t t;
             if (live <= kFewPairs) {
-                const uint64_t node = ring[(head + (lane >> 2)) & mask];
+                const uint32_t e = live <= kDeepPairs ? 2u : 1u, item = lane >> (2u * e);
+                const uint64_t node = ring[(head + item) & mask];
                 const uint32_t n = live;
                 __syncwarp();  // every lane has read its entry before the slots are reused
                 head += n;
                 uint64_t child;
-                const bool keep = expand_few<kOne>(a, wc, (lane >> 2) < n, node, lane, child, t);
+                const bool keep = expand_few<kOne>(a, wc, item < n, node, e, lane, child, t);
                 const uint32_t km = __ballot_sync(0xffffffffu, keep);
                 live = __popc(km);  // at most 32: fits any ring
                 if (keep) ring[(head + __popc(km & ((1u << lane) - 1u))) & mask] = child;

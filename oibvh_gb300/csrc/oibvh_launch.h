@@ -147,7 +147,8 @@ struct DetectArgs {
     int grid;              // CTAs of the grid-stride / persistent kernels
     uint32_t precision;    // 0: float triangle test (reference arithmetic); 1: FP64-filtered
     uint32_t walk_cap;     // per-warp ring entries of the walkers (multiple of 32, <= 512; 0: the default)
-    uint32_t walk_steps = 6;  // steps a warp goes on for when its round has nothing more to claim
+    uint32_t walk_steps = 6;   // steps a warp goes on for when its round has nothing more to claim
+    uint32_t start_steps = 3;  // the same in a round 0 that is dealt out
     uint32_t claim_min = 1;   // a round's pairs are claimed dynamically from this many per warp
     float descend_ratio = kDescendRatio;  // both sides descend while the boxes' squared diagonals are within it
 };

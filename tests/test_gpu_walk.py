@@ -69,3 +69,37 @@ def test_walk_lists_that_overflow_are_regrown(gpu, front):
     want, n = _want(soups)
     sc.detectCollision(DeviceType.GPU0, 0, 1)
     assert np.array_equal(sc.int_tri_pairs(), want) and sc.candidate_count() == n
+
+
+@pytest.mark.parametrize("n_tri", [1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 200])
+def test_few_candidates_on_every_axis(gpu, n_tri):
+    """A round's last candidates, tested by several lanes each: triangles whose
+    float test turns on one axis or another (shared edges, coplanar, lifted)."""
+    from oibvh_gb300 import DeviceType
+    from oibvh_gb300.meshes import Mesh
+    from tests_support import near_degenerate_pair
+
+    a, b = near_degenerate_pair(70 + n_tri, n_tri)
+    soups = [(a.xyz, a.tri), (b.xyz, b.tri)]
+    soups.append(_soup(2 * n_tri, n_tri, 0.1))
+    sc = _scene(soups)
+    want, n = _want(soups)
+    sc.detectCollision(DeviceType.GPU0, 4, 3)
+    assert np.array_equal(sc.int_tri_pairs(), want) and sc.candidate_count() == n
+    sc.set_pairs([(0, 1)])
+    sc.detectCollision(DeviceType.GPU0, 4, 3)
+    assert np.array_equal(sc.int_tri_pairs(), want[(want[:, 0] == 0) & (want[:, 1] == 1)])
+
+
+@pytest.mark.parametrize("sizes", [(1, 9000), (2, 40000), (5, 33000), (16385, 16384), (70000, 300)])
+def test_sparse_trees_two_levels_at_once(gpu, sizes):
+    """Warps with a pair or two, down trees of different depths."""
+    from oibvh_gb300 import DeviceType
+
+    soups = [_soup(n, 40 + i, 0.02) for i, n in enumerate(sizes)]
+    sc = _scene(soups)
+    want, n = _want(soups)
+    for start in (8, 16):
+        sc.set_tuning(start_pairs_log2=start)
+        sc.detectCollision(DeviceType.GPU0, 0, 1)
+        assert np.array_equal(sc.int_tri_pairs(), want) and sc.candidate_count() == n
