@@ -271,20 +271,23 @@ __device__ __forceinline__ uint32_t scan_256(uint32_t v, uint32_t* sh /*[8]*/)
     return pre + x - v;
 }
 
-// One pass of the stable LSD radix sort: a CTA ranks a tile of 4096 items
+// One pass of the stable LSD radix sort: a CTA ranks a tile of 4096 or 2048 items
 // (groups of equal digits in item order), reorders them in shared memory
 // so that each digit's items leave as one run, and writes them behind those of
 // the tree's earlier tiles. kFirst: the values are the item numbers (not read);
 // kLast: the sorted faces are gathered and written with each vertex's first
 // use, instead of keys and values. `swap_hi`: the key written is the item's
 // high word (the pass between the two halves of a 63-bit key).
-constexpr uint32_t kSortThreads = 512, kSortWarps = kSortThreads / 32, kSortItems = kBuildTile / kSortThreads;
+// Builds whose tiles are fewer than the SMs' share cut each in two for the
+// passes (kHalf), so that twice as many CTAs work half as long.
+constexpr uint32_t kSortThreads = 512, kSortWarps = kSortThreads / 32;
 
-template <bool kFirst, bool kLast>
+template <bool kFirst, bool kLast, bool kHalf>
 __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_constant__ BuildArgs a, uint32_t pass, bool swap_hi)
 {
+    constexpr uint32_t kTile = kHalf ? kBuildTile / 2 : kBuildTile, kSortItems = kTile / kSortThreads;
     __shared__ uint16_t s_cnt[kSortWarps][256];
-    __shared__ uint32_t s_key[kBuildTile], s_val[kBuildTile];
+    __shared__ uint32_t s_key[kTile], s_val[kTile];
     __shared__ uint32_t s_base[256], s_start[256], s_sh[8], s_tile, s_bad;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const uint32_t shift = 8 * (pass & 3u);
@@ -297,10 +300,11 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
     if (s_bad) return;
     const uint32_t tile = s_tile;
     uint32_t j;
-    const BuildJob& job = job_of(a, a.ftile_job, tile, j);
-    const uint32_t t0 = tile - job.ftile_begin, n = min(kBuildTile, job.nT - t0 * kBuildTile);
-    const uint32_t* kin = a.sc.keys[pass & 1] + job.face_off + t0 * kBuildTile;
-    const uint32_t* vin = a.sc.vals[pass & 1] + job.face_off + t0 * kBuildTile;
+    const BuildJob& job = job_of(a, a.ftile_job, kHalf ? tile >> 1 : tile, j);
+    const uint32_t chain = kHalf ? 2u * job.ftile_begin : job.ftile_begin, t0 = tile - chain;
+    const uint32_t n = t0 * kTile < job.nT ? min(kTile, job.nT - t0 * kTile) : 0u;  // (a tree's last half may be empty)
+    const uint32_t* kin = a.sc.keys[pass & 1] + job.face_off + t0 * kTile;
+    const uint32_t* vin = a.sc.vals[pass & 1] + job.face_off + t0 * kTile;
     uint32_t* state = a.sc.sort_state[pass & 1];
     uint32_t key[kSortItems], val[kSortItems];
     uint16_t rank[kSortItems];
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
     for (uint32_t r = 0; r < kSortItems; ++r) {
         const uint32_t i = i0 + 32 * r;
         key[r] = i < n ? kin[i] : 0u;
-        val[r] = kFirst ? t0 * kBuildTile + i : i < n ? vin[i] : 0u;
+        val[r] = kFirst ? t0 * kTile + i : i < n ? vin[i] : 0u;
     }
     const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
             uint32_t v[8];
 #pragma unroll
             for (uint32_t q = 0; q < 8; ++q)
-                v[q] = q < k - job.ftile_begin ? ld_state(state + (size_t)(k - q - 1) * 256 + tid) : 0u;
+                v[q] = q < k - chain ? ld_state(state + (size_t)(k - q - 1) * 256 + tid) : 0u;
 #pragma unroll
             for (uint32_t q = 0; q < 8; ++q) {
                 if (done || v[q] == 0) break;
@@ -636,9 +640,9 @@ size_t build_scratch(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t n
     s.hist = (uint32_t*)take((size_t)n_jobs * a.passes * 256 * 4);
     s.order_state = (uint32_t*)take(((size_t)a.f_tiles + a.v_tiles) * 4);
     s.marks = (uint32_t*)take((size_t)a.f_tiles * kTileWords * 4);
-    s.sort_state[0] = (uint32_t*)take((size_t)a.f_tiles * 256 * 4);
+    s.sort_state[0] = (uint32_t*)take((size_t)(a.half_tiles ? 2 : 1) * a.f_tiles * 256 * 4);
     s.zero_bytes = off;
-    s.sort_state[1] = (uint32_t*)take((size_t)a.f_tiles * 256 * 4);
+    s.sort_state[1] = (uint32_t*)take((size_t)(a.half_tiles ? 2 : 1) * a.f_tiles * 256 * 4);
     for (int i = 0; i < 2; ++i) {
         s.keys[i] = (uint32_t*)take((size_t)n_faces * 4);
         s.vals[i] = (uint32_t*)take((size_t)n_faces * 4);
@@ -653,6 +657,15 @@ size_t build_scratch(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t n
     return off;
 }
 
+template <bool kHalf>
+static void launch_sort(const BuildArgs& a, uint32_t p, cudaStream_t s)
+{
+    const uint32_t tiles = kHalf ? 2 * a.f_tiles : a.f_tiles;
+    if (p == 0) k_build_sort<true, false, kHalf><<<tiles, kSortThreads, 0, s>>>(a, p, false);
+    else if (p + 1 < a.passes) k_build_sort<false, false, kHalf><<<tiles, kSortThreads, 0, s>>>(a, p, p == 3);
+    else k_build_sort<false, true, kHalf><<<tiles, kSortThreads, 0, s>>>(a, p, false);
+}
+
 cudaError_t launch_build(const BuildArgs& a, cudaStream_t s)
 {
     cudaError_t e = cudaMemsetAsync(a.sc.fail, 0, a.sc.zero_bytes, s);
@@ -663,9 +676,8 @@ cudaError_t launch_build(const BuildArgs& a, cudaStream_t s)
     if (wide) k_build_codes<true><<<4 * a.f_tiles, 256, 0, s>>>(a);
     else k_build_codes<false><<<4 * a.f_tiles, 256, 0, s>>>(a);
     for (uint32_t p = 0; p < a.passes; ++p) {
-        if (p == 0) k_build_sort<true, false><<<a.f_tiles, kSortThreads, 0, s>>>(a, p, false);
-        else if (p + 1 < a.passes) k_build_sort<false, false><<<a.f_tiles, kSortThreads, 0, s>>>(a, p, p == 3);
-        else k_build_sort<false, true><<<a.f_tiles, kSortThreads, 0, s>>>(a, p, false);
+        if (a.half_tiles) launch_sort<true>(a, p, s);
+        else launch_sort<false>(a, p, s);
     }
     k_build_mark<<<4 * a.v_tiles, 256, 0, s>>>(a);
     k_build_count<<<a.f_tiles + a.v_tiles, 128, 0, s>>>(a);

@@ -71,7 +71,7 @@ struct BuildScratch {
     uint32_t* marks;          // a bit per face corner (sorted faces): a vertex's first use
     uint32_t* counts;         // per word of marks: the tree's marks before it
     uint32_t* unused;         // per 1024 vertices: the tree's unused vertices before them
-    uint32_t* sort_state[2];  // per face tile: 256 look-back states, in turn between passes
+    uint32_t* sort_state[2];  // per sort tile: 256 look-back states, in turn between passes
     size_t zero_bytes;
     uint32_t *keys[2], *vals[2], *hi;  // n_faces each (hi: 63-bit keys only)
     uint32_t *first, *inv, *vperm_new; // n_verts: first-use slot, new number, caller-order map in the new order
@@ -82,6 +82,7 @@ struct BuildArgs {
     BuildJob one;
     const uint32_t *ftile_job, *vtile_job;  // tile -> job
     uint32_t f_tiles, v_tiles;
+    uint32_t half_tiles;    // the sort's tiles are of kBuildTile / 2 faces
     uint32_t passes;        // 4: the reference's 30-bit keys; 8: 63 bits (21 per axis)
     uint32_t* host_error;   // pinned word, set when the build gave up
     BuildScratch sc;

@@ -125,3 +125,18 @@ def test_refits_in_a_row(gpu, n, where):
     for _ in range(2):  # the positions now held, again
         t.refit()
         assert np.array_equal(t.aabb_tree(), got)
+
+
+# the sort's tiles: 2048 faces up to half as many tiles of 4096 as there are SMs, then 4096
+@pytest.mark.parametrize("n", [6143, 6145, 10240, 10241, 311296, 311297, 319488])
+@pytest.mark.parametrize("kind", ["unused", "equal"])
+def test_tree_build_sort_tiles(gpu, n, kind):
+    from oibvh_gb300 import OibvhTree
+
+    xyz, tri = _mesh(n, n, kind)
+    t = OibvhTree(xyz=xyz, tri=tri)
+    for bits in (30, 63):
+        t.set_morton_bits(bits)
+        t.build()
+        _check(t, xyz, tri, bits)
+    assert np.array_equal(t.sorted_faces()[1], _order63(xyz, tri))
