@@ -233,17 +233,25 @@ __global__ void __launch_bounds__(256) k_build_codes(const __grid_constant__ Bui
     }
     __syncthreads();
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) {
-        const uint32_t i = base + k * 256u + threadIdx.x;
-        if (i >= job.nT) continue;
-        const float4 p0 = __ldg(job.pos + f[k][0]), p1 = __ldg(job.pos + f[k][1]), p2 = __ldg(job.pos + f[k][2]);
-        const float va[3] = {p0.x, p0.y, p0.z}, vb[3] = {p1.x, p1.y, p1.z}, vc[3] = {p2.x, p2.y, p2.z};
-        uint32_t lo, hi;
-        leaf_code(va, vb, vc, bmin, bmax, kWide, lo, hi);
-        a.sc.keys[0][job.face_off + i] = lo;
-        if (kWide) a.sc.hi[job.face_off + i] = hi;
+    for (uint32_t h = 0; h < 4; h += 2) {
+        float4 p[2][3];
 #pragma unroll
-        for (uint32_t p = 0; p < P; ++p) atomicAdd(&s_hist[p * 256 + (((p < 4 ? lo : hi) >> (8 * (p & 3))) & 255u)], 1u);
+        for (uint32_t k = 0; k < 2; ++k)
+#pragma unroll
+            for (uint32_t c = 0; c < 3; ++c) p[k][c] = __ldg(job.pos + f[h + k][c]);
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t i = base + (h + k) * 256u + threadIdx.x;
+            if (i >= job.nT) continue;
+            const float va[3] = {p[k][0].x, p[k][0].y, p[k][0].z}, vb[3] = {p[k][1].x, p[k][1].y, p[k][1].z},
+                        vc[3] = {p[k][2].x, p[k][2].y, p[k][2].z};
+            uint32_t lo, hi;
+            leaf_code(va, vb, vc, bmin, bmax, kWide, lo, hi);
+            a.sc.keys[0][job.face_off + i] = lo;
+            if (kWide) a.sc.hi[job.face_off + i] = hi;
+#pragma unroll
+            for (uint32_t p = 0; p < P; ++p) atomicAdd(&s_hist[p * 256 + (((p < 4 ? lo : hi) >> (8 * (p & 3))) & 255u)], 1u);
+        }
     }
     __syncthreads();
     uint32_t* hist = a.sc.hist + (size_t)j * P * 256;
@@ -449,21 +457,34 @@ __device__ __forceinline__ bool lookback(const BuildArgs& a, uint32_t* state, ui
 // (of unused vertices) before its own: a bit per face corner marks the first
 // uses, running counts are kept per 32 corners, and everything that follows
 // works vertex by vertex. (Going through the faces instead, each corner looking
-// up whether it is its vertex's first use, took 361 us for 14 M faces against
-// 64 us for these three kernels.)
+// up whether it is its vertex's first use, took 361 us for 12.9 M faces against
+// 113 us for these three kernels.) What bounds them is chains of loads with little
+// to do in between, so a thread issues those of its four vertices together
+// (k_build_place 71 to 63 us, k_build_apply 159 to 151), and the unused are counted
+// here, where first uses are read anyway (k_build_count 48 to 23).
 __global__ void __launch_bounds__(256) k_build_mark(const __grid_constant__ BuildArgs a)
 {
+    __shared__ uint32_t s_unused;
     if (ld_state(a.sc.fail)) return;
+    if (threadIdx.x == 0) s_unused = 0;
+    __syncthreads();
     uint32_t j;
     const BuildJob& job = job_of(a, a.vtile_job, blockIdx.x >> 2, j);
     const uint32_t base = ((blockIdx.x >> 2) - job.vtile_begin) * kBuildTile + (blockIdx.x & 3u) * 1024u + threadIdx.x;
     uint32_t* marks = a.sc.marks + (size_t)job.ftile_begin * kTileWords;
+    uint32_t n_unused = 0;
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) {
         const uint32_t v = base + 256u * k;
-        const uint32_t s = v < job.nV ? __ldg(a.sc.first + job.vert_off + v) : kNoUse;
+        const uint32_t s = v < job.nV ? __ldg(a.sc.first + job.vert_off + v) : 0u;
+        if (v >= job.nV) continue;
         if (s != kNoUse) atomicOr(marks + (s >> 5), 1u << (s & 31));
+        else ++n_unused;
     }
+    n_unused = __reduce_add_sync(0xffffffffu, n_unused);
+    if ((threadIdx.x & 31) == 0 && n_unused) atomicAdd(&s_unused, n_unused);
+    __syncthreads();
+    if (threadIdx.x == 0) a.sc.unused[blockIdx.x] = s_unused;
 }
 
 // Running counts: CTAs [0, f_tiles) of the marks (per word), the rest of the
@@ -492,10 +513,8 @@ __global__ void __launch_bounds__(128) k_build_count(const __grid_constant__ Bui
             cnt += c[k];
         }
     } else {
-        // thread t: 32 vertices; a warp's 1024 are one block of k_build_place
-        const uint32_t v0 = (tile - chain) * kBuildTile + 32u * tid;
-        const uint32_t* first = a.sc.first + job.vert_off;
-        for (uint32_t k = 0; k < 32 && v0 + k < job.nV; ++k) cnt += __ldg(first + v0 + k) == kNoUse ? 1u : 0u;
+        // a warp: one block (1024 vertices) of k_build_mark and k_build_place
+        if (lane == 0) cnt = a.sc.unused[4 * tile + w];
     }
     uint32_t x = cnt;  // inclusive scan over the CTA
 #pragma unroll
@@ -555,6 +574,14 @@ __global__ void __launch_bounds__(256) k_build_place(const __grid_constant__ Bui
         s[k] = v[k] < job.nV ? __ldg(a.sc.first + job.vert_off + v[k]) : 0u;
         unused |= v[k] < job.nV && s[k] == kNoUse ? 1u << k : 0u;
     }
+    float4 p[4];
+    uint32_t u[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {  // (early: they wait for nothing)
+        const uint32_t at = min(v[k], job.nV - 1u);
+        p[k] = __ldg(job.pos_out + at);
+        u[k] = job.vperm ? __ldg(job.vperm + at) : at;
+    }
     if (__syncthreads_or(unused)) {
         // number the unused ones after the used ones: in vertex order, 256 at a time
         const uint32_t last = job.ftile_begin + (job.nT + kBuildTile - 1) / kBuildTile;
@@ -576,13 +603,15 @@ __global__ void __launch_bounds__(256) k_build_place(const __grid_constant__ Bui
         }
     }
 #pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+        if (!((unused >> k) & 1u))
+            s[k] = __ldg(counts + (s[k] >> 5)) + __popc(__ldg(marks + (s[k] >> 5)) & ((1u << (s[k] & 31)) - 1u));
+#pragma unroll
     for (uint32_t k = 0; k < 4; ++k) {
         if (v[k] >= job.nV) continue;
-        const uint32_t nv = (unused >> k) & 1u ? s[k]
-                                               : __ldg(counts + (s[k] >> 5)) + __popc(__ldg(marks + (s[k] >> 5)) & ((1u << (s[k] & 31)) - 1u));
-        a.sc.inv[job.vert_off + v[k]] = nv;
-        a.sc.pos_new[job.vert_off + nv] = __ldg(job.pos_out + v[k]);
-        a.sc.vperm_new[job.vert_off + nv] = job.vperm ? __ldg(job.vperm + v[k]) : v[k];
+        a.sc.inv[job.vert_off + v[k]] = s[k];
+        a.sc.pos_new[job.vert_off + s[k]] = p[k];
+        a.sc.vperm_new[job.vert_off + s[k]] = u[k];
     }
 }
 
@@ -598,27 +627,40 @@ __global__ void __launch_bounds__(256) k_build_apply(const __grid_constant__ Bui
     const uint32_t base = (block - 4 * (faces ? job.ftile_begin : job.vtile_begin)) * 1024u + threadIdx.x;
     if (faces) {
         const uint32_t* inv = a.sc.inv + job.vert_off;
+        // (all four faces are loaded before the first is written: one chain of loads, not four)
+        uint4 r[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) r[k] = base + 256u * k < job.nT ? job.face_out[base + 256u * k] : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k) {
-            const uint32_t f = base + 256u * k;
-            if (f >= job.nT) break;
-            uint4 r = job.face_out[f];
-            r.x = __ldg(inv + r.x);
-            r.y = __ldg(inv + r.y);
-            r.z = __ldg(inv + r.z);
-            job.face_out[f] = r;
-            uint32_t* t = job.tri_rw + 3 * (size_t)r.w;
-            t[0] = r.x;
-            t[1] = r.y;
-            t[2] = r.z;
+            r[k].x = __ldg(inv + r[k].x);
+            r[k].y = __ldg(inv + r[k].y);
+            r[k].z = __ldg(inv + r[k].z);
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (base + 256u * k >= job.nT) break;
+            job.face_out[base + 256u * k] = r[k];
+            uint32_t* t = job.tri_rw + 3 * (size_t)r[k].w;
+            t[0] = r[k].x;
+            t[1] = r[k].y;
+            t[2] = r[k].z;
         }
     } else {
+        float4 p[4];
+        uint32_t u[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t v = job.vert_off + min(base + 256u * k, job.nV - 1u);
+            p[k] = a.sc.pos_new[v];
+            u[k] = a.sc.vperm_new[v];
+        }
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k) {
             const uint32_t v = base + 256u * k;
             if (v >= job.nV) break;
-            job.pos_out[v] = a.sc.pos_new[job.vert_off + v];
-            job.vperm_out[v] = a.sc.vperm_new[job.vert_off + v];
+            job.pos_out[v] = p[k];
+            job.vperm_out[v] = u[k];
         }
     }
 }
