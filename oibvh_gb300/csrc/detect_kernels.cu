@@ -351,24 +351,6 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool pred, ui
     return base + __popc(mask & ((1u << lane) - 1u));
 }
 
-// Children of implicit node `ia` (level la) `e` levels down, clamped at the
-// leaf level: the first child and the count of real ones
-// (src/cuda/collide.cu:165-176). A leaf is its own only child.
-__device__ __forceinline__ void expand_side(const TreeShape& S, uint32_t ia, uint32_t la, uint32_t e,
-                                            uint32_t& first, uint32_t& count)
-{
-    if (la == S.L) {
-        first = ia;
-        count = 1;
-        return;
-    }
-    const uint32_t nl = min(S.L, la + e);
-    const uint32_t d = nl - la;
-    first = ((ia + 1u) << d) - 1u;
-    const uint32_t right_valid = (2u << nl) - 2u - (S.vl >> (S.L - nl));
-    count = min(1u << d, right_valid - first + 1u);
-}
-
 // Descendant x of implicit node i (level l), d levels down (d = 0: the node
 // itself, for x = 0); false: there is none (x past the 2^d, or past the level's
 // last real node).
@@ -556,75 +538,100 @@ __device__ __forceinline__ void drain_candidates(const DetectArgs& a, WarpCands&
 
 // One BVTT pair per lane, one level down on the sides its key names (both,
 // or the larger box's; a leaf never descends): the up to 2 + 2 boxes (a side
-// that stays contributes its own node) are loaded first (independent loads),
-// the up to 4 child pairs are tested and overlapping leaf pairs become
-// candidates. Returns the overlapping internal child pairs (bit 2x + y: child
-// pair (fa + x, fb + y)) with how each of them expands next (bits 2k, 2k + 1
-// of dm); `tested` gets the warp's number of child pairs tested (lane 0 only).
+// that stays contributes its own node) are loaded first (independent loads)
+// and the up to 4 child pairs are tested. `m`: the overlapping ones (bit 2x + y:
+// first child of A + x, of B + y); child pair k's key is `key` + child_step(k)
+// and, in bits 2k and 2k + 1 of `dm`, how it expands next. Leaf pairs
+// (`leaves`): keys of candidates, with leaf indices. `tested` gets the warp's
+// number of child pairs tested (lane 0 only).
 struct Expansion {
-    uint32_t pair, fa, fb, m, dm;
+    uint64_t key;
+    uint32_t m, dm;
+    bool leaves;
 };
-template <bool kOne>
-__device__ __forceinline__ Expansion expand_test(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node,
-                                                 uint32_t lane, uint32_t& tested)
+__device__ __forceinline__ uint64_t child_step(uint32_t k) { return (uint64_t)(k >> 1) << 24 | (k & 1u); }
+
+// A side of an expansion: the first child (or the node itself), its level, whether
+// there is a second one, and the first's place among the level's real nodes.
+struct Side {
+    uint32_t first, level, real;
+    bool two;
+};
+__device__ __forceinline__ Side side_of(const TreeRef& T, uint32_t i, uint32_t l, bool down)
 {
-    uint32_t pair = 0, fa = 0, fb = 0, na = 0, nb = 0, leaf_a = 0, leaf_b = 0;
-    bool leaves = false, a_leaf = false, b_leaf = false;
-    Box A0{}, A1{}, B0{}, B1{};
+    Side s;
+    s.level = down ? l + 1u : l;
+    s.first = down ? 2u * i + 1u : i;
+    const uint32_t w = T.vl >> (T.L - s.level);  // virtual nodes of the level
+    s.two = down && s.first < (2u << s.level) - 2u - w;
+    s.real = s.first - ((w & ~1u) - __popc(w >> 1));  // less the virtual nodes above it
+    return s;
+}
+
+// Boxes of a side's first child and, where there is one, its second.
+// Leaves: sibling leaves 2j and 2j+1 have adjacent 16-byte face records, read
+// as one 32-byte load (face arrays hold one record past the last face, so the
+// load stays inside the array when the sibling is virtual); an odd leaf index
+// only occurs for a leaf that stays put, read on its own.
+__device__ __forceinline__ void side_boxes(const TreeRef& T, const Side& s, Box& b0, Box& b1)
+{
+    if (s.level == T.L) {
+        const uint32_t i = s.first - ((1u << s.level) - 1u);
+        uint4 f0, f1;
+        if ((i & 1u) == 0) {
+            load_face_pair(T.face + i, f0, f1);
+        } else {
+            f0 = __ldg(T.face + i);
+            f1 = f0;
+        }
+        b0 = leaf_box(T.pos, f0);
+        if (s.two) b1 = leaf_box(T.pos, f1);
+    } else {
+        const float4* p = T.box + 2 * (size_t)s.real;
+        b0 = load_node_nc(p);
+        if (s.two) b1 = load_node_nc(p + 2);  // same level: the next real node
+    }
+}
+
+template <bool kOne>
+__device__ __forceinline__ Expansion expand_test(const DetectArgs& a, bool valid, uint64_t node, uint32_t lane,
+                                                 uint32_t& tested)
+{
+    Expansion e{0, 0, 0, false};
+    uint32_t n = 0;
     if (valid) {
-        pair = bvtt_pair(node);
-        const uint32_t ia = bvtt_a(node), ib = bvtt_b(node);
+        const uint32_t pair = bvtt_pair(node), ia = bvtt_a(node), ib = bvtt_b(node);
         TreeRef TA, TB;
         pair_refs<kOne>(a, pair, TA, TB);
         const uint32_t la = ilog2(ia + 1u), lb = ilog2(ib + 1u);
         // the sides to descend: the key's, never a leaf (a leaf side stays and
         // the other one descends), so every expansion goes one level down
         const uint32_t d = bvtt_desc(node);
-        const bool down_a = la != TA.L && (d != kDescendB || lb == TB.L);
-        const bool down_b = lb != TB.L && (d != kDescendA || la == TA.L);
-        if (down_a) expand_side(TA.shape(), ia, la, 1, fa, na);
-        else fa = ia, na = 1;
-        if (down_b) expand_side(TB.shape(), ib, lb, 1, fb, nb);
-        else fb = ib, nb = 1;
-        const uint32_t lca = ilog2(fa + 1u), lcb = ilog2(fb + 1u);
-        a_leaf = lca == TA.L;
-        b_leaf = lcb == TB.L;
-        leaves = a_leaf && b_leaf;
-        leaf_a = fa - ((1u << lca) - 1u);  // Morton-order leaf index when lca is the leaf level
-        leaf_b = fb - ((1u << lcb) - 1u);
-        node_boxes(TA, fa, lca, na > 1, A0, A1);
-        node_boxes(TB, fb, lcb, nb > 1, B0, B1);
-    }
-    // bit (2x + y): child pair (fa + x, fb + y) overlaps
-    uint32_t m = 0, dm = 0;
-    if (valid) {
-        m |= overlap(A0, B0) ? 1u : 0u;
-        if (nb > 1) m |= overlap(A0, B1) ? 2u : 0u;
-        if (na > 1) m |= overlap(A1, B0) ? 4u : 0u;
-        if (na > 1 && nb > 1) m |= overlap(A1, B1) ? 8u : 0u;
-        if (!leaves) {
+        const Side sa = side_of(TA, ia, la, la != TA.L && (d != kDescendB || lb == TB.L));
+        const Side sb = side_of(TB, ib, lb, lb != TB.L && (d != kDescendA || la == TA.L));
+        Box A0, A1{}, B0, B1{};
+        side_boxes(TA, sa, A0, A1);
+        side_boxes(TB, sb, B0, B1);
+        n = (sa.two ? 2u : 1u) * (sb.two ? 2u : 1u);
+        e.m = (overlap(A0, B0) ? 1u : 0u) | (sb.two && overlap(A0, B1) ? 2u : 0u) | (sa.two && overlap(A1, B0) ? 4u : 0u) |
+              (sa.two && sb.two && overlap(A1, B1) ? 8u : 0u);
+        const bool a_leaf = sa.level == TA.L, b_leaf = sb.level == TB.L;
+        e.leaves = a_leaf && b_leaf;
+        if (e.leaves) {  // leaf indices, in Morton order
+            e.key = bvtt_pack(pair, sa.first - ((1u << sa.level) - 1u), sb.first - ((1u << sb.level) - 1u));
+        } else {
+            e.key = bvtt_pack(pair, sa.first, sb.first);
             const float r = a.descend_ratio;
-            dm |= descend_side(A0, a_leaf, B0, b_leaf, r);
-            if (nb > 1) dm |= descend_side(A0, a_leaf, B1, b_leaf, r) << 2;
-            if (na > 1) dm |= descend_side(A1, a_leaf, B0, b_leaf, r) << 4;
-            if (na > 1 && nb > 1) dm |= descend_side(A1, a_leaf, B1, b_leaf, r) << 6;
+            const float za0 = box_size2(A0), za1 = box_size2(A1), zb0 = box_size2(B0), zb1 = box_size2(B1);
+            e.dm = a_leaf   ? 0x55u * kDescendB
+                   : b_leaf ? 0x55u * kDescendA
+                            : descend_of(za0, zb0, r) | descend_of(za0, zb1, r) << 2 | descend_of(za1, zb0, r) << 4 |
+                                descend_of(za1, zb1, r) << 6;
         }
     }
-    const uint32_t t = __reduce_add_sync(0xffffffffu, na * nb);
+    const uint32_t t = __reduce_add_sync(0xffffffffu, n);
     tested = lane == 0 ? t : 0u;
-    // candidates, one bit per round (at most 4 rounds); every lane joins each round
-    uint32_t cm = leaves ? m : 0u;
-    while (__any_sync(0xffffffffu, cm != 0)) {
-        const bool pred = cm != 0;
-        uint64_t c = 0;
-        if (pred) {
-            const uint32_t k = __ffs(cm) - 1;
-            cm &= cm - 1;
-            c = bvtt_pack(pair, leaf_a + (k >> 1), leaf_b + (k & 1));
-        }
-        push_candidate(wc, pred, c, lane);
-    }
-    return Expansion{pair, fa, fb, leaves ? 0u : m, dm};
+    return e;
 }
 
 // The same for up to 8 pairs, four lanes each: lane 2x + y of an item tests its
@@ -674,14 +681,7 @@ __device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, b
     return ov && !leaves;
 }
 
-// The key of child pair k (bit 2x + y) of an expansion.
-__device__ __forceinline__ uint64_t child_key(const Expansion& e, uint32_t k)
-{
-    return bvtt_pack(e.pair, e.fa + (k >> 1), e.fb + (k & 1), (e.dm >> (2 * k)) & 3u);
-}
-
-// Exclusive prefix over the warp of each lane's child count; `total` = the
-// warp's sum.
+// Exclusive prefix over the warp of each lane's count; `total` = the warp's sum.
 __device__ __forceinline__ uint32_t child_prefix(uint32_t cnt, uint32_t lane, uint32_t& total)
 {
     uint32_t incl = cnt;
@@ -692,29 +692,6 @@ __device__ __forceinline__ uint32_t child_prefix(uint32_t cnt, uint32_t lane, ui
     }
     total = __shfl_sync(0xffffffffu, incl, 31);
     return incl - cnt;
-}
-
-// Children of position `pos` onward go to `slot(pos)` while pos < fit, the
-// rest to the spill list from sbase.
-template <typename Slot>
-__device__ __forceinline__ void write_children(const DetectArgs& a, const Expansion& e, uint32_t pos, uint32_t fit,
-                                               uint64_t* __restrict__ spill, uint32_t sbase, Slot slot)
-{
-    bool overflow = false;
-    uint32_t mm = e.m;
-    while (mm) {
-        const uint32_t k = __ffs(mm) - 1;
-        mm &= mm - 1;
-        const uint64_t child = child_key(e, k);
-        if (pos < fit) *slot(pos) = child;
-        else {
-            const uint32_t sp = sbase + (pos - fit);
-            if (sp < a.work_cap) spill[sp] = child;
-            else overflow = true;
-        }
-        ++pos;
-    }
-    if (overflow) atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
 }
 
 // ---------------------------------------------------------------------------
@@ -847,20 +824,23 @@ constexpr uint32_t kClaimMin = 16;
 // of the warp's ring (one per lane), expands them and appends the overlapping
 // children at the tail, with no barrier between tree levels.
 //
-// What bounds it: the latency of a step's chain (ring entry, boxes, at the
-// leaves faces and then vertices; 1.5 us with few warps busy) times the steps
-// in a row of the busiest warp; DRAM stays below 10 %. So a warp cuts its walk
-// six steps after it has last claimed something and the rest is shared out
-// anew: a barrier costs about 2 us, a warp left alone with a deep subtree tens
-// (2, 4, 6, 8, 12 steps: two meshes of 1.31 M triangles 141, 104, 96, 103, 119 us
-// a detect); three steps after start tests that were dealt out, which leave pairs
-// to one warp in ten (six against three: 1.31 M triangles 77 to 71 us, 24 bodies
-// 72 to 66, 20 k triangles 39 to 36, with pairs taken two levels at once). Measured, whole detects, against one kernel for the start tests,
-// one CTA for the top levels and several launches that each walk to the leaves:
-// two meshes of 20 k triangles 91 to 44 us, of 1.31 M 158 to 79, 24 bodies
-// 115 to 78, a frame of 64 pairs 360 to 270 us for the traversal, of 512
-// pairs 1.52 to 1.50 ms. A queue that idle warps wait on, instead of rounds,
-// was slower (20 k: 112 us): a hand-over costs its giver about 3 us.
+// What bounds it: in small traversals the latency of a step's chain (ring entry,
+// boxes, at the leaves faces and then vertices; 1.1 to 1.5 us) times the steps in
+// a row of the busiest warp; in large ones the instructions (3 us a step with
+// every warp busy; about 450 for 32 pairs, 554 before a side's arithmetic was
+// written out and a step's children and candidates were given their places by one
+// scan: a frame of 64 pairs 228 to 197 us, of 512 pairs 1254 to 1088). DRAM stays
+// below 10 %. A warp cuts its walk six steps after it has last claimed something
+// and the rest is shared out anew: a barrier costs about 2 us, a warp left alone
+// with a deep subtree tens (2, 4, 6, 8, 12 steps: two meshes of 1.31 M triangles
+// 141, 104, 96, 103, 119 us a detect); three steps after start tests that were
+// dealt out, which leave pairs to one warp in ten (six against three: 1.31 M
+// triangles 77 to 71 us, 24 bodies 72 to 66, 20 k triangles 39 to 36, with pairs
+// taken two levels at once). Measured, whole detects, against one kernel for the
+// start tests, one CTA for the top levels and several launches that each walk to
+// the leaves: two meshes of 20 k triangles 91 to 36 us, of 1.31 M 158 to 67, 24
+// bodies 115 to 60. A queue that idle warps wait on, instead of rounds, was slower
+// (20 k: 112 us): a hand-over costs its giver about 3 us.
 template <bool kFused, bool kOne>
 __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32_t total0, uint32_t first, uint32_t last)
 {
@@ -967,16 +947,37 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
                 __syncwarp();
                 head += n;
                 live -= n;
-                const Expansion e = expand_test<kOne>(a, wc, valid, node, lane, t);
+                const Expansion e = expand_test<kOne>(a, valid, node, lane, t);
+                // places for both kinds at once: children in the low half, candidates in the high one
                 uint32_t total;
-                const uint32_t ex = child_prefix((uint32_t)__popc(e.m), lane, total);
-                const uint32_t fit = live < cap ? min(total, cap - live) : 0u;
+                const uint32_t cnt = (uint32_t)__popc(e.m);
+                const uint32_t ex = child_prefix(e.leaves ? cnt << 16 : cnt, lane, total);
+                const uint32_t kids = total & 0xffffu, cands = total >> 16;
+                const uint32_t fit = live < cap ? min(kids, cap - live) : 0u;
                 uint32_t sbase = 0;
-                if (total > fit) {
-                    if (lane == 31) sbase = atomicAdd(spill_cnt, total - fit);
+                if (kids > fit) {
+                    if (lane == 31) sbase = atomicAdd(spill_cnt, kids - fit);
                     sbase = __shfl_sync(0xffffffffu, sbase, 31);
+                    if (sbase + (kids - fit) > a.work_cap && lane == 0) atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
                 }
-                write_children(a, e, ex, fit, spill, sbase, [&](uint32_t p) { return ring + ((head + live + p) & mask); });
+                if (e.leaves) {
+                    uint64_t* to = wc.buf + wc.n + (ex >> 16);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k)
+                        if ((e.m >> k) & 1u) *to++ = e.key + child_step(k);
+                } else {
+                    uint32_t at = ex & 0xffffu;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        if (!((e.m >> k) & 1u)) continue;
+                        const uint64_t child = e.key + child_step(k) + ((uint64_t)((e.dm >> (2 * k)) & 3u) << 48);
+                        if (at < fit) ring[(head + live + at) & mask] = child;
+                        else if (sbase + (at - fit) < a.work_cap) spill[sbase + (at - fit)] = child;
+                        ++at;
+                    }
+                }
+                wc.n += cands;
+                wc.found += cands;
                 live += fit;
             }
             tested += t;

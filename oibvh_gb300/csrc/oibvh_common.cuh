@@ -259,32 +259,6 @@ __device__ __forceinline__ Box node_box(const TreeRef& T, uint32_t implicit, uin
     return load_node_nc(T.box + 2 * (size_t)T.shape().real_index(implicit));
 }
 
-// Boxes of `first` and, when `two`, its right neighbour on the same level.
-// Leaves: sibling leaves 2j and 2j+1 have adjacent 16-byte face records, read
-// as one 32-byte load (face arrays hold one record past the last face, so the
-// load stays inside the array when the sibling is virtual); an odd leaf index
-// only occurs for a leaf that stays put, read on its own.
-__device__ __forceinline__ void node_boxes(const TreeRef& T, uint32_t first, uint32_t level, bool two, Box& b0,
-                                           Box& b1)
-{
-    if (level == T.L) {
-        const uint32_t i = first - ((1u << level) - 1u);
-        uint4 f0, f1;
-        if ((i & 1u) == 0) {
-            load_face_pair(T.face + i, f0, f1);
-        } else {
-            f0 = __ldg(T.face + i);
-            f1 = two ? __ldg(T.face + i + 1) : f0;
-        }
-        b0 = leaf_box(T.pos, f0);
-        if (two) b1 = leaf_box(T.pos, f1);
-    } else {
-        const float4* p = T.box + 2 * (size_t)T.shape().real_index(first);
-        b0 = load_node_nc(p);
-        if (two) b1 = load_node_nc(p + 2);  // same level: the next real node
-    }
-}
-
 // A tree view's first 32 bytes as one 256-bit read-only load (the views are
 // written by the host before the kernels that read them run).
 __device__ __forceinline__ TreeRef load_tree_ref(const TreeView& T)
@@ -327,14 +301,13 @@ __device__ __forceinline__ float box_size2(const Box& b)
     const float x = b.xx - b.nx, y = b.xy - b.ny, z = b.xz - b.nz;
     return x * x + y * y + z * z;
 }
+__device__ __forceinline__ uint32_t descend_of(float sa, float sb, float ratio)
+{
+    return sa > ratio * sb ? kDescendA : sb > ratio * sa ? kDescendB : kDescendBoth;
+}
 __device__ __forceinline__ uint32_t descend_side(const Box& a, bool a_leaf, const Box& b, bool b_leaf, float ratio)
 {
-    if (a_leaf) return kDescendB;
-    if (b_leaf) return kDescendA;
-    const float sa = box_size2(a), sb = box_size2(b);
-    if (sa > ratio * sb) return kDescendA;
-    if (sb > ratio * sa) return kDescendB;
-    return kDescendBoth;
+    return a_leaf ? kDescendB : b_leaf ? kDescendA : descend_of(box_size2(a), box_size2(b), ratio);
 }
 
 // aabb_box_t::overlap (include/utils/utils.h:39-44; src/cuda/collide.cu:12-17)
