@@ -295,7 +295,13 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
 {
     constexpr uint32_t kTile = kHalf ? kBuildTile / 2 : kBuildTile, kSortItems = kTile / kSortThreads;
     __shared__ uint16_t s_cnt[kSortWarps][256];
-    __shared__ uint32_t s_key[kTile], s_val[kTile];
+    __shared__ union {
+        uint32_t peers[kSortWarps][256];  // of a row of 32 items: the lanes with this digit
+        struct {
+            uint32_t key[kTile], val[kTile];
+        } out;
+    } sh;
+    uint32_t *s_key = sh.out.key, *s_val = sh.out.val;
     __shared__ uint32_t s_base[256], s_start[256], s_sh[8], s_tile, s_bad;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const uint32_t shift = 8 * (pass & 3u);
@@ -304,6 +310,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
         s_bad = ld_state(a.sc.fail);
     }
     for (uint32_t i = tid; i < kSortWarps * 128; i += kSortThreads) ((uint32_t*)s_cnt)[i] = 0;
+    for (uint32_t i = tid; i < kSortWarps * 256; i += kSortThreads) (&sh.peers[0][0])[i] = 0;
     __syncthreads();
     if (s_bad) return;
     const uint32_t tile = s_tile;
@@ -328,18 +335,21 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
     for (uint32_t r = 0; r < kSortItems; ++r) {
         const bool valid = i0 + 32 * r < n;
         const uint32_t d = (key[r] >> shift) & 255u;
-        // the valid lanes of the same digit (eight ballots; __match_any_sync was twice as slow a pass)
-        uint32_t peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-        for (uint32_t b = 0; b < 8; ++b) {
-            const uint32_t set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-            peers &= (d >> b) & 1u ? set : ~set;
+        // the row's lanes of the same digit, by a bit each in the digit's word (with eight ballots
+        // instead a pass took 100 us, not 92, for 12.9 M faces; __match_any_sync: 140)
+        if (valid) atomicOr(&sh.peers[w][d], 1u << lane);
+        __syncwarp();
+        uint32_t peers = 0, b = 0;
+        if (valid) {
+            peers = sh.peers[w][d];
+            b = s_cnt[w][d];
         }
-        uint32_t b = 0;
-        if (valid) b = s_cnt[w][d];
         rank[r] = (uint16_t)(b + __popc(peers & lt));
         __syncwarp();
-        if (valid && (peers & lt) == 0) s_cnt[w][d] = (uint16_t)(b + __popc(peers));
+        if (valid && (peers & lt) == 0) {
+            s_cnt[w][d] = (uint16_t)(b + __popc(peers));
+            sh.peers[w][d] = 0;
+        }
         __syncwarp();
     }
     __syncthreads();
