@@ -339,7 +339,7 @@ int walk_grid(const oibvh_scene_s* s, bool fused = true)
     return sm_count(s->device) * std::max(1, per);
 }
 
-int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_t st);
+int size_fp64_setups(oibvh_scene_s* s, uint32_t fp64_list);
 
 // Whether a pass's float narrow phase runs as a kernel of its own after the
 // walk instead of inside it: for several pairs of a million triangles in all.
@@ -380,7 +380,8 @@ int ensure_lists(oibvh_scene_s* s)
 // Broad phase (+ narrow phase unless kDetectBroad) over every pair, pass by pass.
 int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expand, int mode, cudaStream_t st)
 {
-    const bool narrow = mode == kDetectFused;  // narrow phase inside the traversal kernels
+    const bool narrow = mode != kDetectBroad;
+    const bool exact = mode == kDetectSplit;
     if (device_type < 0)
         return fail(OIBVH_ERR_UNSUPPORTED,
                     "device type CPU: the reference's detectCollisionOnCPU is empty; this library has no CPU path");
@@ -391,15 +392,15 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
     DeviceGuard g(s->device);
     struct StaleIfMoved {
         oibvh_scene_s* s;
-        const void* p[6];
+        const void* p[7];
         explicit StaleIfMoved(oibvh_scene_s* sc)
-            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->pairv.p, sc->cand.p}
+            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->pairv.p, sc->cand.p, sc->prec_lists.p}
         {
         }
         ~StaleIfMoved()
         {
-            const void* q[6] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->pairv.p, s->cand.p};
-            for (int i = 0; i < 6; ++i)
+            const void* q[7] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->pairv.p, s->cand.p, s->prec_lists.p};
+            for (int i = 0; i < 7; ++i)
                 if (p[i] != q[i]) s->frame_stale = true;
         }
     } stale_guard(s);
@@ -425,18 +426,22 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         OK_TRY(s->h_hits.ensure(kHostHits, "cudaMallocHost(hits)"));
         OK_TRY(s->h_pairs.ensure(np, "cudaMallocHost(pairs)"));
         OK_TRY(s->pairv.ensure(np, "cudaMalloc(pairs)"));
-        if (np > 1 || !narrow) {  // one pair goes with the walk's arguments; the narrow-phase kernels read the table
+        // one pair goes with the walk's arguments; the narrow-phase kernels read the table
+        if (np > 1 || mode != kDetectFused) {
             CUDA_TRY(cudaStreamSynchronize(st));  // the staging buffer may feed an earlier copy
             std::memcpy(s->h_pairs.p, plan.pv.data(), np * sizeof(PairView));
             CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
         }
         const uint64_t hits_before = s->hit_count;
-        bool split = narrow && split_narrow(s, plan);
+        // (precision mode: the passes follow the walk at once; waiting for its counters first, and copying them
+        // back and forth, took 25 us more for one pair of sheets of 131 k triangles)
+        bool split = exact || (narrow && split_narrow(s, plan));
         for (int attempt = 0;; ++attempt) {
             if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "BVTT queues kept overflowing after regrowing");
             OK_TRY(ensure_lists(s));
-            if (split && s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)") != OIBVH_OK) split = false;
-            if (!narrow) OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
+            if (exact) OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
+            if (exact || !narrow) OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
+            else if (split && s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)") != OIBVH_OK) split = false;
             const bool fused = narrow && !split;
             DetectArgs a{};
             a.pairs = s->pairv.p;
@@ -454,6 +459,9 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.grid = walk_grid(s, fused);
             a.walk_cap = s->tune_walk_cap;
             a.precision = s->precision;
+            a.prec_lists = exact ? s->prec_lists.p : nullptr;
+            a.fp64_tri = exact ? s->fp64_tri.p : nullptr;
+            a.fp64_tri_cap = exact ? s->fp64_tri_cap : 0u;
             a.claim_min = s->tune_claim;
             a.descend_ratio = (float)s->tune_descend;
             const uint32_t front0 = (uint32_t)plan.front0;
@@ -509,6 +517,8 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             s->stats.fp64_axes += c[kCountFp64Axes];
             s->stats.fp64_candidates += c[kCountFp64Cands];
             s->stats.fp32_disagreements += c[kCountDisagree];
+            s->stats.bounded_candidates += (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck];
+            if (exact) OK_TRY(size_fp64_setups(s, c[kCountPrecLeft]));
             s->stats.front_peak = std::max(s->stats.front_peak, peak);
             s->stats.steps = rounds;
             s->cand_count += c[kCountCands];
@@ -519,9 +529,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             break;
         }
         s->stats.passes++;
-        if (mode == kDetectSplit) {
-            OK_TRY(narrow_pass(s, np, hits_before, st));
-        } else if (!narrow) {
+        if (!narrow) {
             if (n_pairs > kMaxPairsPerPass)
                 return fail(OIBVH_ERR_UNSUPPORTED, "the split broad phase handles at most 16384 pairs");
             s->last_pairs = plan.pv;
@@ -549,15 +557,14 @@ int size_fp64_setups(oibvh_scene_s* s, uint32_t fp64_list)
 }
 
 // Narrow phase over the stored candidates of the last broad pass (pairv holds
-// that pass's pair table); hits are appended after the first `hits_before`.
-int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_t st)
+// that pass's pair table).
+int narrow_pass(oibvh_scene_s* s, uint32_t np, cudaStream_t st)
 {
     for (int attempt = 0;; ++attempt) {
         if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "hit queue kept overflowing");
         // counts[kCountCandSlots] still holds the candidate count of the broad phase;
-        // hits (from hits_before), flags and the precision-mode counters are reset
+        // hits, flags and the precision-mode counters are reset
         std::memset(s->h_counts.p, 0, kCountNarrowEnd * sizeof(uint32_t));
-        s->h_counts.p[kCountHits] = (uint32_t)hits_before;
         CUDA_TRY(cudaMemcpyAsync(s->counts.p, s->h_counts.p, 2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(s->counts.p + kCountFp64Axes, s->h_counts.p + kCountFp64Axes,
                                  (kCountNarrowEnd - kCountFp64Axes) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
@@ -586,7 +593,7 @@ int narrow_pass(oibvh_scene_s* s, uint32_t np, uint64_t hits_before, cudaStream_
         const uint32_t* c = s->h_counts.p;
         if (c[kCountFlags] & kFlagHitOverflow) {
             const uint32_t want = grow_cap(c[kCountHits], s->hit_cap);
-            OK_TRY(s->hits.grow_keep(want, hits_before, st, "cudaMalloc(hits)"));
+            OK_TRY(s->hits.ensure(want, "cudaMalloc(hits)"));
             s->hit_cap = want;
             continue;
         }
@@ -607,7 +614,7 @@ int narrow_impl(oibvh_scene_s* s, cudaStream_t st)
     if (!s->cands_valid) return fail(OIBVH_ERR_STATE, "narrow phase needs a broad phase first");
     DeviceGuard g(s->device);
     s->stats.fp64_axes = s->stats.fp64_candidates = s->stats.fp32_disagreements = s->stats.bounded_candidates = 0;
-    return narrow_pass(s, (uint32_t)s->last_pairs.size(), 0, st);
+    return narrow_pass(s, (uint32_t)s->last_pairs.size(), st);
 }
 
 }  // namespace
