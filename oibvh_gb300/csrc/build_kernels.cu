@@ -633,12 +633,17 @@ __global__ void __launch_bounds__(256) k_build_place(const __grid_constant__ Bui
 // the map back into each tree's own buffers.
 __global__ void __launch_bounds__(256) k_build_apply(const __grid_constant__ BuildArgs a)
 {
-    if (ld_state(a.sc.fail)) return;
     const bool faces = blockIdx.x < 4 * a.f_tiles;
     const uint32_t block = faces ? blockIdx.x : blockIdx.x - 4 * a.f_tiles;
     uint32_t j;
     const BuildJob& job = faces ? job_of(a, a.ftile_job, block >> 2, j) : job_of(a, a.vtile_job, block >> 2, j);
     const uint32_t base = (block - 4 * (faces ? job.ftile_begin : job.vtile_begin)) * 1024u + threadIdx.x;
+    if (ld_state(a.sc.fail)) {
+        // the build gave up and its faces may be anything: the refit that follows reads these
+        for (uint32_t k = 0; k < 4 && faces; ++k)
+            if (base + 256u * k < job.nT) job.face_out[base + 256u * k] = make_uint4(0, 0, 0, 0);
+        return;
+    }
     if (faces) {
         const uint32_t* inv = a.sc.inv + job.vert_off;
         // (all four faces are loaded before the first is written: one chain of loads, not four)

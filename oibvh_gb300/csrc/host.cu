@@ -162,10 +162,10 @@ static int tree_build_impl(oibvh_tree_t t, cudaStream_t s)
     OK_TRY(build_impl(a, 1, t->nT, t->nV, t->device, s));
     CUDA_TRY(launch_refit_one(t->job(), RefitSource{}, s));
     CUDA_TRY(cudaStreamSynchronize(s));
-    OK_TRY(build_check(a));
-    t->reordered = true;
-    t->built = true;
-    return OIBVH_OK;
+    const int r = build_check(a);
+    if (r == OIBVH_OK) t->reordered = true;
+    t->built = r == OIBVH_OK;
+    return r;
 }
 
 // ============================================================================
@@ -1221,9 +1221,11 @@ API int oibvh_scene_build(oibvh_scene_t s, void* stream)
     a.v_tiles = s->v_tiles;
     a.passes = wide ? 8 : 4;
     OK_TRY(build_impl(a, n, s->n_faces, s->n_verts, s->device, st));
-    for (auto t : s->trees) {
-        t->reordered = true;
-        t->built = true;
+    std::vector<char> before(n);
+    for (uint32_t i = 0; i < n; ++i) {
+        before[i] = s->trees[i]->reordered;
+        s->trees[i]->reordered = true;
+        s->trees[i]->built = true;
     }
     int r = oibvh_scene_refit(s, stream);
     if (r == OIBVH_OK) {
@@ -1231,7 +1233,10 @@ API int oibvh_scene_build(oibvh_scene_t s, void* stream)
         r = build_check(a);
     }
     if (r != OIBVH_OK)
-        for (auto t : s->trees) t->built = false;
+        for (uint32_t i = 0; i < n; ++i) {
+            s->trees[i]->built = false;
+            if (r == OIBVH_ERR_TIMEOUT) s->trees[i]->reordered = before[i];  // (given up: the old numbers stand)
+        }
     return r;
     GUARD_END
 }
