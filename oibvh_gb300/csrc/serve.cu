@@ -463,7 +463,11 @@ int oibvh_server_s::enqueue_detect(Lane& L)
     a.hit_cap = L.hit_cap;
     a.counts = L.counts.p;
     a.fuse_narrow = 1;
-    a.grid = sm_count(device) * walk_blocks_per_sm();
+    // A lane's share of the CTAs that fit: the walk is a cooperative launch, which starts only when
+    // all of its CTAs do, so with the whole GPU each the lanes' walks queued up (2,000 meshes, four
+    // lanes: 127 k queries/s at most and p99 2.5 ms at 100 k/s; so 150 k, which was all that came,
+    // and 1.0 ms; one batch alone takes as long either way).
+    a.grid = sm_count(device) * std::max(1, walk_blocks_per_sm() / (int)lanes.size());
     CUDA_TRY(launch_begin(a, 0, st));
     CUDA_TRY(launch_walk(a, (uint32_t)L.front0_count, 0, kAllRounds, st));
     // the hits grouped by query (discarded if the batch is redone)
