@@ -332,24 +332,11 @@ uint32_t grow_cap(uint64_t need, uint32_t cur)
     return (uint32_t)c;
 }
 
-int walk_grid(const oibvh_scene_s* s, bool fused = true)
-{
-    const int fit = walk_blocks_per_sm(s->tune_walk_cap, fused);
-    const int per = s->tune_walk_per_sm ? std::min<int>(fit, (int)s->tune_walk_per_sm) : fit;
-    return sm_count(s->device) * std::max(1, per);
-}
-
 int size_fp64_setups(oibvh_scene_s* s, uint32_t fp64_list);
 
-// Whether a pass's float narrow phase runs as a kernel of its own after the
-// walk instead of inside it: for several pairs of a million triangles in all.
-// The walk then carries no triangle test, and the tests run with every lane
-// busy: a frame of 512 pairs 3.13 to 3.06 ms, of 64 pairs 461 to 446 us, of 4
-// pairs 101 to 96 us. Below that, and for one pair, the launch costs what it
-// gives. Without room for the candidates the walk tests them itself.
-bool split_narrow(const oibvh_scene_s* s, const PassPlan& plan)
+// The triangles of a pass's trees, each tree counted once.
+uint64_t pass_triangles(const oibvh_scene_s* s, const PassPlan& plan)
 {
-    if (plan.pv.size() == 1) return false;
     std::vector<bool> seen(s->trees.size(), false);
     uint64_t triangles = 0;
     for (const PairView& v : plan.pv)
@@ -358,7 +345,40 @@ bool split_narrow(const oibvh_scene_s* s, const PassPlan& plan)
                 seen[t] = true;
                 triangles += s->trees[t]->nT;
             }
-    return triangles >= kSplitTriangles;
+    return triangles;
+}
+
+// Whether a pass's float narrow phase runs as a kernel of its own after the
+// walk instead of inside it: for several pairs of a million triangles in all.
+// The walk then carries no triangle test, and the tests run with every lane
+// busy: a frame of 512 pairs 3.13 to 3.06 ms, of 64 pairs 461 to 446 us, of 4
+// pairs 101 to 96 us. Below that, and for one pair, the launch costs what it
+// gives. Without room for the candidates the walk tests them itself.
+bool split_narrow(const PassPlan& plan, uint64_t triangles)
+{
+    return plan.pv.size() > 1 && triangles >= kSplitTriangles;
+}
+
+// CTAs of a pass's walk. A cooperative launch starts only when all of its CTAs
+// do, so a grid for the whole GPU keeps the walks of other streams out: with
+// eight threads, a scene and a stream each, two meshes of 20 k triangles came to
+// 46 k detects/s (62 k with several smaller launches), so to 81 k; of 300 k 24 k
+// (51 k), so to 74 k. Alone, one pair of up to 2^20 triangles loses little by one
+// CTA an SM against all that fit (4): 20 k triangles 32.9 and 34.2 us, 300 k 52.1
+// and 53.9, two coincident meshes of 20 k 64 and 57. Larger ones and several
+// pairs take half: one pair of 1 M triangles 67.7 and 68.5 (73 with one an SM),
+// 24 bodies 61.8 and 64, 32 larger ones 89 and 91 (105), 24 coincident ones 700
+// and 574 (1016). From 2^20 triangles on several pairs take all: 64 pairs 282
+// with two, 237 with all. (A count of CTAs that the caller chose stands.)
+constexpr uint64_t kSmallPair = 1u << 20;
+int walk_grid(const oibvh_scene_s* s, const PassPlan& plan, uint64_t triangles, bool fused)
+{
+    const int fit = std::max(1, walk_blocks_per_sm(s->tune_walk_cap, fused));
+    int per = fit;
+    if (s->tune_walk_per_sm) per = std::min<int>(fit, (int)s->tune_walk_per_sm);
+    else if (!s->precision && plan.pv.size() == 1 && triangles < kSmallPair) per = 1;
+    else if (plan.pv.size() == 1 || triangles < kSplitTriangles) per = std::max(1, fit / 2);
+    return sm_count(s->device) * per;
 }
 
 // How detect_impl runs the narrow phase: fused into the traversal (float
@@ -435,7 +455,8 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         const uint64_t hits_before = s->hit_count;
         // (precision mode: the passes follow the walk at once; waiting for its counters first, and copying them
         // back and forth, took 25 us more for one pair of sheets of 131 k triangles)
-        bool split = exact || (narrow && split_narrow(s, plan));
+        const uint64_t triangles = pass_triangles(s, plan);
+        bool split = exact || (narrow && split_narrow(plan, triangles));
         for (int attempt = 0;; ++attempt) {
             if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "BVTT queues kept overflowing after regrowing");
             OK_TRY(ensure_lists(s));
@@ -456,7 +477,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.hit_cap = s->hit_cap;
             a.counts = s->counts.p;
             a.fuse_narrow = fused ? 1u : 0u;
-            a.grid = walk_grid(s, fused);
+            a.grid = walk_grid(s, plan, triangles, fused);
             a.walk_cap = s->tune_walk_cap;
             a.precision = s->precision;
             a.prec_lists = exact ? s->prec_lists.p : nullptr;
@@ -1543,7 +1564,8 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     }
     PassPlan plan;
     OK_TRY(plan_pass(s, pr.data(), np, s->frame_entry, plan));
-    bool split = s->precision || split_narrow(s, plan);
+    const uint64_t triangles = pass_triangles(s, plan);
+    bool split = s->precision || split_narrow(plan, triangles);
     if (split) {
         // a narrow phase of its own: the candidates of the whole frame are stored
         const uint32_t cap = s->cand_cap;
@@ -1587,7 +1609,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     a.prec_lists = s->precision ? s->prec_lists.p : nullptr;
     a.fp64_tri = s->precision ? s->fp64_tri.p : nullptr;
     a.fp64_tri_cap = s->precision ? s->fp64_tri_cap : 0u;
-    a.grid = walk_grid(s, !split);
+    a.grid = walk_grid(s, plan, triangles, !split);
     a.walk_cap = s->tune_walk_cap;
     a.precision = s->precision;
     a.claim_min = s->tune_claim;
