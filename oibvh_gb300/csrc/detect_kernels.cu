@@ -1258,19 +1258,21 @@ struct WarpList {
 __global__ void __launch_bounds__(kDetectThreads) k_prec_classify(DetectArgs a)
 {
     __shared__ uint4 s_hit[kWarps][64];
-    __shared__ uint2 s_recheck[kWarps][64];
+    __shared__ uint2 s_recheck[kWarps][64], s_other[kWarps][64];
     __shared__ uint32_t s_float[kWarps][64];
     const uint32_t n = min(a.counts[kCountCandSlots], a.cand_cap);
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const PrecLists lists(a);
     WarpList<uint4> hits{s_hit[w]};
-    WarpList<uint2> rechecks{s_recheck[w]};
+    WarpList<uint2> rechecks{s_recheck[w]}, others{s_other[w]};
     WarpList<uint32_t> floats{s_float[w]};
     auto put_hit = [&](uint32_t at, const uint4& rec) {
         if (at < a.hit_cap) a.hits[at] = rec;
         else atomicOr(a.counts + kCountFlags, (uint32_t)kFlagHitOverflow);
     };
+    // (the normals from the front, the other axes from the back: together no more than there are candidates)
     auto put_recheck = [&](uint32_t at, const uint2& e) { lists.recheck[at] = e; };
+    auto put_other = [&](uint32_t at, const uint2& e) { lists.recheck[a.cand_cap - 1u - at] = e; };
     auto put_float = [&](uint32_t at, uint32_t i) { lists.hits[at] = i; };
     for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + lane;
@@ -1292,11 +1294,13 @@ __global__ void __launch_bounds__(kDetectThreads) k_prec_classify(DetectArgs a)
         }
         hits.push(hit, rec, a.counts + kCountHits, lane, put_hit);
         floats.push(to_floats, i, a.counts + kCountPrecHits, lane, put_float);
-        rechecks.push(to_recheck, make_uint2(i, k), a.counts + kCountPrecRecheck, lane, put_recheck);
+        rechecks.push(to_recheck && k < 2u, make_uint2(i, k), a.counts + kCountPrecRecheck, lane, put_recheck);
+        others.push(to_recheck && k >= 2u, make_uint2(i, k), a.counts + kCountPrecOther, lane, put_other);
     }
     if (hits.n > 0) hits.flush(hits.n, a.counts + kCountHits, lane, put_hit);
     if (floats.n > 0) floats.flush(floats.n, a.counts + kCountPrecHits, lane, put_float);
     if (rechecks.n > 0) rechecks.flush(rechecks.n, a.counts + kCountPrecRecheck, lane, put_recheck);
+    if (others.n > 0) others.flush(others.n, a.counts + kCountPrecOther, lane, put_other);
 }
 
 __global__ void __launch_bounds__(kDetectThreads) k_prec_settle(DetectArgs a)
@@ -1577,18 +1581,21 @@ __device__ __forceinline__ float max_abs_diff(const V3& a, const V3& b)
 // candidate is done, else it needs every axis. (Sending them all through the 17
 // bounded axes and then through the double-float pass took 190 us for the
 // 553 k of 16 pairs of sheets, whose margins of 1e-8 to 1e-7 no float bound
-// decides; with this pass 85 us, 57 of them here.) The normals, nearly every axis here, take one cross product with
-// its factors picked by selects.
+// decides; with this pass 62 us, 35 of them here.) Normals take one cross product
+// with its factors picked by selects; they and the other axes are listed from the
+// two ends, so that a warp has one kind (57 us mixed, half the lanes idle).
 __global__ void __launch_bounds__(kDetectThreads) k_prec_recheck(DetectArgs a)
 {
-    const uint32_t n = min(a.counts[kCountPrecRecheck], a.cand_cap);
-    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t n = min(a.counts[kCountPrecRecheck], a.cand_cap), n_other = min(a.counts[kCountPrecOther], a.cand_cap - n);
+    const uint32_t lane = threadIdx.x & 31, rows = (n + 31u) / 32u, all_rows = rows + (n_other + 31u) / 32u;
     const PrecLists lists(a);
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
+    for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < all_rows; row += gridDim.x * (blockDim.x >> 5)) {
+        const bool normals = row < rows;  // a row's lanes have the same kind of axis
+        const uint32_t at = 32u * (normals ? row : row - rows) + lane;
         bool again = false;
         uint2 item = make_uint2(0, 0);
-        if (base + lane < n) {
-            item = lists.recheck[base + lane];
+        if (at < (normals ? n : n_other)) {
+            item = lists.recheck[normals ? at : a.cand_cap - 1u - at];
             V3 P1, P2, P3, Q1, Q2, Q3;
             uint4 rec;
             load_tris(a, a.cand[item.x], P1, P2, P3, Q1, Q2, Q3, rec);
@@ -1605,7 +1612,7 @@ __global__ void __launch_bounds__(kDetectThreads) k_prec_recheck(DetectArgs a)
                 t.q1 = dfb3_rel(Q1, P1);
                 t.q2 = dfb3_rel(Q2, P1);
                 t.q3 = dfb3_rel(Q3, P1);
-                if (item.y < 2) {
+                if (normals) {
                     const bool nrm = item.y == 0;  // n1 = p2 x (p3 - p2), m1 = (q2 - q1) x (q3 - q2)
                     const DFB3 c = dfb3_cross(dfb3_sel(nrm, t.p2, dfb3_sub(t.q2, t.q1)),
                                               dfb3_sub(dfb3_sel(nrm, t.p3, t.q3), dfb3_sel(nrm, t.p2, t.q2)));

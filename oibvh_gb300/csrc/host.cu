@@ -538,7 +538,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             s->stats.fp64_axes += c[kCountFp64Axes];
             s->stats.fp64_candidates += c[kCountFp64Cands];
             s->stats.fp32_disagreements += c[kCountDisagree];
-            s->stats.bounded_candidates += (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck];
+            s->stats.bounded_candidates += (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck] + c[kCountPrecOther];
             if (exact) OK_TRY(size_fp64_setups(s, c[kCountPrecLeft]));
             s->stats.front_peak = std::max(s->stats.front_peak, peak);
             s->stats.steps = rounds;
@@ -624,7 +624,7 @@ int narrow_pass(oibvh_scene_s* s, uint32_t np, cudaStream_t st)
         s->stats.fp64_axes += c[kCountFp64Axes];
         s->stats.fp64_candidates += c[kCountFp64Cands];
         s->stats.fp32_disagreements += c[kCountDisagree];
-        s->stats.bounded_candidates += (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck];
+        s->stats.bounded_candidates += (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck] + c[kCountPrecOther];
         if (s->precision) OK_TRY(size_fp64_setups(s, c[kCountPrecLeft]));
         return OIBVH_OK;
     }
@@ -1702,7 +1702,7 @@ API int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream)
     s->stats.fp64_axes = c[kCountFp64Axes];
     s->stats.fp64_candidates = c[kCountFp64Cands];
     s->stats.fp32_disagreements = c[kCountDisagree];
-    s->stats.bounded_candidates = (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck];
+    s->stats.bounded_candidates = (uint64_t)c[kCountPrecHits] + c[kCountPrecRecheck] + c[kCountPrecOther];
     s->stats.front_peak = c[kCountPeak];
     s->hit_count = c[kCountHits];
     s->h_hits_valid = s->hit_count <= kHostHits;

@@ -174,14 +174,15 @@ constexpr uint32_t kFp64TriRows = 23;
 // BVTT pairs tested, (precision mode) axes evaluated in FP64, candidates with
 // at least one such axis, candidates whose float and FP64 answers differ,
 // the sizes of the float-hit, recheck and FP64 lists of the precision narrow phase
-// of the list its double-float pass leaves to FP64, and of what its recheck
-// leaves to the bounded pass; then the largest list
+// of the list its double-float pass leaves to FP64, of what its recheck
+// leaves to the bounded pass, and of the rechecks of axes other than normals
+// (not counted with the others); then the largest list
 // of a walk round and the rounds walked. Past the words that the host reads:
 // the walk's control words, each on a cache line of its own.
 constexpr uint32_t kCountHits = 0, kCountFlags = 1, kCountCands = 2, kCountCandSlots = 3, kCountTested = 4,
                    kCountFp64Axes = 5, kCountFp64Cands = 6, kCountDisagree = 7, kCountPrecHits = 8,
                    kCountPrecRecheck = 9, kCountPrecFp64 = 10, kCountPrecLeft = 11, kCountPrecAgain = 12,
-                   kCountNarrowEnd = 13, kCountPeak = 13, kCountRounds = 14, kCountHost = 16,
+                   kCountPrecOther = 13, kCountNarrowEnd = 14, kCountPeak = 14, kCountRounds = 15, kCountHost = 16,
                    kCtlRelease = 32,
                    kCtlRound = 64, kCtlRoundWords = 64, kCtlRoundClaim = 32,  // four slots
                    kCountTotal = kCtlRound + 4 * kCtlRoundWords;
