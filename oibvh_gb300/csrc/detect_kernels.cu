@@ -1910,7 +1910,13 @@ cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, ui
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = first != last ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, walk_kernel(a.fuse_narrow, a.n_pairs == 1), a, total0, first, last);
+    for (;;) {
+        e = cudaLaunchKernelEx(&cfg, walk_kernel(a.fuse_narrow, a.n_pairs == 1), a, total0, first, last);
+        // (a stream may have fewer SMs than the device: a smaller grid does the same)
+        if (e != cudaErrorCooperativeLaunchTooLarge || cfg.gridDim.x == 1) return e;
+        cudaGetLastError();
+        cfg.gridDim.x /= 2;
+    }
 }
 
 int walk_blocks_per_sm(uint32_t walk_cap, bool fused)
