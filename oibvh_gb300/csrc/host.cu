@@ -369,14 +369,15 @@ bool split_narrow(const PassPlan& plan, uint64_t triangles)
 // pairs take half: one pair of 1 M triangles 67.7 and 68.5 (73 with one an SM),
 // 24 bodies 61.8 and 64, 32 larger ones 89 and 91 (105), 24 coincident ones 700
 // and 574 (1016). From 2^20 triangles on several pairs take all: 64 pairs 282
-// with two, 237 with all. (A count of CTAs that the caller chose stands.)
-constexpr uint64_t kSmallPair = 1u << 20;
+// with two, 237 with all. (In precision mode one pair takes half from 2^17 triangles on: 131 k
+// each 113 with one an SM, 95 with two. A count of CTAs that the caller chose stands.)
+constexpr uint64_t kSmallPair = 1u << 20, kSmallExactPair = 1u << 17;
 int walk_grid(const oibvh_scene_s* s, const PassPlan& plan, uint64_t triangles, bool fused)
 {
     const int fit = std::max(1, walk_blocks_per_sm(s->tune_walk_cap, fused));
     int per = fit;
     if (s->tune_walk_per_sm) per = std::min<int>(fit, (int)s->tune_walk_per_sm);
-    else if (!s->precision && plan.pv.size() == 1 && triangles < kSmallPair) per = 1;
+    else if (plan.pv.size() == 1 && triangles < (s->precision ? kSmallExactPair : kSmallPair)) per = 1;
     else if (plan.pv.size() == 1 || triangles < kSplitTriangles) per = std::max(1, fit / 2);
     return sm_count(s->device) * per;
 }
@@ -1513,8 +1514,14 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
     if (e == cudaSuccess) e = launch_begin(a, 0, st);
     ++k;
     mark(3);
-    for (uint32_t r = 0; r < s->frame_rounds && e == cudaSuccess; ++r) {  // the last launch walks all rounds left
-        e = launch_walk(a, s->frame_front0, r, r + 1 < s->frame_rounds ? r : kAllRounds, st);
+    // The last launch walks all rounds left, usually none: a cooperative one, so it takes one CTA an SM
+    // and fits beside other streams' kernels (three launches, the last with the whole GPU: frames of 32
+    // pairs from eight threads 4.2 k/s, so 5.1 k; alone 2 us longer for 64 pairs).
+    for (uint32_t r = 0; r < s->frame_rounds && e == cudaSuccess; ++r) {
+        const bool rest = r + 1 == s->frame_rounds;
+        DetectArgs w = a;
+        if (rest) w.grid = std::min(w.grid, sm_count(s->device));
+        e = launch_walk(w, s->frame_front0, r, rest ? kAllRounds : r, st);
         ++k;
     }
     mark(4);
@@ -1617,6 +1624,8 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
 
     s->frame_args = a;
     s->frame_front0 = (uint32_t)plan.front0;
+    // a plain launch for each round that the warm-up frame walked, one launch for what is left
+    s->frame_rounds = std::max(3u, std::min(16u, (uint32_t)s->stats.steps + 1u));
 
     // capture on a private non-blocking stream (the legacy default stream
     // cannot be captured); the graph is launched on the caller's stream
