@@ -9,7 +9,7 @@
 // Here one stable sort of (code, face index) replaces the two payload sorts
 // and the permutation is kept, so faces are gathered once into a 16-byte
 // record (v0, v1, v2, original index). Keys are the reference's 30 bits, or
-// 63 bits (21 per axis) as an option, sorted as two stable 32-bit passes.
+// 63 bits (21 per axis) as an option, sorted 8 bits a pass.
 #include "oibvh_common.cuh"
 #include "oibvh_launch.h"
 #include "refit_device.cuh"

@@ -19,8 +19,8 @@
 // and, 32 at a time, tested inside the traversal (the kernels' <true>
 // instantiation, the float test) or stored for a separate kernel (<false>,
 // fewer registers): k_narrow (float test, split API) or, in precision mode,
-// the FP64-filtered test's passes (k_prec_classify, k_prec_settle,
-// k_prec_fp64_setup, k_prec_fp64).
+// the FP64-filtered test's passes (k_prec_classify, k_prec_recheck,
+// k_prec_settle, k_prec_df, k_prec_fp64_setup, k_prec_fp64).
 //
 // The float triangle test reproduces the reference's CPU arithmetic
 // (src/utils/utils.cpp:71-169, glm scalar dot/cross): every product, sum and

@@ -12,8 +12,8 @@
 //   * arrivals queue FIFO; whenever a lane (a CUDA stream with its own work
 //     lists) is idle and queries are waiting, all waiting queries whose slots
 //     fit in the arena (up to max_batch) form a batch and are launched at
-//     once: one transform launch for all slots, one refit launch for all
-//     slots, one detect for all pairs,
+//     once: one refit launch for all slots, which moves their vertices, one
+//     detect for all pairs,
 //     and the counters copied back; so queries that arrive while earlier
 //     batches are on the GPU are admitted as lanes and memory free up, and
 //     batches on different lanes overlap on the device;
