@@ -640,16 +640,11 @@ __device__ __forceinline__ Expansion expand_test(const DetectArgs& a, bool valid
 // them four times over, a scan and loops: 2.2x fewer cycles from a step's start
 // to its end. Warps of small traversals mostly hold fewer than 8 pairs.
 // Returns whether `child` is an overlapping pair to expand next.
-//
-// With e = 2: up to 2 pairs, 16 lanes each and two levels at once: the pairs between
-// are not tested (their boxes contain the children's, so nothing is missed), and a
-// warp with a pair or two, as most in small traversals, is down in half the steps.
 constexpr uint32_t kFewPairs = 8, kDeepPairs = 2;
 template <bool kOne>
-__device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node, uint32_t e,
-                                           uint32_t lane, uint64_t& child, uint32_t& tested)
+__device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, bool valid, uint64_t node, uint32_t lane,
+                                           uint64_t& child, uint32_t& tested)
 {
-    const uint32_t x = (lane >> e) & ((1u << e) - 1u), y = lane & ((1u << e) - 1u);
     bool ov = false, leaves = false, active = false;
     uint64_t cval = 0;
     child = 0;
@@ -662,8 +657,8 @@ __device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, b
         const bool down_a = la != TA.L && (d != kDescendB || lb == TB.L);
         const bool down_b = lb != TB.L && (d != kDescendA || la == TA.L);
         uint32_t ca, lca, cb, lcb;
-        const bool va = child_of(TA, ia, la, down_a ? min(e, TA.L - la) : 0u, x, ca, lca);
-        const bool vb = child_of(TB, ib, lb, down_b ? min(e, TB.L - lb) : 0u, y, cb, lcb);
+        const bool va = child_of(TA, ia, la, down_a, (lane >> 1) & 1u, ca, lca);
+        const bool vb = child_of(TB, ib, lb, down_b, lane & 1u, cb, lcb);
         active = va && vb;
         if (active) {
             const Box A = node_box(TA, ca, lca), B = node_box(TB, cb, lcb);
@@ -679,6 +674,66 @@ __device__ __forceinline__ bool expand_few(const DetectArgs& a, WarpCands& wc, b
     tested = lane == 0 ? t : 0u;
     push_candidate(wc, ov && leaves, cval, lane);
     return ov && !leaves;
+}
+
+// Up to 2 pairs, 16 lanes each and two levels at once, so that a warp with a
+// pair or two, as most in small traversals, is down in half the steps: lane
+// 4x + y of an item follows child x / 2 of A and then its child x % 2, and so in
+// B. The loads of both levels are issued together, but the pair in between is
+// tested and decides how it descends, as in two steps: a box does not hold its
+// children's where positions are NaN or were set without a refit, and the
+// candidates must not depend on how many pairs a warp happens to hold.
+// Internal nodes only, as two_levels_left() says for the warp: next to the leaves,
+// whose boxes are two loads away, the four boxes of a lane in a row took longer
+// than two steps (two meshes of 1.31 M triangles 72.5 us a detect, 70.7 so; 67.1
+// with the pairs in between not tested).
+template <bool kOne>
+__device__ __forceinline__ bool two_levels_left(const DetectArgs& a, bool valid, uint64_t node)
+{
+    bool left = true;
+    if (valid) {
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, bvtt_pair(node), TA, TB);
+        left = ilog2(bvtt_a(node) + 1u) + 2u < TA.L && ilog2(bvtt_b(node) + 1u) + 2u < TB.L;
+    }
+    return __all_sync(0xffffffffu, left);
+}
+template <bool kOne>
+__device__ __forceinline__ bool expand_two_levels(const DetectArgs& a, bool valid, uint64_t node, uint32_t lane,
+                                                  uint64_t& child, uint32_t& tested)
+{
+    const uint32_t x = (lane >> 2) & 3u, y = lane & 3u;
+    bool ov = false;
+    uint32_t n = 0;  // pairs tested by this lane
+    child = 0;
+    if (valid) {
+        TreeRef TA, TB;
+        pair_refs<kOne>(a, bvtt_pair(node), TA, TB);
+        const uint32_t la = ilog2(bvtt_a(node) + 1u), lb = ilog2(bvtt_b(node) + 1u), d = bvtt_desc(node);
+        uint32_t ca, lca, cb, lcb, ga, lga, gb, lgb;  // the pair in between, and its children
+        const bool va = child_of(TA, bvtt_a(node), la, d != kDescendB, x >> 1, ca, lca);
+        const bool vb = child_of(TB, bvtt_b(node), lb, d != kDescendA, y >> 1, cb, lcb);
+        if (va && vb) {
+            const bool wa = child_of(TA, ca, lca, 1u, x & 1u, ga, lga), wb = child_of(TB, cb, lcb, 1u, y & 1u, gb, lgb);
+            Box A = load_node_nc(TA.box + 2 * (size_t)TA.shape().real_index(ca));
+            Box B = load_node_nc(TB.box + 2 * (size_t)TB.shape().real_index(cb));
+            const Box A2 = load_node_nc(TA.box + 2 * (size_t)TA.shape().real_index(wa ? ga : ca));
+            const Box B2 = load_node_nc(TB.box + 2 * (size_t)TB.shape().real_index(wb ? gb : cb));
+            n = ((x | y) & 1u) == 0 ? 1u : 0u;  // (one lane counts the pair in between)
+            const uint32_t side = descend_side(A, false, B, false, a.descend_ratio);
+            const bool sa = side != kDescendB, sb = side != kDescendA;
+            if (overlap(A, B) && (sa ? wa : (x & 1u) == 0) && (sb ? wb : (y & 1u) == 0)) {
+                ++n;
+                if (sa) A = A2;
+                if (sb) B = B2;
+                ov = overlap(A, B);
+                child = bvtt_pack(bvtt_pair(node), sa ? ga : ca, sb ? gb : cb, descend_side(A, false, B, false, a.descend_ratio));
+            }
+        }
+    }
+    const uint32_t t = __reduce_add_sync(0xffffffffu, n);
+    tested = lane == 0 ? t : 0u;
+    return ov;
 }
 
 // Exclusive prefix over the warp of each lane's count; `total` = the warp's sum.
@@ -930,13 +985,15 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             }
             uint32_t t;
             if (live <= kFewPairs) {
-                const uint32_t e = live <= kDeepPairs ? 2u : 1u, item = lane >> (2u * e);
+                const bool two = live <= kDeepPairs && two_levels_left<kOne>(a, lane >> 4 < live, ring[(head + (lane >> 4)) & mask]);
+                const uint32_t item = lane >> (two ? 4 : 2);
                 const uint64_t node = ring[(head + item) & mask];
                 const uint32_t n = live;
                 __syncwarp();  // every lane has read its entry before the slots are reused
                 head += n;
                 uint64_t child;
-                const bool keep = expand_few<kOne>(a, wc, item < n, node, e, lane, child, t);
+                const bool keep = two ? expand_two_levels<kOne>(a, item < n, node, lane, child, t)
+                                      : expand_few<kOne>(a, wc, item < n, node, lane, child, t);
                 const uint32_t km = __ballot_sync(0xffffffffu, keep);
                 live = __popc(km);  // at most 32: fits any ring
                 if (keep) ring[(head + __popc(km & ((1u << lane) - 1u))) & mask] = child;
