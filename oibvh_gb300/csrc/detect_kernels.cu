@@ -816,7 +816,7 @@ __device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t 
             }
             st_release(release, (uint64_t)(r + 1u) << 32 | next);
             ctl[kCountPeak] = max(ctl[kCountPeak], (uint32_t)w);
-            ctl[kCountRounds] = r + 1u;
+            if ((uint32_t)w > 0) ctl[kCountRounds] = r + 2u;
         } else {
             uint64_t v = 0;
             uint32_t polls = 0;
@@ -910,7 +910,12 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
     uint64_t* ring = s_ring + (size_t)wib * R;
     const uint32_t W = gridDim.x * kWarps;
     const uint32_t w = wib * gridDim.x + blockIdx.x;  // neighbouring items go to different SMs
-    uint32_t n_src = first == 0 ? total0 : min(*(volatile uint32_t*)round_slot(a.counts, first), a.work_cap);
+    const uint32_t listed = first == 0 ? total0 : *(volatile uint32_t*)round_slot(a.counts, first);
+    uint32_t n_src = first == 0 ? total0 : min(listed, a.work_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && listed > 0) {  // (the launch before, of one round, had no barrier to do it)
+        a.counts[kCountRounds] = first + 1u;
+        if (first > 0) a.counts[kCountPeak] = max(a.counts[kCountPeak], listed);
+    }
     for (uint32_t r = first;; ++r) {
         uint32_t* claim = round_slot(a.counts, r) + kCtlRoundClaim;
         uint32_t* spill_cnt = round_slot(a.counts, r + 1);

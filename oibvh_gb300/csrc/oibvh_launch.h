@@ -177,7 +177,7 @@ constexpr uint32_t kFp64TriRows = 23;
 // of the list its double-float pass leaves to FP64, of what its recheck
 // leaves to the bounded pass, and of the rechecks of axes other than normals
 // (not counted with the others); then the largest list
-// of a walk round and the rounds walked. Past the words that the host reads:
+// of a walk round and the rounds that had anything to walk. Past the words that the host reads:
 // the walk's control words, each on a cache line of its own.
 constexpr uint32_t kCountHits = 0, kCountFlags = 1, kCountCands = 2, kCountCandSlots = 3, kCountTested = 4,
                    kCountFp64Axes = 5, kCountFp64Cands = 6, kCountDisagree = 7, kCountPrecHits = 8,

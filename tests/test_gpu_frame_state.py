@@ -1,0 +1,56 @@
+"""What a captured frame reports and what it depends on: its statistics are a
+direct detect's, and calls between frames do not reach into the next one."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _soup(n, seed, size=0.4):
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-1.0, 1.0, (n, 1, 3))
+    xyz = (c + rng.uniform(-size, size, (n, 3, 3))).astype(np.float32).reshape(-1, 3)
+    return xyz, np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+
+
+def _scene(soups):
+    from oibvh_gb300 import OibvhTree, Scene
+
+    trees = [OibvhTree(xyz=x, tri=t) for x, t in soups]
+    sc = Scene()
+    for t in trees:
+        t.build()
+        sc.addOibvhTree(t)
+    return sc, trees
+
+
+def test_frame_statistics_are_the_detects(gpu):
+    """Lists between rounds of the size a direct detect of the same state has:
+    which pairs share a warp depends on their order in the lists, so the sizes
+    agree roughly (a factor of two), not exactly."""
+    from oibvh_gb300 import DeviceType
+
+    sc, _ = _scene([_soup(1500, 1), _soup(1700, 2)])
+    sc.set_tuning(start_pairs_log2=8, walk_front=64)
+    sc.detectCollision(DeviceType.GPU0, 0, 1)
+    direct = sc.stats()
+    assert direct["front_peak"] > 100 and direct["steps"] > 1
+    sc.capture_frame(0, 1, True)
+    sc.launch_frame()
+    sc.finish_frame()
+    frame = sc.stats()
+    assert frame["candidates"] == direct["candidates"] and frame["hits"] == direct["hits"]
+    assert direct["front_peak"] / 2 <= frame["front_peak"] <= 2 * direct["front_peak"]
+    assert abs(frame["steps"] - direct["steps"]) <= 1
+
+
+def test_frame_steps_of_a_single_round(gpu):
+    from oibvh_gb300 import DeviceType
+
+    sc, _ = _scene([_soup(1, 3), _soup(1, 4)])
+    sc.detectCollision(DeviceType.GPU0, 0, 1)
+    assert sc.stats()["steps"] == 1
+    sc.capture_frame(0, 1, True)
+    sc.launch_frame()
+    sc.finish_frame()
+    assert sc.stats()["steps"] == 1 and sc.stats()["front_peak"] == 0
