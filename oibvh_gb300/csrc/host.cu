@@ -1680,6 +1680,7 @@ API int oibvh_scene_launch_frame(oibvh_scene_t s, void* stream)
     if (!s) return fail(OIBVH_ERR_ARG, "scene is NULL");
     DeviceGuard g(s->device);
     if (s->frame_stale || !s->frame_exec) OK_TRY(capture_frame_impl(s, (cudaStream_t)stream));
+    s->h_hits_valid = false;  // the frame writes the pinned records; until it is finished they are read behind its work
     CUDA_TRY(cudaGraphLaunch(s->frame_exec, (cudaStream_t)stream));
     note_launches(s->frame_kernels);
     return OIBVH_OK;
@@ -1740,6 +1741,7 @@ API int oibvh_scene_profile_frame(oibvh_scene_t s, void* stream, oibvh_frame_pro
     } ev;
     for (auto& x : ev.e) CUDA_TRY(cudaEventCreate(&x));
     uint32_t kernels = 0;
+    s->h_hits_valid = false;
     CUDA_TRY(enqueue_frame(s, st, ev.e, &kernels));
     CUDA_TRY(cudaStreamSynchronize(st));
     float ms[5] = {};

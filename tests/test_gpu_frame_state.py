@@ -54,3 +54,33 @@ def test_frame_steps_of_a_single_round(gpu):
     sc.launch_frame()
     sc.finish_frame()
     assert sc.stats()["steps"] == 1 and sc.stats()["front_peak"] == 0
+
+
+def test_pairs_read_while_a_frame_runs_are_whole_records(gpu):
+    """Between launch and finish the count is still the one before, and the
+    records are read behind the frame's work: all of them are the new frame's."""
+    import torch
+
+    sc, trees = _scene([_soup(600, 5, 0.2), _soup(600, 6, 0.2)])
+    sc.capture_frame(0, 1, True)
+
+    def frame(seed):
+        rng = np.random.default_rng(seed)
+        for t in trees:
+            t.set_positions(rng.permutation(_soup(600, seed, 0.2)[0].reshape(600, 9)).reshape(-1, 3))
+            seed += 1
+        sc.launch_frame()
+
+    frame(10)
+    sc.finish_frame()
+    first = sc.int_tri_pairs()
+    assert 0 < first.shape[0] <= 4096
+    torch.cuda._sleep(20_000_000)  # (some 10 ms ahead of the frame on its stream)
+    frame(20)
+    seen = sc.int_tri_pairs()
+    sc.finish_frame()
+    second = sc.int_tri_pairs()
+    assert seen.shape[0] == first.shape[0]
+    got, new = {tuple(r) for r in seen}, {tuple(r) for r in second}
+    assert new != {tuple(r) for r in first}
+    assert len(got & new) == min(len(first), len(second))  # (records past the new count are left over)
