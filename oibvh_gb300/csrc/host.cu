@@ -177,7 +177,8 @@ struct oibvh_scene_s {
     bool all_pairs = true;
     std::vector<uint32_t> pairs;  // flattened (a, b)
 
-    DevBuf<PairView> pairv;
+    DevBuf<PairView> pairv;        // of the last direct pass
+    DevBuf<PairView> frame_pairv;  // of the captured frame: a detect between two frames may start from other levels
     DevBuf<uint64_t> work0, work1, cand;
     DevBuf<uint4> hits;
     DevBuf<uint32_t> counts;
@@ -413,15 +414,15 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
     DeviceGuard g(s->device);
     struct StaleIfMoved {
         oibvh_scene_s* s;
-        const void* p[7];
+        const void* p[6];
         explicit StaleIfMoved(oibvh_scene_s* sc)
-            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->pairv.p, sc->cand.p, sc->prec_lists.p}
+            : s(sc), p{sc->work0.p, sc->work1.p, sc->hits.p, sc->counts.p, sc->cand.p, sc->prec_lists.p}
         {
         }
         ~StaleIfMoved()
         {
-            const void* q[7] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->pairv.p, s->cand.p, s->prec_lists.p};
-            for (int i = 0; i < 7; ++i)
+            const void* q[6] = {s->work0.p, s->work1.p, s->hits.p, s->counts.p, s->cand.p, s->prec_lists.p};
+            for (int i = 0; i < 6; ++i)
                 if (p[i] != q[i]) s->frame_stale = true;
         }
     } stale_guard(s);
@@ -1585,10 +1586,11 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
         }
     }
     if (s->precision) OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
+    OK_TRY(s->frame_pairv.ensure(np, "cudaMalloc(frame pairs)"));
     OK_TRY(s->h_frame_counts.ensure(kCountHost, "cudaMallocHost(frame counts)"));
     CUDA_TRY(cudaStreamSynchronize(st));
     std::memcpy(s->h_pairs.p, plan.pv.data(), np * sizeof(PairView));
-    CUDA_TRY(cudaMemcpyAsync(s->pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(s->frame_pairv.p, s->h_pairs.p, np * sizeof(PairView), cudaMemcpyHostToDevice, st));
     if (s->frame_rest) {
         OK_TRY(ensure_build_jobs(s, st));
         // the graph reads the rest positions in each tree's vertex order: one
@@ -1601,7 +1603,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     CUDA_TRY(cudaStreamSynchronize(st));
 
     DetectArgs a{};
-    a.pairs = s->pairv.p;
+    a.pairs = s->frame_pairv.p;
     a.n_pairs = np;
     a.one = plan.pv[0];
     a.work[0] = s->work0.p;

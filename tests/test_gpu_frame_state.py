@@ -84,3 +84,22 @@ def test_pairs_read_while_a_frame_runs_are_whole_records(gpu):
     got, new = {tuple(r) for r in seen}, {tuple(r) for r in second}
     assert new != {tuple(r) for r in first}
     assert len(got & new) == min(len(first), len(second))  # (records past the new count are left over)
+
+
+@pytest.mark.parametrize("captured,between", [(0, 6), (6, 0), (0, 9), (9, 4)])
+@pytest.mark.parametrize("call", ["detect", "broad"])
+def test_a_detect_from_another_level_leaves_the_frame_alone(gpu, captured, between, call):
+    from oibvh_gb300 import DeviceType
+
+    soups = [_soup(n, 30 + n, 0.2) for n in (700, 900, 1100)]
+    sc, _ = _scene(soups)
+    sc.set_tuning(start_pairs_log2=8)
+    sc.detectCollision(DeviceType.GPU0, captured, 1)
+    want, n = sc.int_tri_pairs(), sc.candidate_count()
+    sc.capture_frame(captured, 1, True)
+    for _ in range(2):
+        sc.launch_frame()
+        sc.finish_frame()
+        assert np.array_equal(sc.int_tri_pairs(), want) and sc.candidate_count() == n
+        getattr(sc, "detectCollision" if call == "detect" else "broad")(DeviceType.GPU0, between, 1)
+        assert sc.candidate_count() == n
