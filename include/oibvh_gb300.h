@@ -260,7 +260,8 @@ int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t reps, o
  * 16384 pairs, results to pinned memory).
  * capture_frame runs one ordinary frame first (it sizes the queues with 2x
  * headroom and uploads the tables), then captures. launch_frame replays the
- * graph (re-capturing first if the scene or tuning changed); finish_frame
+ * graph (re-capturing first if the scene or tuning changed, or a tree was
+ * built anew: the rest positions are then copied again); finish_frame
  * waits for it and validates: if a queue overflowed, it reruns the detect the
  * synchronous way and marks the graph for re-capture, so results are always
  * complete. Matrix contents at d_mats may change between launches; the rest

@@ -38,6 +38,7 @@ namespace oibvh_host {
 thread_local std::string g_last_error;
 std::atomic<int64_t> g_fail_alloc{-1};
 std::atomic<uint64_t> g_alloc_attempts{0};
+std::atomic<uint64_t> g_builds{0};
 }  // namespace oibvh_host
 
 static int tree_alloc(oibvh_tree_t t)
@@ -147,6 +148,7 @@ static int tree_build_impl(oibvh_tree_t t, cudaStream_t s)
     DeviceGuard g(t->device);
     OK_TRY(t->vperm.ensure(t->nV, "cudaMalloc(vertex order)"));
     OK_TRY(sync_positions(t, s));
+    t->begin_build();
     if (build_is_small(t->nT, t->nV)) {
         CUDA_TRY(launch_build_small(t->build_job(), t->shape, t->box.p, t->morton_bits == 63, s));
         CUDA_TRY(cudaStreamSynchronize(s));
@@ -225,6 +227,8 @@ struct oibvh_scene_s {
     // captured frame (CUDA graph): [transform] + refit + detect
     cudaGraphExec_t frame_exec = nullptr;
     bool frame_stale = true;
+    uint64_t frame_builds = 0;  // the trees' builds at the capture
+    uint64_t frame_builds_seen = 0;  // g_builds when they were last added up
     uint32_t frame_entry = 0, frame_expand = 1, frame_rounds = 3, frame_kernels = 0, frame_redos = 0;
     bool frame_refit = true;
     const float4* frame_rest = nullptr;
@@ -1243,6 +1247,7 @@ API int oibvh_scene_build(oibvh_scene_t s, void* stream)
     a.f_tiles = s->f_tiles;
     a.v_tiles = s->v_tiles;
     a.passes = wide ? 8 : 4;
+    for (auto t : s->trees) t->begin_build();
     OK_TRY(build_impl(a, n, s->n_faces, s->n_verts, s->device, st));
     std::vector<char> before(n);
     for (uint32_t i = 0; i < n; ++i) {
@@ -1546,9 +1551,17 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
     return e;
 }
 
+uint64_t tree_builds(const oibvh_scene_s* s)
+{
+    uint64_t n = 0;
+    for (auto t : s->trees) n += t->builds;
+    return n;
+}
+
 // Capture [transform] + refit + detect of every pair (one pass) into a graph.
 int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
 {
+    const uint64_t seen = g_builds.load(std::memory_order_relaxed);
     if (s->frame_exec) {
         cudaGraphExecDestroy(s->frame_exec);
         s->frame_exec = nullptr;
@@ -1651,8 +1664,23 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     }
     s->frame_kernels = kernels;
     s->frame_stale = false;
+    s->frame_builds_seen = seen;
+    s->frame_builds = tree_builds(s);
     s->last_pairs = plan.pv;
     return OIBVH_OK;
+}
+
+// The graph captured again where it no longer fits the scene: queues moved, settings
+// changed, or a tree was built anew, whose vertices (the order of the captured rest
+// positions) then have other numbers.
+int refresh_frame(oibvh_scene_s* s, cudaStream_t st)
+{
+    const uint64_t seen = g_builds.load(std::memory_order_relaxed);
+    if (!s->frame_stale && s->frame_exec && seen != s->frame_builds_seen) {
+        if (tree_builds(s) != s->frame_builds) s->frame_stale = true;
+        s->frame_builds_seen = seen;
+    }
+    return s->frame_stale || !s->frame_exec ? capture_frame_impl(s, st) : OIBVH_OK;
 }
 
 }  // namespace
@@ -1681,7 +1709,7 @@ API int oibvh_scene_launch_frame(oibvh_scene_t s, void* stream)
     GUARD_BEGIN
     if (!s) return fail(OIBVH_ERR_ARG, "scene is NULL");
     DeviceGuard g(s->device);
-    if (s->frame_stale || !s->frame_exec) OK_TRY(capture_frame_impl(s, (cudaStream_t)stream));
+    OK_TRY(refresh_frame(s, (cudaStream_t)stream));
     s->h_hits_valid = false;  // the frame writes the pinned records; until it is finished they are read behind its work
     CUDA_TRY(cudaGraphLaunch(s->frame_exec, (cudaStream_t)stream));
     note_launches(s->frame_kernels);
@@ -1732,7 +1760,7 @@ API int oibvh_scene_profile_frame(oibvh_scene_t s, void* stream, oibvh_frame_pro
     if (!s || !out) return fail(OIBVH_ERR_ARG, "scene or out is NULL");
     DeviceGuard g(s->device);
     cudaStream_t st = (cudaStream_t)stream;
-    if (s->frame_stale || !s->frame_exec) OK_TRY(capture_frame_impl(s, st));
+    OK_TRY(refresh_frame(s, st));
     struct Events {
         cudaEvent_t e[6] = {};
         ~Events()

@@ -24,6 +24,8 @@ extern thread_local std::string g_last_error;
 // cudaErrorMemoryAllocation without calling CUDA, then the hook is off again.
 extern std::atomic<int64_t> g_fail_alloc;
 extern std::atomic<uint64_t> g_alloc_attempts;  // device + pinned allocation attempts
+// Builds begun of any tree: a captured frame looks its trees over only when it has changed.
+extern std::atomic<uint64_t> g_builds;
 inline bool injected_alloc_failure()
 {
     g_alloc_attempts.fetch_add(1, std::memory_order_relaxed);
@@ -245,8 +247,14 @@ struct oibvh_tree_s {
     DevBuf<float4> box;         // 2 * (size - nT): internal nodes only
     DevBuf<uint32_t> counters;  // refit climbing counters
     bool built = false;
+    uint32_t builds = 0;        // builds begun: each may renumber the vertices
     uint32_t morton_bits = 30;  // 30 (the reference's key) or 63 (21 bits per axis)
 
+    void begin_build()
+    {
+        ++builds;
+        g_builds.fetch_add(1, std::memory_order_relaxed);
+    }
     const uint32_t* vmap() const { return reordered ? vperm.p : nullptr; }
 
     // this tree alone (a scene sets the first tiles and offsets)

@@ -103,3 +103,39 @@ def test_a_detect_from_another_level_leaves_the_frame_alone(gpu, captured, betwe
         assert np.array_equal(sc.int_tri_pairs(), want) and sc.candidate_count() == n
         getattr(sc, "detectCollision" if call == "detect" else "broad")(DeviceType.GPU0, between, 1)
         assert sc.candidate_count() == n
+
+
+@pytest.mark.parametrize("by", ["scene", "tree"])
+@pytest.mark.parametrize("n", [300, 6000])
+def test_a_build_between_frames_is_followed(gpu, by, n):
+    """A build renumbers the vertices: the rest positions that a frame moves
+    have to be in the new order."""
+    import torch
+
+    from oibvh_gb300 import DeviceType
+
+    soups = [_soup(n, 50 + i, 0.1) for i in range(3)]
+    packed = torch.from_numpy(np.concatenate([np.pad(x, ((0, 0), (0, 1))) for x, _ in soups], 0)).cuda()
+    mats = torch.tensor(np.tile(np.eye(3, 4, dtype=np.float32).reshape(12), (3, 1))).cuda()
+    sc, trees = _scene(soups)
+    sc.capture_frame(0, 1, True, packed.data_ptr(), mats.data_ptr())
+    other, _ = _scene(soups)
+    rng = np.random.default_rng(n)
+    for _ in range(2):
+        # the order depends on the positions built from: others than at the capture
+        moved = [rng.permutation(x.reshape(-1, 9)).reshape(-1, 3).copy() for x, _ in soups]
+        for t, x in zip(trees, moved):
+            t.set_positions(x)
+        if by == "scene":
+            sc.build()
+        else:
+            trees[1].build()
+        mats.copy_(torch.from_numpy(rng.normal(0, 0.6, (3, 12)).astype(np.float32)))
+        sc.launch_frame()
+        sc.finish_frame()
+        other.transform(packed.data_ptr(), mats.data_ptr())
+        other.refit()
+        other.detectCollision(DeviceType.GPU0, 0, 1)
+        want = other.int_tri_pairs()
+        assert want.shape[0] > 0 and np.array_equal(sc.int_tri_pairs(), want)
+        assert sc.candidate_count() == other.candidate_count()
