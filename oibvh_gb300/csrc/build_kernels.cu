@@ -962,16 +962,17 @@ bool build_is_small(uint32_t nT, uint32_t nV) { return nT <= kSmallMax && nV <= 
 
 cudaError_t launch_build_small(const BuildJob& job, const TreeShape& shape, float4* box, bool wide, cudaStream_t s)
 {
-    static std::atomic<bool> configured[64];
+    static std::atomic<unsigned long long> configured[64];  // the context it was done for
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+    const unsigned long long ctx = current_context_id();
+    if (dev < 0 || dev >= 64 || ctx == 0 || configured[dev].load(std::memory_order_acquire) != ctx) {
         e = cudaFuncSetAttribute(k_build_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared));
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_build_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared));
         if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+        if (dev >= 0 && dev < 64) configured[dev].store(ctx, std::memory_order_release);
     }
     note_launches(1);
     if (wide) k_build_small<true><<<1, kSmallThreads, sizeof(SmallShared), s>>>(job, shape, box);

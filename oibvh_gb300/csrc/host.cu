@@ -18,6 +18,8 @@
 #include <cstdio>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -32,6 +34,25 @@ using namespace oibvh;
 namespace oibvh {
 static std::atomic<uint64_t> g_launches{0};
 void note_launches(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+// cuCtxGetId through the runtime's driver entry point (no link to libcuda).
+typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
+
+// Id of the current context (0 when it cannot be read).
+unsigned long long current_context_id()
+{
+    static CtxGetIdFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return (CtxGetIdFn) nullptr;
+        return (CtxGetIdFn)f;
+    }();
+    unsigned long long id = 0;
+    if (!fn || fn(nullptr, &id) != 0) return 0;
+    return id;
+}
 }  // namespace oibvh
 
 namespace oibvh_host {
@@ -39,6 +60,49 @@ thread_local std::string g_last_error;
 std::atomic<int64_t> g_fail_alloc{-1};
 std::atomic<uint64_t> g_alloc_attempts{0};
 std::atomic<uint64_t> g_builds{0};
+}  // namespace oibvh_host
+
+// What builds keep between calls, for each context they have run in (gone with it).
+struct BuildContext {
+    cudaMemPool_t pool = nullptr;
+    uint32_t* errors = nullptr;  // a pinned page of error words
+    uint32_t next = 0;
+};
+static std::mutex g_build_mu;
+static std::map<unsigned long long, BuildContext> g_build_contexts;
+
+// The current context's id, with a context made where this thread has none yet.
+static unsigned long long context_id()
+{
+    unsigned long long id = current_context_id();
+    if (id == 0) {
+        cudaFree(nullptr);
+        id = current_context_id();
+    }
+    return id;
+}
+
+namespace oibvh_host {
+cudaMemPool_t scratch_pool(int dev)
+{
+    std::lock_guard<std::mutex> lock(g_build_mu);
+    BuildContext& c = g_build_contexts[context_id()];
+    if (!c.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        uint64_t keep = 512ull << 20;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        c.pool = pool;
+    }
+    return c.pool;
+}
 }  // namespace oibvh_host
 
 static int tree_alloc(oibvh_tree_t t)
@@ -106,16 +170,17 @@ static int sync_positions(oibvh_tree_t t, cudaStream_t s)
 }
 
 // A pinned word per build that a build kernel sets when it gives up (a wait
-// that ran out). The words outlive the builds: one page, taken in turn.
+// that ran out). The words outlive the builds: one page a context, taken in turn.
 static uint32_t* build_error_word()
 {
-    static uint32_t* page = [] {
+    std::lock_guard<std::mutex> lock(g_build_mu);
+    BuildContext& c = g_build_contexts[context_id()];
+    if (!c.errors) {
         void* p = nullptr;
-        return cudaHostAlloc(&p, 4096, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess ? (uint32_t*)p : nullptr;
-    }();
-    static std::atomic<uint32_t> next{0};
-    if (!page) return nullptr;
-    uint32_t* w = page + next.fetch_add(1, std::memory_order_relaxed) % 1024u;
+        if (cudaHostAlloc(&p, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return nullptr;
+        c.errors = (uint32_t*)p;
+    }
+    uint32_t* w = c.errors + c.next++ % 1024u;
     *(volatile uint32_t*)w = 0;
     return w;
 }

@@ -144,32 +144,9 @@ struct DevBuf {
 };
 
 // Scratch memory for one call, stream-ordered, from a pool of its own per
-// device that keeps up to 512 MB between calls (cudaMalloc and cudaFree of a
+// context that keeps up to 512 MB between calls (cudaMalloc and cudaFree of a
 // call's scratch cost more than a small build, and synchronise the device).
-inline cudaMemPool_t scratch_pool(int dev)
-{
-    struct Pools {
-        cudaMemPool_t p[64] = {};
-        std::once_flag once[64];
-    };
-    static Pools pools;
-    if (dev < 0 || dev >= 64) return nullptr;
-    std::call_once(pools.once[dev], [dev] {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-            cudaGetLastError();
-            return;
-        }
-        uint64_t keep = 512ull << 20;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        pools.p[dev] = pool;
-    });
-    return pools.p[dev];
-}
+cudaMemPool_t scratch_pool(int dev);  // nullptr: none could be made
 struct PoolBuf {
     uint8_t* p = nullptr;
     int dev;

@@ -50,25 +50,6 @@ std::mutex g_scratch_mu;
 unsigned char* g_scratch_addr[64] = {};
 unsigned long long g_scratch_ctx[64] = {};  // id of the context the address belongs to
 
-// cuCtxGetId through the runtime's driver entry point (no link to libcuda).
-typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
-
-// Id of the current context (0 when it cannot be read).
-unsigned long long current_context_id()
-{
-    static CtxGetIdFn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return (CtxGetIdFn) nullptr;
-        return (CtxGetIdFn)f;
-    }();
-    unsigned long long id = 0;
-    if (!fn || fn(nullptr, &id) != 0) return 0;
-    return id;
-}
-
 // Device address of g_noalloc_scratch on `dev` (the current device, its
 // context already initialised by the caller).
 int scratch_address(int dev, unsigned char** out)

@@ -60,6 +60,11 @@ struct BuildJob {
     uint32_t* tri_rw;       // the tree's faces (3 * nT), rewritten by the renumbering (tri, writable)
 };
 
+// Id of the current context, 0 when it cannot be read (host.cu). What lives as
+// long as a context (pools, pinned pages, kernel attributes, symbol addresses) is
+// kept under it: after cudaDeviceReset the next context starts without them.
+unsigned long long current_context_id();
+
 // build_kernels.cu
 constexpr uint32_t kBuildTile = 4096;  // faces (vertices) of a tile
 struct BuildScratch {

@@ -1,0 +1,77 @@
+"""What builds keep for the life of a context (a pool, a pinned page, a kernel
+attribute) is made anew in the next one: the library works on after
+cudaDeviceReset, in a process of its own."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _run(code):
+    code = "import sys\nsys.path.insert(0, %r)\nsys.path.insert(0, %r)\n" % (ROOT, os.path.join(ROOT, "tests")) + textwrap.dedent(code)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+    assert "done" in r.stdout
+
+
+def test_builds_and_detects_after_a_device_reset(gpu):
+    _run('''
+        import ctypes, glob, os
+        import numpy as np
+        from oibvh_gb300 import DeviceType, OibvhTree, Scene
+        from oibvh_gb300 import _native as N
+
+        def soup(n, seed):
+            rng = np.random.default_rng(seed)
+            c = rng.uniform(-1, 1, (n, 1, 3))
+            return ((c + rng.uniform(-0.05, 0.05, (n, 3, 3))).astype(np.float32).reshape(-1, 3),
+                    np.arange(3 * n, dtype=np.uint32).reshape(-1, 3))
+
+        def everything():
+            out = []
+            trees = []
+            for n in (900, 6000, 5000):  # both sides of the builds in one launch
+                for bits in (30, 63):
+                    t = OibvhTree(xyz=soup(n, n)[0], tri=soup(n, n)[1])
+                    t.set_morton_bits(bits)
+                    t.build()
+                    out.append(t.aabb_tree())
+                    out.append(t.sorted_faces()[1])
+                    trees.append(t)
+            sc = Scene()
+            for t in trees[::2]:
+                t.set_morton_bits(30)
+                sc.addOibvhTree(t)
+            sc.build()
+            sc.detectCollision(DeviceType.GPU0, 4, 3)
+            out.append(sc.int_tri_pairs())
+            sc.capture_frame(4, 3, True)
+            sc.launch_frame()
+            sc.finish_frame()
+            out.append(sc.int_tri_pairs())
+            return out, trees + [sc]
+
+        cudart = None
+        for name in ("libcudart.so.13", "/usr/local/cuda/lib64/libcudart.so.13", "/usr/local/cuda/lib64/libcudart.so"):
+            try:
+                cudart = ctypes.CDLL(name)
+                break
+            except OSError:
+                pass
+        assert cudart is not None
+        kept = []
+        want, handles = everything()
+        for _ in range(2):
+            for h in handles:  # their memory goes with the context: nothing is left to free
+                h._h = ctypes.c_void_p(None)
+            assert cudart.cudaDeviceReset() == 0
+            got, handles = everything()
+            assert len(got) == len(want) and all(np.array_equal(a, b) for a, b in zip(got, want))
+        print("done", flush=True)
+        os._exit(0)
+    ''')
