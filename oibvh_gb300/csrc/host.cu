@@ -173,11 +173,15 @@ static int sync_positions(oibvh_tree_t t, cudaStream_t s)
 // that ran out). The words outlive the builds: one page a context, taken in turn.
 static uint32_t* build_error_word()
 {
+    if (injected_alloc_failure()) return nullptr;  // (counted for every build, also where the page is there)
     std::lock_guard<std::mutex> lock(g_build_mu);
     BuildContext& c = g_build_contexts[context_id()];
     if (!c.errors) {
         void* p = nullptr;
-        if (cudaHostAlloc(&p, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return nullptr;
+        if (cudaHostAlloc(&p, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();  // (not for the next launch to report)
+            return nullptr;
+        }
         c.errors = (uint32_t*)p;
     }
     uint32_t* w = c.errors + c.next++ % 1024u;

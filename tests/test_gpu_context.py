@@ -75,3 +75,60 @@ def test_builds_and_detects_after_a_device_reset(gpu):
         print("done", flush=True)
         os._exit(0)
     ''')
+
+
+def test_a_build_that_gets_no_memory_fails_alone(gpu):
+    """The first builds of a process, with the error words, then the scratch not
+    to be had: each reports it, and the next one works."""
+    _run('''
+        import numpy as np
+        from oibvh_gb300 import OibvhTree, Scene
+        from oibvh_gb300 import _native as N
+        from oracle.oracle import Port
+
+        rng = np.random.default_rng(3)
+        xyz = rng.uniform(-1, 1, (18000, 3)).astype(np.float32)
+        tri = np.arange(18000, dtype=np.uint32).reshape(-1, 3)
+        L = N.lib()
+        trees = [OibvhTree(xyz=xyz, tri=tri) for _ in range(3)]
+        want = Port.oibvh_build(xyz, tri)
+
+        def check(t):
+            assert np.array_equal(t.sorted_faces()[1], want[2])
+            assert np.array_equal(t.aabb_tree().view(np.uint32), want[0].view(np.uint32))
+
+        def fails(n, build):
+            L.oibvh_debug_fail_alloc_after(n)
+            try:
+                build()
+            except N.OibvhError as e:
+                assert e.status == N.ERR_OOM, e
+                return True
+            finally:
+                L.oibvh_debug_fail_alloc_after(-1)
+            return False
+
+        for n in (0, 1):
+            assert fails(n, trees[n].build), n
+        for t in trees:
+            t.build()
+            check(t)
+        a0 = L.oibvh_debug_alloc_attempts()
+        trees[0].build()
+        assert L.oibvh_debug_alloc_attempts() - a0 == 2
+        check(trees[0])
+        sc = Scene()
+        for t in trees:
+            sc.addOibvhTree(t)
+        sc.build()
+        a0 = L.oibvh_debug_alloc_attempts()
+        sc.build()
+        k = L.oibvh_debug_alloc_attempts() - a0
+        assert k == 2
+        for n in range(k):
+            assert fails(n, sc.build), n
+        sc.build()
+        for t in trees:
+            check(t)
+        print("done")
+    ''')
