@@ -413,8 +413,9 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
 #pragma unroll
     for (uint32_t r = 0; r < kSortItems; ++r) {
         const uint32_t q = r * kSortThreads + tid;
+        if (q - lane >= n) break;  // (the whole warp: the ballot names every lane)
         const uint32_t row = __ballot_sync(0xffffffffu, q < n);
-        if (q >= n) break;
+        if (q >= n) continue;
         const uint32_t k = s_key[q], o = s_val[q], dst = s_base[(k >> shift) & 255u] + q;
         if (kLast) {
             const uint32_t* t = job.tri + 3 * (size_t)o;
