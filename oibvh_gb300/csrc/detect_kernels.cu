@@ -9,9 +9,9 @@
 // The broad phase is one kernel, k_walk, after k_begin has set its counters:
 // warps claim start-level node pairs 32 at a time, test them, and walk the
 // overlapping ones down through a private ring in shared memory. It goes in
-// rounds with a grid-wide barrier between them (a cooperative launch): a warp
-// that has nothing more to claim goes on for a few levels only and leaves the
-// rest to the next round's list, which all warps share out anew. Appends
+// rounds of a launch each: a warp that has nothing more to claim goes on for a
+// few levels only and leaves the rest to the next round's list, which all warps
+// share out anew. No CTA waits for another one. Appends
 // (next list, hits, candidates) are warp-aggregated: one atomic per warp,
 // positions from ballot/shuffle prefix sums.
 //
@@ -751,21 +751,10 @@ __device__ __forceinline__ uint32_t child_prefix(uint32_t cnt, uint32_t lane, ui
 
 // ---------------------------------------------------------------------------
 // The traversal's rounds. Round 0 takes the start tests, round r >= 1 the list
-// that round r - 1 appended (two arrays in turn). A round's words (list size
-// and, in the upper half of the same 64 bits, the CTAs that have finished
-// appending to it; items claimed) are one of four slots in turn: round r
-// appends to slot r + 1 and clears slot r + 2, which nobody looks at then.
+// that round r - 1 appended (two arrays in turn). A round's words (list size,
+// items claimed) are one of four slots in turn: round r appends to slot r + 1 and
+// clears slot r + 2, which nobody looks at then.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t ld_acquire(const uint64_t* p)
-{
-    uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(uint64_t* p, uint64_t v)
-{
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 __device__ __forceinline__ uint32_t* round_slot(uint32_t* counts, uint32_t r)
 {
     return counts + kCtlRound + (r & 3u) * kCtlRoundWords;
@@ -788,50 +777,6 @@ __device__ __forceinline__ void publish(const DetectArgs& a)
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) a.host_hits[i] = __ldcg(a.hits + i);
 }
 __global__ void __launch_bounds__(256) k_publish(DetectArgs a) { publish(a); }
-
-// The grid's barrier after round r (every CTA is resident: a cooperative
-// launch). The CTA that arrives last has the list's final size from the word
-// it arrives at, and releases the others with it: one atomic and one poll
-// between a CTA's last append and the next round's first load. Returns the
-// next round's items, kStop to stop: after a round that may be the last and
-// left nothing, or when the list has overflowed. A CTA
-// that has polled for several seconds raises kFlagTimeout and stops.
-constexpr uint32_t kBarrierPolls = 1u << 24;
-constexpr uint32_t kStop = 0xffffffffu;
-__device__ __forceinline__ uint32_t round_barrier(const DetectArgs& a, uint32_t r, bool may_stop, uint32_t* s_next,
-                                                  uint32_t* s_last)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *s_last = 0;
-        uint32_t* ctl = a.counts;
-        uint64_t* release = (uint64_t*)(ctl + kCtlRelease);  // (rounds finished, items of the next)
-        __threadfence();
-        const uint64_t w = atomicAdd((unsigned long long*)round_slot(ctl, r + 1), 1ull << 32);
-        uint32_t next = (uint32_t)w;
-        if ((uint32_t)(w >> 32) == gridDim.x - 1u) {
-            if (next > a.work_cap || (next == 0 && may_stop)) {
-                next = kStop;
-                *s_last = 1;
-            }
-            st_release(release, (uint64_t)(r + 1u) << 32 | next);
-            ctl[kCountPeak] = max(ctl[kCountPeak], (uint32_t)w);
-            if ((uint32_t)w > 0) ctl[kCountRounds] = r + 2u;
-        } else {
-            uint64_t v = 0;
-            uint32_t polls = 0;
-            while ((uint32_t)((v = ld_acquire(release)) >> 32) <= r && ++polls < kBarrierPolls) __nanosleep(20);
-            next = (uint32_t)v;
-            if ((uint32_t)(v >> 32) <= r) {
-                atomicOr(ctl + kCountFlags, (uint32_t)kFlagTimeout);
-                next = kStop;
-            }
-        }
-        *s_next = next;
-    }
-    __syncthreads();
-    return *s_next;
-}
 
 // One start pair per lane (test i of the start-level cross products, the
 // reference's Scene::expandBvttNodes, src/cuda/scene.cu:192-223): overlapping
@@ -874,10 +819,20 @@ __device__ __forceinline__ uint32_t start_pairs(const DetectArgs& a, WarpCands& 
 // meshes 94 to 81 us a detect, 24 bodies 92 to 80, 64 pairs 306 to 297).
 constexpr uint32_t kClaimMin = 16;
 
-// Rounds first .. last of the traversal (fewer when a round leaves nothing);
-// more than one round needs a cooperative launch. Each step pops up to 32 pairs
-// of the warp's ring (one per lane), expands them and appends the overlapping
-// children at the tail, with no barrier between tree levels.
+// Round r of the traversal. Each step pops up to 32 pairs of the warp's ring (one
+// per lane), expands them and appends the overlapping children at the tail, with
+// no barrier between tree levels. `last`: the last round that the host has
+// launched; its CTA that finishes last writes what is left for a next one, and
+// hands over the results.
+//
+// A round is a launch, not a barrier in one launch: the CTAs of a grid barrier
+// all have to be resident at once (a cooperative launch starts when they can be),
+// so a detect waited for the end of whatever else held the SMs. The next round's
+// CTAs are scheduled while this one's last warps finish (programmatic launch:
+// they wait at the start for its end), which a round's launch latency hides
+// behind. Two meshes of 20 k triangles 31.6 us a detect with the barrier, 35.0
+// with plain launches, 31.5 so; of 1.31 M 67, 72 and 65; a scene of 64 pairs 275,
+// 276 and 268.
 //
 // What bounds it: in small traversals the latency of a step's chain (ring entry,
 // boxes, at the leaves faces and then vertices; 1.1 to 1.5 us) times the steps in
@@ -886,7 +841,7 @@ constexpr uint32_t kClaimMin = 16;
 // written out and a step's children and candidates were given their places by one
 // scan: a frame of 64 pairs 228 to 197 us, of 512 pairs 1254 to 1088). DRAM stays
 // below 10 %. A warp cuts its walk six steps after it has last claimed something
-// and the rest is shared out anew: a barrier costs about 2 us, a warp left alone
+// and the rest is shared out anew: the next round costs about 2 us, a warp left alone
 // with a deep subtree tens (2, 4, 6, 8, 12 steps: two meshes of 1.31 M triangles
 // 141, 104, 96, 103, 119 us a detect); three steps after start tests that were
 // dealt out, which leave pairs to one warp in ten (six against three: 1.31 M
@@ -897,34 +852,37 @@ constexpr uint32_t kClaimMin = 16;
 // bodies 115 to 60. A queue that idle warps wait on, instead of rounds, was slower
 // (20 k: 112 us): a hand-over costs its giver about 3 us.
 template <bool kFused, bool kOne>
-__global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32_t total0, uint32_t first, uint32_t last)
+__global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32_t total0, uint32_t r, bool last)
 {
     extern __shared__ uint64_t s_ring[];  // [warp][walk_ring(cap)]
     __shared__ uint64_t s_cand[kWarps][kCandBuf], s_late[kFused ? kWarps : 1][kLateBuf];
-    __shared__ uint32_t s_next, s_last, s_found, s_tested;
+    __shared__ uint32_t s_last, s_found, s_tested;
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_found = s_tested = 0;
+    // (with a programmatic launch only: the round before is done and its writes are here; then
+    // the next round's CTAs may come as this one's leave)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
     WarpCands wc{s_cand[wib], s_late[kFused ? wib : 0], 0};
     const uint32_t R = walk_ring(a.walk_cap), mask = R - 1u;
     uint64_t* ring = s_ring + (size_t)wib * R;
     const uint32_t W = gridDim.x * kWarps;
     const uint32_t w = wib * gridDim.x + blockIdx.x;  // neighbouring items go to different SMs
-    const uint32_t listed = first == 0 ? total0 : *(volatile uint32_t*)round_slot(a.counts, first);
-    uint32_t n_src = first == 0 ? total0 : min(listed, a.work_cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && listed > 0) {  // (the launch before, of one round, had no barrier to do it)
-        a.counts[kCountRounds] = first + 1u;
-        if (first > 0) a.counts[kCountPeak] = max(a.counts[kCountPeak], listed);
+    const uint32_t listed = r == 0 ? total0 : *(volatile uint32_t*)round_slot(a.counts, r);
+    const uint32_t n_src = r == 0 ? total0 : min(listed, a.work_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        round_slot(a.counts, r + 2)[0] = 0;
+        round_slot(a.counts, r + 2)[kCtlRoundClaim] = 0;
+        if (listed > 0) a.counts[kCountRounds] = r + 1u;
+        if (r > 0) a.counts[kCountPeak] = max(a.counts[kCountPeak], listed);
     }
-    for (uint32_t r = first;; ++r) {
+    if (n_src > 0) {
         uint32_t* claim = round_slot(a.counts, r) + kCtlRoundClaim;
         uint32_t* spill_cnt = round_slot(a.counts, r + 1);
-        const uint64_t* src = r & 1u ? a.work[1] : a.work[0];
-        uint64_t* spill = r & 1u ? a.work[0] : a.work[1];
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *(uint64_t*)round_slot(a.counts, r + 2) = 0;
-            round_slot(a.counts, r + 2)[kCtlRoundClaim] = 0;
-        }
+        // (where they are used: kept, the two pointers are spilled, 28 B a thread and more)
+        auto src = [&]() { return r & 1u ? a.work[1] : a.work[0]; };
+        auto spill = [&]() { return r & 1u ? a.work[0] : a.work[1]; };
         // A long list is claimed `chunk` consecutive items at a time; a short one (start tests:
         // at most a warp's worth per warp; pairs: fewer than kClaimMin per warp) is dealt out
         // statically, items w, w + W, .., so that it spreads over all warps.
@@ -959,7 +917,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
                     live += start_pairs<kOne>(a, wc, i, lane < n_take, ring, mask, head + live, lane);
                     drain_candidates<kFused, kOne>(a, wc, lane);
                 } else {
-                    if (lane < n_take) ring[(head + live + lane) & mask] = __ldcg(src + i);
+                    if (lane < n_take) ring[(head + live + lane) & mask] = __ldcg(src() + i);
                     live += n_take;
                     __syncwarp();
                 }
@@ -984,7 +942,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
                 if (lane == 0) base = atomicAdd(spill_cnt, live);
                 base = __shfl_sync(0xffffffffu, base, 0);
                 for (uint32_t k = lane; k < live; k += 32)
-                    if (base + k < a.work_cap) spill[base + k] = ring[(head + k) & mask];
+                    if (base + k < a.work_cap) spill()[base + k] = ring[(head + k) & mask];
                 if (lane == 0 && base + live > a.work_cap) atomicOr(a.counts + kCountFlags, (uint32_t)kFlagFrontOverflow);
                 break;
             }
@@ -1034,7 +992,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
                         if (!((e.m >> k) & 1u)) continue;
                         const uint64_t child = e.key + child_step(k) + ((uint64_t)((e.dm >> (2 * k)) & 3u) << 48);
                         if (at < fit) ring[(head + live + at) & mask] = child;
-                        else if (sbase + (at - fit) < a.work_cap) spill[sbase + (at - fit)] = child;
+                        else if (sbase + (at - fit) < a.work_cap) spill()[sbase + (at - fit)] = child;
                         ++at;
                     }
                 }
@@ -1048,32 +1006,36 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
             // queued, where little else is live
             drain_candidates<kFused, kOne>(a, wc, lane);
         }
-        // before the wait for the slowest warp: the warp's last candidates (but for rounds that
-        // claim: a partial buffer costs as much as a full one, so those keep theirs, and
-        // another round follows even if nothing is left), and the CTA's totals
-        if (!claiming || r == last) flush_candidates<kFused, kOne>(a, wc, lane);
+        flush_candidates<kFused, kOne>(a, wc, lane);
         if (lane == 0 && (tested | wc.found)) {
             atomicAdd(&s_tested, tested);
             atomicAdd(&s_found, wc.found);
         }
-        wc.found = 0;
         __syncthreads();
         if (threadIdx.x == 0) {
             if (r == 0 && blockIdx.x == 0) s_tested += total0;
             if (s_tested) atomicAdd(a.counts + kCountTested, s_tested);
             if (s_found) atomicAdd(a.counts + kCountCands, s_found);
-            s_tested = s_found = 0;
         }
-        if (r == last) break;
-        n_src = round_barrier(a, r, !claiming, &s_next, &s_last);
-        if (n_src == kStop) break;
     }
-    // the CTA that was last to finish hands over the results, and clears the
-    // other counter block for the next traversal (nobody uses it now)
-    if (a.host && s_last) {
-        publish(a);
+    if (!last) return;
+    // the CTA that is last to finish hands over the results, and clears the other
+    // counter block for the next traversal (nobody uses it now)
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(a.counts + kCtlDone, gridDim.x - 1u) == gridDim.x - 1u;  // (wraps to 0)
+        if (s_last) {
+            __threadfence();
+            a.counts[kCountLeft] = __ldcg(round_slot(a.counts, r + 1));
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (!s_last || !a.host) return;
+    publish(a);
+    if (a.counts_next)
         for (uint32_t i = threadIdx.x; i < kCountTotal; i += blockDim.x) a.counts_next[i] = 0;
-    }
 }
 
 // Narrow phase over stored candidates (the split broad/narrow API):
@@ -1934,7 +1896,7 @@ cudaError_t launch_publish(const DetectArgs& a, cudaStream_t s)
 
 static size_t walk_smem(uint32_t cap) { return (size_t)kWarps * walk_ring(cap) * 8; }  // one ring per warp
 
-typedef void (*WalkKernel)(DetectArgs, uint32_t, uint32_t, uint32_t);
+typedef void (*WalkKernel)(DetectArgs, uint32_t, uint32_t, bool);
 static WalkKernel walk_kernel(bool fused, bool one)
 {
     return fused ? (one ? k_walk<true, true> : k_walk<true, false>) : (one ? k_walk<false, true> : k_walk<false, false>);
@@ -1955,30 +1917,26 @@ static cudaError_t walk_configure()
     return cudaSuccess;
 }
 
-cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, uint32_t last, cudaStream_t s)
+cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t from, uint32_t to, bool hand_over, cudaStream_t s)
 {
     if (fused_precision(a)) return cudaErrorInvalidValue;
     if (a.walk_cap > kWalkCapMax || (a.walk_cap % 32) != 0) return cudaErrorInvalidValue;
     cudaError_t e = walk_configure();
-    if (e != cudaSuccess) return e;
-    note_launches(1);
     cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)a.grid);
     cfg.blockDim = dim3(kDetectThreads);
     cfg.dynamicSmemBytes = walk_smem(a.walk_cap);
     cfg.stream = s;
     cfg.attrs = &attr;
-    cfg.numAttrs = first != last ? 1 : 0;
-    for (;;) {
-        e = cudaLaunchKernelEx(&cfg, walk_kernel(a.fuse_narrow, a.n_pairs == 1), a, total0, first, last);
-        // (a stream may have fewer SMs than the device: a smaller grid does the same)
-        if (e != cudaErrorCooperativeLaunchTooLarge || cfg.gridDim.x == 1) return e;
-        cudaGetLastError();
-        cfg.gridDim.x /= 2;
+    for (uint32_t r = from; r < to && e == cudaSuccess; ++r) {
+        note_launches(1);
+        cfg.numAttrs = r > from ? 1 : 0;  // (behind a round of this call; the first one waits for all before it)
+        e = cudaLaunchKernelEx(&cfg, walk_kernel(a.fuse_narrow, a.n_pairs == 1), a, total0, r, hand_over && r + 1 == to);
     }
+    return e;
 }
 
 int walk_blocks_per_sm(uint32_t walk_cap, bool fused)

@@ -5,7 +5,7 @@
 // (include/cuda/scene.cuh:44-61, src/cuda/scene.cu). Differences by design:
 //   * the tree stays resident in device memory; nothing is copied back to
 //     the host after build or refit unless asked (oibvh_tree_get_aabbs);
-//   * the BVTT loop is one launch, so detect reads counters back once per
+//   * the BVTT loop is enqueued whole, so detect reads counters back once per
 //     pass, not once per level (the reference reads after every level,
 //     src/cuda/scene.cu:302);
 //   * queues are sized by demand: an overflow is detected, the queue grows,
@@ -259,6 +259,7 @@ struct oibvh_scene_s {
     DevBuf<uint32_t> walk_counts;  // two counter blocks, in turn between direct detects: each clears the other one
     uint32_t walk_turn = 0;
     bool walk_clean = false;       // the block of this turn is zero
+    uint32_t walk_rounds = 4;      // walk rounds that go out before the host looks: as many as the last detect took
     PinnedBuf<PairView> h_pairs;
     PinnedBuf<uint32_t> h_counts;
     PinnedBuf<uint4> h_hits;       // the last detect's hits, when there are at most kHostHits
@@ -468,7 +469,7 @@ int ensure_lists(oibvh_scene_s* s)
 {
     OK_TRY(s->work0.ensure(s->front_cap, "cudaMalloc(work list)"));
     OK_TRY(s->work1.ensure(s->front_cap, "cudaMalloc(work list)"));
-    OK_TRY(s->counts.ensure(2 * kCountTotal, "cudaMalloc(counts)"));
+    OK_TRY(s->counts.ensure(kCountTotal, "cudaMalloc(counts)"));
     return OIBVH_OK;
 }
 
@@ -561,43 +562,51 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.claim_min = s->tune_claim;
             a.descend_ratio = (float)s->tune_descend;
             const uint32_t front0 = (uint32_t)plan.front0;
-            s->h_counts.p[kCountFlags] = kFlagTimeout;  // overwritten when the walk hands over its counters
             a.host = s->h_counts.p;
             a.host_hits = s->h_hits.p;
             a.host_hit_cap = narrow ? kHostHits : 0u;
-            if (fused && hits_before == 0) {
-                // one launch: the counter block was cleared by the detect before
-                if (!s->walk_counts.p) {
-                    OK_TRY(s->walk_counts.ensure(2 * kCountTotal, "cudaMalloc(counts)"));
-                    s->walk_clean = false;
-                }
-                a.counts = s->walk_counts.p + s->walk_turn * kCountTotal;
-                a.counts_next = s->walk_counts.p + (s->walk_turn ^ 1u) * kCountTotal;
-                if (!s->walk_clean) CUDA_TRY(launch_begin(a, 0, st));
-                s->walk_clean = false;
-                CUDA_TRY(launch_walk(a, front0, 0, kAllRounds, st));
-                CUDA_TRY(cudaStreamSynchronize(st));
-                s->walk_clean = !(s->h_counts.p[kCountFlags] & kFlagTimeout);
-                if (s->walk_clean) s->walk_turn ^= 1u;
-            } else if (split) {
-                DetectArgs w = a, n = a;
-                w.host = nullptr;
+            const uint32_t* c = s->h_counts.p;
+            const uint32_t batch = s->walk_rounds;
+            if (split) {
+                DetectArgs n = a;
                 n.grid = sm_count(s->device) * 8;
                 CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
-                CUDA_TRY(launch_walk(w, front0, 0, kAllRounds, st));
+                DetectArgs w = a;
+                w.host = nullptr;
+                CUDA_TRY(launch_walk(w, front0, 0, batch + 1, true, st));  // (one more: a pass that lacks one runs again)
                 CUDA_TRY(launch_narrow(n, st));
                 CUDA_TRY(launch_publish(a, st));
                 CUDA_TRY(cudaStreamSynchronize(st));
+                if (!c[kCountFlags] && c[kCountLeft]) {  // candidates are missing: again, with more rounds
+                    s->walk_rounds = batch + 8;
+                    continue;
+                }
             } else {
-                a.counts_next = a.counts + kCountTotal;  // (cleared to no purpose)
-                CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
-                CUDA_TRY(launch_walk(a, front0, 0, kAllRounds, st));
-                CUDA_TRY(cudaStreamSynchronize(st));
+                // (in turn: the detect before has cleared this one's counters)
+                const bool in_turn = fused && hits_before == 0;
+                if (in_turn) {
+                    if (!s->walk_counts.p) {
+                        OK_TRY(s->walk_counts.ensure(2 * kCountTotal, "cudaMalloc(counts)"));
+                        s->walk_clean = false;
+                    }
+                    a.counts = s->walk_counts.p + s->walk_turn * kCountTotal;
+                    a.counts_next = s->walk_counts.p + (s->walk_turn ^ 1u) * kCountTotal;
+                }
+                if (!in_turn || !s->walk_clean) CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
+                if (in_turn) s->walk_clean = false;
+                for (uint32_t r = 0, to = batch;; r = to, to += 2) {
+                    CUDA_TRY(launch_walk(a, front0, r, to, true, st));
+                    CUDA_TRY(cudaStreamSynchronize(st));
+                    if (c[kCountFlags] || !c[kCountLeft]) break;
+                }
+                if (in_turn) {
+                    s->walk_clean = true;
+                    s->walk_turn ^= 1u;
+                }
             }
-            const uint32_t* c = s->h_counts.p;
+            s->walk_rounds = std::max(1u, c[kCountRounds]);
             const uint32_t flags = c[kCountFlags], rounds = c[kCountRounds];
             const uint64_t peak = c[kCountPeak];
-            if (flags & kFlagTimeout) return fail(OIBVH_ERR_TIMEOUT, "the BVTT traversal's barrier timed out");
             if (flags) {
                 s->stats.retries++;
                 if (flags & kFlagFrontOverflow) s->front_cap = grow_cap(peak, s->front_cap);
@@ -1589,16 +1598,8 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
     if (e == cudaSuccess) e = launch_begin(a, 0, st);
     ++k;
     mark(3);
-    // The last launch walks all rounds left, usually none: a cooperative one, so it takes one CTA an SM
-    // and fits beside other streams' kernels (three launches, the last with the whole GPU: frames of 32
-    // pairs from eight threads 4.2 k/s, so 5.1 k; alone 2 us longer for 64 pairs).
-    for (uint32_t r = 0; r < s->frame_rounds && e == cudaSuccess; ++r) {
-        const bool rest = r + 1 == s->frame_rounds;
-        DetectArgs w = a;
-        if (rest) w.grid = std::min(w.grid, sm_count(s->device));
-        e = launch_walk(w, s->frame_front0, r, rest ? kAllRounds : r, st);
-        ++k;
-    }
+    if (e == cudaSuccess) e = launch_walk(a, s->frame_front0, 0, s->frame_rounds, true, st);
+    k += s->frame_rounds;
     mark(4);
     if (!a.fuse_narrow && e == cudaSuccess) {
         DetectArgs n = a;
@@ -1708,8 +1709,8 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
 
     s->frame_args = a;
     s->frame_front0 = (uint32_t)plan.front0;
-    // a plain launch for each round that the warm-up frame walked, one launch for what is left
-    s->frame_rounds = std::max(3u, std::min(16u, (uint32_t)s->stats.steps + 1u));
+    // the rounds that the warm-up frame took and one more (a round with nothing to walk returns at once)
+    s->frame_rounds = std::max(3u, (uint32_t)s->stats.steps + 1u);
 
     // capture on a private non-blocking stream (the legacy default stream
     // cannot be captured); the graph is launched on the caller's stream
@@ -1795,8 +1796,8 @@ API int oibvh_scene_finish_frame(oibvh_scene_t s, void* stream)
     CUDA_TRY(cudaStreamSynchronize(st));
     const uint32_t* c = s->h_frame_counts.p;
     if (!c) return fail(OIBVH_ERR_STATE, "no frame was launched");
-    if (c[kCountFlags]) {
-        // the captured queues were too small for this frame: redo the detect the
+    if (c[kCountFlags] || c[kCountLeft]) {
+        // the captured queues or rounds were too few for this frame: redo the detect the
         // synchronous way (the refit already ran) and capture again next frame
         s->frame_stale = true;
         s->frame_redos++;

@@ -32,6 +32,8 @@ namespace oibvh {
 
 // Fixed capacity of each of the two traversal work lists (BVTT node pairs).
 constexpr uint32_t kNoAllocItems = 1u << 18;
+// Rounds that go out before the host looks whether anything is left (most pairs take three or four).
+constexpr uint32_t kNoAllocRounds = 4;
 // Header: the counters, rounded up (the pair's record goes with the kernels' arguments).
 constexpr size_t kNoAllocHeader = 4096;
 constexpr size_t kNoAllocBytes = kNoAllocHeader + 2 * (size_t)kNoAllocItems * sizeof(uint64_t);
@@ -151,11 +153,13 @@ extern "C" __attribute__((visibility("default"))) int oibvh_pair_detect_noalloc(
         args.grid = sms * per_sm;
 
         NA_CUDA(launch_begin(args, 0, s));
-        NA_CUDA(launch_walk(args, (uint32_t)total0, 0, kAllRounds, s));
         uint32_t counts[kCountHost];
-        NA_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
-        NA_CUDA(cudaStreamSynchronize(s));
-        if (counts[kCountFlags] & kFlagTimeout) return noalloc_fail(OIBVH_ERR_TIMEOUT, "the traversal's barrier timed out");
+        for (uint32_t r = 0;; r += kNoAllocRounds) {
+            NA_CUDA(launch_walk(args, (uint32_t)total0, r, r + kNoAllocRounds, true, s));
+            NA_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
+            NA_CUDA(cudaStreamSynchronize(s));
+            if (counts[kCountFlags] || counts[kCountLeft] == 0) break;
+        }
         *n_hits = counts[kCountHits];
         if (counts[kCountFlags] & kFlagFrontOverflow)
             return noalloc_fail(OIBVH_ERR_OVERFLOW, "the pair needs more than " + std::to_string(kNoAllocItems) +

@@ -159,7 +159,6 @@ enum DeviceFlag : uint32_t {
     kFlagCandOverflow = 1u << 1,
     kFlagHitOverflow = 1u << 2,
     kFlagBadInput = 1u << 3,
-    kFlagTimeout = 1u << 4,
 };
 
 // glm::min / glm::max semantics (third/glm/detail/func_common.inl:17-29).

@@ -141,10 +141,10 @@ struct DetectArgs {
     uint4* hits;
     uint32_t hit_cap;
     uint32_t* counts;      // see kCount* below
-    uint32_t* host;        // pinned: where the walk of all rounds (or launch_publish) puts the counters; nullptr: nowhere
+    uint32_t* host;        // pinned: where the last walk round (or launch_publish) puts the counters; nullptr: nowhere
     uint4* host_hits;      // pinned: and the hits, when there are at most host_hit_cap
     uint32_t host_hit_cap;
-    uint32_t* counts_next; // with host: the counter block that the walk clears for the next traversal
+    uint32_t* counts_next; // with host: the counter block that the walk clears for the next traversal (nullptr: none)
     uint32_t* prec_lists;  // precision mode, 4 x cand_cap words: the passes' lists (PrecLists)
     double* fp64_tri;      // precision mode: the FP64 list's setups, kFp64TriRows rows of fp64_tri_cap
                            // (structure of arrays; nullptr: each is formed where it is used)
@@ -159,11 +159,11 @@ struct DetectArgs {
     float descend_ratio = kDescendRatio;  // both sides descend while the boxes' squared diagonals are within it
 };
 // A traversal of `total0` start pairs: counters cleared (launch_begin, which
-// sets the hits to hits_before, or the traversal before), then launch_walk of round 0 .. kAllRounds, or of rounds 0, 1,
-// .. one at a time and then r .. kAllRounds.
+// sets the hits to hits_before, or the traversal before), then rounds 0, 1, .. in any number of calls of
+// launch_walk (rounds from .. to - 1), until one leaves nothing. hand_over: the last of them writes kCountLeft,
+// and the counters and few hits to the pinned host memory where there is any.
 cudaError_t launch_begin(const DetectArgs& a, uint32_t hits_before, cudaStream_t s);
-constexpr uint32_t kAllRounds = 0xffffffffu;  // until a round leaves nothing (a cooperative launch)
-cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t first, uint32_t last, cudaStream_t s);
+cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t from, uint32_t to, bool hand_over, cudaStream_t s);
 // the counters (and few hits) to the pinned host memory
 cudaError_t launch_publish(const DetectArgs& a, cudaStream_t s);
 // walker CTAs that fit on one SM with rings of `walk_cap` entries (0:
@@ -182,13 +182,14 @@ constexpr uint32_t kFp64TriRows = 23;
 // of the list its double-float pass leaves to FP64, of what its recheck
 // leaves to the bounded pass, and of the rechecks of axes other than normals
 // (not counted with the others); then the largest list
-// of a walk round and the rounds that had anything to walk. Past the words that the host reads:
+// of a walk round, the rounds that had anything to walk, and what the last round
+// that was launched has left to a next one. Past the words that the host reads:
 // the walk's control words, each on a cache line of its own.
 constexpr uint32_t kCountHits = 0, kCountFlags = 1, kCountCands = 2, kCountCandSlots = 3, kCountTested = 4,
                    kCountFp64Axes = 5, kCountFp64Cands = 6, kCountDisagree = 7, kCountPrecHits = 8,
                    kCountPrecRecheck = 9, kCountPrecFp64 = 10, kCountPrecLeft = 11, kCountPrecAgain = 12,
-                   kCountPrecOther = 13, kCountNarrowEnd = 14, kCountPeak = 14, kCountRounds = 15, kCountHost = 16,
-                   kCtlRelease = 32,
+                   kCountPrecOther = 13, kCountNarrowEnd = 14, kCountPeak = 14, kCountRounds = 15, kCountLeft = 16,
+                   kCountHost = 17, kCtlDone = 32,
                    kCtlRound = 64, kCtlRoundWords = 64, kCtlRoundClaim = 32,  // four slots
                    kCountTotal = kCtlRound + 4 * kCtlRoundWords;
 

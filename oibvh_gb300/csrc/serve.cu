@@ -22,8 +22,8 @@
 //     the grouped pairs, 8 B each) tracked by events, each query's pairs then
 //     one block copy on the host; the loop never waits on the device while
 //     other work can be launched;
-//   * a batch whose queues were too small is redone on its lane with larger
-//     queues, so results are never truncated.
+//   * a batch whose queues or launched walk rounds were too few is redone on
+//     its lane with more, so results are never truncated.
 //
 // A query's pair set does not depend on what it was batched with: the
 // traversal and the triangle test of a pair read only that pair's trees.
@@ -46,6 +46,9 @@ using Clock = std::chrono::steady_clock;
 
 constexpr size_t kArenaAlign = 256;
 static_assert(kArenaAlign % 32 == 0, "node arrays in the arena must be 32-byte aligned (256-bit node loads)");
+
+// Walk rounds launched for a batch (most take three to five); one that needs more is redone with more.
+constexpr uint32_t kServeRounds = 6;
 
 size_t align_up(size_t x) { return (x + kArenaAlign - 1) / kArenaAlign * kArenaAlign; }
 
@@ -133,6 +136,7 @@ struct Lane {
     PinnedBuf<uint2> h_out;
     uint32_t front_cap = 0, hit_cap = 0;  // set from the server's capacities at the first batch
     uint32_t cap_gen = ~0u;  // queue capacities follow the server's settings of this generation
+    uint32_t rounds = kServeRounds;
     uint64_t front0_count = 0;
     uint32_t n_pairs = 0;
     uint64_t n_hits = 0;
@@ -469,7 +473,7 @@ int oibvh_server_s::enqueue_detect(Lane& L)
     // and 1.0 ms; one batch alone takes as long either way).
     a.grid = sm_count(device) * std::max(1, walk_blocks_per_sm() / (int)lanes.size());
     CUDA_TRY(launch_begin(a, 0, st));
-    CUDA_TRY(launch_walk(a, (uint32_t)L.front0_count, 0, kAllRounds, st));
+    CUDA_TRY(launch_walk(a, (uint32_t)L.front0_count, 0, L.rounds, true, st));
     // the hits grouped by query (discarded if the batch is redone)
     const uint32_t bgrid = (uint32_t)sm_count(device) * 2;
     k_bucket_count<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, L.counts.p, L.hit_cap, L.qcount.p);
@@ -509,11 +513,12 @@ int oibvh_server_s::advance(Lane& L)
 {
     if (L.phase == 1) {
         const uint32_t* c = L.h_counts.p;
-        if (c[kCountFlags]) {
-            // queues too small: grow and redo the detect
+        if (c[kCountFlags] || c[kCountLeft]) {
+            // queues too small, or more walk rounds needed: grow and redo the detect
             const uint64_t peak = c[kCountPeak];
             if (c[kCountFlags] & kFlagFrontOverflow) L.front_cap = grow(peak, L.front_cap);
             if (c[kCountFlags] & kFlagHitOverflow) L.hit_cap = grow(c[kCountHits], L.hit_cap);
+            if (c[kCountLeft]) L.rounds += 4;
             if (c[kCountFlags] & ~(uint32_t)(kFlagFrontOverflow | kFlagHitOverflow))
                 return fail(OIBVH_ERR_CUDA, "unexpected traversal flags");
             if (L.front_cap == 0x7fffffffu && (c[kCountFlags] & kFlagFrontOverflow))
