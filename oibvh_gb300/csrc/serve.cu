@@ -22,8 +22,9 @@
 //     the grouped pairs, 8 B each) tracked by events, each query's pairs then
 //     one block copy on the host; the loop never waits on the device while
 //     other work can be launched;
-//   * a batch whose queues or launched walk rounds were too few is redone on
-//     its lane with more, so results are never truncated.
+//   * a batch that needs more walk rounds than were launched goes on on its
+//     lane, one whose queues were too small is redone there with larger ones,
+//     so results are never truncated.
 //
 // A query's pair set does not depend on what it was batched with: the
 // traversal and the triangle test of a pair read only that pair's trees.
@@ -46,9 +47,6 @@ using Clock = std::chrono::steady_clock;
 
 constexpr size_t kArenaAlign = 256;
 static_assert(kArenaAlign % 32 == 0, "node arrays in the arena must be 32-byte aligned (256-bit node loads)");
-
-// Walk rounds launched for a batch (most take three to five); one that needs more is redone with more.
-constexpr uint32_t kServeRounds = 6;
 
 size_t align_up(size_t x) { return (x + kArenaAlign - 1) / kArenaAlign * kArenaAlign; }
 
@@ -136,7 +134,11 @@ struct Lane {
     PinnedBuf<uint2> h_out;
     uint32_t front_cap = 0, hit_cap = 0;  // set from the server's capacities at the first batch
     uint32_t cap_gen = ~0u;  // queue capacities follow the server's settings of this generation
-    uint32_t rounds = kServeRounds;
+    uint32_t rounds = 4;  // walk rounds that go out before the host looks: the most that recent batches took
+    uint32_t walked = 0;  // rounds of this batch so far
+    uint32_t batches = 0;
+    uint32_t turn = 0;    // of two counter blocks: a batch's last round clears the next one's
+    bool clean = false;   // the block of this turn is zero
     uint64_t front0_count = 0;
     uint32_t n_pairs = 0;
     uint64_t n_hits = 0;
@@ -146,7 +148,7 @@ struct Lane {
     {
         OK_TRY(work0.ensure(front_cap, "cudaMalloc(work list)"));
         OK_TRY(work1.ensure(front_cap, "cudaMalloc(work list)"));
-        return counts.ensure(kCountTotal, "cudaMalloc(counts)");
+        return counts.ensure(2 * kCountTotal, "cudaMalloc(counts)");
     }
     ~Lane()
     {
@@ -285,6 +287,7 @@ struct oibvh_server_s {
     int reserve_lanes();
     int launch(Lane& L, std::vector<Query*>& batch);
     int enqueue_detect(Lane& L);
+    int enqueue_rounds(Lane& L, uint32_t n);
     int advance(Lane& L);
     void finish(Lane& L, int status, const std::string& msg);
     size_t slot_bytes(uint32_t b) const
@@ -448,13 +451,21 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
     return enqueue_detect(L);
 }
 
-// Broad + fused narrow phase of the lane's batch; counters copied back.
+// Broad + fused narrow phase of the lane's batch, from the start.
 int oibvh_server_s::enqueue_detect(Lane& L)
 {
-    cudaStream_t st = L.st;
     OK_TRY(L.ensure_lists());
     OK_TRY(L.hits.ensure(L.hit_cap, "cudaMalloc(hits)"));
     OK_TRY(L.out.ensure(L.hit_cap, "cudaMalloc(grouped pairs)"));
+    L.walked = 0;
+    return enqueue_rounds(L, L.rounds);
+}
+
+// The next `n` walk rounds of the lane's batch, its hits so far grouped by query,
+// and the counters copied back.
+int oibvh_server_s::enqueue_rounds(Lane& L, uint32_t n)
+{
+    cudaStream_t st = L.st;
     CUDA_TRY(cudaMemsetAsync(L.qcount.p, 0, L.n_pairs * sizeof(uint32_t), st));
     DetectArgs a{};
     a.pairs = L.pairv.p;
@@ -465,23 +476,29 @@ int oibvh_server_s::enqueue_detect(Lane& L)
     a.work_cap = L.front_cap;
     a.hits = L.hits.p;
     a.hit_cap = L.hit_cap;
-    a.counts = L.counts.p;
+    a.counts = L.counts.p + L.turn * kCountTotal;
+    a.counts_next = L.counts.p + (L.turn ^ 1u) * kCountTotal;
+    a.host = L.h_counts.p;
     a.fuse_narrow = 1;
-    // A lane's share of the CTAs that fit: the walk is a cooperative launch, which starts only when
-    // all of its CTAs do, so with the whole GPU each the lanes' walks queued up (2,000 meshes, four
-    // lanes: 127 k queries/s at most and p99 2.5 ms at 100 k/s; so 150 k, which was all that came,
-    // and 1.0 ms; one batch alone takes as long either way).
+    // A lane's share of the CTAs that fit: the others' batches walk at the same time (2,000 meshes, four
+    // lanes, 100 k queries/s: p99 2.1 ms with the whole GPU each; one batch alone takes as long either way).
     a.grid = sm_count(device) * std::max(1, walk_blocks_per_sm() / (int)lanes.size());
-    CUDA_TRY(launch_begin(a, 0, st));
-    CUDA_TRY(launch_walk(a, (uint32_t)L.front0_count, 0, L.rounds, true, st));
-    // the hits grouped by query (discarded if the batch is redone)
+    // (CTAs scheduled ahead wait where other lanes' batches could run: 150 k queries/s offered, 144 k served
+    // with them, all without; alone, 10 k/s: p50 126 us without them, 120 with)
+    a.ahead = 1;
+    for (auto& o : lanes)
+        if (o.get() != &L && o->phase) a.ahead = 0;
+    if (L.walked == 0 && !L.clean) CUDA_TRY(launch_begin(a, 0, st));
+    L.clean = false;
+    CUDA_TRY(launch_walk(a, (uint32_t)L.front0_count, L.walked, L.walked + n, true, st));
+    L.walked += n;
+    // the hits grouped by query (discarded if the batch goes on or is redone)
     const uint32_t bgrid = (uint32_t)sm_count(device) * 2;
-    k_bucket_count<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, L.counts.p, L.hit_cap, L.qcount.p);
+    k_bucket_count<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, a.counts, L.hit_cap, L.qcount.p);
     k_bucket_scan<<<1, 1024, 0, st>>>(L.qcount.p, L.n_pairs, L.qoff.p, L.qcursor.p);
-    k_bucket_scatter<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, L.counts.p, L.hit_cap, L.qcursor.p, L.out.p);
+    k_bucket_scatter<<<bgrid, kBucketThreads, 0, st>>>(L.hits.p, a.counts, L.hit_cap, L.qcursor.p, L.out.p);
     CUDA_TRY(cudaGetLastError());
     note_launches(3);
-    CUDA_TRY(cudaMemcpyAsync(L.h_counts.p, L.counts.p, kCountHost * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaMemcpyAsync(L.h_qoff.p, L.qoff.p, ((size_t)L.n_pairs + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaEventRecord(L.ev, st));
     L.phase = 1;
@@ -513,12 +530,15 @@ int oibvh_server_s::advance(Lane& L)
 {
     if (L.phase == 1) {
         const uint32_t* c = L.h_counts.p;
-        if (c[kCountFlags] || c[kCountLeft]) {
-            // queues too small, or more walk rounds needed: grow and redo the detect
+        if (!c[kCountFlags] && c[kCountLeft]) return enqueue_rounds(L, 2);  // more rounds needed than were launched
+        L.rounds = std::max(c[kCountRounds], ++L.batches % 32u ? L.rounds : std::max(2u, L.rounds) - 1u);
+        L.turn ^= 1u;
+        L.clean = true;
+        if (c[kCountFlags]) {
+            // queues too small: grow and redo the detect
             const uint64_t peak = c[kCountPeak];
             if (c[kCountFlags] & kFlagFrontOverflow) L.front_cap = grow(peak, L.front_cap);
             if (c[kCountFlags] & kFlagHitOverflow) L.hit_cap = grow(c[kCountHits], L.hit_cap);
-            if (c[kCountLeft]) L.rounds += 4;
             if (c[kCountFlags] & ~(uint32_t)(kFlagFrontOverflow | kFlagHitOverflow))
                 return fail(OIBVH_ERR_CUDA, "unexpected traversal flags");
             if (L.front_cap == 0x7fffffffu && (c[kCountFlags] & kFlagFrontOverflow))

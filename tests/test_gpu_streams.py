@@ -141,3 +141,63 @@ def test_detects_of_several_threads(gpu, precision):
         if isinstance(r, BaseException):
             raise r
         assert r[0] > 0 and r[1] >= r[0]
+
+
+def _dense():
+    """Two soups whose walk takes more rounds than are launched at first."""
+    return [_soup(200000, 1, 0.02), _soup(200000, 2, 0.02)]
+
+
+def test_walks_go_on_for_as_many_rounds_as_they_need(gpu):
+    """A detect's, a frame's and a server batch's first launches cover the
+    rounds of lighter work; the rest follows."""
+    import torch
+
+    from oibvh_gb300 import DeviceType, OibvhTree, Scene, Server
+
+    soups = _dense()
+    trees = [OibvhTree(xyz=x, tri=t) for x, t in soups]
+    for t in trees:
+        t.build()
+    sc = Scene()
+    for t in trees:
+        sc.addOibvhTree(t)
+    sc.detectCollision(DeviceType.GPU0, 4, 3)  # its queues grow
+    want, n = sc.int_tri_pairs(), sc.candidate_count()
+    assert sc.stats()["steps"] > 4 and want.shape[0] > 10000
+
+    fresh = Scene()
+    for t in trees:
+        fresh.addOibvhTree(t)
+    fresh.set_tuning(front_capacity=sc.tuning()["front_capacity"], hit_capacity=sc.tuning()["hit_capacity"])
+    fresh.detectCollision(DeviceType.GPU0, 4, 3)
+    assert fresh.stats()["retries"] == 0
+    assert np.array_equal(fresh.int_tri_pairs(), want) and fresh.candidate_count() == n
+
+    # a frame captured with the bodies apart
+    packed = torch.from_numpy(np.concatenate([np.pad(x, ((0, 0), (0, 1))) for x, _ in soups], 0)).cuda()
+    mats = np.tile(np.eye(3, 4, dtype=np.float32).reshape(12), (2, 1))
+    mats[1, 3] = 100.0
+    d_mats = torch.from_numpy(mats).cuda()
+    fresh.capture_frame(4, 3, True, packed.data_ptr(), d_mats.data_ptr())
+    fresh.launch_frame()
+    fresh.finish_frame()
+    assert fresh.candidate_count() == 0 and fresh.stats()["frame_redos"] == 0
+    mats[1, 3] = 0.0
+    d_mats.copy_(torch.from_numpy(mats))
+    for _ in range(2):  # redone, then captured again
+        fresh.launch_frame()
+        fresh.finish_frame()
+        assert np.array_equal(fresh.int_tri_pairs(), want) and fresh.candidate_count() == n
+
+    server = Server(memory_budget=1 << 30, max_batch=16, lanes=2)
+    ids = [server.add_mesh(t) for t in trees]
+    server.set_queue_capacity(front=sc.tuning()["front_capacity"], hits=sc.tuning()["hit_capacity"])
+    server.start()
+    for b in (1, 3):
+        tickets = [server.submit(ids[0], ids[1], np.eye(3, 4, dtype=np.float32)) for _ in range(b)]
+        for t in tickets:
+            assert int(server.wait(t)["n_pairs"]) == want.shape[0]
+            assert np.array_equal(server.pairs(t), want[:, 2:])
+            server.release(t)
+    server.close()
