@@ -288,7 +288,7 @@ struct oibvh_scene_s {
     uint32_t tune_start_log2 = 16;  // start cross product ~ 2^this node pairs per pass
     uint32_t tune_handoff = 2048;   // kept for callers: the traversal has no separate top walk
     uint32_t precision = 0;         // OIBVH_PRECISION_*
-    uint32_t tune_walk_per_sm = 0;  // walker CTAs per SM, 0 = as many as fit
+    uint32_t tune_walk_per_sm = 0;  // walker CTAs per SM, 0 = by the pass (walk_grid)
     uint32_t tune_walk_cap = 128;   // per-warp front entries of the walkers
     uint32_t tune_refit_log = 10;   // refit level-group depth (levels per CTA: 9, 10 or 11)
     uint32_t tune_descend = 16;     // both sides descend while the boxes' squared diagonals are within it
@@ -434,26 +434,22 @@ bool split_narrow(const PassPlan& plan, uint64_t triangles)
     return plan.pv.size() > 1 && triangles >= kSplitTriangles;
 }
 
-// CTAs of a pass's walk. A cooperative launch starts only when all of its CTAs
-// do, so a grid for the whole GPU keeps the walks of other streams out: with
-// eight threads, a scene and a stream each, two meshes of 20 k triangles came to
-// 46 k detects/s (62 k with several smaller launches), so to 81 k; of 300 k 24 k
-// (51 k), so to 74 k. Alone, one pair of up to 2^20 triangles loses little by one
-// CTA an SM against all that fit (4): 20 k triangles 32.9 and 34.2 us, 300 k 52.1
-// and 53.9, two coincident meshes of 20 k 64 and 57. Larger ones and several
-// pairs take half: one pair of 1 M triangles 67.7 and 68.5 (73 with one an SM),
-// 24 bodies 61.8 and 64, 32 larger ones 89 and 91 (105), 24 coincident ones 700
-// and 574 (1016). From 2^20 triangles on several pairs take all: 64 pairs 282
-// with two, 237 with all. (In precision mode one pair takes half from 2^17 triangles on: 131 k
-// each 113 with one an SM, 95 with two. A count of CTAs that the caller chose stands.)
-constexpr uint64_t kSmallPair = 1u << 20, kSmallExactPair = 1u << 17;
-int walk_grid(const oibvh_scene_s* s, const PassPlan& plan, uint64_t triangles, bool fused)
+// CTAs of a pass's walk: all that fit, half of them for one pair in float mode (a
+// count that the caller chose stands). How much a pass walks depends on how its
+// bodies touch, which nobody knows before, so the rule does not go by their sizes:
+// two coincident meshes of 20 k triangles take 111 us with one CTA an SM, 98 with
+// half (2), 89 with all (4); 24 coincident bodies 1457, 990 and 829; 64 pairs 472,
+// 328 and 267. For one pair that touches lightly half is no slower than all (20 k
+// triangles 34.4 and 34.7 us, 1.31 M 69.4 and 69.5) and leaves room for other
+// streams' walks: eight threads with meshes of 300 k triangles, a scene and a
+// stream each, come to 67 k detects/s with it, to 49 k with all. (In precision mode
+// one pair of 131 k triangles takes 108 us with half, 98 with all.)
+int walk_grid(const oibvh_scene_s* s, const PassPlan& plan, bool fused)
 {
     const int fit = std::max(1, walk_blocks_per_sm(s->tune_walk_cap, fused));
     int per = fit;
     if (s->tune_walk_per_sm) per = std::min<int>(fit, (int)s->tune_walk_per_sm);
-    else if (plan.pv.size() == 1 && triangles < (s->precision ? kSmallExactPair : kSmallPair)) per = 1;
-    else if (plan.pv.size() == 1 || triangles < kSplitTriangles) per = std::max(1, fit / 2);
+    else if (plan.pv.size() == 1 && !s->precision) per = std::max(1, fit / 2);
     return sm_count(s->device) * per;
 }
 
@@ -553,7 +549,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.hit_cap = s->hit_cap;
             a.counts = s->counts.p;
             a.fuse_narrow = fused ? 1u : 0u;
-            a.grid = walk_grid(s, plan, triangles, fused);
+            a.grid = walk_grid(s, plan, fused);
             a.walk_cap = s->tune_walk_cap;
             a.precision = s->precision;
             a.prec_lists = exact ? s->prec_lists.p : nullptr;
@@ -1701,7 +1697,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     a.prec_lists = s->precision ? s->prec_lists.p : nullptr;
     a.fp64_tri = s->precision ? s->fp64_tri.p : nullptr;
     a.fp64_tri_cap = s->precision ? s->fp64_tri_cap : 0u;
-    a.grid = walk_grid(s, plan, triangles, !split);
+    a.grid = walk_grid(s, plan, !split);
     a.walk_cap = s->tune_walk_cap;
     a.precision = s->precision;
     a.claim_min = s->tune_claim;
