@@ -870,7 +870,8 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
     const uint32_t W = gridDim.x * kWarps;
     const uint32_t w = wib * gridDim.x + blockIdx.x;  // neighbouring items go to different SMs
     const uint32_t listed = r == 0 ? total0 : *(volatile uint32_t*)round_slot(a.counts, r);
-    const uint32_t n_src = r == 0 ? total0 : min(listed, a.work_cap);
+    // (a list that was too small: the pass is given up here, and runs again or fails)
+    const uint32_t n_src = r == 0 || listed <= a.work_cap ? listed : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         round_slot(a.counts, r + 2)[0] = 0;
         round_slot(a.counts, r + 2)[kCtlRoundClaim] = 0;
@@ -892,7 +893,7 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
         uint32_t next = w;  // static share: the next item
         bool more = claiming ? n_src > 0 : w < n_src;
         // pairs a warp may queue (the rest goes to the next round): few items, few pairs each
-        const uint32_t cap = claiming ? R - 32u : 32u;
+        const uint32_t cap = claiming || a.stay ? R - 32u : 32u;
         const uint32_t limit = r == 0 && !claiming ? a.start_steps : a.walk_steps;
         uint32_t head = 0, live = 0, steps = 0, tested = 0;
         for (;;) {

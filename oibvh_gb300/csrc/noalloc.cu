@@ -32,8 +32,8 @@ namespace oibvh {
 
 // Fixed capacity of each of the two traversal work lists (BVTT node pairs).
 constexpr uint32_t kNoAllocItems = 1u << 18;
-// Rounds that go out before the host looks whether anything is left (most pairs take three or four).
-constexpr uint32_t kNoAllocRounds = 4;
+// Rounds that go out before the host looks whether anything is left (most pairs take two to four).
+constexpr uint32_t kNoAllocRounds = 3;
 // Header: the counters, rounded up (the pair's record goes with the kernels' arguments).
 constexpr size_t kNoAllocHeader = 4096;
 constexpr size_t kNoAllocBytes = kNoAllocHeader + 2 * (size_t)kNoAllocItems * sizeof(uint64_t);
@@ -152,13 +152,20 @@ extern "C" __attribute__((visibility("default"))) int oibvh_pair_detect_noalloc(
         NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_a));
         args.grid = sms * per_sm;
 
-        NA_CUDA(launch_begin(args, 0, s));
         uint32_t counts[kCountHost];
-        for (uint32_t r = 0;; r += kNoAllocRounds) {
-            NA_CUDA(launch_walk(args, (uint32_t)total0, r, r + kNoAllocRounds, true, s));
-            NA_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
-            NA_CUDA(cudaStreamSynchronize(s));
-            if (counts[kCountFlags] || counts[kCountLeft] == 0) break;
+        for (;;) {
+            NA_CUDA(launch_begin(args, 0, s));
+            for (uint32_t r = 0;; r += kNoAllocRounds) {
+                NA_CUDA(launch_walk(args, (uint32_t)total0, r, r + kNoAllocRounds, true, s));
+                NA_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
+                NA_CUDA(cudaStreamSynchronize(s));
+                if (counts[kCountFlags] || counts[kCountLeft] == 0) break;
+            }
+            // The lists cannot grow. Sharing the pairs out every few steps takes more of them than walking on
+            // from where they are, so a pair whose lists ran over is walked again that way before it is refused.
+            if (!(counts[kCountFlags] & kFlagFrontOverflow) || args.stay) break;
+            args.stay = 1;
+            args.start_steps = args.walk_steps = 0xffffffffu;
         }
         *n_hits = counts[kCountHits];
         if (counts[kCountFlags] & kFlagFrontOverflow)

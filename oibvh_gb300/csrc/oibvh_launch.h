@@ -156,6 +156,8 @@ struct DetectArgs {
     uint32_t walk_steps = 6;   // steps a warp goes on for when its round has nothing more to claim
     uint32_t start_steps = 3;  // the same in a round 0 that is dealt out
     uint32_t claim_min = 1;   // a round's pairs are claimed dynamically from this many per warp
+    uint32_t stay = 0;        // 1: warps keep what their rings hold, also of items dealt out (with steps without end:
+                              // the lists take the fewest pairs, and a pass the longest)
     uint32_t ahead = 1;       // a round's CTAs are scheduled while the round before still runs (launch_walk)
     float descend_ratio = kDescendRatio;  // both sides descend while the boxes' squared diagonals are within it
 };
