@@ -1641,14 +1641,13 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     if (s->frame_rest) OK_TRY(oibvh_scene_transform(s, (const float*)s->frame_rest, s->frame_mats, st));
     if (s->frame_refit) OK_TRY(oibvh_scene_refit(s, st));
     OK_TRY(detect_impl(s, s->device, s->frame_entry, s->frame_expand, full_detect_mode(s), st));
-    // headroom, then the exact tables the graph will read
-    s->front_cap = std::max(s->front_cap, grow_cap(2 * s->stats.front_peak, s->front_cap));
+    // headroom (where a capture before has not left it), then the exact tables the graph will read
+    auto headroom = [](uint64_t used, uint32_t cap) { return 2 * used > cap ? grow_cap(2 * used, cap) : cap; };
+    s->front_cap = headroom(s->stats.front_peak, s->front_cap);
     OK_TRY(ensure_lists(s));
-    if (s->hit_count * 2 > s->hit_cap) {
-        const uint32_t want = grow_cap(2 * s->hit_count, s->hit_cap);
-        OK_TRY(s->hits.ensure(want, "cudaMalloc(hits)"));
-        s->hit_cap = want;
-    }
+    const uint32_t want_hits = headroom(s->hit_count, s->hit_cap);
+    OK_TRY(s->hits.ensure(want_hits, "cudaMalloc(hits)"));
+    s->hit_cap = want_hits;
     PassPlan plan;
     OK_TRY(plan_pass(s, pr.data(), np, s->frame_entry, plan));
     const uint64_t triangles = pass_triangles(s, plan);
@@ -1656,7 +1655,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     if (split) {
         // a narrow phase of its own: the candidates of the whole frame are stored
         const uint32_t cap = s->cand_cap;
-        s->cand_cap = std::max(s->cand_cap, grow_cap(2 * s->cand_count, s->cand_cap));
+        s->cand_cap = headroom(s->cand_count, s->cand_cap);
         const int r = s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)");
         if (r != OIBVH_OK && s->precision) return r;
         if (r != OIBVH_OK) {

@@ -139,3 +139,26 @@ def test_a_build_between_frames_is_followed(gpu, by, n):
         want = other.int_tri_pairs()
         assert want.shape[0] > 0 and np.array_equal(sc.int_tri_pairs(), want)
         assert sc.candidate_count() == other.candidate_count()
+
+
+@pytest.mark.parametrize("sizes,precision", [((400000, 350000, 300000), 0), ((2000, 3000, 2500), 0), ((2000, 3000, 2500), 1)])
+def test_captures_in_a_row_do_not_grow_the_queues(gpu, sizes, precision):
+    """A frame that is captured again (here: because its tuning was set) has the
+    headroom of its last capture; only a larger frame needs more."""
+    import torch
+
+    sc, _ = _scene([_soup(n, n, 0.01) for n in sizes])
+    sc.set_precision(precision)
+
+    def again():
+        sc.set_tuning(descend_ratio=16)
+        sc.launch_frame()
+        sc.finish_frame()
+        return sc.tuning()["front_capacity"], torch.cuda.mem_get_info()[0]
+
+    sc.capture_frame(0, 1, True)
+    front, free = again()
+    for _ in range(6):
+        f, now = again()
+        assert f == front
+        assert free - now < 32 << 20, (free, now)
