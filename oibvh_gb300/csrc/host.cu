@@ -268,6 +268,8 @@ struct oibvh_scene_s {
     uint32_t front_cap = 1u << 20;
     uint32_t cand_cap = 1u << 20;
     uint32_t hit_cap = 1u << 18;
+    bool cands_fit = true;  // false: a float pass' candidates found no room, so that the walk tests them itself
+                            // (until the trees, the pairs or the capacities change)
 
     // multi-tree refit: job table as last uploaded
     DevBuf<RefitJob> refit_jobs;
@@ -325,6 +327,7 @@ struct oibvh_scene_s {
 namespace {
 
 constexpr uint64_t kSplitTriangles = 1ull << 20;  // split_narrow
+constexpr uint32_t kMaxCandidates = 0x7fffffffu;  // grow_cap
 // Hits that come to the host with the counters (64 KB).
 constexpr uint32_t kHostHits = 4096;
 
@@ -528,13 +531,19 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         // (precision mode: the passes follow the walk at once; waiting for its counters first, and copying them
         // back and forth, took 25 us more for one pair of sheets of 131 k triangles)
         const uint64_t triangles = pass_triangles(s, plan);
-        bool split = exact || (narrow && split_narrow(plan, triangles));
+        bool split = exact || (narrow && s->cands_fit && split_narrow(plan, triangles));
+        const uint32_t had_room = s->cand_cap;
+        bool grown = false;
+        auto no_room = [&] {
+            s->cands_fit = split = false;
+            s->cand_cap = had_room;
+        };
         for (int attempt = 0;; ++attempt) {
             if (attempt > 12) return fail(OIBVH_ERR_OVERFLOW, "BVTT queues kept overflowing after regrowing");
             OK_TRY(ensure_lists(s));
             if (exact) OK_TRY(s->prec_lists.ensure(4 * (size_t)s->cand_cap, "cudaMalloc(precision lists)"));
             if (exact || !narrow) OK_TRY(s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)"));
-            else if (split && s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)") != OIBVH_OK) split = false;
+            else if (split && s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)") != OIBVH_OK) no_room();
             const bool fused = narrow && !split;
             DetectArgs a{};
             a.pairs = s->pairv.p;
@@ -606,7 +615,13 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             if (flags) {
                 s->stats.retries++;
                 if (flags & kFlagFrontOverflow) s->front_cap = grow_cap(peak, s->front_cap);
-                if (flags & kFlagCandOverflow) s->cand_cap = grow_cap(c[kCountCandSlots], s->cand_cap);
+                if (flags & kFlagCandOverflow) {
+                    // (the count wraps at 2^32, so a list that a whole walk has measured and that runs over again
+                    // cannot be had either)
+                    if (split && !exact && (c[kCountCandSlots] > kMaxCandidates || grown)) no_room();
+                    else s->cand_cap = grow_cap(c[kCountCandSlots], s->cand_cap);
+                    grown = !(flags & kFlagFrontOverflow);
+                }
                 if (flags & kFlagHitOverflow) {
                     const uint32_t want = grow_cap(c[kCountHits], s->hit_cap);
                     OK_TRY(s->hits.grow_keep(want, hits_before, st, "cudaMalloc(hits)"));
@@ -1016,7 +1031,7 @@ API int oibvh_scene_add_tree(oibvh_scene_t s, oibvh_tree_t t, uint32_t* id)
     // the reference asserts a built tree (src/cuda/scene.cu:97); here a tree may
     // also be added unbuilt and built with the others by oibvh_scene_build
     s->trees.push_back(t);
-    s->frame_stale = true;
+    s->frame_stale = s->cands_fit = true;
     if (id) *id = (uint32_t)(s->trees.size() - 1);
     return OIBVH_OK;
     GUARD_END
@@ -1029,7 +1044,7 @@ API int oibvh_scene_set_pairs(oibvh_scene_t s, const uint32_t* pairs, uint32_t n
     if (!pairs) {
         s->all_pairs = true;
         s->pairs.clear();
-        s->frame_stale = true;
+        s->frame_stale = s->cands_fit = true;
         return OIBVH_OK;
     }
     for (uint32_t i = 0; i < n_pairs; ++i)
@@ -1037,7 +1052,7 @@ API int oibvh_scene_set_pairs(oibvh_scene_t s, const uint32_t* pairs, uint32_t n
             return fail(OIBVH_ERR_ARG, "pair " + std::to_string(i) + " is not two distinct trees of this scene");
     s->all_pairs = false;
     s->pairs.assign(pairs, pairs + 2 * (size_t)n_pairs);
-    s->frame_stale = true;
+    s->frame_stale = s->cands_fit = true;
     return OIBVH_OK;
     GUARD_END
 }
@@ -1175,6 +1190,7 @@ API int oibvh_scene_set_queue_capacity(oibvh_scene_t s, uint32_t front, uint32_t
     }
     if (candidates) {
         s->cand_cap = candidates;
+        s->cands_fit = true;
         s->cand.release();
         s->cands_valid = false;
     }
@@ -1651,7 +1667,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     PassPlan plan;
     OK_TRY(plan_pass(s, pr.data(), np, s->frame_entry, plan));
     const uint64_t triangles = pass_triangles(s, plan);
-    bool split = s->precision || split_narrow(plan, triangles);
+    bool split = s->precision || (s->cands_fit && split_narrow(plan, triangles));
     if (split) {
         // a narrow phase of its own: the candidates of the whole frame are stored
         const uint32_t cap = s->cand_cap;
@@ -1659,7 +1675,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
         const int r = s->cand.ensure(s->cand_cap, "cudaMalloc(candidates)");
         if (r != OIBVH_OK && s->precision) return r;
         if (r != OIBVH_OK) {
-            split = false;
+            s->cands_fit = split = false;
             s->cand_cap = cap;
         }
     }
