@@ -323,7 +323,9 @@ typedef struct oibvh_detect_stats {
     uint64_t fp64_candidates;     /* precision mode: candidates with at least one such axis */
     uint64_t fp32_disagreements;  /* precision mode: candidates where float and FP64 answers differ */
     uint64_t bounded_candidates;  /* precision mode: candidates the plain float test and its margin bound
-                                     left open, which took the bounded float pass */
+                                     left open; those that an axis separates by too little to be sure are
+                                     first tested on that axis in double-float arithmetic, which decides
+                                     most, the others take the bounded float pass on all axes */
 } oibvh_detect_stats;
 int oibvh_scene_get_stats(oibvh_scene_t s, oibvh_detect_stats* out);
 
