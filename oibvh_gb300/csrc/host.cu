@@ -1511,8 +1511,22 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
         if (ms < best) best = ms, b_claim = c;
     }
     s->tune_claim = b_claim;
-    const int fit = walk_blocks_per_sm(b_cap);
-    for (int per = 1; per < fit && st == OIBVH_OK; ++per) {
+    // every count that fits the walker of this scene's passes, but for the one that 0 stands for (timed above)
+    PassPlan plan;
+    bool fused = true;
+    if (st == OIBVH_OK) {
+        std::vector<uint32_t> pr;
+        list_pairs(s, pr);
+        const uint32_t np = (uint32_t)std::min<size_t>(pr.size() / 2, kMaxPairsPerPass);
+        if (np) {
+            st = plan_pass(s, pr.data(), np, entry_level, plan);
+            fused = !s->precision && !(s->cands_fit && split_narrow(plan, pass_triangles(s, plan)));
+        }
+    }
+    const int fit = plan.pv.empty() ? 0 : walk_blocks_per_sm(b_cap, fused);
+    const int automatic = plan.pv.empty() ? 0 : walk_grid(s, plan, fused) / sm_count(s->device);
+    for (int per = 1; per <= fit && st == OIBVH_OK; ++per) {
+        if (per == automatic) continue;
         s->tune_walk_per_sm = (uint32_t)per;
         float ms;
         if (!time_setting(ms)) break;
@@ -1551,7 +1565,7 @@ API int oibvh_scene_autotune(oibvh_scene_t s, uint32_t entry_level, uint32_t rep
     oibvh_tuning bt{};
     bt.start_pairs_log2 = b_start;
     bt.handoff = b_handoff;
-    bt.walk_blocks_per_sm = b_per ? b_per : (uint32_t)walk_blocks_per_sm(b_cap);
+    bt.walk_blocks_per_sm = b_per;
     bt.walk_front = b_cap;
     bt.refit_group_log2 = b_group;
     bt.descend_ratio = b_desc;
