@@ -851,7 +851,7 @@ static int stage_xyz(oibvh_tree_t t, const float* xyz, bool on_device, bool refi
         CUDA_TRY(cudaMemcpyAsync(t->xyz.p, xyz, 3 * (size_t)t->nV * sizeof(float), cudaMemcpyHostToDevice, s));
         src = t->xyz.p;
     }
-    const bool direct = refit && refit_takes_xyz(t->nT);
+    const bool direct = refit && refit_takes_xyz(t->nT, t->nV);
     if (!direct) CUDA_TRY(launch_xyz_to_pos4(src, t->vmap(), t->nV, t->pos4.p, s));
     t->cur_pos = t->pos4.p;
     t->borrowed = nullptr;

@@ -117,7 +117,7 @@ cudaError_t launch_gather_pos4(const float4* src, const uint32_t* vperm, uint32_
 // (9, 10 or 11; 0 = 10, the single-tree refit's)
 uint32_t refit_blocks_for(uint32_t nT, uint32_t group_log2 = 0);
 uint32_t refit_counters_per_tree();
-bool refit_takes_xyz(uint32_t nT);  // whether launch_refit_one should be given `src` rather than converted positions
+bool refit_takes_xyz(uint32_t nT, uint32_t nV);  // whether launch_refit_one should be given `src` rather than converted positions
 cudaError_t launch_refit_one(const RefitJob& job, const RefitSource& src, cudaStream_t s);
 cudaError_t launch_leaf_boxes(const uint4* face, const float4* pos, uint32_t nT, float4* out, cudaStream_t s);
 // block_job: optional host-built map from a refit CTA to its job (nullptr:

@@ -178,9 +178,18 @@ uint32_t refit_blocks_for(uint32_t nT, uint32_t group_log2)
 }
 uint32_t refit_counters_per_tree() { return 4 * kStageCounters; }
 
-// A tree of up to this many faces is refitted from the caller's positions in one launch.
-constexpr uint32_t kRefitXyzMax = 32768;
-bool refit_takes_xyz(uint32_t nT) { return nT <= kRefitXyzMax; }
+// A tree of up to this many faces is refitted from the caller's positions in one
+// launch, if it has no more vertices than faces (a closed mesh has half as many; or
+// a thousand, which one CTA converts as fast as a launch starts). A CTA converts its
+// share of the vertices, and there is one for 1024 faces only: 300 faces over 2948
+// vertices took 19.4 us in one launch and 19.0 in two, over a million 1315 and 22;
+// 4096 faces over 12,288 23.2 and 21.6, over 2050 19.0 (20.9 in two); 32,768 over
+// 98,304 24.2 and 23.9, over 16,386 20.1 (22.8).
+constexpr uint32_t kRefitXyzMax = 32768, kRefitXyzFew = 1024;
+bool refit_takes_xyz(uint32_t nT, uint32_t nV)
+{
+    return nT <= kRefitXyzMax && nV <= (nT < kRefitXyzFew ? kRefitXyzFew : nT);
+}
 
 cudaError_t launch_refit_one(const RefitJob& job, const RefitSource& src, cudaStream_t s)
 {
