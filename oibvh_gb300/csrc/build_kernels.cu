@@ -1034,9 +1034,10 @@ __global__ void __launch_bounds__(256, 8) k_transform_multi(const BuildJob* __re
         if (v >= jobs[j].nV) continue;
         jj[k] = j;
         vv[k] = v;
-        // packed rest positions of all jobs, in the caller's vertex order (through vperm) or the trees'
+        // packed rest positions of all jobs, in the caller's vertex order (through vperm) or the trees',
+        // or (rest == nullptr) each job's own source in the tree's order
         const uint32_t* vp = rest_tree_order ? nullptr : jobs[j].vperm;
-        p[k] = __ldg(rest + jobs[j].vert_off + (vp ? __ldg(vp + v) : v));
+        p[k] = rest ? __ldg(rest + jobs[j].vert_off + (vp ? __ldg(vp + v) : v)) : __ldg(jobs[j].pos + v);
     }
 #pragma unroll
     for (uint32_t k = 0; k < kTransformUnroll; ++k) {

@@ -285,6 +285,7 @@ struct oibvh_scene_s {
     DevBuf<uint32_t> ftile_job, vtile_job;  // kBuildTile-face / -vertex tile -> job
     std::vector<BuildJob> build_cache;
     uint32_t v_blocks = 0, f_tiles = 0, v_tiles = 0, n_faces = 0, n_verts = 0;
+    bool refit_moves = true;  // no tree has many more vertices than its faces can use (transform_refit_takes)
 
     // tuning (oibvh_scene_set_tuning / oibvh_scene_autotune)
     uint32_t tune_start_log2 = 16;  // start cross product ~ 2^this node pairs per pass
@@ -1268,6 +1269,7 @@ int ensure_build_jobs(oibvh_scene_s* s, cudaStream_t st)
     const size_t n = s->trees.size();
     std::vector<BuildJob> jobs(n);
     uint32_t vb = 0, ft = 0, vt = 0, fo = 0, vo = 0;
+    bool moves = true;
     for (size_t i = 0; i < n; ++i) {
         const oibvh_tree_t t = s->trees[i];
         BuildJob j = t->build_job();
@@ -1283,8 +1285,10 @@ int ensure_build_jobs(oibvh_scene_s* s, cudaStream_t st)
             return fail(OIBVH_ERR_ARG, "the scene holds more than 2^32 faces or vertices");
         fo += t->nT;
         vo += t->nV;
+        moves = moves && transform_refit_takes(t->nT, t->nV);
         jobs[i] = j;
     }
+    s->refit_moves = moves;
     s->v_blocks = vb;
     s->f_tiles = ft;
     s->v_tiles = vt;
@@ -1604,7 +1608,7 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
         if (ev && e == cudaSuccess) e = cudaEventRecord(ev[i], st);
     };
     mark(0);
-    const bool together = s->frame_rest && s->frame_refit && transform_refit_pays(s->n_faces);
+    const bool together = s->frame_rest && s->frame_refit && s->refit_moves && transform_refit_pays(s->n_faces);
     if (s->frame_rest && !together && e == cudaSuccess) {
         e = launch_transform_multi(s->build_jobs.p, (uint32_t)s->trees.size(), s->v_blocks, s->vblock_job.p,
                                    s->frame_rest_tree.p, s->frame_mats, true, st);

@@ -103,7 +103,8 @@ cudaError_t launch_build(const BuildArgs& a, cudaStream_t s);
 bool build_is_small(uint32_t nT, uint32_t nV);
 cudaError_t launch_build_small(const BuildJob& job, const TreeShape& shape, float4* box, bool wide, cudaStream_t s);
 // rest: packed positions of all jobs in each caller's vertex order (read
-// through the jobs' vperm), or in each tree's order (rest_tree_order). Writes each job's pos_out.
+// through the jobs' vperm), or in each tree's order (rest_tree_order); nullptr: each job's own pos.
+// Writes each job's pos_out.
 cudaError_t launch_transform_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, const uint32_t* vjob,
                                    const float4* rest, const float* mats, bool rest_tree_order, cudaStream_t s);
 cudaError_t launch_gather_rest_multi(const BuildJob* d_jobs, uint32_t n_jobs, uint32_t v_blocks, const uint32_t* vjob,
@@ -128,6 +129,7 @@ cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total
 cudaError_t launch_transform_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks,
                                    const uint32_t* block_job, uint32_t group_log2, const RefitRest& rest, cudaStream_t s);
 bool transform_refit_pays(uint64_t n_faces);  // whether a captured frame should
+bool transform_refit_takes(uint32_t nT, uint32_t nV);  // whether it should with such a tree (and a server batch)
 
 // detect_kernels.cu
 struct DetectArgs {

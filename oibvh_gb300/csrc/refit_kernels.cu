@@ -229,6 +229,11 @@ cudaError_t launch_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total
 // the launch saved is about 2 us, and a frame's profile keeps the two stages apart.
 constexpr uint64_t kTransformRefitFaces = 1u << 20;
 bool transform_refit_pays(uint64_t n_faces) { return n_faces >= kTransformRefitFaces; }
+// A tree's vertices are moved by the CTAs of its faces, 1024 each: one with many more
+// vertices than its faces can use would keep the others waiting (300 faces over a
+// million vertices: over a millisecond), so that a frame or a server batch with such a
+// tree is moved in a launch of its own.
+bool transform_refit_takes(uint32_t nT, uint32_t nV) { return nV <= (nT < 1024u ? 4096u : 3u * nT); }
 
 cudaError_t launch_transform_refit(const RefitJob* d_jobs, uint32_t n_jobs, uint32_t total_blocks,
                                    const uint32_t* block_job, uint32_t group_log2, const RefitRest& rest, cudaStream_t s)

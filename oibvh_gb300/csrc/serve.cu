@@ -369,7 +369,8 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
     const uint32_t lg = ilog2(std::max(1u, n));
     const uint32_t auto_level = lg >= start_log2 ? 0u : (start_log2 - lg) / 2u;
     uint64_t front0 = 0;
-    uint32_t rblocks = 0;
+    uint32_t rblocks = 0, vblocks = 0;
+    bool refit_moves = true;
     for (uint32_t i = 0; i < n; ++i) {
         Query* q = batch[i];
         const oibvh_tree_t A = pool[q->a];
@@ -404,6 +405,9 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
         j.pos_out = q->pos;
         j.nV = B->nV;
         j.nT = B->nT;
+        j.vblock_begin = vblocks;
+        vblocks += (B->nV + 255) / 256;
+        refit_moves = refit_moves && transform_refit_takes(B->nT, B->nV);
         L.h_jobs.p[i] = j;
         std::memcpy(L.h_mats.p + 12 * (size_t)i, q->mat, 12 * sizeof(float));
         RefitJob r{};
@@ -439,8 +443,13 @@ int oibvh_server_s::launch(Lane& L, std::vector<Query*>& batch)
     CUDA_TRY(cudaMemcpyAsync(L.jobs.p, L.h_jobs.p, n * sizeof(BuildJob), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(L.rjobs.p, L.h_rjobs.p, n * sizeof(RefitJob), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(L.mats.p, L.h_mats.p, 12 * n * sizeof(float), cudaMemcpyHostToDevice, st));
-    // a batch has few jobs: the CTAs binary-search them (no block map)
-    CUDA_TRY(launch_transform_refit(L.rjobs.p, n, rblocks, nullptr, 0, RefitRest{L.jobs.p, nullptr, L.mats.p}, st));
+    // a batch has few jobs: the CTAs binary-search them (no block maps)
+    if (refit_moves) {
+        CUDA_TRY(launch_transform_refit(L.rjobs.p, n, rblocks, nullptr, 0, RefitRest{L.jobs.p, nullptr, L.mats.p}, st));
+    } else {
+        CUDA_TRY(launch_transform_multi(L.jobs.p, n, vblocks, nullptr, nullptr, L.mats.p, false, st));
+        CUDA_TRY(launch_refit(L.rjobs.p, n, rblocks, nullptr, 0, st));
+    }
     L.batch = batch;
     const auto now = Clock::now();
     for (uint32_t i = 0; i < n; ++i) {
