@@ -71,6 +71,12 @@ int oibvh_debug_fail_alloc_after(int64_t n);
 /* Device and pinned-host allocations attempted so far (process-wide). */
 uint64_t oibvh_debug_alloc_attempts(void);
 
+/* Test hook for the waits between a build's tiles: how often a tile of the
+ * builds from now on looks for its predecessors' counts before the build is
+ * given up with OIBVH_ERR_TIMEOUT (0: at the first look that does not find
+ * them; 0xffffffff: the default, about a second). Process-wide. */
+int oibvh_debug_set_build_polls(uint32_t n);
+
 /* ------------------------------------------------------------------ tree */
 
 /* OibvhTree::OibvhTree(std::shared_ptr<Mesh>) + setup()

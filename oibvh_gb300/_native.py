@@ -102,6 +102,7 @@ SIGNATURES = [
     ("oibvh_get_launch_count", _u64, []),
     ("oibvh_debug_fail_alloc_after", ctypes.c_int, [ctypes.c_int64]),
     ("oibvh_debug_alloc_attempts", _u64, []),
+    ("oibvh_debug_set_build_polls", ctypes.c_int, [ctypes.c_uint32]),
     ("oibvh_tree_create", ctypes.c_int, [_f32p, _u32, _u32p, _u32, ctypes.c_int, ctypes.POINTER(_vp)]),
     ("oibvh_tree_create_copy", ctypes.c_int, [_vp, _f32p, _u32, ctypes.POINTER(_vp)]),
     ("oibvh_tree_build", ctypes.c_int, [_vp, _vp]),

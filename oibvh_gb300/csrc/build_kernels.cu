@@ -135,7 +135,6 @@ __device__ __forceinline__ void morton_key(const float u[3], bool wide, uint32_t
 constexpr uint32_t kNoUse = 0xffffffffu;
 constexpr uint32_t kTileWords = 3 * kBuildTile / 32;  // a bit per face corner of a tile
 constexpr uint32_t kStateSum = 1u << 30, kStateTotal = 2u << 30, kStateValue = kStateSum - 1u;
-constexpr uint32_t kLookbackPolls = 1u << 20;
 
 __device__ __forceinline__ const BuildJob& job_of(const BuildArgs& a, const uint32_t* map, uint32_t tile, uint32_t& j)
 {
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_build_sort(const __grid_con
                 done = (v[q] & kStateTotal) != 0;
                 --k;
             }
-            if (!done && ++polls > kLookbackPolls) {
+            if (!done && ++polls > a.polls) {
                 s_bad = 1;
                 break;
             }
@@ -454,7 +453,7 @@ __device__ __forceinline__ bool lookback(const BuildArgs& a, uint32_t* state, ui
         const uint32_t empty = __ballot_sync(0xffffffffu, v == 0), total = __ballot_sync(0xffffffffu, (v & kStateTotal) != 0);
         const uint32_t upto = total ? (uint32_t)__ffs(total) - 1u : 31u;  // lanes 0 .. upto count
         if (empty & (0xffffffffu >> (31u - upto))) {
-            if (++polls > kLookbackPolls) return false;
+            if (++polls > a.polls) return false;
             continue;
         }
         before += __reduce_add_sync(0xffffffffu, lane <= upto ? v & kStateValue : 0u);

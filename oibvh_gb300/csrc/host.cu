@@ -59,6 +59,7 @@ namespace oibvh_host {
 thread_local std::string g_last_error;
 std::atomic<int64_t> g_fail_alloc{-1};
 std::atomic<uint64_t> g_alloc_attempts{0};
+std::atomic<uint32_t> g_build_polls{oibvh::kLookbackPolls};
 std::atomic<uint64_t> g_builds{0};
 }  // namespace oibvh_host
 
@@ -195,6 +196,7 @@ static int build_impl(BuildArgs& a, uint32_t n_jobs, uint32_t n_faces, uint32_t 
 {
     a.host_error = build_error_word();
     if (!a.host_error) return fail(OIBVH_ERR_OOM, "cudaHostAlloc(build error words)");
+    a.polls = g_build_polls.load(std::memory_order_relaxed);
     // Tiles for at most half of the SMs are cut in two for the sort: a pass is then a tile's
     // own chain of loads, ranks and look-back, not throughput (30-bit keys, whole builds:
     // 5 k faces 94 to 84 us, 150 k 109 to 100, 300 k 116 to 115; 500 k would take 143, not 138).
@@ -777,6 +779,12 @@ API uint64_t oibvh_get_launch_count(void) { return g_launches.load(std::memory_o
 API int oibvh_debug_fail_alloc_after(int64_t n)
 {
     g_fail_alloc.store(n < 0 ? -1 : n, std::memory_order_relaxed);
+    return OIBVH_OK;
+}
+
+API int oibvh_debug_set_build_polls(uint32_t n)
+{
+    g_build_polls.store(n == 0xffffffffu ? kLookbackPolls : n, std::memory_order_relaxed);
     return OIBVH_OK;
 }
 

@@ -24,6 +24,8 @@ extern thread_local std::string g_last_error;
 // cudaErrorMemoryAllocation without calling CUDA, then the hook is off again.
 extern std::atomic<int64_t> g_fail_alloc;
 extern std::atomic<uint64_t> g_alloc_attempts;  // device + pinned allocation attempts
+// Polls of a build's waits between tiles (oibvh_debug_set_build_polls).
+extern std::atomic<uint32_t> g_build_polls;
 // Builds begun of any tree: a captured frame looks its trees over only when it has changed.
 extern std::atomic<uint64_t> g_builds;
 inline bool injected_alloc_failure()

@@ -82,6 +82,7 @@ struct BuildScratch {
     uint32_t *first, *inv, *vperm_new; // n_verts: first-use slot, new number, caller-order map in the new order
     float4* pos_new;                   // n_verts
 };
+constexpr uint32_t kLookbackPolls = 1u << 20;
 struct BuildArgs {
     const BuildJob* jobs;   // one job: nullptr, and the job in `one`
     BuildJob one;
@@ -90,6 +91,7 @@ struct BuildArgs {
     uint32_t half_tiles;    // the sort's tiles are of kBuildTile / 2 faces
     uint32_t passes;        // 4: the reference's 30-bit keys; 8: 63 bits (21 per axis)
     uint32_t* host_error;   // pinned word, set when the build gave up
+    uint32_t polls;         // looks at a tile's predecessors before it gives up (kLookbackPolls: about a second)
     BuildScratch sc;
 };
 // Bytes of the build's scratch, and its parts set from `p`.
