@@ -61,6 +61,7 @@ std::atomic<int64_t> g_fail_alloc{-1};
 std::atomic<uint64_t> g_alloc_attempts{0};
 std::atomic<uint32_t> g_build_polls{oibvh::kLookbackPolls};
 std::atomic<uint64_t> g_builds{0};
+std::atomic<int64_t> g_trees{0};
 }  // namespace oibvh_host
 
 // What builds keep between calls, for each context they have run in (gone with it).
@@ -69,8 +70,9 @@ struct BuildContext {
     uint32_t* errors = nullptr;  // a pinned page of error words
     uint32_t next = 0;
 };
-static std::mutex g_build_mu;
-static std::map<unsigned long long, BuildContext> g_build_contexts;
+// (never destroyed: trees may outlive the statics of a program that ends)
+static std::mutex& g_build_mu = *new std::mutex;
+static std::map<unsigned long long, BuildContext>& g_build_contexts = *new std::map<unsigned long long, BuildContext>;
 
 // The current context's id, with a context made where this thread has none yet.
 static unsigned long long context_id()
@@ -103,6 +105,13 @@ cudaMemPool_t scratch_pool(int dev)
         c.pool = pool;
     }
     return c.pool;
+}
+
+void release_scratch()
+{
+    std::lock_guard<std::mutex> lock(g_build_mu);
+    auto c = g_build_contexts.find(current_context_id());
+    if (c != g_build_contexts.end() && c->second.pool) cudaMemPoolTrimTo(c->second.pool, 0);
 }
 }  // namespace oibvh_host
 

@@ -28,6 +28,7 @@ extern std::atomic<uint64_t> g_alloc_attempts;  // device + pinned allocation at
 extern std::atomic<uint32_t> g_build_polls;
 // Builds begun of any tree: a captured frame looks its trees over only when it has changed.
 extern std::atomic<uint64_t> g_builds;
+extern std::atomic<int64_t> g_trees;  // trees alive
 inline bool injected_alloc_failure()
 {
     g_alloc_attempts.fetch_add(1, std::memory_order_relaxed);
@@ -87,6 +88,19 @@ inline int sm_count(int dev)
     return n;
 }
 
+// The scratch that builds keep between calls, back to the device (what no build is using).
+void release_scratch();
+
+// cudaMalloc, or the scratch's memory where there is none left.
+inline cudaError_t device_malloc(void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    release_scratch();
+    return cudaMalloc(p, bytes);
+}
+
 template <class T>
 struct DevBuf {
     T* p = nullptr;
@@ -107,7 +121,7 @@ struct DevBuf {
         if (want <= n && p) return OIBVH_OK;
         release();
         if (want == 0) want = 1;
-        cudaError_t e = injected_alloc_failure() ? cudaErrorMemoryAllocation : cudaMalloc(&p, want * sizeof(T));
+        cudaError_t e = injected_alloc_failure() ? cudaErrorMemoryAllocation : device_malloc((void**)&p, want * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
             cudaGetLastError();
@@ -121,7 +135,7 @@ struct DevBuf {
     {
         if (want <= n && p) return OIBVH_OK;
         T* q = nullptr;
-        cudaError_t e = injected_alloc_failure() ? cudaErrorMemoryAllocation : cudaMalloc(&q, want * sizeof(T));
+        cudaError_t e = injected_alloc_failure() ? cudaErrorMemoryAllocation : device_malloc((void**)&q, want * sizeof(T));
         if (e != cudaSuccess) {
             cudaGetLastError();
             return cuda_fail(e, what);
@@ -147,7 +161,8 @@ struct DevBuf {
 
 // Scratch memory for one call, stream-ordered, from a pool of its own per
 // context that keeps up to 512 MB between calls (cudaMalloc and cudaFree of a
-// call's scratch cost more than a small build, and synchronise the device).
+// call's scratch cost more than a small build, and synchronise the device), until
+// the last tree is destroyed or memory runs out.
 cudaMemPool_t scratch_pool(int dev);  // nullptr: none could be made
 struct PoolBuf {
     uint8_t* p = nullptr;
@@ -212,6 +227,11 @@ using namespace oibvh;
 // Tree
 // ============================================================================
 struct oibvh_tree_s {
+    oibvh_tree_s() { g_trees.fetch_add(1, std::memory_order_relaxed); }
+    ~oibvh_tree_s()
+    {
+        if (g_trees.fetch_sub(1, std::memory_order_relaxed) == 1) release_scratch();
+    }
     int device = 0;
     uint32_t nV = 0, nT = 0;
     TreeShape shape{};

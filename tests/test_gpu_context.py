@@ -132,3 +132,34 @@ def test_a_build_that_gets_no_memory_fails_alone(gpu):
             check(t)
         print("done")
     ''')
+
+
+def test_the_last_tree_gives_the_scratch_back(gpu):
+    _run('''
+        import numpy as np, torch
+        from oibvh_gb300 import OibvhTree
+
+        rng = np.random.default_rng(1)
+        small = OibvhTree(xyz=rng.uniform(-1, 1, (30, 3)).astype(np.float32), tri=np.arange(30, dtype=np.uint32).reshape(-1, 3))
+        small.build()
+        torch.cuda.synchronize()
+        n = 4000000
+        xyz = rng.uniform(-1, 1, (n // 2, 3)).astype(np.float32)
+        tri = rng.integers(0, n // 2, (n, 3)).astype(np.uint32)
+        warm = OibvhTree(xyz=xyz[:9000], tri=np.arange(9000, dtype=np.uint32).reshape(-1, 3))
+        warm.build()
+        free = torch.cuda.mem_get_info()[0]
+        for _ in range(2):
+            t = OibvhTree(xyz=xyz, tri=tri)
+            t.build()
+            t.close()
+        kept = free - torch.cuda.mem_get_info()[0]
+        assert 32 << 20 < kept < 768 << 20, kept  # kept for the next build, within its bound
+        warm.close()
+        small.close()
+        kept = free - torch.cuda.mem_get_info()[0]
+        assert kept < 32 << 20, kept
+        t = OibvhTree(xyz=xyz, tri=tri)  # and had again
+        t.build()
+        print("done")
+    ''')
