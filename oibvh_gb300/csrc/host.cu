@@ -270,7 +270,8 @@ struct oibvh_scene_s {
     DevBuf<uint32_t> walk_counts;  // two counter blocks, in turn between direct detects: each clears the other one
     uint32_t walk_turn = 0;
     bool walk_clean = false;       // the block of this turn is zero
-    uint32_t walk_rounds = 4;      // walk rounds that go out before the host looks: as many as the last detect took
+    uint32_t walk_rounds = 4;      // walk rounds that go out before the host looks: the most that recent detects took
+    uint32_t walks = 0;
     PinnedBuf<PairView> h_pairs;
     PinnedBuf<uint32_t> h_counts;
     PinnedBuf<uint4> h_hits;       // the last detect's hits, when there are at most kHostHits
@@ -621,7 +622,8 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
                     s->walk_turn ^= 1u;
                 }
             }
-            s->walk_rounds = std::max(1u, c[kCountRounds]);
+            // (how many a pass takes varies by one; one too many costs it 1 us, one too few 10)
+            s->walk_rounds = std::max(c[kCountRounds], ++s->walks % 32u ? s->walk_rounds : std::max(2u, s->walk_rounds) - 1u);
             const uint32_t flags = c[kCountFlags], rounds = c[kCountRounds];
             const uint64_t peak = c[kCountPeak];
             if (flags) {
