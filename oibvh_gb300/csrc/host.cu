@@ -834,7 +834,6 @@ API int oibvh_tree_create_copy(oibvh_tree_t other, const float* xyz, uint32_t n_
         }
         if (e == cudaSuccess) e = cudaMemcpy(t->xyz.p, xyz, 3 * (size_t)t->nV * sizeof(float), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = launch_xyz_to_pos4(t->xyz.p, t->vmap(), t->nV, t->pos4.p, 0);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         if (e == cudaSuccess)
             e = cudaMemcpy(t->tri.p, other->tri.p, 3 * (size_t)t->nT * sizeof(uint32_t), cudaMemcpyDeviceToDevice);
         if (e == cudaSuccess)
@@ -842,6 +841,7 @@ API int oibvh_tree_create_copy(oibvh_tree_t other, const float* xyz, uint32_t n_
         if (e == cudaSuccess)
             e = cudaMemcpy(t->box.p, other->box.p, 2 * (size_t)(t->shape.size - t->nT) * sizeof(float4),
                            cudaMemcpyDeviceToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // (copies on the device return before they are done)
         if (e != cudaSuccess) st = cuda_fail(e, "cudaMemcpy(copy tree)");
     }
     if (st != OIBVH_OK) {
