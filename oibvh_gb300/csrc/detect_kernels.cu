@@ -1028,7 +1028,9 @@ __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32
         s_last = atomicInc(a.counts + kCtlDone, gridDim.x - 1u) == gridDim.x - 1u;  // (wraps to 0)
         if (s_last) {
             __threadfence();
-            a.counts[kCountLeft] = __ldcg(round_slot(a.counts, r + 1));
+            const uint32_t left = __ldcg(round_slot(a.counts, r + 1));
+            a.counts[kCountLeft] = left;
+            a.counts[kCountPeak] = max(__ldcg(a.counts + kCountPeak), left);  // (no next round to note it)
             __threadfence();
         }
     }

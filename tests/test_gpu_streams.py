@@ -201,3 +201,26 @@ def test_walks_go_on_for_as_many_rounds_as_they_need(gpu):
             assert np.array_equal(server.pairs(t), want[:, 2:])
             server.release(t)
     server.close()
+
+
+def test_a_list_that_runs_over_in_the_last_round_is_measured(gpu):
+    """Its size is known although no further round was launched: the queue is
+    grown to it, not doubled until it fits."""
+    from oibvh_gb300 import DeviceType
+
+    near = _soup(3000, 5, 0.4)
+    sc = _scene([near, _soup(3000, 6, 0.4)])
+    apart = (near[0] + np.float32(50.0)).astype(np.float32)
+    sc._trees[0].refit(apart)
+    for _ in range(140):  # light detects: fewer and fewer rounds are launched
+        sc.detectCollision(DeviceType.GPU0, 4, 3)
+    assert sc.candidate_count() == 0
+    sc.set_queue_capacity(front=16)
+    sc._trees[0].refit(near[0])
+    sc.detectCollision(DeviceType.GPU0, 4, 3)
+    st = sc.stats()
+    assert st["front_peak"] > 30000  # eleven doublings from 16
+    assert st["retries"] <= 4
+    want = _scene([near, _soup(3000, 6, 0.4)])
+    want.detectCollision(DeviceType.GPU0, 4, 3)
+    assert sc.candidate_count() == want.candidate_count() and np.array_equal(sc.int_tri_pairs(), want.int_tri_pairs())
