@@ -238,8 +238,8 @@ int oibvh_scene_transform(oibvh_scene_t s, const float* d_rest_xyzw, const float
 typedef struct oibvh_tuning {
     uint32_t start_pairs_log2;    /* start cross product ~ 2^this node pairs per pass (8..24, default 16) */
     uint32_t handoff;             /* 32..8192 (2048); no effect: the traversal has no separate top walk */
-    uint32_t walk_blocks_per_sm;  /* walker CTAs per SM, 0 = by the pass (half of what fits for one pair in float
-                                     mode, else as many as fit) */
+    uint32_t walk_blocks_per_sm;  /* walker CTAs per SM, 0 = by the pass (as many as fit where the scene's last pass
+                                     tested many node pairs, else half as many) */
     uint32_t front_capacity;      /* starting work-list capacity (entries), 0 = keep */
     uint32_t hit_capacity;        /* starting hit-queue capacity (records), 0 = keep */
     uint32_t walk_front;          /* per-warp queue of the walkers, node pairs (multiple of 32, <= 512, at least 64 used; 128; 0 = keep) */

@@ -270,8 +270,8 @@ struct oibvh_scene_s {
     DevBuf<uint32_t> walk_counts;  // two counter blocks, in turn between direct detects: each clears the other one
     uint32_t walk_turn = 0;
     bool walk_clean = false;       // the block of this turn is zero
-    uint32_t walk_rounds = 4;      // walk rounds that go out before the host looks: the most that recent detects took
-    uint32_t walks = 0;
+    WalkRounds walk_rounds;
+    uint32_t tested = 0;           // node pairs that the last pass tested (0: none yet)
     PinnedBuf<PairView> h_pairs;
     PinnedBuf<uint32_t> h_counts;
     PinnedBuf<uint4> h_hits;       // the last detect's hits, when there are at most kHostHits
@@ -341,6 +341,7 @@ namespace {
 
 constexpr uint64_t kSplitTriangles = 1ull << 20;  // split_narrow
 constexpr uint32_t kMaxCandidates = 0x7fffffffu;  // grow_cap
+constexpr uint32_t kMuchOnePair = 3u << 18, kMuchTested = 1u << 21;  // walk_grid
 // Hits that come to the host with the counters (64 KB).
 constexpr uint32_t kHostHits = 4096;
 
@@ -450,22 +451,24 @@ bool split_narrow(const PassPlan& plan, uint64_t triangles)
     return plan.pv.size() > 1 && triangles >= kSplitTriangles;
 }
 
-// CTAs of a pass's walk: all that fit, half of them for one pair in float mode (a
-// count that the caller chose stands). How much a pass walks depends on how its
-// bodies touch, which nobody knows before, so the rule does not go by their sizes:
-// two coincident meshes of 20 k triangles take 111 us with one CTA an SM, 98 with
-// half (2), 89 with all (4); 24 coincident bodies 1457, 990 and 829; 64 pairs 472,
-// 328 and 267. For one pair that touches lightly half is no slower than all (20 k
-// triangles 34.4 and 34.7 us, 1.31 M 69.4 and 69.5) and leaves room for other
-// streams' walks: eight threads with meshes of 300 k triangles, a scene and a
-// stream each, come to 67 k detects/s with it, to 49 k with all. (In precision mode
-// one pair of 131 k triangles takes 108 us with half, 98 with all.)
+// CTAs of a pass's walk: all that fit (4 an SM) where the scene's last pass has
+// tested many node pairs, half of them otherwise, and a count that the caller chose
+// in any case. How much a pass walks depends on how its bodies touch, not on their
+// sizes; before the first one the sizes have to do. us a detect with half and with all,
+// by pairs tested: one pair of 0.06 M 34.8 and 35.9, 0.19 M 53.4 and 54.5, 0.89 M
+// (sheets, precision mode) 110 and 99, 1.2 M 99 and 89, 4.9 M 179 and 196, 19 M 437
+// and 410, 77 M 1479 and 1173; several pairs of 0.3 M 66.5 and 68.2, 0.8 M 82 and 84,
+// 1.9 M 117 and 112, 5.8 M 172 and 160, 69 M 973 and 814; frames of 0.6 M and 1.9 M
+// walk as long with either. Half leaves room for other streams' walks: eight threads,
+// each with a scene and a stream, come to 67 k and 49 k detects/s with pairs of 0.19 M,
+// to 18.7 k and 16.4 k frames/s of 0.6 M, 14.4 k and 12.3 k of 1.9 M.
 int walk_grid(const oibvh_scene_s* s, const PassPlan& plan, bool fused)
 {
     const int fit = std::max(1, walk_blocks_per_sm(s->tune_walk_cap, fused));
-    int per = fit;
+    const bool one = plan.pv.size() == 1;
+    const bool much = s->tested ? s->tested >= (one ? kMuchOnePair : kMuchTested) : !one && pass_triangles(s, plan) >= kSplitTriangles;
+    int per = much ? fit : std::max(1, fit / 2);
     if (s->tune_walk_per_sm) per = std::min<int>(fit, (int)s->tune_walk_per_sm);
-    else if (plan.pv.size() == 1 && !s->precision) per = std::max(1, fit / 2);
     return sm_count(s->device) * per;
 }
 
@@ -584,7 +587,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.host_hits = s->h_hits.p;
             a.host_hit_cap = narrow ? kHostHits : 0u;
             const uint32_t* c = s->h_counts.p;
-            const uint32_t batch = s->walk_rounds;
+            const uint32_t batch = s->walk_rounds.count();
             if (split) {
                 DetectArgs n = a;
                 n.grid = sm_count(s->device) * 8;
@@ -596,7 +599,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
                 CUDA_TRY(launch_publish(a, st));
                 CUDA_TRY(cudaStreamSynchronize(st));
                 if (!c[kCountFlags] && c[kCountLeft]) {  // candidates are missing: again, with more rounds
-                    s->walk_rounds = batch + 8;
+                    s->walk_rounds.took(batch + 8);
                     continue;
                 }
             } else {
@@ -622,8 +625,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
                     s->walk_turn ^= 1u;
                 }
             }
-            // (how many a pass takes varies by one; one too many costs it 1 us, one too few 10)
-            s->walk_rounds = std::max(c[kCountRounds], ++s->walks % 32u ? s->walk_rounds : std::max(2u, s->walk_rounds) - 1u);
+            s->walk_rounds.took(c[kCountRounds]);
             const uint32_t flags = c[kCountFlags], rounds = c[kCountRounds];
             const uint64_t peak = c[kCountPeak];
             if (flags) {
@@ -644,6 +646,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
                 continue;
             }
             s->stats.nodes_tested += c[kCountTested];
+            s->tested = std::max(1u, c[kCountTested]);
             s->stats.fp64_axes += c[kCountFp64Axes];
             s->stats.fp64_candidates += c[kCountFp64Cands];
             s->stats.fp32_disagreements += c[kCountDisagree];
@@ -1647,7 +1650,11 @@ cudaError_t enqueue_frame(oibvh_scene_s* s, cudaStream_t st, cudaEvent_t* ev, ui
     if (e == cudaSuccess) e = launch_begin(a, 0, st);
     ++k;
     mark(3);
-    if (e == cudaSuccess) e = launch_walk(a, s->frame_front0, 0, s->frame_rounds, true, st);
+    if (e == cudaSuccess) e = launch_walk(a, s->frame_front0, 0, s->frame_rounds - 1, false, st);
+    // the round that the warm-up frame did not need, usually with nothing to walk: a CTA an SM
+    DetectArgs spare = a;
+    spare.grid = std::min(a.grid, sm_count(s->device));
+    if (e == cudaSuccess) e = launch_walk(spare, s->frame_front0, s->frame_rounds - 1, s->frame_rounds, true, st);
     k += s->frame_rounds;
     mark(4);
     if (!a.fuse_narrow && e == cudaSuccess) {

@@ -189,6 +189,21 @@ struct PoolBuf {
     }
 };
 
+// How many walk rounds go out before the host looks whether any is left: the most
+// that the last 8 to 16 walks took. It varies by one from walk to walk; one too many
+// costs 1 to 2 us, one too few a second trip to the host, 10.
+struct WalkRounds {
+    uint32_t now = 0, before = 0, n = 0;
+    uint32_t count() const { return std::max(now, before) ? std::max(now, before) : 4u; }
+    void took(uint32_t rounds)
+    {
+        now = std::max(now, std::max(1u, rounds));
+        if (++n % 8u) return;
+        before = now;
+        now = 0;
+    }
+};
+
 template <class T>
 struct PinnedBuf {
     T* p = nullptr;

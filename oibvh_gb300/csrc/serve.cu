@@ -134,9 +134,8 @@ struct Lane {
     PinnedBuf<uint2> h_out;
     uint32_t front_cap = 0, hit_cap = 0;  // set from the server's capacities at the first batch
     uint32_t cap_gen = ~0u;  // queue capacities follow the server's settings of this generation
-    uint32_t rounds = 4;  // walk rounds that go out before the host looks: the most that recent batches took
+    WalkRounds rounds;
     uint32_t walked = 0;  // rounds of this batch so far
-    uint32_t batches = 0;
     uint32_t turn = 0;    // of two counter blocks: a batch's last round clears the next one's
     bool clean = false;   // the block of this turn is zero
     uint64_t front0_count = 0;
@@ -467,7 +466,7 @@ int oibvh_server_s::enqueue_detect(Lane& L)
     OK_TRY(L.hits.ensure(L.hit_cap, "cudaMalloc(hits)"));
     OK_TRY(L.out.ensure(L.hit_cap, "cudaMalloc(grouped pairs)"));
     L.walked = 0;
-    return enqueue_rounds(L, L.rounds);
+    return enqueue_rounds(L, L.rounds.count());
 }
 
 // The next `n` walk rounds of the lane's batch, its hits so far grouped by query,
@@ -540,7 +539,7 @@ int oibvh_server_s::advance(Lane& L)
     if (L.phase == 1) {
         const uint32_t* c = L.h_counts.p;
         if (!c[kCountFlags] && c[kCountLeft]) return enqueue_rounds(L, 2);  // more rounds needed than were launched
-        L.rounds = std::max(c[kCountRounds], ++L.batches % 32u ? L.rounds : std::max(2u, L.rounds) - 1u);
+        L.rounds.took(c[kCountRounds]);
         L.turn ^= 1u;
         L.clean = true;
         if (c[kCountFlags]) {
