@@ -550,6 +550,7 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
         bool split = exact || (narrow && s->cands_fit && split_narrow(plan, triangles));
         const uint32_t had_room = s->cand_cap;
         bool grown = false;
+        uint32_t more_rounds = 0;
         auto no_room = [&] {
             s->cands_fit = split = false;
             s->cand_cap = had_room;
@@ -587,19 +588,20 @@ int detect_impl(oibvh_scene_s* s, int device_type, uint32_t entry, uint32_t expa
             a.host_hits = s->h_hits.p;
             a.host_hit_cap = narrow ? kHostHits : 0u;
             const uint32_t* c = s->h_counts.p;
-            const uint32_t batch = s->walk_rounds.count();
+            // (a pass with a narrow phase behind it runs again when it lacks a round: one more, and more at first)
+            const uint32_t batch = !split ? s->walk_rounds.count() : s->walk_rounds.n ? s->walk_rounds.count() + 1 + more_rounds : 8 + more_rounds;
             if (split) {
                 DetectArgs n = a;
                 n.grid = sm_count(s->device) * 8;
                 CUDA_TRY(launch_begin(a, (uint32_t)hits_before, st));
                 DetectArgs w = a;
                 w.host = nullptr;
-                CUDA_TRY(launch_walk(w, front0, 0, batch + 1, true, st));  // (one more: a pass that lacks one runs again)
+                CUDA_TRY(launch_walk(w, front0, 0, batch, true, st));
                 CUDA_TRY(launch_narrow(n, st));
                 CUDA_TRY(launch_publish(a, st));
                 CUDA_TRY(cudaStreamSynchronize(st));
                 if (!c[kCountFlags] && c[kCountLeft]) {  // candidates are missing: again, with more rounds
-                    s->walk_rounds.took(batch + 8);
+                    more_rounds += 8;
                     continue;
                 }
             } else {
