@@ -224,3 +224,31 @@ def test_a_list_that_runs_over_in_the_last_round_is_measured(gpu):
     want = _scene([near, _soup(3000, 6, 0.4)])
     want.detectCollision(DeviceType.GPU0, 4, 3)
     assert sc.candidate_count() == want.candidate_count() and np.array_equal(sc.int_tri_pairs(), want.int_tri_pairs())
+
+
+@pytest.mark.parametrize("sizes,precision", [((420000, 400000, 300000), 0), ((200000, 200000), 1), ((3000, 2500, 2000), 1)])
+def test_passes_with_a_narrow_phase_behind_them_run_again(gpu, sizes, precision):
+    """After light passes too few rounds are launched for a heavy one: its
+    narrow phase must not take what the walk has found so far for all of it."""
+    from oibvh_gb300 import DeviceType
+
+    near = [_soup(n, 60 + i, 0.01 if n > 10000 else 0.2) for i, n in enumerate(sizes)]
+    scenes = [_scene(near) for _ in range(2)]
+    for sc in scenes:
+        sc.set_precision(precision)
+    sc, other = scenes
+    other.detectCollision(DeviceType.GPU0, 4, 3)
+    want, n, steps = other.int_tri_pairs(), other.candidate_count(), other.stats()["steps"]
+    assert want.shape[0] > 0 and steps > 2
+    sc.set_tuning(front_capacity=other.tuning()["front_capacity"])
+    for _ in range(2):
+        for i, t in enumerate(sc._trees):
+            t.refit((near[i][0] + np.float32(50.0 * i)).astype(np.float32))
+        for _ in range(20):
+            sc.detectCollision(DeviceType.GPU0, 4, 3)
+            assert sc.candidate_count() == 0
+        for i, t in enumerate(sc._trees):
+            t.refit(near[i][0])
+        for _ in range(2):
+            sc.detectCollision(DeviceType.GPU0, 4, 3)
+            assert sc.candidate_count() == n and np.array_equal(sc.int_tri_pairs(), want)
