@@ -1936,7 +1936,7 @@ cudaError_t launch_walk(const DetectArgs& a, uint32_t total0, uint32_t from, uin
     cfg.attrs = &attr;
     for (uint32_t r = from; r < to && e == cudaSuccess; ++r) {
         note_launches(1);
-        cfg.numAttrs = a.ahead && r > from ? 1 : 0;  // (behind a round of this call; the first one waits for all before it)
+        cfg.numAttrs = a.ahead && r > 0 ? 1 : 0;  // (round 0 waits for all before it, as does one behind anything but a round)
         e = cudaLaunchKernelEx(&cfg, walk_kernel(a.fuse_narrow, a.n_pairs == 1), a, total0, r, hand_over && r + 1 == to);
     }
     return e;

@@ -1767,7 +1767,7 @@ int capture_frame_impl(oibvh_scene_s* s, cudaStream_t st)
     s->frame_args = a;
     s->frame_front0 = (uint32_t)plan.front0;
     // the rounds that the warm-up frame took and one more (a round with nothing to walk returns at once)
-    s->frame_rounds = std::max(3u, (uint32_t)s->stats.steps + 1u);
+    s->frame_rounds = std::max(2u, (uint32_t)s->stats.steps + 1u);
 
     // capture on a private non-blocking stream (the legacy default stream
     // cannot be captured); the graph is launched on the caller's stream
