@@ -56,8 +56,8 @@ TRANSFORM_DRAM_BYTES_PER_VERTEX = (124.32e6 + 73.98e6) / 7760256
 MOVE_REFIT_DRAM_BYTES_PER_TRIANGLE = (307.60e6 + 500.34e6) / 12808960
 # DRAM bytes (read + written) of the traversal kernels (k_begin, the k_walk
 # launches and k_narrow) of one frame per BVTT node pair tested, measured with
-# ncu on 64 batched pairs (146.1 MB per frame, 12,582,398 pairs tested)
-TRAVERSAL_DRAM_BYTES_PER_TESTED = (6.48e6 + 26.00e6 + 85.46e6 + 28.15e6) / 12582398
+# ncu on 64 batched pairs (143.7 MB per frame, 12,582,398 pairs tested)
+TRAVERSAL_DRAM_BYTES_PER_TESTED = (88.78e6 + 54.89e6) / 12582398
 
 
 def parse():

@@ -830,26 +830,29 @@ constexpr uint32_t kClaimMin = 16;
 // so a detect waited for the end of whatever else held the SMs. The next round's
 // CTAs are scheduled while this one's last warps finish (programmatic launch:
 // they wait at the start for its end), which a round's launch latency hides
-// behind. Two meshes of 20 k triangles 31.6 us a detect with the barrier, 35.0
+// behind: two meshes of 20 k triangles 31.6 us a detect with the barrier, 35.0
 // with plain launches, 31.5 so; of 1.31 M 67, 72 and 65; a scene of 64 pairs 275,
-// 276 and 268.
+// 276 and 268 (all three before the pairs between two levels were tested).
 //
-// What bounds it: in small traversals the latency of a step's chain (ring entry,
-// boxes, at the leaves faces and then vertices; 1.1 to 1.5 us) times the steps in
-// a row of the busiest warp; in large ones the instructions (3 us a step with
-// every warp busy; about 450 for 32 pairs, 554 before a side's arithmetic was
-// written out and a step's children and candidates were given their places by one
-// scan: a frame of 64 pairs 228 to 197 us, of 512 pairs 1254 to 1088). DRAM stays
-// below 10 %. A warp cuts its walk six steps after it has last claimed something
-// and the rest is shared out anew: the next round costs about 2 us, a warp left alone
-// with a deep subtree tens (2, 4, 6, 8, 12 steps: two meshes of 1.31 M triangles
-// 141, 104, 96, 103, 119 us a detect); three steps after start tests that were
-// dealt out, which leave pairs to one warp in ten (six against three: 1.31 M
-// triangles 77 to 71 us, 24 bodies 72 to 66, 20 k triangles 39 to 36, with pairs
-// taken two levels at once). Measured, whole detects, against one kernel for the
+// What bounds it is latency: a step's chain of loads (ring entry, boxes, at the
+// leaves faces and then vertices), 1.1 to 1.5 us, times the steps in a row of the
+// busiest warp in small traversals; in large ones the same chain at the warps that 64
+// registers leave. Four CTAs an SM keep 45 to 47 % of the warps active, the schedulers
+// issue in 41 to 51 % of the cycles, and a warp waits 7 to 10 cycles of 14 to 17 for a
+// load between two instructions (a frame of 64 pairs; DRAM 2 to 12 %, the L1's data
+// pipe 18 to 47 %). Fewer instructions a step help all the same, as each is in the
+// chain: about 450 for 32 pairs, 554 before a side's arithmetic was written out and a
+// step's children and candidates were given their places by one scan (a frame of 64
+// pairs 228 to 197 us, of 512 pairs 1254 to 1088). A warp cuts its walk six steps
+// after it has last claimed something and the rest is shared out anew: the next round
+// costs about 2 us, a warp left alone with a deep subtree tens (2, 4, 6, 8, 12 steps:
+// two meshes of 1.31 M triangles 141, 104, 96, 103, 119 us a detect); three steps after
+// start tests that were dealt out, which leave pairs to one warp in ten (six against
+// three: 1.31 M triangles 77 to 71 us, 24 bodies 72 to 66, 20 k triangles 39 to 36, with
+// pairs taken two levels at once). Measured, whole detects, against one kernel for the
 // start tests, one CTA for the top levels and several launches that each walk to
-// the leaves: two meshes of 20 k triangles 91 to 36 us, of 1.31 M 158 to 67, 24
-// bodies 115 to 60. A queue that idle warps wait on, instead of rounds, was slower
+// the leaves: two meshes of 20 k triangles 91 to 34 us, of 1.31 M 158 to 68, 24
+// bodies 115 to 67. A queue that idle warps wait on, instead of rounds, was slower
 // (20 k: 112 us): a hand-over costs its giver about 3 us.
 template <bool kFused, bool kOne>
 __global__ void __launch_bounds__(kDetectThreads, 4) k_walk(DetectArgs a, uint32_t total0, uint32_t r, bool last)
